@@ -135,6 +135,11 @@ void      *tlb_buffer_device_ptr(tlb_buffer *b);
  * the reference only writes buffers from host memory). For callers whose data is already in HBM. */
 tlb_status tlb_buffer_copy_device(tlb_buffer *b, uint64_t offset, const void *device_src, uint64_t n);
 void       tlb_buffer_free(tlb_buffer *b);
+/* Pinned host memory for results and inputs (no counterpart: the reference copies through pageable vectors). Copies
+ * between it and the device run at the link's rate and need no staging. Blocks come from a bounded pool that keeps up to 256 MB for
+ * reuse; TLB_ALLOC when 1 GB is handed out (use ordinary memory then). Any thread may free. */
+tlb_status tlb_host_alloc(uint64_t bytes, void **out);
+void       tlb_host_free(void *p);
 
 /* ------------------------------------------------------------------ programs
  * Executor::compile (crates/kernels/src/cuda/exec.rs:27-62): plans every tensor into one arena
@@ -155,7 +160,8 @@ void       tlb_program_free(tlb_program *prog);
 tlb_status tlb_plan_only(const tlb_graph *graph, const tlb_leaves *leaves, const uint64_t *node_scratch, uint64_t *arena_size,
                          uint64_t *io_size, uint8_t *tensor_buffer, uint64_t *tensor_offset, int64_t *scratch_offset);
 /* Program::set_input (exec.rs:91-98): n must equal the input tensor's byte size, else
- * "input i takes N bytes, got M". Blocking host-to-device copy into the program's io buffer. */
+ * "input i takes N bytes, got M". When it returns the bytes have been taken over; the next run, read or device-side
+ * copy of the program sees them (and so does the device memory itself, if tlb_program_tensor_ptr gave its address out). */
 tlb_status tlb_program_set_input(tlb_program *prog, uint32_t i, const void *bytes, uint64_t n);
 /* Device-side feedback for loops: copies the bytes of a KEPT tensor of the arena into graph input `input` (same byte
  * size), on the device stream, without waiting -- the next run sees them. A decode loop feeds the ARGMAX of a step

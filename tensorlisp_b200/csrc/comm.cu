@@ -108,7 +108,7 @@ __device__ __forceinline__ void ar_body(const ArRank &a, int n, int n_ranks, int
     __syncthreads();
     if (s_fail) {
         if (tid == 0) {
-            atomicExch(a.err, 3);
+            report_error(a.err, 3);
             seqs[c] = seq;
         }
         return;

@@ -228,6 +228,18 @@ using namespace tlb;
         if (e__ != cudaSuccess) return fail(st, std::string(#expr) + " failed: " + cuda_msg(e__)); \
     } while (0)
 
+// Waits for the stream; every sequence enqueued before the call is done afterwards.
+static cudaError_t sync_stream(tlb_device *dev) {
+    const uint64_t w = dev->work.load();
+    const cudaError_t e = cudaStreamSynchronize(dev->stream);
+    if (e == cudaSuccess) {
+        uint64_t d = dev->done.load();
+        while (d < w && !dev->done.compare_exchange_weak(d, w)) {}
+    }
+    return e;
+}
+static void quant_space_free(tlb_device *dev);
+
 extern "C" {
 
 const char *tlb_last_error(void) { return g_last_error.c_str(); }
@@ -252,10 +264,21 @@ tlb_status tlb_device_open(int ordinal, tlb_device **dev) {
     TLB_TRY_CUDA(cudaSetDevice(ordinal), TLB_NO_DEVICE);
     tlb_device *d = new tlb_device;
     d->ordinal = ordinal;
-    e = cudaGetDeviceProperties(&d->prop, ordinal);
-    if (e != cudaSuccess) {
-        delete d;
-        return fail(TLB_NO_DEVICE, "cudaGetDeviceProperties: " + cuda_msg(e));
+    {   // asked for once per ordinal: the query takes 3 to 9 ms
+        static std::mutex m;
+        static std::map<int, cudaDeviceProp> known;
+        std::lock_guard<std::mutex> lock(m);
+        auto it = known.find(ordinal);
+        if (it == known.end()) {
+            e = cudaGetDeviceProperties(&d->prop, ordinal);
+            if (e != cudaSuccess) {
+                delete d;
+                return fail(TLB_NO_DEVICE, "cudaGetDeviceProperties: " + cuda_msg(e));
+            }
+            known[ordinal] = d->prop;
+        } else {
+            d->prop = it->second;
+        }
     }
     if (d->prop.major != 10) {
         const std::string m = "this library is built for sm_100a only; device " + std::string(d->prop.name) + " is sm_" +
@@ -278,6 +301,7 @@ void tlb_device_close(tlb_device *dev) {
     if (!dev) return;
     tlb_comm_destroy(dev);
     cudaSetDevice(dev->ordinal);
+    quant_space_free(dev);
     if (dev->stream) cudaStreamDestroy(dev->stream);
     delete dev;
 }
@@ -291,7 +315,7 @@ tlb_status tlb_device_name(tlb_device *dev, char *out, size_t n) {
 tlb_status tlb_device_sync(tlb_device *dev) {
     if (!dev) return fail(TLB_INVALID, "null device");
     cudaSetDevice(dev->ordinal);
-    TLB_TRY_CUDA(cudaStreamSynchronize(dev->stream), TLB_EXECUTION);
+    TLB_TRY_CUDA(sync_stream(dev), TLB_EXECUTION);
     return TLB_OK;
 }
 
@@ -451,8 +475,8 @@ tlb_status tlb_buffer_write(tlb_buffer *b, uint64_t offset, const void *host, ui
         return fail(TLB_INVALID, "write of " + std::to_string(n) + " bytes at " + std::to_string(offset) + " past a buffer of " + std::to_string(b->size));
     if (n == 0) return TLB_OK;
     cudaSetDevice(b->dev->ordinal);
-    TLB_TRY_CUDA(cudaMemcpyAsync((char *)b->ptr + offset, host, n, cudaMemcpyHostToDevice, b->dev->stream), TLB_EXECUTION);
-    TLB_TRY_CUDA(cudaStreamSynchronize(b->dev->stream), TLB_EXECUTION);
+    TLB_TRY_CUDA(copy_h2d(b->ordinal, (char *)b->ptr + offset, host, n, b->dev->stream), TLB_EXECUTION);
+    TLB_TRY_CUDA(sync_stream(b->dev), TLB_EXECUTION);
     return TLB_OK;
 }
 
@@ -462,8 +486,7 @@ tlb_status tlb_buffer_read(tlb_buffer *b, uint64_t offset, void *host, uint64_t 
         return fail(TLB_INVALID, "read of " + std::to_string(n) + " bytes at " + std::to_string(offset) + " past a buffer of " + std::to_string(b->size));
     if (n == 0) return TLB_OK;
     cudaSetDevice(b->dev->ordinal);
-    TLB_TRY_CUDA(cudaMemcpyAsync(host, (char *)b->ptr + offset, n, cudaMemcpyDeviceToHost, b->dev->stream), TLB_EXECUTION);
-    TLB_TRY_CUDA(cudaStreamSynchronize(b->dev->stream), TLB_EXECUTION);
+    TLB_TRY_CUDA(copy_d2h(b->ordinal, host, (char *)b->ptr + offset, n, b->dev->stream), TLB_EXECUTION);
     return TLB_OK;
 }
 
@@ -486,6 +509,13 @@ void tlb_buffer_free(tlb_buffer *b) {
     cudaFree(b->ptr);
     delete b;
 }
+
+tlb_status tlb_host_alloc(uint64_t bytes, void **out) {
+    if (!out) return fail(TLB_INVALID, "tlb_host_alloc: null output");
+    *out = pinned_alloc(std::max<uint64_t>(bytes, 1));
+    return *out ? TLB_OK : fail(TLB_ALLOC, "no " + std::to_string(bytes) + " bytes of pinned host memory");
+}
+void tlb_host_free(void *p) { pinned_free(p); }
 
 // Copies and validates the IR of a caller (tensor ids in range, views of roots only, known types, leaves present).
 // Returns an empty string, or what is wrong.
@@ -539,6 +569,82 @@ static std::string import_graph(const tlb_graph *graph, const tlb_leaves *leaves
         for (uint32_t i = 0; i < leaves->n_states; i++) lv.states.push_back(leaves->state_offset[i]);
     }
     return "";
+}
+
+// ------------------------------------------------------------------ the pinned page of a program
+// Inputs of at most IO_SMALL bytes wait in the page until the program's launch sequence fetches them (k_io_page):
+// a blocking copy of the same bytes takes 10 to 12 us, most of it the wait. Kept results of at most IO_SMALL bytes that
+// the caller reads after its runs are pushed into the page by the sequence itself. The sequence's kernels also write
+// their error word there, so run() needs no copy to see it.
+static bool is_small_out(const tlb_program *p, uint32_t tensor) {
+    const Place pl = p->layout.place[tensor];
+    const uint64_t n = p->graph.tensors[tensor].nbytes();
+    if (pl.buf != BUF_ARENA || pl.off % 16 || n == 0 || n > IO_SMALL) return false;
+    for (int32_t k : p->graph.keep)
+        if ((uint32_t)k == tensor) return true;
+    return false;
+}
+static bool page_create(tlb_program *p) {
+    uint64_t at = (sizeof(IoPage) + 255) / 256 * 256;
+    const uint64_t in_end = at + IO_IN_TOTAL;
+    p->in_host_off.assign(p->layout.inputs.size(), 0);
+    int n = 0;
+    for (size_t i = 0; i < p->layout.inputs.size(); i++) {
+        const uint64_t bytes = align_up(p->layout.inputs[i].second);
+        if (bytes == 0 || p->layout.inputs[i].second > IO_SMALL || at + bytes > in_end || n == IO_MAX_IN) continue;
+        p->in_host_off[i] = (uint32_t)at;
+        at += bytes;
+        n++;
+    }
+    for (int32_t k : p->graph.keep)
+        if ((uint32_t)k < p->n_user_tensors && is_small_out(p, (uint32_t)k)) p->out_host_off = (uint32_t)at;
+    if (p->out_host_off) at += IO_OUT_TOTAL;
+    p->page = (IoPage *)pinned_alloc(at, true);
+    if (!p->page) return false;
+    std::memset((void *)p->page, 0, sizeof(IoPage));
+    return true;
+}
+// no sequence in flight uses the page
+static cudaError_t page_idle(tlb_program *p) { return p->page_seq > p->dev->done.load() ? sync_stream(p->dev) : cudaSuccess; }
+static void page_in_use(tlb_program *p) { p->page_seq = ++p->dev->work; }
+// inputs that wait in the page go to the io buffer now, in front of something else that touches it
+static cudaError_t flush_inputs(tlb_program *p) {
+    if (!p->in_dirty) return cudaSuccess;
+    p->in_dirty = false;
+    const cudaError_t e = launch_fetch_inputs(p->page, p->io, p->dev->stream);
+    page_in_use(p);
+    return e;
+}
+// the table of pushed results, rewritten while no sequence uses the page
+static void push_table(tlb_program *p) {
+    int n = 0;
+    for (const auto &o : p->pushed)
+        p->page->out[n++] = {p->layout.place[o.tensor].off, o.host_off, (uint32_t)((o.bytes + 15) / 16)};
+    p->page->n_out = n;
+}
+static void push_add(tlb_program *p, uint32_t tensor, uint64_t bytes) {
+    if (!p->out_host_off || bytes != p->graph.tensors[tensor].nbytes() || !is_small_out(p, tensor) || p->pushed.size() >= IO_MAX_OUT) return;
+    for (uint32_t t : p->no_push)
+        if (t == tensor) return;
+    uint32_t at = p->out_host_off;   // first gap that holds it
+    for (bool moved = true; moved;) {
+        moved = false;
+        for (const auto &o : p->pushed) {
+            const uint32_t end = o.host_off + (uint32_t)align_up(o.bytes);
+            if (at < end && o.host_off < at + align_up(bytes)) {
+                at = end;
+                moved = true;
+            }
+        }
+    }
+    if (at + align_up(bytes) > p->out_host_off + IO_OUT_TOTAL) return;
+    p->pushed.push_back({tensor, at, bytes, p->runs + 1, 0});
+    push_table(p);
+}
+static void push_drop_unread(tlb_program *p) {
+    const size_t before = p->pushed.size();
+    p->pushed.erase(std::remove_if(p->pushed.begin(), p->pushed.end(), [](const tlb_program::Pushed &o) { return o.unread > 64; }), p->pushed.end());
+    if (p->pushed.size() != before) push_table(p);
 }
 
 // ------------------------------------------------------------------ programs
@@ -614,9 +720,14 @@ tlb_status tlb_program_compile(tlb_device *dev, const tlb_graph *graph, const tl
         tlb_program_free(p);
         return bad(TLB_ALLOC, "buffer allocation of " + std::to_string(want) + " bytes failed");
     }
-    // the last 256 bytes of the arena allocation hold the device error word of bounded waits
-    cudaMemsetAsync((char *)p->arena + std::max<uint64_t>(p->layout.arena_size, 1), 0, 256, dev->stream);
-    cudaStreamSynchronize(dev->stream);
+    if (!page_create(p)) {
+        tlb_program_free(p);
+        return bad(TLB_ALLOC, "no pinned host memory for a program");
+    }
+    for (const Place &pl : p->layout.place) {
+        if (pl.buf == BUF_WEIGHTS) p->need_weights = std::max(p->need_weights, pl.index + 1);
+        if (pl.buf == BUF_STATE) p->need_state = true;
+    }
     const char *ng = getenv("TLB_NO_CUDA_GRAPH");
     p->use_graph = !(ng && ng[0] == '1');
     *prog = p;
@@ -654,6 +765,10 @@ void tlb_program_free(tlb_program *prog) {
         if (c.exec) cudaGraphExecDestroy(c.exec);
     if (prog->arena) cudaFree(prog->arena);
     if (prog->io) cudaFree(prog->io);
+    if (prog->page) {
+        cudaDeviceSynchronize();   // the page goes back to the pool: no kernel may still write to it
+        pinned_free(prog->page);
+    }
     delete prog;
 }
 
@@ -665,8 +780,23 @@ tlb_status tlb_program_set_input(tlb_program *prog, uint32_t i, const void *byte
     if (n == 0) return TLB_OK;
     if (!bytes) return fail(TLB_INVALID, "null input data");
     cudaSetDevice(prog->dev->ordinal);
-    TLB_TRY_CUDA(cudaMemcpyAsync((char *)prog->io + in.first, bytes, n, cudaMemcpyHostToDevice, prog->dev->stream), TLB_EXECUTION);
-    TLB_TRY_CUDA(cudaStreamSynchronize(prog->dev->stream), TLB_EXECUTION);
+    const uint32_t at = prog->in_host_off[i];
+    if (at == 0) {
+        TLB_TRY_CUDA(copy_h2d(prog->ordinal, (char *)prog->io + in.first, bytes, n, prog->dev->stream), TLB_EXECUTION);
+    } else {
+        TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
+        IoPage *pg = prog->page;
+        std::memcpy((char *)pg + at, bytes, n);
+        int e = 0;
+        while (e < pg->n_in && pg->in[e].host_off != at) e++;
+        pg->in[e] = {in.first, at, (uint32_t)((n + 15) / 16)};
+        if (e == pg->n_in) pg->n_in = e + 1;
+        prog->in_dirty = true;
+    }
+    if (prog->io_exposed) {   // the caller may look at the io buffer from another stream
+        TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
+        TLB_TRY_CUDA(sync_stream(prog->dev), TLB_EXECUTION);
+    }
     return TLB_OK;
 }
 
@@ -686,19 +816,15 @@ tlb_status tlb_program_feed_input(tlb_program *prog, uint32_t input, uint32_t te
     if (!kept) return fail(TLB_INVALID, "tensor " + std::to_string(tensor_id) + " is not kept: its bytes may be reused before the run ends");
     if (n == 0) return TLB_OK;
     cudaSetDevice(prog->dev->ordinal);
+    TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
     TLB_TRY_CUDA(cudaMemcpyAsync((char *)prog->io + in.first, (char *)prog->arena + pl.off, n, cudaMemcpyDeviceToDevice, prog->dev->stream), TLB_EXECUTION);
     return TLB_OK;
 }
 
 static tlb_status make_ctx(tlb_program *prog, tlb_buffer *const *weights, uint32_t n_weights, tlb_buffer *state, RunCtx &rc) {
-    uint32_t need_w = 0;
-    bool need_state = false;
-    for (const Place &pl : prog->layout.place) {
-        if (pl.buf == BUF_WEIGHTS) need_w = std::max(need_w, pl.index + 1);
-        if (pl.buf == BUF_STATE) need_state = true;
-    }
+    const uint32_t need_w = prog->need_weights;
     if (need_w > n_weights) return fail(TLB_INVALID, "the program reads weight buffer " + std::to_string(need_w - 1) + " but only " + std::to_string(n_weights) + " were given");
-    if (need_state && !state) return fail(TLB_INVALID, "the program reads state tensors but no state block was given");
+    if (prog->need_state && !state) return fail(TLB_INVALID, "the program reads state tensors but no state block was given");
     for (uint32_t i = 0; i < n_weights; i++) {
         if (!weights[i]) return fail(TLB_INVALID, "null weight buffer");
         rc.weights.push_back((char *)weights[i]->ptr);
@@ -708,7 +834,7 @@ static tlb_status make_ctx(tlb_program *prog, tlb_buffer *const *weights, uint32
     rc.arena = (char *)prog->arena;
     rc.stream = prog->dev->stream;
     rc.dev = prog->dev;
-    rc.err = (int *)((char *)prog->arena + std::max<uint64_t>(prog->layout.arena_size, 1));
+    rc.err = &prog->page->err;
     return TLB_OK;
 }
 
@@ -732,7 +858,33 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     tlb_status st = make_ctx(prog, weights, n_weights, state, rc);
     if (st != TLB_OK) return st;
     const bool profile = getenv("TL_NATIVE_PROFILE") != nullptr;
-    if (!prog->use_graph || profile || prog->dispatches.size() < 2) return launch_all(prog, rc, profile);
+    const bool idle = prog->page_seq <= prog->dev->done.load();
+    for (auto &o : prog->pushed) o.unread++;
+    if (idle) push_drop_unread(prog);
+    // Small inputs come in, the launches, results that are read after every run go out. A captured sequence always has
+    // the two page kernels (their tables say what moves), a direct one launches them when there is something to move.
+    auto sequence = [&](bool captured, bool prof) {
+        cudaError_t e = cudaSuccess;
+        const bool any_in = std::any_of(prog->in_host_off.begin(), prog->in_host_off.end(), [](uint32_t o) { return o != 0; });
+        if (captured ? any_in : prog->in_dirty) e = launch_fetch_inputs(prog->page, prog->io, rc.stream);
+        tlb_status s = e == cudaSuccess ? launch_all(prog, rc, prof) : fail(TLB_EXECUTION, "fetching inputs: " + cuda_msg(e));
+        if (s == TLB_OK && (captured ? prog->out_host_off != 0 : !prog->pushed.empty())) {
+            e = launch_push_outputs(prog->page, prog->arena, rc.stream);
+            if (e != cudaSuccess) s = fail(TLB_EXECUTION, "pushing results: " + cuda_msg(e));
+        }
+        return s;
+    };
+    auto enqueued = [&] {
+        prog->in_dirty = false;
+        prog->runs++;
+        page_in_use(prog);
+    };
+    auto direct = [&](bool prof) {
+        const tlb_status s = sequence(false, prof);
+        enqueued();
+        return s;
+    };
+    if (!prog->use_graph || profile || prog->dispatches.empty()) return direct(profile);
     // replay a captured CUDA graph, one per set of buffer addresses (sessions switch state blocks)
     std::vector<void *> key;
     for (char *w : rc.weights) key.push_back(w);
@@ -741,22 +893,23 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     for (auto &c : prog->captured)
         if (c.key == key) {
             TLB_TRY_CUDA(cudaGraphLaunch(c.exec, rc.stream), TLB_EXECUTION);
+            enqueued();
             return TLB_OK;
         }
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(rc.stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        return launch_all(prog, rc, false);
+        return direct(false);
     }
-    st = launch_all(prog, rc, false);
+    st = sequence(true, false);
     e = cudaStreamEndCapture(rc.stream, &graph);
     if (st != TLB_OK || e != cudaSuccess || !graph) {
         cudaGetLastError();
         if (graph) cudaGraphDestroy(graph);
         if (st != TLB_OK) return st;
         prog->use_graph = false;
-        return launch_all(prog, rc, false);
+        return direct(false);
     }
     {   // how many kernels one run of the program launches (tlb_program_kernel_count)
         size_t n_nodes = 0;
@@ -777,7 +930,7 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     if (e != cudaSuccess) {
         cudaGetLastError();
         prog->use_graph = false;
-        return launch_all(prog, rc, false);
+        return direct(false);
     }
     if (prog->captured.size() >= 8) {
         cudaGraphExecDestroy(prog->captured.front().exec);
@@ -785,6 +938,7 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     }
     prog->captured.push_back({key, exec});
     TLB_TRY_CUDA(cudaGraphLaunch(exec, rc.stream), TLB_EXECUTION);
+    enqueued();
     return TLB_OK;
 }
 
@@ -797,6 +951,8 @@ tlb_status tlb_program_profile(tlb_program *prog, tlb_buffer *const *weights, ui
     RunCtx rc;
     tlb_status st = make_ctx(prog, weights, n_weights, state, rc);
     if (st != TLB_OK) return st;
+    TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
+    for (auto &o : prog->pushed) o.valid_from = prog->runs + 1;   // this run pushes nothing
     std::vector<cudaEvent_t> ev(n + 1);
     for (auto &e : ev) TLB_TRY_CUDA(cudaEventCreate(&e), TLB_EXECUTION);
     cudaError_t e = cudaEventRecord(ev[0], rc.stream);
@@ -819,15 +975,14 @@ tlb_status tlb_program_profile(tlb_program *prog, tlb_buffer *const *weights, ui
 tlb_status tlb_program_run(tlb_program *prog, tlb_buffer *const *weights, uint32_t n_weights, tlb_buffer *state) {
     tlb_status st = tlb_program_enqueue(prog, weights, n_weights, state);
     if (st != TLB_OK) return st;
-    cudaError_t e = cudaStreamSynchronize(prog->dev->stream);
+    cudaError_t e = sync_stream(prog->dev);
     if (e != cudaSuccess)
         return fail(TLB_EXECUTION, cuda_msg(e) + " (graph of " + std::to_string(prog->dispatches.size()) + " dispatches)");
-    // bounded waits inside kernels report through the error word behind the arena
-    int flag = 0;
-    e = cudaMemcpy(&flag, (char *)prog->arena + std::max<uint64_t>(prog->layout.arena_size, 1), 4, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return fail(TLB_EXECUTION, cuda_msg(e));
+    // bounded waits inside kernels report through the error word of the page
+    volatile int *word = &prog->page->err;
+    const int flag = *word;
     if (flag != 0) {
-        cudaMemset((char *)prog->arena + std::max<uint64_t>(prog->layout.arena_size, 1), 0, 4);
+        *word = 0;
         if (flag == TLB_ERR_INDEX)
             return fail(TLB_EXECUTION, "a context length, block id or cache slot from the caller was out of range (skipped on the device; device error word 4)");
         return fail(TLB_EXECUTION, "a kernel gave up waiting for its own copies (device error word " + std::to_string(flag) + ")");
@@ -853,8 +1008,19 @@ tlb_status tlb_program_read(tlb_program *prog, uint32_t tensor_id, uint64_t byte
     if (pl.off + bytes > size) return fail(TLB_INVALID, "tensor " + std::to_string(tensor_id) + " reads past its buffer");
     if (bytes == 0) return TLB_OK;
     cudaSetDevice(prog->dev->ordinal);
-    TLB_TRY_CUDA(cudaMemcpyAsync(out, base + pl.off, bytes, cudaMemcpyDeviceToHost, prog->dev->stream), TLB_EXECUTION);
-    TLB_TRY_CUDA(cudaStreamSynchronize(prog->dev->stream), TLB_EXECUTION);
+    for (auto &o : prog->pushed)
+        if (o.tensor == tensor_id && o.bytes == bytes && prog->runs >= o.valid_from) {
+            TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
+            std::memcpy(out, (const char *)prog->page + o.host_off, bytes);
+            o.unread = 0;
+            return TLB_OK;
+        }
+    if (pl.buf == BUF_IO) TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
+    TLB_TRY_CUDA(copy_d2h(prog->ordinal, out, base + pl.off, bytes, prog->dev->stream), TLB_EXECUTION);
+    if (prog->out_host_off && bytes <= IO_SMALL && std::none_of(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; })) {
+        TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
+        push_add(prog, tensor_id, bytes);
+    }
     return TLB_OK;
 }
 
@@ -871,8 +1037,24 @@ void *tlb_program_tensor_ptr(tlb_program *prog, uint32_t tensor_id, uint64_t *by
     if (!prog || tensor_id >= prog->n_user_tensors) return nullptr;
     const Place pl = prog->layout.place[tensor_id];
     if (bytes) *bytes = prog->graph.tensors[tensor_id].nbytes();
-    if (pl.buf == BUF_ARENA) return (char *)prog->arena + pl.off;
-    if (pl.buf == BUF_IO) return (char *)prog->io + pl.off;
+    if (pl.buf == BUF_ARENA) {
+        // the caller may write there: what read() returns comes from the tensor itself from now on
+        cudaSetDevice(prog->ordinal);
+        if (page_idle(prog) == cudaSuccess) {
+            prog->pushed.erase(std::remove_if(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; }), prog->pushed.end());
+            push_table(prog);
+        }
+        prog->no_push.push_back(tensor_id);
+        return (char *)prog->arena + pl.off;
+    }
+    if (pl.buf == BUF_IO) {
+        if (!prog->io_exposed) {
+            prog->io_exposed = true;
+            cudaSetDevice(prog->ordinal);
+            if (flush_inputs(prog) == cudaSuccess) sync_stream(prog->dev);
+        }
+        return (char *)prog->io + pl.off;
+    }
     return nullptr;
 }
 
@@ -903,6 +1085,49 @@ tlb_status tlb_selftest_wait_runs_out(tlb_device *dev, uint32_t limit, uint32_t 
 }
 
 // ------------------------------------------------------------------ quantizers
+}  // extern "C"
+
+constexpr uint64_t QUANT_PIECE = 16 << 20;   // f32 bytes of a piece: staged in 1 MB chunks at the link's rate, short enough to overlap
+struct QuantSpace {
+    static constexpr int SLOTS = 3;
+    uint64_t in_bytes = 0, out_bytes = 0;
+    void *in[SLOTS] = {}, *out[SLOTS] = {};
+    cudaStream_t up = nullptr, down = nullptr;
+    cudaEvent_t arrived[SLOTS] = {}, done[SLOTS] = {}, left[SLOTS] = {};
+};
+static void quant_space_free(tlb_device *dev) {
+    QuantSpace *q = dev->quant;
+    dev->quant = nullptr;
+    if (!q) return;
+    for (int s = 0; s < QuantSpace::SLOTS; s++) {
+        if (q->in[s]) cudaFree(q->in[s]);
+        if (q->out[s]) cudaFree(q->out[s]);
+        for (cudaEvent_t ev : {q->arrived[s], q->done[s], q->left[s]})
+            if (ev) cudaEventDestroy(ev);
+    }
+    if (q->up) cudaStreamDestroy(q->up);
+    if (q->down) cudaStreamDestroy(q->down);
+    delete q;
+}
+static QuantSpace *quant_space(tlb_device *dev, uint64_t in_bytes, uint64_t out_bytes) {
+    QuantSpace *q = dev->quant;
+    if (q && q->in_bytes >= in_bytes && q->out_bytes >= out_bytes) return q;
+    if (q) quant_space_free(dev);
+    q = dev->quant = new QuantSpace;
+    q->in_bytes = std::max<uint64_t>(in_bytes, QUANT_PIECE);
+    q->out_bytes = std::max<uint64_t>(out_bytes, QUANT_PIECE / 2);
+    bool ok = cudaStreamCreateWithFlags(&q->up, cudaStreamNonBlocking) == cudaSuccess && cudaStreamCreateWithFlags(&q->down, cudaStreamNonBlocking) == cudaSuccess;
+    for (int s = 0; s < QuantSpace::SLOTS && ok; s++) {
+        ok = cudaMalloc(&q->in[s], q->in_bytes) == cudaSuccess && cudaMalloc(&q->out[s], q->out_bytes) == cudaSuccess;
+        for (cudaEvent_t *ev : {&q->arrived[s], &q->done[s], &q->left[s]}) ok = ok && cudaEventCreateWithFlags(ev, cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (ok) return q;
+    cudaGetLastError();
+    quant_space_free(dev);
+    return nullptr;
+}
+
+extern "C" {
 tlb_status tlb_quantize_rows_device(tlb_device *dev, uint32_t type, const void *src, int64_t rows, int64_t n_per_row, void *out) {
     if (!dev) return fail(TLB_INVALID, "null device");
     const TypeTraits *tr = type_traits(type);
@@ -918,30 +1143,59 @@ tlb_status tlb_quantize_rows_device(tlb_device *dev, uint32_t type, const void *
     return TLB_OK;
 }
 
+// f32 rows of host memory, in pieces: the piece after the one that is being quantized is on its way up, the one before
+// it on its way down. The device buffers and the two copy streams are kept between calls (three pieces, 72 MB).
 tlb_status tlb_quantize_rows(tlb_device *dev, uint32_t type, const float *src, int64_t rows, int64_t n_per_row, void *out) {
     if (!dev || (!src && rows * n_per_row) || (!out && rows * n_per_row)) return fail(TLB_INVALID, "tlb_quantize_rows: bad arguments");
     const uint64_t rs = tlb_row_size(type, n_per_row);
-    if (rows * n_per_row == 0) return tlb_quantize_rows_device(dev, type, nullptr, rows, n_per_row, nullptr);
-    if (rs == 0) return tlb_quantize_rows_device(dev, type, nullptr, rows, n_per_row, nullptr);  // reports the reason
+    if (rows <= 0 || n_per_row <= 0 || rs == 0) return tlb_quantize_rows_device(dev, type, nullptr, rows, n_per_row, nullptr);   // reports the reason
     cudaSetDevice(dev->ordinal);
-    const uint64_t in_bytes = (uint64_t)rows * n_per_row * 4, out_bytes = (uint64_t)rows * rs;
-    void *din = nullptr, *dout = nullptr;
-    if (cudaMalloc(&din, in_bytes) != cudaSuccess || cudaMalloc(&dout, out_bytes) != cudaSuccess) {
-        cudaGetLastError();
-        if (din) cudaFree(din);
-        return fail(TLB_ALLOC, "buffer allocation of " + std::to_string(in_bytes + out_bytes) + " bytes failed");
-    }
+    const uint64_t row_in = (uint64_t)n_per_row * 4;
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(rows, (int64_t)(QUANT_PIECE / row_in)));
+    const uint64_t in_bytes = (uint64_t)per * row_in, out_bytes = (uint64_t)per * rs;
+    std::lock_guard<std::mutex> lock(dev->quant_mutex);
+    QuantSpace *q = quant_space(dev, in_bytes, out_bytes);
+    if (!q) return fail(TLB_ALLOC, "buffer allocation of " + std::to_string(in_bytes + out_bytes) + " bytes failed");
     tlb_status st = TLB_OK;
-    cudaError_t e = cudaMemcpyAsync(din, src, in_bytes, cudaMemcpyHostToDevice, dev->stream);
-    if (e == cudaSuccess) {
-        st = tlb_quantize_rows_device(dev, type, din, rows, n_per_row, dout);
-        if (st == TLB_OK) e = cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, dev->stream);
+    cudaError_t e = cudaSuccess;
+    auto step = [&](cudaError_t r) { return (e = r) == cudaSuccess; };
+    const bool direct = pinned_owns(out, (uint64_t)rows * rs);   // results can be written where they belong while later pieces run
+    int64_t piece = 0;
+    char *to_prev = nullptr;
+    int s_prev = 0;
+    uint64_t n_prev = 0;
+    for (int64_t r0 = 0; r0 < rows && e == cudaSuccess && st == TLB_OK; r0 += per, piece++) {
+        const int64_t n = std::min(per, rows - r0);
+        const int s = (int)(piece % QuantSpace::SLOTS);
+        // the kernel that read this slot's rows, and the copy that read its blocks, are behind these events
+        if (piece >= QuantSpace::SLOTS && !step(cudaStreamWaitEvent(q->up, q->done[s], 0))) break;
+        if (!step(copy_h2d(dev->ordinal, q->in[s], src + r0 * n_per_row, (uint64_t)n * row_in, q->up))) break;
+        if (!step(cudaEventRecord(q->arrived[s], q->up)) || !step(cudaStreamWaitEvent(dev->stream, q->arrived[s], 0))) break;
+        if (piece >= QuantSpace::SLOTS && !step(cudaStreamWaitEvent(dev->stream, q->left[s], 0))) break;
+        st = tlb_quantize_rows_device(dev, type, q->in[s], n, n_per_row, q->out[s]);
+        if (st != TLB_OK || !step(cudaEventRecord(q->done[s], dev->stream))) break;
+        if (direct && !step(cudaStreamWaitEvent(q->down, q->done[s], 0))) break;
+        char *to = (char *)out + (uint64_t)r0 * rs;
+        if (direct) {
+            if (!step(cudaMemcpyAsync(to, q->out[s], (uint64_t)n * rs, cudaMemcpyDeviceToHost, q->down)) || !step(cudaEventRecord(q->left[s], q->down))) break;
+        } else {
+            // a blocking copy: of the piece before this one, so that this one's kernel and the next upload are not kept waiting
+            if (to_prev && (!step(cudaStreamWaitEvent(q->down, q->done[s_prev], 0)) || !step(copy_d2h(dev->ordinal, to_prev, q->out[s_prev], n_prev * rs, q->down)) || !step(cudaEventRecord(q->left[s_prev], q->down)))) break;
+            to_prev = to;
+            s_prev = s;
+            n_prev = (uint64_t)n;
+        }
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
-    cudaFree(din);
-    cudaFree(dout);
+    if (to_prev && e == cudaSuccess && st == TLB_OK && step(cudaStreamWaitEvent(q->down, q->done[s_prev], 0))) e = copy_d2h(dev->ordinal, to_prev, q->out[s_prev], n_prev * rs, q->down);
+    // everything has left the buffers, whatever happened
+    const cudaError_t e1 = cudaStreamSynchronize(q->up), e2 = sync_stream(dev), e3 = cudaStreamSynchronize(q->down);
+    if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
+    if (q->in_bytes > 2 * QUANT_PIECE) quant_space_free(dev);   // one very long row: not kept
     if (st != TLB_OK) return st;
-    if (e != cudaSuccess) return fail(TLB_EXECUTION, "tlb_quantize_rows: " + cuda_msg(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(TLB_EXECUTION, "tlb_quantize_rows: " + cuda_msg(e));
+    }
     return TLB_OK;
 }
 

@@ -1,0 +1,52 @@
+// Host <-> device traffic of the C ABI: pinned memory that is kept between calls, staged copies of pageable memory
+// that several host threads fill, and the two small kernels that move a program's small inputs and results
+// between pinned host memory and the device inside the program's own launch sequence.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <functional>
+
+namespace tlb {
+
+// ---- pinned host memory. Blocks are kept for reuse up to a bound (HOST_CACHE_LIMIT); what is handed out at any time
+// is bounded too (HOST_LIVE_LIMIT): beyond it, and when pinning fails, pinned_alloc returns null and the caller uses
+// pageable memory (`always`: a block the library itself cannot do without, whatever is handed out). Safe to use from
+// several threads.
+void *pinned_alloc(uint64_t bytes, bool always = false);
+void pinned_free(void *p);
+bool pinned_owns(const void *p, uint64_t bytes);   // [p, p + bytes) lies in a block that is handed out
+
+// ---- host threads: runs fn(0) .. fn(n - 1), on the calling thread and up to `threads` - 1 others. When another caller
+// has the helpers, everything runs on the calling thread.
+void host_parallel(int n, int threads, const std::function<void(int)> &fn);
+
+// ---- copies between caller memory (pageable or pinned) and the device on `st`.
+// h2d: when it returns, the source has been read (the copy itself may still be on its way, in stream order).
+// d2h: when it returns, the destination holds the data (everything in front of it on the stream has finished).
+cudaError_t copy_h2d(int ordinal, void *dst, const void *src, uint64_t n, cudaStream_t st);
+cudaError_t copy_d2h(int ordinal, void *dst, const void *src, uint64_t n, cudaStream_t st);
+
+// ---- a program's pinned page
+constexpr int IO_MAX_IN = 32, IO_MAX_OUT = 8;          // entries of the two tables
+constexpr uint64_t IO_SMALL = 64 << 10;                // a tensor of at most this many bytes travels through the page
+constexpr uint64_t IO_IN_TOTAL = 128 << 10, IO_OUT_TOTAL = 64 << 10;
+struct IoPiece {
+    uint64_t dev_off;    // byte offset in the program's io buffer (inputs) or arena (outputs), a multiple of 16
+    uint32_t host_off;   // byte offset in the page, a multiple of 16
+    uint32_t n16;        // 16-byte pieces
+};
+struct IoPage {
+    int err;             // error word of the program's kernels (bounded waits, indices out of range)
+    int pad0[15];
+    int n_in, n_out, pad1[14];
+    IoPiece in[IO_MAX_IN];
+    IoPiece out[IO_MAX_OUT];
+};
+// moves the n_in listed inputs from the page to the io buffer and sets n_in to 0
+cudaError_t launch_fetch_inputs(IoPage *page, void *io, cudaStream_t st);
+// moves the n_out listed outputs from the arena to the page
+cudaError_t launch_push_outputs(IoPage *page, const void *arena, cudaStream_t st);
+
+}  // namespace tlb

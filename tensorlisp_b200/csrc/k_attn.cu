@@ -78,7 +78,7 @@ struct PagedParams {
 __device__ __forceinline__ int paged_ctx(const PagedParams &p, int seq) {
     const int n = p.lens[seq];
     if (n < 0 || n > p.ctx_cap) {
-        if (p.err) atomicExch(p.err, TLB_ERR_INDEX);
+        if (p.err) report_error(p.err, TLB_ERR_INDEX);
         return n < 0 ? 0 : p.ctx_cap;
     }
     return n;
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(PA_WARPS * 32) k_paged_attn(PagedParams p) {
             for (int b = (c_begin >> p.block_shift) + (int)threadIdx.x; b <= ((c_end - 1) >> p.block_shift); b += PA_WARPS * 32)
                 bad |= (uint32_t)table[b] >= p.pool_blocks;   // negative ids are large here
         if (__syncthreads_or(bad)) {
-            if (threadIdx.x == 0 && p.err) atomicExch(p.err, TLB_ERR_INDEX);
+            if (threadIdx.x == 0 && p.err) report_error(p.err, TLB_ERR_INDEX);
             return;
         }
     }
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(PA_WARPS * 32) k_paged_attn_any(PagedParams p)
             for (int b = (int)threadIdx.x; b <= ((ctx - 1) >> p.block_shift); b += PA_WARPS * 32)
                 bad |= (uint32_t)table[b] >= p.pool_blocks;
         if (__syncthreads_or(bad)) {
-            if (threadIdx.x == 0 && p.err) atomicExch(p.err, TLB_ERR_INDEX);
+            if (threadIdx.x == 0 && p.err) report_error(p.err, TLB_ERR_INDEX);
             return;
         }
     }
@@ -627,7 +627,7 @@ __global__ void k_cache_write(int kv_heads, int hs, int block_size, const uint4 
     const int64_t slot = slots[tok];
     if (slot < 0) return;
     if (slot >= pool_slots) {   // beyond the pools: nothing is written, the host hears of it
-        if (threadIdx.x == 0 && err) atomicExch(err, TLB_ERR_INDEX);
+        if (threadIdx.x == 0 && err) report_error(err, TLB_ERR_INDEX);
         return;
     }
     const int64_t blk = slot / block_size, off = slot % block_size;

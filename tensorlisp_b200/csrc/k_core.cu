@@ -337,7 +337,7 @@ __global__ void k_rope_kv(RopeKvArgs p, const uint8_t *q, const uint8_t *k, cons
             const int64_t slot = slots[tok];
             if (slot < 0) return;
             if (slot >= p.pool_slots) {   // beyond the pools: nothing is written, the host hears of it
-                if (pr == 0 && err) atomicExch(err, TLB_ERR_INDEX);
+                if (pr == 0 && err) report_error(err, TLB_ERR_INDEX);
                 return;
             }
             src = k + h * p.k.nb[1] + tok * p.k.nb[2];

@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(fat::THREADS, 1) k_fa_tc(FaTcParams p) {
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, 512);
-    if (tid == 0 && s_fail && p.err) atomicExch(p.err, 2);
+    if (tid == 0 && s_fail && p.err) report_error(p.err, 2);
 }
 
 // ---------------------------------------------------------------- host side

@@ -337,7 +337,7 @@ __device__ __forceinline__ void xr_body(const ArRank &a, const RowQuantArgs &p, 
     __syncthreads();
     if (s_fail) {
         if (tid == 0) {
-            atomicExch(a.err, 3);
+            report_error(a.err, 3);
             seqs[n] = seq;
         }
         return;

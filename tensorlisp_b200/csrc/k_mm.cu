@@ -274,7 +274,7 @@ k_gemv_stream(const uint8_t *__restrict__ W, int row_bytes, int64_t M, int K, co
         if (!ok) {
             // the consumers stopped releasing stages: record it, then wait (bounded) for the copies
             // still in flight before the CTA's shared memory is released
-            atomicExch(err, 1);
+            report_error(err, 1);
             for (int j = max(0, issued - GEMV_STAGES); j < issued; j++)
                 mbar_wait(&full[j & (GEMV_STAGES - 1)], (uint32_t)((j / GEMV_STAGES) & 1));
         }
@@ -302,7 +302,7 @@ k_gemv_stream(const uint8_t *__restrict__ W, int row_bytes, int64_t M, int K, co
     for (int i = 0; i < my_tiles; i++) {
         const int s = i & (GEMV_STAGES - 1);
         if (!mbar_wait(&full[s], (uint32_t)((i / GEMV_STAGES) & 1))) {
-            if (lane == 0) atomicExch(err, 1);
+            if (lane == 0) report_error(err, 1);
             break;  // this warp stops releasing stages; the producer's bounded wait ends the CTA
         }
         const int64_t r0 = (blockIdx.x + (int64_t)i * gridDim.x) * rows_per_tile;

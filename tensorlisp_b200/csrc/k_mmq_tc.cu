@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(Q4K_THREADS, 1) k_mmq_tc_q4k(const __grid_cons
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
-    if (tid == 0 && s_fail) atomicExch(p.err, 2);
+    if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
 // y[n][m] = sum over the K splits, in split order. Up to three matrices per launch: element i of the
@@ -705,7 +705,7 @@ __global__ void k_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsig
     __syncthreads();
     if (threadIdx.x == 0) {
         *ns = t1 - t0;
-        if (s_fail) atomicExch(err, 2);
+        if (s_fail) report_error(err, 2);
     }
 }
 cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsigned long long *ns, cudaStream_t st) {

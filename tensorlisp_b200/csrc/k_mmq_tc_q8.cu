@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(tc8::THREADS, 1) k_mmq_tc_q80(const __grid_con
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, tc8::TMEM_COLS);
-    if (tid == 0 && s_fail) atomicExch(p.err, 2);
+    if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
 // ---------------------------------------------------------------- many activation columns (prompt pass)
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, tc8::TMEM_COLS);
-    if (tid == 0 && s_fail) atomicExch(p.err, 2);
+    if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
 // ---------------------------------------------------------------- many activation columns, one accumulator (prompt pass)
@@ -913,7 +913,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, 512);
-    if (tid == 0 && s_fail) atomicExch(p.err, 2);
+    if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
 static size_t tc8f_smem() { return (size_t)tc8f::B_STAGES * tc8f::B_STAGE + (size_t)tc8f::RAW_STAGES * tc8::RAW_BYTES + 1024; }   // the larger raw stage (Q8_0)

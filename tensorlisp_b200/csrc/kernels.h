@@ -204,6 +204,10 @@ void flash_tc_configure();
 // pipelines, the peer exchange); 4 is a context length, block id or cache slot from the caller that a kernel skipped
 // because it pointed outside the tables or pools.
 #define TLB_ERR_INDEX 4
+#ifdef __CUDACC__
+// The error word may lie in pinned host memory (a program's page): a plain store, no atomic over the link.
+__device__ __forceinline__ void report_error(int *err, int code) { *(volatile int *)err = code; }
+#endif
 
 // ---------------------------------------------------------------- k_attn.cu
 // KV pools are private to the executor (only the two paged nodes touch them): f16

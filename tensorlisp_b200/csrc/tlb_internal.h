@@ -5,14 +5,17 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/tlb200.h"
+#include "hostio.h"
 
 namespace tlb {
 
@@ -122,6 +125,13 @@ struct tlb_device {
     // a captured CUDA graph have the communicator's state baked in (which all-reduce path, the peers' mapped
     // pointers), so the generation is part of the key a captured graph is replayed under.
     uint64_t comm_generation = 0;
+    // Launch sequences enqueued on the stream so far, and how many of them are known to have finished: whoever waits
+    // for the stream raises `done` to what `work` was before the wait. A program may touch its pinned page again once
+    // the last sequence that uses it is done, without asking the driver.
+    std::atomic<uint64_t> work{0}, done{0};
+    // device buffers and streams of tlb_quantize_rows, kept between calls
+    struct QuantSpace *quant = nullptr;
+    std::mutex quant_mutex;
 };
 
 struct tlb_buffer {
@@ -197,4 +207,22 @@ struct tlb_program {
     std::vector<Captured> captured;
     uint32_t kernel_nodes = 0;   // kernel launches in the most recently captured graph
     bool use_graph = true;
+    uint32_t need_weights = 0;   // weight buffers the graph reads, and whether it reads state
+    bool need_state = false;
+    // ---- the pinned page: error word, and the small inputs and results (hostio.h)
+    tlb::IoPage *page = nullptr;
+    std::vector<uint32_t> in_host_off;   // per input: where it waits in the page, 0 = it is copied instead
+    uint32_t out_host_off = 0;           // where results start in the page, 0 = none is small enough
+    bool in_dirty = false;               // inputs wait in the page that no fetch has been enqueued for
+    uint64_t page_seq = 0;               // device work number of the last sequence that uses the page
+    bool io_exposed = false;             // the caller holds an address in the io buffer: set_input then waits for its copy
+    // results the caller reads after every run: pushed into the page at the end of the sequence
+    struct Pushed {
+        uint32_t tensor, host_off;
+        uint64_t bytes, valid_from;      // first run that pushes it
+        int unread;                      // runs since it was last read
+    };
+    std::vector<Pushed> pushed;
+    std::vector<uint32_t> no_push;       // tensors whose device address the caller holds
+    uint64_t runs = 0;
 };

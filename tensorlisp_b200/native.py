@@ -7,6 +7,7 @@ CUDA library.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 
 import numpy as np
 
@@ -21,6 +22,39 @@ _NP_OF = {0: np.float32, 1: np.float16, 26: np.int32, 27: np.int64, 24: np.int8,
 
 def row_size(ty: int, ne0: int) -> int:
     return int(_lib.lib().tlb_row_size(ty, ne0))
+
+
+class _HostBlock:
+    """A block of pinned host memory as numpy takes it; given back when the last array over it goes away."""
+
+    __slots__ = ("ptr", "__array_interface__")
+
+    def __init__(self, ptr: int, nbytes: int) -> None:
+        self.ptr = ptr
+        self.__array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (ptr, False), "version": 3}
+
+    def __del__(self) -> None:
+        try:
+            _lib.lib().tlb_host_free(self.ptr)
+        except Exception:
+            pass
+
+
+_PINNED_FROM = 64 << 10     # smaller results come through the program's page: an ordinary array is as good
+
+
+def _result_bytes(nbytes: int) -> np.ndarray:
+    """Uninitialised bytes for a result: pinned where that pays (the copy goes straight there, and no page of the array
+    is touched for the first time while the caller waits), ordinary memory when the pool has none."""
+    if nbytes >= _PINNED_FROM:
+        p = C.c_void_p()
+        if _lib.lib().tlb_host_alloc(nbytes, C.byref(p)) == 0:
+            return np.asarray(_HostBlock(p.value, nbytes))
+    return np.empty(nbytes, np.uint8)
+
+
+def _address(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
 
 
 class StateBlock:
@@ -45,8 +79,8 @@ class StateBlock:
         check(_lib.lib().tlb_buffer_write(self.h, offset, data.ctypes.data_as(C.c_void_p), data.nbytes))
 
     def read(self, offset: int, nbytes: int) -> np.ndarray:
-        out = np.empty(nbytes, np.uint8)
-        check(_lib.lib().tlb_buffer_read(self.h, offset, out.ctypes.data_as(C.c_void_p), nbytes))
+        out = _result_bytes(nbytes)
+        check(_lib.lib().tlb_buffer_read(self.h, offset, _address(out), nbytes))
         return out
 
     def copy_blocks(self, k_pool_offset: int, v_pool_offset: int, pool_blocks: int, bytes_per_block: int, pairs) -> None:
@@ -203,6 +237,8 @@ class NativeProgram:
         self.h = handle
         self.graph = graph
         self._outputs = outputs
+        self._result = {}       # tensor -> (bytes, element type, shape) of what read() returns
+        self._given = (None,)   # (weights, state) of the last run, with the arguments made from them
 
     @classmethod
     def compile(cls, native: Native, graph: Graph, outputs: list[tuple[str, int]] | None = None) -> "NativeProgram":
@@ -227,14 +263,17 @@ class NativeProgram:
     def set_input(self, i: int, data: np.ndarray | bytes) -> None:
         if isinstance(data, (bytes, bytearray)):
             data = np.frombuffer(data, np.uint8)
-        data = np.ascontiguousarray(data)
-        check(self.native.L.tlb_program_set_input(self.h, i, data.ctypes.data_as(C.c_void_p), data.nbytes))
+        if type(data) is not np.ndarray or not data.flags.c_contiguous:
+            data = np.ascontiguousarray(data)
+        check(self.native.L.tlb_program_set_input(self.h, i, _address(data), data.nbytes))
 
     def _buffers(self, state: StateBlock | None):
         st = state if state is not None else self.native.state
         w = self.native.weights
-        arr = (C.c_void_p * 1)(w.h if w else None)
-        return arr, (1 if w else 0), (st.h if st else None)
+        key = (w.h.value if w else None, st.h.value if st else None)
+        if self._given[0] != key:
+            self._given = (key, (C.c_void_p * 1)(w.h if w else None), 1 if w else 0, st.h if st else None)
+        return self._given[1:]
 
     def feed_input(self, i: int, tensor: int) -> None:
         """The bytes of a kept arena tensor become input i of the next run (device-side copy, enqueued)."""
@@ -258,17 +297,17 @@ class NativeProgram:
 
     def read(self, tensor: int, dtype=None) -> np.ndarray:
         """The tensor's bytes as an array of its own element type, in ndarray (outermost first) order."""
-        T = self.graph.tensors[tensor]
-        n = T.nbytes()
-        out = np.empty(n, np.uint8)
-        check(self.native.L.tlb_program_read(self.h, tensor, n, out.ctypes.data_as(C.c_void_p)))
-        dt = dtype or _NP_OF.get(T.ty)
-        if dt is None:
-            return out
-        shape = [d for d in reversed(T.ne)]
-        while len(shape) > 1 and shape[0] == 1:
-            shape.pop(0)
-        return out.view(dt).reshape(shape)
+        known = self._result.get((tensor, dtype))
+        if known is None:
+            T = self.graph.tensors[tensor]
+            shape = [d for d in reversed(T.ne)]
+            while len(shape) > 1 and shape[0] == 1:
+                shape.pop(0)
+            known = self._result[(tensor, dtype)] = (T.nbytes(), dtype or _NP_OF.get(T.ty), tuple(shape))
+        n, dt, shape = known
+        out = _result_bytes(n)
+        check(self.native.L.tlb_program_read(self.h, tensor, n, _address(out)))
+        return out if dt is None else out.view(dt).reshape(shape)
 
     def outputs(self) -> list[tuple[str, np.ndarray]]:
         return [(name, self.read(t)) for name, t in self._outputs]
@@ -329,6 +368,7 @@ class EntryCache:
         self.native, self.build = native, build
         self.compile = compile or (lambda native, graph: NativeProgram.compile(native, graph))
         self.programs: dict[str, list[tuple[tuple, object]]] = {}
+        self.declared = weakref.WeakKeyDictionary()     # program -> its declared inputs, in input order
 
     def program(self, name: str, shapes: tuple):
         lst = self.programs.setdefault(name, [])
@@ -346,15 +386,17 @@ class EntryCache:
         """inputs: arrays in the entry's input order. f32 goes in as it is; an input the graph declares i32 takes
         whole-number values. Returns the outputs as (name, array) pairs."""
         arrays = [np.asarray(a) for a in inputs]
-        prog = self.program(name, tuple(tuple(a.shape) for a in arrays))
-        declared = [t for t in prog.graph.tensors if t.storage_kind == INPUT]
-        declared.sort(key=lambda t: t.storage_index)
+        prog = self.program(name, tuple([a.shape for a in arrays]))
+        declared = self.declared.get(prog)
+        if declared is None:
+            declared = sorted((t for t in prog.graph.tensors if t.storage_kind == INPUT), key=lambda t: t.storage_index)
+            self.declared[prog] = declared
         for i, a in enumerate(arrays):
             t = declared[i] if i < len(declared) else None
             if t is not None and t.ty in (I32, I64):
                 a = to_i32(t.name, a) if t.ty == I32 else to_i32(t.name, a).astype(np.int64)
-            elif t is not None and t.ty == F32:
-                a = np.ascontiguousarray(a, np.float32)
+            elif t is not None and t.ty == F32 and a.dtype != np.float32:
+                a = a.astype(np.float32)
             prog.set_input(i, a)
         prog.run(state)
         return prog.outputs()
@@ -371,7 +413,8 @@ def quantize_rows(native: Native, ty: int, x: np.ndarray) -> np.ndarray:
     x = np.ascontiguousarray(x, np.float32)
     rows, n = x.shape
     name, blck, size = TYPE_TRAITS.get(ty, ("?", 1, 0))      # an unknown type is refused by name by the library
-    out = np.zeros((rows, size * n // blck if n % blck == 0 else 0), np.uint8)
+    row = size * n // blck if n % blck == 0 else 0
+    out = _result_bytes(rows * row).reshape(rows, row)
     check(native.L.tlb_quantize_rows(native.dev, ty, x.ctypes.data_as(C.c_void_p), rows, n,
                                      out.ctypes.data_as(C.c_void_p)))
     return out

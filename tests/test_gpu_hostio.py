@@ -1,0 +1,116 @@
+"""Inputs and results on their way between the host and the device: the pinned page of a program (tensors of at most
+64 KB), staged copies above it, results in pinned memory, quantize_rows in pieces. Values are compared for equality."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tensorlisp_b200 import graph as G
+from tensorlisp_b200._lib import check
+from tensorlisp_b200.native import Native, NativeProgram, quantize_rows
+
+pytestmark = pytest.mark.gpu
+
+# around the page's limit (16384 f32), its 16-byte pieces, the chunk sizes and thread counts of the staged copies
+SIZES = [1, 3, 4, 1023, 4097, 16383, 16384, 16385, 65536, 65537, 262144, 262145, 524287, 524289, 4194304, 4194305]
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_every_run_sees_the_inputs_set_last(n):
+    native = Native.load([])
+    g = G.Graph()
+    x, z = g.input(G.F32, [n], "x"), g.input(G.F32, [4], "z")
+    y, w = g.output(g.scale(x, 2.0)), g.output(g.scale(z, 3.0))
+    prog = NativeProgram.compile(native, g)
+    rng = np.random.default_rng(n)
+    held = []
+    for i in range(4):      # from the second run on the small results come through the page
+        a, b = rng.standard_normal(n).astype(np.float32), rng.standard_normal(4).astype(np.float32)
+        prog.set_input(0, np.zeros(n, np.float32))
+        prog.set_input(0, a)
+        if i != 2:
+            prog.set_input(1, b)
+            last = b
+        prog.run()
+        got = prog.read(y)
+        assert np.array_equal(got.reshape(-1), 2 * a)
+        assert np.array_equal(prog.read(w).reshape(-1), 3 * last)
+        held.append((got, 2 * a))
+    prog.enqueue()          # nothing set in between: the same again, and read() waits for it
+    assert np.array_equal(prog.read(y).reshape(-1), 2 * a)
+    for got, want in held:  # results are the caller's: later runs leave them alone
+        assert np.array_equal(got.reshape(-1), want)
+    assert np.array_equal(prog.read(x).reshape(-1), a)
+    prog.free()
+    native.close()
+
+
+def test_a_device_side_input_and_the_page_keep_their_order():
+    native = Native.load([])
+    g = G.Graph()
+    x = g.input(G.F32, [8], "x")
+    y = g.output(g.scale(x, 2.0))
+    prog = NativeProgram.compile(native, g)
+    ones = np.ones(8, np.float32)
+    prog.set_input(0, ones)
+    prog.run()
+    prog.set_input(0, 5 * ones)     # overtaken by the copy behind it
+    prog.feed_input(0, y)
+    prog.run()
+    assert np.array_equal(prog.read(y).reshape(-1), 4 * ones)
+    prog.feed_input(0, y)           # overtaken by the input set behind it
+    prog.set_input(0, 7 * ones)
+    prog.enqueue()
+    prog.enqueue()
+    assert np.array_equal(prog.read(y).reshape(-1), 14 * ones)
+    for _ in range(3):              # a loop that never waits
+        prog.feed_input(0, y)
+        prog.enqueue()
+    assert np.array_equal(prog.read(y).reshape(-1), 112 * ones)
+    prog.free()
+    native.close()
+
+
+def test_a_known_device_address_sees_every_input_and_every_result():
+    import torch
+
+    class At:
+        def __init__(self, ptr, n):
+            self.__cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(ptr, False), version=3, strides=None)
+
+    native = Native.load([])
+    g = G.Graph()
+    x = g.input(G.F32, [16], "x")
+    y = g.output(g.scale(x, 2.0))
+    prog = NativeProgram.compile(native, g)
+    a = np.arange(16, dtype=np.float32)
+    prog.set_input(0, a)
+    prog.run()
+    prog.read(y)
+    prog.run()
+    dx, dy = torch.as_tensor(At(prog.tensor_ptr(x)[0], 16), device="cuda"), torch.as_tensor(At(prog.tensor_ptr(y)[0], 16), device="cuda")
+    prog.set_input(0, a + 1)
+    assert np.array_equal(dx.cpu().numpy(), a + 1)
+    dx.add_(1)
+    torch.cuda.synchronize()
+    prog.run()
+    assert np.array_equal(prog.read(y).reshape(-1), 2 * (a + 2))
+    dy.fill_(9)
+    torch.cuda.synchronize()
+    assert np.array_equal(prog.read(y).reshape(-1), np.full(16, 9, np.float32))
+    prog.free()
+    native.close()
+
+
+@pytest.mark.parametrize("ty,name", [(G.Q8_0, "q8_0"), (G.Q4_K, "q4_K")])
+@pytest.mark.parametrize("rows,n", [(1, 256), (300, 256), (1025, 4096), (5000, 4096), (7, 1 << 20)])
+def test_quantize_rows_in_pieces(oracle, ty, name, rows, n):
+    native = Native(0)
+    x = np.random.default_rng(rows).standard_normal((rows, n)).astype(np.float32)
+    got = quantize_rows(native, ty, x)
+    plain = np.zeros_like(np.empty(got.shape, np.uint8))        # ordinary memory takes the staged way down
+    check(native.L.tlb_quantize_rows(native.dev, ty, x.ctypes.data_as(C.c_void_p), rows, n, plain.ctypes.data_as(C.c_void_p)))
+    assert np.array_equal(got, plain)
+    some = np.unique(np.concatenate([[0, rows - 1], np.random.default_rng(1).integers(0, rows, 40)]))
+    assert np.array_equal(got[some], oracle.quantize(ty, x[some]))
+    native.close()
