@@ -675,6 +675,20 @@ cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes,
     return cudaSuccess;
 }
 
+// 2-D tensor map of 16-bit elements, boxes of at most 64 columns (one 128-byte swizzled line) x box_rows; rows and columns
+// outside the matrix read as zero
+cudaError_t tc_encode_2d_sw128(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t cols, uint64_t rows, uint32_t box_cols, uint32_t box_rows, bool bf16) {
+    if (encode_tiled() == nullptr) return cudaErrorNotSupported;
+    const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {box_cols, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    if (encode_tiled()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), gdim, gstride, box, estr,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    return cudaSuccess;
+}
+
 void launch_mmq_reduce(const float *partial, float *y, int64_t total, int n_split, cudaStream_t st) {
     ReduceSegs g{};
     g.n_segs = 1;

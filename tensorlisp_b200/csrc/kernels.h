@@ -82,6 +82,19 @@ cudaError_t launch_mm_fold_f16(bool q4k, const void *W, int64_t K, int64_t M, in
                                cudaStream_t st);
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st);
 
+// ---------------------------------------------------------------- k_mm_plain.cu
+// f16 / bf16 weights x f32 activations (as three terms of the weights' type) on tcgen05, any number of columns
+struct PlainPlan {
+    int passes, cols;        // activation columns are processed `cols` at a time
+    int steps, tiles, ctas;
+    uint64_t bytes;          // scratch: the parts of cut tiles (0: no tile is cut)
+};
+bool mm_plain_supported(uint32_t type, int64_t K, int64_t M, int64_t N, uint64_t w_row_bytes);
+PlainPlan mm_plain_plan(int64_t K, int64_t M, int64_t N, int sm_count);
+cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64_t w_row_bytes, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx,
+                            float *y, int64_t ldy, void *scratch, int *err, cudaStream_t st);
+void mm_plain_configure();
+
 // ---------------------------------------------------------------- k_fused.cu
 // One row (= activation column n) per CTA: produce the f32 row, quantize it to Q8_K into an ActLayout
 // block at `out`, optionally also pack the tensor-core blobs behind it.

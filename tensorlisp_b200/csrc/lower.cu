@@ -364,6 +364,17 @@ bool allreduce_follows(const L &l) {
     return nx.op == "ALLREDUCE" && nx.src[0] == l.id;
 }
 
+// f16 / bf16 weights of an unbatched product whose rows and columns the copies of the tensor-core kernel can address
+bool plain_tc(const Graph &g, const Tensor &t) {
+    if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || getenv("TLB_MM_GENERIC") || getenv("TLB_NO_TC")) return false;
+    const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
+    if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1 || tx.ne[2] * tx.ne[3] != 1 || tx.ty != TLB_TYPE_F32 || t.ty != TLB_TYPE_F32 || !t.is_contiguous()) return false;
+    uint64_t wo = 0, xo = 0;
+    g.root(t.src[0], &wo);
+    g.root(t.src[1], &xo);
+    return tx.nb[0] == 4 && tx.nb[1] % 16 == 0 && wo % 16 == 0 && xo % 16 == 0 && mm_plain_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1], tw.nb[1]);
+}
+
 // ---- MUL_MAT (lower.rs:543-571). Quantized weights take int8 activations quantized once per
 // distinct activation tensor by a QUANT_ACT node that rewrite_graph put in src[2].
 void lower_mul_mat(L &l) {
@@ -387,6 +398,22 @@ void lower_mul_mat(L &l) {
     g.y = view_of(t);
     g.r2 = t.ne[2] / tw.ne[2];
     g.r3 = t.ne[3] / tw.ne[3];
+    if (plain_tc(*l.c.g, t)) {
+        const PlainPlan pp = mm_plain_plan(K, M, N, sm);
+        const int64_t sc = l.c.layout->scratch[l.pos];
+        if (pp.bytes > 0 && sc < 0) throw std::string("mul_mat scratch was not planned");
+        Place ps;
+        ps.buf = BUF_ARENA;
+        ps.off = sc < 0 ? 0 : (uint64_t)sc;
+        const bool bf16 = tw.ty == TLB_TYPE_BF16;
+        const uint64_t wrow = tw.nb[1];
+        const int64_t ldx = N > 1 ? (int64_t)tx.nb[1] / 4 : K;
+        l.push([=](const RunCtx &r) {
+            if (((uintptr_t)r.at(pw) | (uintptr_t)r.at(px)) & 15) return launch_mm_generic(g, r.at(pw), r.at(px), r.at(pd), r.stream);   // a state block laid out by the caller
+            return launch_mm_plain(pp, bf16, r.at(pw), wrow, K, M, N, (const float *)r.at(px), ldx, (float *)r.at(pd), M, r.at(ps), r.err, r.stream);
+        });
+        return;
+    }
     if (!gemv_type(tw.ty)) {
         l.push([=](const RunCtx &r) { return launch_mm_generic(g, r.at(pw), r.at(px), r.at(pd), r.stream); });
         return;
@@ -873,6 +900,10 @@ uint64_t node_scratch_bytes(const Graph &g, int32_t id, int sm_count) {
         for (int s : {0, 3, 5})
             if (t.src[s] >= 0) Msum += g.tensors[t.src[s]].ne[1];
         return mmq_tc_plan(tx.ne[0], Msum, tx.ne[1], sm_count).partial_bytes;
+    }
+    if (plain_tc(g, t)) {
+        const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
+        return mm_plain_plan(tw.ne[0], tw.ne[1], tx.ne[1], sm_count).bytes;
     }
     if (t.op == "MUL_MAT" && t.src[0] >= 0 && t.src[1] >= 0 && t.src[2] >= 0 && is_qact(g.tensors[t.src[2]].op) &&
         g.tensors[t.src[2]].op_params[1] > 0) {
