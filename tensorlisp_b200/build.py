@@ -3,8 +3,8 @@
     python -m tensorlisp_b200.build [--force] [--verbose]
 
 Every .cu under csrc/ is compiled to an object (in parallel) and linked into one shared library
-that exports exactly the C ABI of include/tlb200.h. k_quant.cu is compiled with -fmad=false: the
-row quantizers must round every intermediate the way the reference's no-FMA build does.
+that exports exactly the C ABI of include/tlb200.h. k_quant.cu, k_fused.cu and k_gemv.cu are compiled with
+-fmad=false: the row quantizers must round every intermediate the way the reference's no-FMA build does.
 """
 from __future__ import annotations
 
@@ -23,7 +23,7 @@ LIB = HERE / "libtlb200.so"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", 
           "-Xcompiler", "-Wall", "--expt-relaxed-constexpr", "-DTLB_BUILDING"]
-PER_FILE = {"k_quant.cu": ["-fmad=false"], "k_fused.cu": ["-fmad=false"]}
+PER_FILE = {"k_quant.cu": ["-fmad=false"], "k_fused.cu": ["-fmad=false"], "k_gemv.cu": ["-fmad=false"]}
 
 
 def _nvcc() -> str:

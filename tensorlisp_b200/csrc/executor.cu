@@ -330,7 +330,7 @@ static tlb_status buffer_create(tlb_device *dev, uint64_t bytes, bool zero, tlb_
     cudaSetDevice(dev->ordinal);
     void *p = nullptr;
     const uint64_t n = std::max<uint64_t>(bytes, 1);
-    cudaError_t e = cudaMalloc(&p, n);
+    cudaError_t e = cudaMalloc(&p, align_up(n));   // 16-byte copies of a matrix's last rows may end past it
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(TLB_ALLOC, "buffer allocation of " + std::to_string(n) + " bytes failed");

@@ -20,34 +20,6 @@ namespace tlb {
 constexpr int RQ_THREADS = 256;
 constexpr int RQ_WARPS = RQ_THREADS / 32;
 
-// The f32 value at (column n, element k) before any normalisation: a, a + b, act(a) * b or f16 a.
-__device__ __forceinline__ void rq_load8(const RowQuantArgs &p, int n, int64_t k0, float (&x)[8]) {
-    if (p.mode == RQ_GLU) {
-        const float4 g0 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0), g1 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0 + 4);
-        const float4 u0 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0), u1 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0 + 4);
-        const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-#pragma unroll
-        for (int e = 0; e < 8; e++) x[e] = __fmul_rn(__fdiv_rn(g[e], __fadd_rn(1.0f, expf(-g[e]))), u[e]);   // SiLU(g)*u
-    } else if (p.mode == RQ_F16) {
-        const uint4 h = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p.a) + n * p.lda + k0);
-        const __half2 *h2 = reinterpret_cast<const __half2 *>(&h);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float2 f = __half22float2(h2[e]);
-            x[2 * e] = f.x;
-            x[2 * e + 1] = f.y;
-        }
-    } else {
-        const float4 a0 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0), a1 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0 + 4);
-        x[0] = a0.x; x[1] = a0.y; x[2] = a0.z; x[3] = a0.w; x[4] = a1.x; x[5] = a1.y; x[6] = a1.z; x[7] = a1.w;
-        if (p.b) {   // residual add: x = a + b
-            const float4 b0 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0), b1 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0 + 4);
-            x[0] = __fadd_rn(x[0], b0.x); x[1] = __fadd_rn(x[1], b0.y); x[2] = __fadd_rn(x[2], b0.z); x[3] = __fadd_rn(x[3], b0.w);
-            x[4] = __fadd_rn(x[4], b1.x); x[5] = __fadd_rn(x[5], b1.y); x[6] = __fadd_rn(x[6], b1.z); x[7] = __fadd_rn(x[7], b1.w);
-        }
-    }
-}
-
 // Grid (column, slice of 8 blocks): every warp owns ONE 256-element block, so a row of 4096 (14336)
 // elements is spread over 2 (7) CTAs instead of one warp walking several blocks in turn. With a
 // normalisation, every CTA of a row first adds up the squares of the whole row in the same order
@@ -198,8 +170,9 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
         const __half2 t = __floats2half2_rn(__fmul_rn(q0, dh), __fmul_rn(q1, dh));
         h[e] = *reinterpret_cast<const uint32_t *>(&t);
     }
-    *reinterpret_cast<uint4 *>(blob) = make_uint4(h[0], h[1], h[2], h[3]);
-    // the Q8_0 block itself too (int8 codes and f32 scales): a consumer that is not a prompt-sized 2-D mul_mat reads those
+    if (p.npad) *reinterpret_cast<uint4 *>(blob) = make_uint4(h[0], h[1], h[2], h[3]);
+    // the Q8_0 block itself (int8 codes and f32 scales): the few-column mul_mat reads it (npad 0: nothing else is wanted), and any
+    // consumer that is not a prompt-sized 2-D product
     uint2 packed;
     packed.x = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
     packed.y = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
@@ -433,8 +406,8 @@ bool row_quant_supported(int64_t K) { return K % 256 == 0 && K / 256 <= 65535 * 
 cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st) {
     if (p.N == 0 || p.K == 0) return cudaSuccess;
     if (p.q80) {
-        if (p.npad != 256 || !row_quant_q80_supported(p.K, p.mode)) return cudaErrorInvalidValue;
-        const int rows256 = (int)((p.N + 255) / 256) * 256, nb = (int)(p.K / 256);
+        if ((p.npad != 256 && p.npad != 0) || !row_quant_q80_supported(p.K, p.mode)) return cudaErrorInvalidValue;
+        const int rows256 = p.npad ? (int)((p.N + 255) / 256) * 256 : (int)p.N, nb = (int)(p.K / 256);
         if (p.mode == RQ_NORM) return launch_pdl(k_row_quant_q80, dim3(rows256, 1), dim3(nb * 32), 0, st, p);
         return launch_pdl(k_row_quant_q80, dim3(rows256, (nb + 7) / 8), dim3(256), 0, st, p);
     }

@@ -593,7 +593,7 @@ void mmq_tc_configure() {
 }
 
 bool mmq_tc_supported(uint32_t type, int64_t K, int64_t M, int64_t N) {
-    return type == TLB_TYPE_Q4_K && K % 256 == 0 && K >= 256 && M >= 1 && N > 4 && N <= (int64_t)MM_FOLD_NPAD * 65535 && encode_tiled() != nullptr;
+    return type == TLB_TYPE_Q4_K && K % 256 == 0 && K >= 256 && M >= 1 && N > GEMV_MAX_COLS && N <= (int64_t)MM_FOLD_NPAD * 65535 && encode_tiled() != nullptr;
 }
 
 TcPlan mmq_tc_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
@@ -671,6 +671,19 @@ cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes,
     if (encode_tiled()(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), gdim,
                        gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    return cudaSuccess;
+}
+
+// the same over 8-byte elements: boxes of up to 2 KB per row (multiples of 16 bytes; bytes past a row's end read as zero)
+cudaError_t tc_encode_2d_bytes(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows) {
+    if (encode_tiled() == nullptr) return cudaErrorNotSupported;
+    const cuuint64_t gdim[2] = {(cuuint64_t)(row_bytes / 8), (cuuint64_t)rows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {box_bytes / 8, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    if (encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void *>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     return cudaSuccess;
 }

@@ -26,12 +26,10 @@ ActLayout act_layout(int kind, int64_t K, int64_t N);
 cudaError_t launch_quantize_rows(uint32_t type, const float *x, int64_t rows, int64_t n_per_row, void *y, cudaStream_t st);
 cudaError_t launch_act_quantize(const ActLayout &a, const float *x, int64_t ldx, void *out, cudaStream_t st);
 
+// Up to this many activation columns the few-column kernel (k_gemv.cu) is the faster one: its matrix instruction takes eight.
+constexpr int64_t GEMV_MAX_COLS = 8;
+
 // ---------------------------------------------------------------- k_mm.cu
-// y[n*ldy + m] = dot(W row m, quantized activation column n), contiguous W rows of K elements.
-// Returns cudaErrorNotSupported when the shape cannot use the pipelined kernel (caller falls back).
-bool gemv_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
-cudaError_t launch_gemv(uint32_t type, const void *W, int64_t K, int64_t M, const ActLayout &a, const void *act,
-                        float *y, int64_t ldy, int sm_count, int *err_flag, cudaStream_t st);
 // Generic strided / batched product (any supported weight type, f32 activations or a quantized
 // activation block per (i2,i3) batch). dst f32.
 struct MMGeneric {
@@ -42,7 +40,6 @@ struct MMGeneric {
     ActLayout a;
 };
 cudaError_t launch_mm_generic(const MMGeneric &p, const void *W, const void *X, void *Y, cudaStream_t st);
-void gemv_configure();  // sets the dynamic shared-memory attributes once per process
 
 // ---------------------------------------------------------------- k_mmq_tc.cu
 // Q4_K weights x 5..64 activation columns on tcgen05 (f16 operands built from the integer codes).
@@ -98,7 +95,7 @@ void mm_plain_configure();
 // ---------------------------------------------------------------- k_fused.cu
 // One row (= activation column n) per CTA: produce the f32 row, quantize it to Q8_K into an ActLayout
 // block at `out`, optionally also pack the tensor-core blobs behind it.
-enum { RQ_PLAIN = 0, RQ_NORM = 1, RQ_GLU = 2, RQ_F16 = 3 };
+enum { RQ_PLAIN = 0, RQ_NORM = 1, RQ_GLU = 2, RQ_F16 = 3, RQ_READY = 4 };
 struct RowQuantArgs {
     int mode;
     int64_t K, N;
@@ -121,6 +118,27 @@ struct RowQuantArgs {
                          // operand (blobs of 256 columns x 64 elements, value = code x f16 scale) is produced
 };
 bool row_quant_supported(int64_t K);
+
+// ---------------------------------------------------------------- k_gemv.cu
+// Up to three matrices of one block type and row length against a few activation columns (eight per launch). act: mode, sources,
+// eps, norm weight and sum_out as for launch_row_quant, the rows then being produced and quantized in the launch itself; or
+// RQ_READY: `ready` is an ActLayout block (act: its offsets). Q6_K (k_gemv_f32.cu): one matrix, RQ_PLAIN, four columns per launch.
+struct GemvArgs {
+    uint32_t type;
+    int n_mats, glu;             // glu: W[0] and W[1] are gate and up, y[0] = SiLU(gate) * up
+    const void *W[3];
+    float *y[3];
+    int64_t M[3], ldy[3];
+    int64_t K, N;
+    RowQuantArgs act;
+    const void *ready;
+};
+bool gemv_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
+cudaError_t launch_gemv(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
+void gemv_configure();
+bool gemv_f32_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
+cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
+void gemv_f32_configure();
 bool row_quant_q80_supported(int64_t K, int mode);
 cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st);
 // the all-reduce in front of a residual add + RMS norm + quantizer fused into one kernel (tensor parallelism):

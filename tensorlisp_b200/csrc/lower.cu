@@ -43,6 +43,25 @@ TcPlan tc_plan(uint32_t wty, int64_t K, int64_t M, int64_t N, int sm) {
     return wty == TLB_TYPE_Q8_0 ? mmq_tc8_plan(K, M, N, sm) : mmq_tc_plan(K, M, N, sm);
 }
 
+// A product that the few-column kernel takes (k_gemv.cu): a 2-D matrix of whole super-blocks, at most eight columns, or any
+// number of them where no tensor-core kernel reads the type.
+bool gemv_node(const Graph &g, const Tensor &t) {
+    if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || getenv("TLB_MM_GENERIC")) return false;
+    const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
+    if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1 || tx.ne[2] * tx.ne[3] != 1 || tx.ty != TLB_TYPE_F32 || t.ty != TLB_TYPE_F32) return false;
+    if (tw.ne[0] != tx.ne[0] || t.ne[0] != tw.ne[1] || t.ne[1] != tx.ne[1] || t.nelements() == 0) return false;
+    if (tw.nb[1] != tw.row_size() || tw.nb[0] != type_traits(tw.ty)->size || !t.is_contiguous() || tx.nb[0] != 4 || tx.nb[1] % 16) return false;
+    uint64_t wo = 0, xo = 0;
+    g.root(t.src[0], &wo);
+    g.root(t.src[1], &xo);
+    if (wo % 16 || xo % 16 || !gemv_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1])) return false;
+    return getenv("TLB_NO_TC") || !tc_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1]);
+}
+// One or two rows are produced and quantized by the product's own launch; more are a launch of their own, which spreads them over
+// the SMs (a CTA needs about 0.5 us per row of 4096). f32 activations (Q6_K) are read as they are.
+bool gemv_self_quant(const Graph &g, const Tensor &t) { return t.ne[1] <= 2 || g.tensors[t.src[0]].ty == TLB_TYPE_Q6_K; }
+constexpr int GEMV_MARK = 8, GEMV_MODE = 9, GEMV_GLU = 10;   // op_params of such a node once fuse_gemv has seen it; eps in 15
+
 int act_kind_for(uint32_t wty) { return wty == TLB_TYPE_Q4_K ? ACT_Q8_K : ACT_Q8_0; }
 bool is_qact(const std::string &op) { return op == "QUANT_ACT" || op == "ROW_QUANT"; }
 
@@ -449,18 +468,68 @@ void lower_mul_mat(L &l) {
         });
         return;
     }
-    if (!batched && dense_w && dense_y && gemv_supported(tw.ty, K, M, N) && !getenv("TLB_MM_GENERIC")) {
-        const uint32_t wty = tw.ty;
-        l.push([=](const RunCtx &r) {
-            return launch_gemv(wty, r.at(pw), K, M, a, r.at(pq), (float *)r.at(pd), M, sm, r.err, r.stream);
-        });
-        return;
-    }
     g.a = a;
     l.push([=](const RunCtx &r) {
         MMGeneric gg = g;
         gg.act = r.at(pq);
         return launch_mm_generic(gg, r.at(pw), r.at(px), r.at(pd), r.stream);
+    });
+}
+
+// A node that fuse_gemv prepared: src = w0, row source (x, or the a / gate / f16 values its producer read), -, w1, y1, w2, y2,
+// the producer's second operand, its norm weight, its sum; the node's own tensor is y0 (with GEMV_GLU: SiLU(gate) * up).
+void lower_gemv(L &l) {
+    const Tensor &t = l.t();
+    const int32_t a = l.src(1), b = t.src[7], w = t.src[8], sum = t.src[9];
+    GemvArgs p{};
+    const Tensor &tw0 = l.T(l.src(0));
+    p.type = tw0.ty;
+    p.K = tw0.ne[0];
+    p.N = t.ne[1];
+    p.glu = t.op_params[GEMV_GLU];
+    Place pw[3], py[3];
+    const int wslot[3] = {0, 3, 5}, yslot[3] = {-1, 4, 6};
+    for (int j = 0; j < 3 && t.src[wslot[j]] >= 0; j++) {
+        const int32_t y = j == 0 || p.glu ? l.id : l.src(yslot[j]);
+        pw[j] = l.place(t.src[wslot[j]]);
+        py[j] = l.place(y);
+        p.M[j] = p.ldy[j] = l.T(t.src[wslot[j]]).ne[1];
+        p.n_mats++;
+    }
+    p.act.mode = t.op_params[GEMV_MODE];
+    p.act.K = p.K;
+    p.act.N = p.N;
+    p.act.eps = t.param_f32(15);
+    p.act.lda = p.act.mode == RQ_F16 || p.N == 1 ? p.K : (int64_t)l.T(a).nb[1] / 4;
+    if (b >= 0) p.act.ldb = p.N > 1 ? (int64_t)l.T(b).nb[1] / 4 : p.K;
+    if (w >= 0) p.act.wn = l.T(w).ne[0];
+    p.act.ld_sum = p.K;
+    const Place pa = l.place(a);
+    Place pb, pn, ps, pq;
+    if (p.act.mode == RQ_READY) {
+        const ActLayout al = act_layout(act_kind_for(p.type), p.K, p.N);
+        p.act.qs_off = al.qs_off;
+        p.act.d_off = al.d_off;
+        p.act.bsum_off = al.bsum_off;
+        pq = l.place(l.src(2));
+    }
+    if (b >= 0) pb = l.place(b);
+    if (w >= 0) pn = l.place(w);
+    if (sum >= 0) ps = l.place(sum);
+    const int sm = l.c.dev->prop.multiProcessorCount;
+    l.push([=](const RunCtx &r) {
+        GemvArgs q = p;
+        for (int j = 0; j < q.n_mats; j++) {
+            q.W[j] = r.at(pw[j]);
+            q.y[j] = (float *)r.at(py[j]);
+            if ((uintptr_t)q.W[j] & 15) return cudaErrorMisalignedAddress;   // a weight offset that is not what the leaves promise
+        }
+        q.act.a = (const float *)r.at(pa);
+        q.act.b = b >= 0 ? (const float *)r.at(pb) : nullptr;
+        q.act.w = w >= 0 ? (const float *)r.at(pn) : nullptr;
+        q.act.sum_out = sum >= 0 ? (float *)r.at(ps) : nullptr;
+        q.ready = q.act.mode == RQ_READY ? r.at(pq) : nullptr;
+        return launch_gemv(q, sm, r.err, r.stream);
     });
 }
 
@@ -1050,6 +1119,7 @@ void lower_node(const LowerCtx &c, int32_t id, int pos, std::vector<Dispatch> &o
     if (op == "ARGMAX") return lower_argmax(l);
     if (op == "CONCAT" || op == "REPEAT" || op == "SUM_ROWS" || op == "MEAN" || op == "ARANGE") return lower_simple(l);
     if (op == "IM2COL" || op == "UPSCALE" || op == "POOL_2D" || op == "CONV_2D_DW" || op == "PAD" || op == "PAD_REFLECT_1D") return lower_image(l);
+    if ((op == "MUL_MAT" || op == "MUL_MAT_GROUP") && t.op_params[GEMV_MARK]) return lower_gemv(l);
     if (op == "MUL_MAT") return lower_mul_mat(l);
     if (op == "MUL_MAT_GROUP") return lower_mul_mat_group(l);
     if (op == "CUSTOM") return lower_custom(l);
@@ -1063,6 +1133,7 @@ void fuse_row_producers(Graph &g);
 void fuse_rope_cache(Graph &g);
 void fuse_mul_mat_groups(Graph &g);
 void fuse_attn_quant(Graph &g);
+void fuse_gemv(Graph &g, bool groups, bool producers);
 // Readers of every root (views of a tensor count for the root), as fuse.rs:56-63 requires.
 void rewrite_graph(Graph &g) {
     const size_t nt0 = g.tensors.size();
@@ -1158,7 +1229,8 @@ void rewrite_graph(Graph &g) {
             }
         }
         Tensor &t = g.tensors[id];
-        if (t.op == "MUL_MAT" && t.src[0] >= 0 && t.src[1] >= 0 && gemv_type(g.tensors[t.src[0]].ty)) {
+        if (t.op == "MUL_MAT" && t.src[0] >= 0 && t.src[1] >= 0 && gemv_type(g.tensors[t.src[0]].ty) &&
+            !(gemv_node(g, t) && gemv_self_quant(g, t))) {
             const Tensor tw = g.tensors[t.src[0]];   // by value: the tensor vector grows below
             const int32_t x = t.src[1];
             const Tensor tx = g.tensors[x];
@@ -1207,6 +1279,7 @@ void rewrite_graph(Graph &g) {
         nodes.push_back(id);
     }
     g.nodes.swap(nodes);
+    fuse_gemv(g, enabled("MUL_MAT_GROUP"), enabled("ROW_QUANT"));
     if (enabled("ROW_QUANT")) fuse_row_producers(g);
     if (enabled("ROW_QUANT") && enabled("ATTN_QUANT")) fuse_attn_quant(g);
     if (enabled("ROPE_KV_WRITE")) fuse_rope_cache(g);
@@ -1261,7 +1334,7 @@ void fuse_row_producers(Graph &g) {
     for (int32_t k : g.keep) kept[g.root(k)] = 1;
     // a MUL_MAT that carries a QUANT_ACT of its activation never reads the f32 activation itself
     auto really_reads = [&](const Tensor &t, int slot) {
-        return !(t.op == "MUL_MAT" && slot == 1 && t.src[2] >= 0 && is_qact(g.tensors[t.src[2]].op) &&
+        return !((t.op == "MUL_MAT" || t.op == "MUL_MAT_GROUP") && slot == 1 && t.src[2] >= 0 && is_qact(g.tensors[t.src[2]].op) &&
                  gemv_type(g.tensors[t.src[0]].ty));
     };
     // readers of a root among the nodes, by position
@@ -1284,9 +1357,11 @@ void fuse_row_producers(Graph &g) {
     for (size_t qi = 0; qi < nn; qi++) {
         const int32_t qid = g.nodes[qi];
         if (g.tensors[qid].op != "QUANT_ACT") continue;
-        // Q8_K activations (Q4_K weights), or the Q8_0 activations of the prompt mul_mat (operand blobs of 256 columns)
+        // Q8_K activations (Q4_K weights), or the Q8_0 activations of the prompt mul_mat (operand blobs of 256 columns) and of the
+        // few-column kernel (no blobs)
         const bool q80 = g.tensors[qid].op_params[0] == ACT_Q8_0;
-        if (q80 && g.tensors[qid].op_params[1] != 256) continue;
+        if (q80 && g.tensors[qid].op_params[1] != 256 && g.tensors[qid].op_params[1] != 0) continue;
+        if (q80 && !row_quant_q80_supported(g.tensors[g.tensors[qid].src[0]].ne[0], RQ_PLAIN)) continue;
         const int32_t x = g.tensors[qid].src[0];
         const Tensor X = g.tensors[x];
         if (X.ty != 0 || !row_quant_supported(X.ne[0]) || !dense_rows(X, 4)) continue;
@@ -1454,6 +1529,153 @@ void fuse_rope_cache(Graph &g) {
 }
 
 
+// Few-column mul_mats (gemv_node): matrices of one type and row length that read the same activations become one node (wq / wk / wv,
+// gate / up), SiLU(gate) * up its epilogue, and the producer of the activations (RMS norm with the residual add in front
+// of it, the f16 -> f32 cast of the attention output, a gate) its prologue. Legality as for the other fusions: a folded
+// intermediate has no other reader, is not kept, and nothing between the folded nodes and the fused one touches it.
+void fuse_gemv(Graph &g, bool groups, bool producers) {
+    const size_t nn = g.nodes.size();
+    std::vector<char> dead(nn, 0), kept(g.tensors.size(), 0);
+    for (int32_t k : g.keep) kept[g.root(k)] = 1;
+    auto live_readers = [&](int32_t root, std::vector<int> &out) {   // positions; views launch nothing and count through their readers
+        out.clear();
+        for (size_t i = 0; i < nn; i++) {
+            const Tensor &t = g.tensors[g.nodes[i]];
+            if (dead[i] || t.is_view_op()) continue;
+            for (int s = 0; s < 10; s++)
+                if (t.src[s] >= 0 && g.root(t.src[s]) == root) {
+                    out.push_back((int)i);
+                    break;
+                }
+        }
+    };
+    auto dense_rows = [&](const Tensor &t) {
+        return t.ty == TLB_TYPE_F32 && t.nb[0] == 4 && t.nb[1] % 16 == 0 && (t.ne[2] <= 1 || t.nb[2] == t.nb[1] * (uint64_t)t.ne[1]) &&
+               (t.ne[3] <= 1 || t.nb[3] == t.nb[1] * (uint64_t)t.ne[1] * (uint64_t)t.ne[2]);
+    };
+    auto aligned = [&](int32_t id) {
+        uint64_t o = 0;
+        g.root(id, &o);
+        return o % 16 == 0;
+    };
+    const int wslot[3] = {0, 3, 5}, yslot[3] = {-1, 4, 6};
+    std::vector<int> rd;
+    for (size_t i = 0; i < nn; i++) {
+        if (dead[i] || !gemv_node(g, g.tensors[g.nodes[i]])) continue;
+        if (!gemv_self_quant(g, g.tensors[g.nodes[i]]) && g.tensors[g.nodes[i]].src[2] < 0) continue;
+        Tensor &A = g.tensors[g.nodes[i]];
+        const Tensor W0 = g.tensors[A.src[0]];
+        int members = 1;
+        int last = (int)i;
+        if (groups && W0.row_size() % 16 == 0 && A.view_src < 0) {
+            for (size_t j = i + 1; j < nn && members < 3; j++) {
+                const Tensor &B = g.tensors[g.nodes[j]];
+                if (B.is_view_op()) continue;
+                if (!gemv_node(g, B) || B.src[1] != A.src[1] || B.src[2] != A.src[2] || B.view_src >= 0 || g.tensors[B.src[0]].ty != W0.ty) break;
+                A.src[wslot[members]] = B.src[0];
+                A.src[yslot[members]] = g.nodes[j];
+                dead[j] = 1;
+                last = (int)j;
+                members++;
+            }
+        }
+        if (members > 1) A.op = "MUL_MAT_GROUP";
+        A.op_params[GEMV_MARK] = 1;
+        const bool self = gemv_self_quant(g, A);
+        A.op_params[GEMV_MODE] = self ? RQ_PLAIN : RQ_READY;
+        A.op_params[GEMV_GLU] = 0;
+        if (self) A.src[2] = -1;
+        if (!producers) continue;
+        // ---- prologue
+        const int32_t x = A.src[1], xroot = g.root(x);
+        live_readers(xroot, rd);
+        int xp = -1;
+        for (size_t k = 0; k < i; k++)
+            if (!dead[k] && g.nodes[k] == xroot) xp = (int)k;
+        bool only = self && xp >= 0 && !kept[xroot] && g.tensors[xroot].view_src < 0 && W0.ty != TLB_TYPE_Q6_K;
+        for (int r : rd) only = only && (r == (int)i || r == xp);   // (a cast lists itself as a source)
+        if (only) {
+            const Tensor P = g.tensors[xroot];
+            if (P.op == "RMS_NORM_MUL" && xroot == x) {
+                const int32_t a = P.src[0], w = P.src[1];
+                const Tensor &W = g.tensors[w];
+                if (dense_rows(g.tensors[a]) && aligned(a) && aligned(w) && W.ty == TLB_TYPE_F32 && W.nb[0] == 4 && W.ne[0] % 8 == 0 && W.ne[1] * W.ne[2] * W.ne[3] == 1) {
+                    A.op_params[GEMV_MODE] = RQ_NORM;
+                    A.op_params[15] = P.op_params[15];
+                    A.src[1] = a;
+                    A.src[8] = w;
+                    dead[xp] = 1;
+                    int ap = -1;
+                    for (int k = 0; k < xp; k++)
+                        if (!dead[k] && g.nodes[k] == a) ap = k;
+                    if (ap >= 0 && g.tensors[a].op == "ADD" && g.tensors[a].view_src < 0) {
+                        const Tensor R = g.tensors[a];
+                        const int32_t s0 = R.src[0], s1 = R.src[1];
+                        bool ok = s0 >= 0 && s1 >= 0 && R.is_contiguous() && dense_rows(g.tensors[s0]) && dense_rows(g.tensors[s1]) && aligned(s0) && aligned(s1);
+                        for (int k = 0; ok && k < 4; k++) ok = g.tensors[s0].ne[k] == R.ne[k] && g.tensors[s1].ne[k] == R.ne[k];
+                        live_readers(a, rd);   // nobody may read the sum between the add's old place and this node
+                        for (int r : rd) ok = ok && (r >= (int)i || r == ap);
+                        // the operands keep their values until here: nothing in between writes to them in place
+                        for (int k = ap + 1; ok && k < (int)i; k++)
+                            if (!dead[k] && !g.tensors[g.nodes[k]].is_view_op()) ok = g.root(g.nodes[k]) != g.root(s0) && g.root(g.nodes[k]) != g.root(s1);
+                        if (ok) {
+                            A.src[1] = s0;
+                            A.src[7] = s1;
+                            A.src[9] = a;
+                            dead[ap] = 1;
+                        }
+                    }
+                }
+            } else if (P.op == "GLU" && xroot == x && P.op_params[0] == 2 && P.src[0] >= 0 && P.src[1] >= 0 && dense_rows(g.tensors[P.src[0]]) &&
+                       dense_rows(g.tensors[P.src[1]]) && aligned(P.src[0]) && aligned(P.src[1])) {
+                A.op_params[GEMV_MODE] = RQ_GLU;
+                A.src[1] = P.src[0];
+                A.src[7] = P.src[1];
+                dead[xp] = 1;
+            } else if (P.op == "CPY" && P.src[0] >= 0 && g.tensors[P.src[0]].ty == TLB_TYPE_F16 && P.is_contiguous() && g.tensors[P.src[0]].is_contiguous() &&
+                       aligned(P.src[0]) && g.tensors[x].is_contiguous()) {
+                A.op_params[GEMV_MODE] = RQ_F16;
+                A.src[1] = P.src[0];
+                dead[xp] = 1;
+            }
+        }
+        // ---- epilogue: SiLU(gate) * up right behind its two products
+        if (members == 2) {
+            const int32_t gate = g.nodes[i], up = A.src[4];
+            int gp = -1;
+            for (size_t k = last + 1; k < nn && gp < 0; k++) {
+                const Tensor &B = g.tensors[g.nodes[k]];
+                if (B.is_view_op() || dead[k]) continue;
+                if (B.op == "GLU" && B.op_params[0] == 2 && B.src[0] == gate && B.src[1] == up && B.view_src < 0 && B.is_contiguous()) gp = (int)k;
+                break;
+            }
+            if (gp >= 0 && !kept[gate] && !kept[up] && g.tensors[up].ne[0] == A.ne[0]) {
+                bool ok = true;
+                for (int32_t m : {gate, up}) {
+                    live_readers(m, rd);
+                    for (int r : rd) ok = ok && (r == gp || (m == up && r == (int)i));
+                }
+                const int32_t out = g.nodes[gp];
+                for (int k = 0; k < 4; k++) ok = ok && g.tensors[out].ne[k] == A.ne[k];
+                if (ok) {   // the GLU's tensor takes over the node, in the products' place
+                    Tensor &G = g.tensors[out];
+                    G.op = A.op;
+                    for (int k = 0; k < 16; k++) G.op_params[k] = A.op_params[k];
+                    for (int k = 0; k < 10; k++) G.src[k] = A.src[k];
+                    G.src[4] = -1;
+                    G.op_params[GEMV_GLU] = 1;
+                    g.nodes[i] = out;
+                    dead[gp] = 1;
+                }
+            }
+        }
+    }
+    std::vector<int32_t> out;
+    for (size_t i = 0; i < nn; i++)
+        if (!dead[i]) out.push_back(g.nodes[i]);
+    g.nodes.swap(out);
+}
+
 // Consecutive tensor-core mul_mats over the same quantized activations (wq, wk, wv of a layer; gate and up)
 // become one MUL_MAT_GROUP launch: each of wq / wk / wv alone leaves most SMs idle (32 / 8 / 8 row tiles on
 // 148 SMs), and gate + up (2 x 112 tiles) together are enough work for the stream-K schedule, which gives
@@ -1463,6 +1685,7 @@ void fuse_mul_mat_groups(Graph &g) {
     const size_t nn = g.nodes.size();
     std::vector<char> dead(nn, 0);
     auto eligible = [&](const Tensor &t) {
+        if (t.op_params[GEMV_MARK] && (t.op == "MUL_MAT" || t.op == "MUL_MAT_GROUP")) return false;
         if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || t.src[2] < 0) return false;
         const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]], &q = g.tensors[t.src[2]];
         if (!is_qact(q.op) || q.op_params[1] <= 0 || tw.ty != TLB_TYPE_Q4_K) return false;

@@ -1,4 +1,5 @@
-// The Q8_K block quantizer shared by the row-producing kernels (k_fused.cu) and the attention epilogue (k_attn.cu).
+// Row sources and the Q8_K block quantizer shared by the row-producing kernels (k_fused.cu), the few-column mul_mat (k_gemv.cu)
+// and the attention epilogue (k_attn.cu).
 #pragma once
 #include <cuda_fp16.h>
 
@@ -11,6 +12,34 @@ __device__ __forceinline__ int nearest_int_f(float v) {
     return (__float_as_int(t) & 0x007fffff) - 0x00400000;
 }
 
+
+// The f32 value at (column n, element k) before any normalisation: a, a + b, act(a) * b or f16 a.
+__device__ __forceinline__ void rq_load8(const RowQuantArgs &p, int n, int64_t k0, float (&x)[8]) {
+    if (p.mode == RQ_GLU) {
+        const float4 g0 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0), g1 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0 + 4);
+        const float4 u0 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0), u1 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0 + 4);
+        const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+        for (int e = 0; e < 8; e++) x[e] = __fmul_rn(__fdiv_rn(g[e], __fadd_rn(1.0f, expf(-g[e]))), u[e]);   // SiLU(g)*u
+    } else if (p.mode == RQ_F16) {
+        const uint4 h = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p.a) + n * p.lda + k0);
+        const __half2 *h2 = reinterpret_cast<const __half2 *>(&h);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float2 f = __half22float2(h2[e]);
+            x[2 * e] = f.x;
+            x[2 * e + 1] = f.y;
+        }
+    } else {
+        const float4 a0 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0), a1 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0 + 4);
+        x[0] = a0.x; x[1] = a0.y; x[2] = a0.z; x[3] = a0.w; x[4] = a1.x; x[5] = a1.y; x[6] = a1.z; x[7] = a1.w;
+        if (p.b) {   // residual add: x = a + b
+            const float4 b0 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0), b1 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0 + 4);
+            x[0] = __fadd_rn(x[0], b0.x); x[1] = __fadd_rn(x[1], b0.y); x[2] = __fadd_rn(x[2], b0.z); x[3] = __fadd_rn(x[3], b0.w);
+            x[4] = __fadd_rn(x[4], b1.x); x[5] = __fadd_rn(x[5], b1.y); x[6] = __fadd_rn(x[6], b1.z); x[7] = __fadd_rn(x[7], b1.w);
+        }
+    }
+}
 
 // Q8_K quantization of one 256-value block held by a warp (lane l: values l*8 .. l*8+7), its optional f32
 // copy, and its slice of the tensor-core operand blob (quantize_row_q8_K_ref, ggml-quants.c:2768-2805)

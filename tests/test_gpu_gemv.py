@@ -1,0 +1,61 @@
+"""The few-column mul_mat kernels at the edges of their tiles: row groups of 16, row segments of four or eight super-blocks,
+one to eight columns per launch (Q6_K: four), short rows that share a tile, and the nodes folded into a launch."""
+import numpy as np
+import pytest
+
+from helpers import Model, close
+from oracle.bindings import Q4_0, Q4_K, Q6_K, Q8_0
+from tensorlisp_b200 import graph as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ty", [Q4_K, Q8_0, Q4_0, Q6_K])
+@pytest.mark.parametrize("K,M,N", [(256, 1, 1), (256, 2385, 3), (512, 17, 2), (768, 333, 5), (1280, 2369, 1), (2304, 31, 8), (2304, 148 * 16 + 9, 2), (4096, 130, 9), (16384, 40, 4),
+                                   (28672, 65, 7), (1024, 40001, 1)])
+def test_edges(oracle, ty, K, M, N):
+    rng = np.random.default_rng(K + M + N)
+    W = (rng.standard_normal((M, K)) * 0.02).astype(np.float32)
+    X = (rng.standard_normal((N, K)) * np.exp(rng.standard_normal((N, 1)) * 3)).astype(np.float32)
+    X[0, :300] = 0
+    Wq = oracle.quantize(ty, W)
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(ty, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    want = X.astype(np.float64) @ oracle.dequantize(ty, Wq, K).reshape(M, K).astype(np.float64).T if ty == Q6_K else oracle.mul_mat(ty, Wq, K, X)
+    for _ in range(2):   # (the second run finds the first one's stages in shared memory)
+        (got,) = m.run(X)
+        for n in range(N):
+            close(got.reshape(N, M)[n], want.reshape(N, M)[n], 2e-5)
+    m.close()
+
+
+@pytest.mark.parametrize("ty", [Q4_K, Q8_0, Q4_0])
+@pytest.mark.parametrize("d,f,n", [(512, 768, 1), (768, 512, 2), (512, 2560, 3), (2048, 4864, 1), (8448, 256, 2)])
+def test_folded_nodes(oracle, ty, d, f, n):
+    """Residual add, norm, gate and up, SiLU(gate) * up, f16 cast in front of a product: what the launches take in."""
+    rng = np.random.default_rng(d + f + n)
+    mk = lambda k, m: (rng.standard_normal((m, k)) * 0.02).astype(np.float32)
+    ws = [oracle.quantize(ty, mk(k, m)) for k, m in ((d, f), (d, f), (f, d), (d, 96), (d, 40), (d, 24))]
+    wn = (1 + 0.1 * rng.standard_normal(d)).astype(np.float32)
+    g = G.Graph()
+    x, r = g.input(G.F32, [d, n], "x"), g.input(G.F32, [d, n], "r")
+    norm = g.weight(G.F32, [d], "norm")
+    gate, up, down, q, k, v = [g.weight(ty, [a, b], s) for s, a, b in (("gate", d, f), ("up", d, f), ("down", f, d), ("q", d, 96), ("k", d, 40), ("v", d, 24))]
+    h = g.add(x, r, "h")
+    t = g.mul(g.rms_norm(h, 1e-5), norm, "t")
+    y = g.mul_mat(down, g.glu(g.mul_mat(gate, t, "g"), b=g.mul_mat(up, t, "u"), name="a"), "y")
+    o = g.output(g.add(h, y, "o"))
+    c = g.cast(g.cast(o, G.F16), G.F32)
+    outs = [g.output(g.mul_mat(w, c, s)) for w, s in ((q, "yq"), (k, "yk"), (v, "yv"))]
+    m = Model(g, [wn] + ws)
+    X, R = rng.standard_normal((2, n, d)).astype(np.float32)
+    got = m.run(X, R)
+    H = X + R
+    T = oracle.rms_norm(H, 1e-5, wn)
+    O = H + oracle.mul_mat(ty, ws[2], f, oracle.silu_mul(oracle.mul_mat(ty, ws[0], d, T), oracle.mul_mat(ty, ws[1], d, T)))
+    close(got[0].reshape(n, d), O, 1e-3)
+    C = got[0].reshape(n, d).astype(np.float16).astype(np.float32)
+    for y, w in zip(got[1:], ws[3:]):
+        close(y.reshape(n, -1), oracle.mul_mat(ty, w, d, C), 2e-5)
+    m.close()
