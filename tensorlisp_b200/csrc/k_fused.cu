@@ -39,8 +39,7 @@ __global__ void __launch_bounds__(RQ_THREADS) k_row_quant_q8k(RowQuantArgs p) {
         if (p.npad == MM_FOLD_NPAD) {
             if (sb < nblk) {
                 const int64_t kk = (int64_t)sb * 256 + lane * 8;
-                *reinterpret_cast<uint4 *>((uint8_t *)ob + p.blob_off + ((size_t)(n >> 8) * (size_t)(K / 64) + (size_t)(kk >> 6)) * 32768 +
-                                           (size_t)((n & 255) >> 3) * 1024 + (size_t)((kk & 63) >> 3) * 128 + (size_t)(n & 7) * 16) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4 *>((uint8_t *)ob + p.blob_off + mm_fold_at(n, kk, mm_fold_groups(p.N))) = make_uint4(0, 0, 0, 0);
             }
         } else if (p.npad > 0 && sb < nblk) {
             const int ch = n / p.npad, nl = n % p.npad;   // blobs: [chunk of npad columns][block]
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(RQ_THREADS) k_row_quant_q8k(RowQuantArgs p) {
 
 // ---------------------------------------------------------------- the same producers in front of a Q8_0 quantizer (prompt pass)
 // Q8_0 weights against prompt-sized batches read one operand only: f16(code x f16 scale) of the activations' Q8_0
-// quantization, packed in blobs of 256 columns x 64 elements of K (k_mm_q80_f16, k_mmq_tc_q8.cu). This kernel
+// quantization (k_mm_q80_f16, k_mmq_tc_q8.cu). This kernel
 // produces that (and the Q8_0 block itself) from the f32 row source (a, a + b with the sum written back, RMS norm of either, SiLU(g) * u,
 // f16 values), so the normalised / gated f32 row never goes to memory. Quantization follows quantize_row_q8_0_ref
 // (ggml-quants.c): d = amax / 127 over 32 values, codes roundf(x / d), the scale rounded to f16.
@@ -117,9 +116,7 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
     const int sb = blockIdx.y * nwarps + warp;
     const bool live = sb < nblk;
     const int64_t k0 = (int64_t)sb * 256 + lane * 8;
-    // this lane's 16 bytes of the operand: column n of tile n / 256, stage k0 / 64, chunk (k0 % 64) / 8
-    uint8_t *blob = (uint8_t *)p.out + p.blob_off + ((size_t)(n >> 8) * (size_t)(K / 64) + (size_t)(k0 >> 6)) * 32768 +
-                    (size_t)((n & 255) >> 3) * 1024 + (size_t)((k0 & 63) >> 3) * 128 + (size_t)(n & 7) * 16;
+    uint8_t *blob = (uint8_t *)p.out + p.blob_off + mm_fold_at(n, k0, mm_fold_groups(p.N));   // this lane's 16 bytes of the operand
     if (n >= p.N) {   // padding columns of the last tile are zero
         if (live) *reinterpret_cast<uint4 *>(blob) = make_uint4(0, 0, 0, 0);
         return;
@@ -383,10 +380,14 @@ __global__ void __launch_bounds__(XR_THREADS) k_exchange_row_quant_emulated(XrAl
 // (with flagged words a slot holds {value, sequence number} pairs: 8 bytes per element)
 bool exchange_row_quant_supported(int64_t K, int64_t N) { return K % 256 == 0 && K / 256 <= XR_THREADS / 32 && N >= 1 && N <= AR_CTAS && N * K * 8 <= (int64_t)AR_SLOT_BYTES; }
 
-static int xr_rows(const RowQuantArgs &p) { return p.npad > 0 ? (int)((p.N + p.npad - 1) / p.npad) * p.npad : (int)p.N; }
+// rows including the zero columns that fill the operand up
+static int rq_rows(const RowQuantArgs &p) {
+    const int pad = p.npad == MM_FOLD_NPAD ? 16 : p.npad;
+    return pad > 0 ? (int)((p.N + pad - 1) / pad) * pad : (int)p.N;
+}
 
 cudaError_t launch_exchange_row_quant(const ArRank &a, const RowQuantArgs &p, int n_ranks, cudaStream_t st) {
-    return launch_pdl(k_exchange_row_quant, dim3((unsigned)xr_rows(p)), dim3(XR_THREADS), 0, st, a, p, n_ranks);
+    return launch_pdl(k_exchange_row_quant, dim3((unsigned)rq_rows(p)), dim3(XR_THREADS), 0, st, a, p, n_ranks);
 }
 
 // n_ranks <= 4 emulated ranks, one cooperative launch
@@ -398,7 +399,7 @@ cudaError_t launch_exchange_row_quant_emulated(const ArRank *a, const RowQuantAr
         all.p[r] = p[r];
     }
     void *args[] = {&all, &n_ranks};
-    return cudaLaunchCooperativeKernel((void *)k_exchange_row_quant_emulated, dim3(xr_rows(p[0]), n_ranks), dim3(XR_THREADS), args, 0, st);
+    return cudaLaunchCooperativeKernel((void *)k_exchange_row_quant_emulated, dim3(rq_rows(p[0]), n_ranks), dim3(XR_THREADS), args, 0, st);
 }
 
 bool row_quant_supported(int64_t K) { return K % 256 == 0 && K / 256 <= 65535 * RQ_WARPS; }
@@ -407,13 +408,12 @@ cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st) {
     if (p.N == 0 || p.K == 0) return cudaSuccess;
     if (p.q80) {
         if ((p.npad != 256 && p.npad != 0) || !row_quant_q80_supported(p.K, p.mode)) return cudaErrorInvalidValue;
-        const int rows256 = p.npad ? (int)((p.N + 255) / 256) * 256 : (int)p.N, nb = (int)(p.K / 256);
-        if (p.mode == RQ_NORM) return launch_pdl(k_row_quant_q80, dim3(rows256, 1), dim3(nb * 32), 0, st, p);
-        return launch_pdl(k_row_quant_q80, dim3(rows256, (nb + 7) / 8), dim3(256), 0, st, p);
+        const int nb = (int)(p.K / 256);
+        if (p.mode == RQ_NORM) return launch_pdl(k_row_quant_q80, dim3(rq_rows(p), 1), dim3(nb * 32), 0, st, p);
+        return launch_pdl(k_row_quant_q80, dim3(rq_rows(p), (nb + 7) / 8), dim3(256), 0, st, p);
     }
-    const int rows = p.npad > 0 ? (int)((p.N + p.npad - 1) / p.npad) * p.npad : (int)p.N;   // padding columns of the last chunk too
     const int nblk = (int)(p.K / 256);
-    return launch_pdl(k_row_quant_q8k, dim3(rows, (nblk + RQ_WARPS - 1) / RQ_WARPS), dim3(RQ_THREADS), 0, st, p);
+    return launch_pdl(k_row_quant_q8k, dim3(rq_rows(p), (nblk + RQ_WARPS - 1) / RQ_WARPS), dim3(RQ_THREADS), 0, st, p);
 }
 
 }  // namespace tlb

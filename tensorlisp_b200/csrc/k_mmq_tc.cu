@@ -606,9 +606,9 @@ TcPlan mmq_tc_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
         t.n_split = 1;
         t.sb_per_split = t.nsb;
         t.streamk = 0;
-        t.n_col_chunks = (int)((N + t.npad - 1) / t.npad);
-        t.blob_unit = mm_fold_blob_unit();
-        t.blob_bytes = (uint64_t)t.n_col_chunks * t.nsb * t.blob_unit;
+        t.n_col_chunks = 1;
+        t.blob_unit = 0;
+        t.blob_bytes = mm_fold_bytes(K, N);
         t.partial_bytes = 0;
         return t;
     }
@@ -744,8 +744,7 @@ cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsi
 cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs,
                                 float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool leave_partial) {
     if (t.npad == MM_FOLD_NPAD) {
-        if (n_mats != 1) return cudaErrorInvalidValue;
-        return launch_mm_fold_f16(true, W[0], K, M[0], N, blobs, y[0], ldy, err, st);
+        return launch_mm_fold_f16(true, n_mats, W, K, M, N, blobs, y, ldy, err, st);
     }
     if (n_mats < 1 || n_mats > TC_MAX_MATS || (n_mats > 1 && t.n_col_chunks != 1)) return cudaErrorInvalidValue;
     if (t.n_split > 16) return cudaErrorInvalidValue;

@@ -591,12 +591,19 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // Each product carries two f16 roundings (2^-12 relative each, independent across k), so y differs from the reference's
 // integer arithmetic by about 1e-4 of max|y| at K = 4096: inside the 1e-3 bar of mul_mat, not bit-comparable. The exact
 // kernel above stays reachable (TLB_PROMPT_EXACT=1).
-// A persistent CTA walks (row tile, column tile) pairs, 128 weight rows x 256 activation columns each. Per 256 elements
+// A persistent CTA walks (row tile, column tile) pairs, 128 weight rows x up to 256 activation columns each. Per 256 elements
 // of K: TMA brings 128 x 272 raw bytes; eight warps strip the scales, turn the codes into scaled f16 and store them into
-// tensor memory (A operand, 128 columns); the packed B arrives as four 32 KB bulk copies (64 elements of K each, core
-// matrix layout); one warp issues 16 MMAs of 128 x 256 x 16. Eight warps drain the 128 x 256 accumulator once per tile.
+// tensor memory (A operand, 128 columns); the packed B arrives as four bulk copies (64 elements of K each, core
+// matrix layout, 32 KB for 256 columns); one warp issues 16 MMAs of 128 x columns x 16. Eight warps drain the accumulator
+// once per tile; tiles of at most 128 columns have two, so that the next tile's MMAs do not wait for that.
+//
+// What bounds it: the way of B into shared memory, or below about 110 columns the expansion of the weights. So the tile's width is
+// chosen for the number of columns and row tiles at hand (fold_cols): 333 columns as 2 x 256 wasted a third of the MMAs,
+// and 8 row tiles x 2 left 132 SMs idle. Matrices that share the activations are one launch. Measured for 333 columns, Q4_K:
+// [14336 x 4096] 67 -> 56 us, [4096 x 14336] 100 -> 56, [4096 x 4096] 34 -> 16, [1024 x 4096] 33 -> 9.
 namespace tc8f {
-constexpr int NW = 256;                                  // activation columns per tile
+constexpr int NW = MM_FOLD_NPAD;                         // widest column tile
+constexpr int MAX_MATS = 3;
 constexpr int KS = 64;                                   // elements of K per B stage
 constexpr int B_STAGE = NW * KS * 2;                     // 32 KB
 constexpr int B_STAGES = 4, RAW_STAGES = 2, A_RING = 2;
@@ -625,20 +632,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 }
 }  // namespace tc8f
 
-// B operand of the kernel below: blobs [chunk of 256 columns][stage of 64 elements of K] x 32 KB, each
-// [column / 8][8 chunks of 8 elements][column % 8][16 bytes] (K-major core matrices: lbo 128, sbo 1024), values
-// f16(d_a * q8) in the order of K.
+// B operand of the kernel below from an ActLayout block: mm_fold_at, values f16(d_a * q8) in the order of K.
 // `blk`: elements per activation scale (32 for Q8_0 activations, 256 for the Q8_K activations of Q4_K weights).
 __global__ void __launch_bounds__(256) k_act_pack_q80_f16(const int8_t *__restrict__ qs, const float *__restrict__ ds, int64_t K, int N, int blk,
                                                            uint8_t *__restrict__ out) {
     const int st = blockIdx.x;   // stage of 64 elements
-    uint8_t *o = out + ((size_t)blockIdx.y * gridDim.x + st) * tc8f::B_STAGE;
-    const int n0 = (int)blockIdx.y * tc8f::NW;
-    for (int u = threadIdx.x; u < tc8f::NW * 8; u += blockDim.x) {
-        const int nl = u / 8, kc = u % 8, n = n0 + nl;
+    const int groups = mm_fold_groups(N);
+    const int u_end = min(groups * 8, (int)(blockIdx.y + 1) * tc8f::NW) * 8;
+    for (int u = (int)blockIdx.y * tc8f::NW * 8 + threadIdx.x; u < u_end; u += blockDim.x) {
+        const int n = u / 8;
+        const int64_t k0 = (int64_t)st * tc8f::KS + u % 8 * 8;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (n < N) {
-            const int64_t k0 = (int64_t)st * tc8f::KS + kc * 8;
             const uint2 q = *reinterpret_cast<const uint2 *>(qs + (size_t)n * K + k0);
             const float d = ds[(size_t)n * (K / blk) + k0 / blk];
             const uint32_t w[2] = {q.x, q.y};
@@ -653,27 +658,58 @@ __global__ void __launch_bounds__(256) k_act_pack_q80_f16(const int8_t *__restri
             }
             v = make_uint4(h[0], h[1], h[2], h[3]);
         }
-        *reinterpret_cast<uint4 *>(o + (size_t)(nl / 8) * 1024 + kc * 128 + (nl % 8) * 16) = v;
+        *reinterpret_cast<uint4 *>(out + mm_fold_at(n, k0, groups)) = v;
     }
 }
 
-struct Tc8fParams {
-    const uint8_t *act;   // packed B blobs
-    float *out;
-    int64_t M, ldy;
-    int N, nst, row_tiles, col_tiles;
-    int *err;
+struct Tc8fMaps {
+    CUtensorMap m[tc8f::MAX_MATS];
 };
+struct Tc8fParams {
+    const uint8_t *act;   // packed B operand
+    float *out[tc8f::MAX_MATS];
+    int64_t M[tc8f::MAX_MATS], ldy[tc8f::MAX_MATS];
+    int tile0[tc8f::MAX_MATS];   // first row tile of each matrix (past the end: not there)
+    int N, nst, row_tiles, col_tiles, nw, groups;   // nw: columns of a tile
+    int *err;
+    // Tile t: column tiles in bands of eight, the eight of a row tile one after the other. A band's share of B stays in L2 and the
+    // weights come past it once per band (gate and up of a layer, 125 MB in Q8_0, do not fit into L2 beside it).
+    __device__ __forceinline__ void at(int t, int &row_tile, int &col_tile) const {
+        const int per = row_tiles * 8, band = t / per, in = t - band * per, width = min(8, col_tiles - band * 8);
+        row_tile = in / width;
+        col_tile = band * 8 + in - row_tile * width;
+    }
+    __device__ __forceinline__ int mat_of(int row_tile) const { return row_tile >= tile0[2] ? 2 : (row_tile >= tile0[1] ? 1 : 0); }
+};
+// two weights: q * a - b in f32 (one rounding), then f16; q as the f16 1024 + q
+__device__ __forceinline__ uint32_t fold_pair(uint32_t q, uint64_t a, uint64_t nb) {
+    uint32_t r;
+    asm("{\n\t.reg .b16 l, h;\n\t.reg .f32 x, y;\n\t.reg .b64 p;\n\t"
+        "mov.b32 {l, h}, %1;\n\t"
+        "add.rn.f32.f16 x, l, 0fC4800000;\n\t"
+        "add.rn.f32.f16 y, h, 0fC4800000;\n\t"
+        "mov.b64 p, {x, y};\n\t"
+        "fma.rn.f32x2 p, p, %2, %3;\n\t"
+        "mov.b64 {x, y}, p;\n\t"
+        "cvt.rn.f16x2.f32 %0, y, x;\n\t}"
+        : "=r"(r) : "r"(q), "l"(a), "l"(nb));
+    return r;
+}
+__device__ __forceinline__ uint64_t twice(float x) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
 
 // WQ4K = false: Q8_0 weights (raw rows of 8 x 34 bytes per unit); true: Q4_K weights (one 144-byte super-block per unit:
 // f16 d, dmin, twelve bytes of 6-bit scales and mins, 128 bytes of nibbles), expanded to f16(d * sc * q - dmin * m), the f32
 // value that ggml's dequantizer produces (dequantize_row_q4_K, ggml-quants.c) rounded once.
 template <bool WQ4K>
-__global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ CUtensorMap wmap, Tc8fParams p) {
+__global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
     using namespace tc;
     using namespace tc8f;
     constexpr int ROWS = tc8::ROWS;
-    constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(tc8f::NW >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B
+    const uint32_t IDESC = (1u << 4) | ((uint32_t)(p.nw >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
     constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
@@ -681,7 +717,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     uint8_t *bst = smem;                                   // tc8f::B_STAGES x tc8f::B_STAGE
     uint8_t *raw = bst + tc8f::B_STAGES * tc8f::B_STAGE;               // tc8f::RAW_STAGES x RAW_BYTES
     __shared__ uint64_t bar_raw[tc8f::RAW_STAGES], bar_rawfree[tc8f::RAW_STAGES], bar_b[tc8f::B_STAGES], bar_bfree[tc8f::B_STAGES];
-    __shared__ uint64_t bar_aready[tc8f::A_RING], bar_afree[tc8f::A_RING], bar_accfull, bar_accfree;
+    __shared__ uint64_t bar_aready[tc8f::A_RING], bar_afree[tc8f::A_RING], bar_accfull[2], bar_accfree[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_fail;
     volatile int *fail = &s_fail;
@@ -689,6 +725,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nst = p.nst;   // units of 256 elements of K
     const int n_tiles = p.row_tiles * p.col_tiles;
+    const uint32_t accs = p.nw <= 128 ? 2 : 1;   // accumulators, 128 columns apart
     if (tid == 0) {
         for (int i = 0; i < tc8f::RAW_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
@@ -702,8 +739,10 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             mbar_init(&bar_aready[i], tc8f::DEQ_WARPS);
             mbar_init(&bar_afree[i], 1);
         }
-        mbar_init(&bar_accfull, 1);
-        mbar_init(&bar_accfree, tc8f::EPI_WARPS);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bar_accfull[i], 1);
+            mbar_init(&bar_accfree[i], tc8f::EPI_WARPS);
+        }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -719,28 +758,35 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         if (lane == 0) {
             uint32_t g = 0;
             for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-                const int row_tile = t % p.row_tiles;
+                int row_tile, col_tile;
+                p.at(t, row_tile, col_tile);
+                const int mat = p.mat_of(row_tile);
+                const CUtensorMap *wmap = mat == 0 ? &maps.m[0] : (mat == 1 ? &maps.m[1] : &maps.m[2]);
+                const int row0 = (row_tile - p.tile0[mat]) * ROWS;
                 for (int i = 0; i < nst; i++, g++) {
                     const int s = g % tc8f::RAW_STAGES;
                     if (g >= tc8f::RAW_STAGES) mbar_wait_nap(&bar_rawfree[s], ((g / tc8f::RAW_STAGES) - 1) & 1, fail, 64);
                     mbar_expect_tx(&bar_raw[s], RAW_BYTES);
-                    tma_2d(raw + s * RAW_BYTES, &wmap, i * (ROW_CHUNK / 2), row_tile * ROWS, &bar_raw[s]);   // x in 16-bit elements
+                    tma_2d(raw + s * RAW_BYTES, wmap, i * (ROW_CHUNK / 2), row0, &bar_raw[s]);   // x in 16-bit elements
                 }
             }
         }
     } else if (warp == tc8f::TMA_B_WARP) {
-        // ---- packed activations: four 32 KB stages per unit
+        // ---- packed activations: four stages per unit (of the last column tile only what there is: columns do not mix)
         if (lane == 0) {
             griddep_wait();
             uint32_t g = 0;
             for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-                const int col_tile = t / p.row_tiles;
-                const uint8_t *src = p.act + (size_t)col_tile * nst * 4 * tc8f::B_STAGE;
+                int row_tile, col_tile;
+                p.at(t, row_tile, col_tile);
+                const int g0 = col_tile * (p.nw / 8);
+                const uint32_t bytes = (uint32_t)min(p.nw / 8, p.groups - g0) * 1024u;
+                const uint8_t *src = p.act + (size_t)g0 * 1024;
                 for (int i = 0; i < nst * 4; i++, g++) {
                     const int s = g % tc8f::B_STAGES;
                     if (g >= tc8f::B_STAGES) mbar_wait_nap(&bar_bfree[s], ((g / tc8f::B_STAGES) - 1) & 1, fail, 32);
-                    mbar_expect_tx(&bar_b[s], tc8f::B_STAGE);
-                    bulk_g2s(bst + s * tc8f::B_STAGE, src + (size_t)i * tc8f::B_STAGE, tc8f::B_STAGE, &bar_b[s]);
+                    mbar_expect_tx(&bar_b[s], bytes);
+                    bulk_g2s(bst + s * tc8f::B_STAGE, src + (size_t)i * p.groups * 1024, bytes, &bar_b[s]);
                 }
             }
         }
@@ -749,8 +795,9 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         const bool leader = elect_one();
         uint32_t g = 0, gb = 0, it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
-            if (it > 0) {
-                mbar_wait_nap(&bar_accfree, (it - 1) & 1, fail, 32);   // the accumulator of the tile before has been drained
+            const uint32_t ai = it % accs, acc = tmem_base + tc8f::ACC_COL0 + ai * 128u;
+            if (it >= accs) {
+                mbar_wait_nap(&bar_accfree[ai], (it / accs - 1) & 1, fail, 32);   // the tile before in this accumulator has been drained
                 tc_fence_after();
             }
             for (int i = 0; i < nst; i++, g++) {
@@ -767,12 +814,12 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                         const uint64_t b_desc0 = smem_desc(su32(bst + bs * tc8f::B_STAGE), 128, 1024);
 #pragma unroll
                         for (int k = 0; k < 4; k++)
-                            umma_f16_ta(tmem_base + tc8f::ACC_COL0, a0 + (uint32_t)((s4 * 4 + k) * 8), b_desc0 + (uint64_t)(k * 16), IDESC,
+                            umma_f16_ta(acc, a0 + (uint32_t)((s4 * 4 + k) * 8), b_desc0 + (uint64_t)(k * 16), IDESC,
                                         (i | s4 | k) ? 1u : 0u);
                         umma_commit(&bar_bfree[bs]);
                         if (s4 == 3) {
                             umma_commit(&bar_afree[slot]);
-                            if (i == nst - 1) umma_commit(&bar_accfull);
+                            if (i == nst - 1) umma_commit(&bar_accfull[ai]);
                         }
                     }
                     __syncwarp();
@@ -817,8 +864,8 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                         int sc0, mn0, sc1, mn1;
                         scale_min(2 * j, sc0, mn0);
                         scale_min(2 * j + 1, sc1, mn1);
-                        const float a0 = __fmul_rn(d, (float)sc0), b0 = __fmul_rn(dmin, (float)mn0);
-                        const float a1 = __fmul_rn(d, (float)sc1), b1 = __fmul_rn(dmin, (float)mn1);
+                        const uint64_t a0 = twice(__fmul_rn(d, (float)sc0)), b0 = twice(-__fmul_rn(dmin, (float)mn0));
+                        const uint64_t a1 = twice(__fmul_rn(d, (float)sc1)), b1 = twice(-__fmul_rn(dmin, (float)mn1));
                         uint32_t lo[16], hi[16];
 #pragma unroll
                         for (int u = 0; u < 2; u++) {
@@ -827,18 +874,11 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
 #pragma unroll
                             for (int wi = 0; wi < 4; wi++) {
                                 const uint32_t w = w4[wi];
-                                float fl[4], fh[4];
-#pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    fl[e] = __fsub_rn(__fmul_rn(a0, (float)((w >> (8 * e)) & 0xF)), b0);
-                                    fh[e] = __fsub_rn(__fmul_rn(a1, (float)((w >> (8 * e + 4)) & 0xF)), b1);
-                                }
-                                const __half2 l0 = __floats2half2_rn(fl[0], fl[1]), l1 = __floats2half2_rn(fl[2], fl[3]);
-                                const __half2 h0 = __floats2half2_rn(fh[0], fh[1]), h1 = __floats2half2_rn(fh[2], fh[3]);
-                                lo[(u * 4 + wi) * 2] = *reinterpret_cast<const uint32_t *>(&l0);
-                                lo[(u * 4 + wi) * 2 + 1] = *reinterpret_cast<const uint32_t *>(&l1);
-                                hi[(u * 4 + wi) * 2] = *reinterpret_cast<const uint32_t *>(&h0);
-                                hi[(u * 4 + wi) * 2 + 1] = *reinterpret_cast<const uint32_t *>(&h1);
+                                const uint32_t x = w & 0x0f0f0f0fu, y = (w >> 4) & 0x0f0f0f0fu;
+                                lo[(u * 4 + wi) * 2] = fold_pair(__byte_perm(x, 0x64646464u, 0x4140), a0, b0);
+                                lo[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(x, 0x64646464u, 0x4342), a0, b0);
+                                hi[(u * 4 + wi) * 2] = fold_pair(__byte_perm(y, 0x64646464u, 0x4140), a1, b1);
+                                hi[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(y, 0x64646464u, 0x4342), a1, b1);
                             }
                         }
                         tmem_st16(a_lane + (uint32_t)(slot * 128 + j * 32), lo);
@@ -880,32 +920,40 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             }
         }
     } else if (warp >= tc8f::EPI_WARP0) {
-        // ---- draining warps: lane quadrant warp % 4, column half (warp - tc8f::EPI_WARP0) / 4; once per tile
+        // ---- draining warps: lane quadrant warp % 4, every other 32 columns from (warp - tc8f::EPI_WARP0) / 4 on; once per tile
         const int q = warp & 3, ch = (warp - tc8f::EPI_WARP0) >> 2;
-        const int row_in_tile = q * 32 + lane;
-        const uint32_t lane_addr = tmem_base + tc8f::ACC_COL0 + ((uint32_t)(q * 32) << 16) + (uint32_t)(ch * 128);
+        const int row_in_tile = q * 32 + lane, chunks = (p.nw + 31) / 32;
         uint32_t it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
-            const int row_tile = t % p.row_tiles, col_tile = t / p.row_tiles;
-            mbar_wait_nap(&bar_accfull, it & 1, fail, 128);
+            int row_tile, col_tile;
+            p.at(t, row_tile, col_tile);
+            const int col0 = col_tile * p.nw, mat = p.mat_of(row_tile);
+            const uint32_t ai = it % accs;
+            const uint32_t lane_addr = tmem_base + tc8f::ACC_COL0 + ai * 128u + ((uint32_t)(q * 32) << 16);
+            mbar_wait_nap(&bar_accfull[ai], (it / accs) & 1, fail, 128);
             tc_fence_after();
-            const int64_t row = (int64_t)row_tile * ROWS + row_in_tile;
-            const int col0 = col_tile * tc8f::NW + ch * 128;
-            float *o = p.out + (size_t)col0 * p.ldy + row;
+            const int64_t row = (int64_t)(row_tile - p.tile0[mat]) * ROWS + row_in_tile, M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]);
+            const int64_t ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
+            float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + (size_t)col0 * ldy + row;
+            if (ch >= chunks) {
+                if (lane == 0) mbar_arrive(&bar_accfree[ai]);
+                continue;
+            }
+            const int cols = min(p.nw, p.N - col0);
 #pragma unroll 1
-            for (int c = 0; c < 4; c++) {
+            for (int c = ch; c < chunks; c += 2) {
                 uint32_t v[32];
-                tmem_ld32(lane_addr + (uint32_t)(c * 32), v);
+                tmem_ld32(lane_addr + (uint32_t)(c * 32), v);   // (past the tile's last column: other columns of the same 512, not used)
                 tmem_ld_wait();
-                if (c == 3) {   // everything of this warp's part is in registers: the accumulator may be overwritten
+                if (c + 2 >= chunks) {   // everything of this warp's part is in registers: the accumulator may be overwritten
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_accfree);
+                    if (lane == 0) mbar_arrive(&bar_accfree[ai]);
                 }
-                if (row < p.M) {
+                if (row < M) {
 #pragma unroll
                     for (int j = 0; j < 32; j++)
-                        if (col0 + c * 32 + j < p.N) o[(size_t)(c * 32 + j) * p.ldy] = __uint_as_float(v[j]);
+                        if (c * 32 + j < cols) o[(size_t)(c * 32 + j) * ldy] = __uint_as_float(v[j]);
                 }
             }
         }
@@ -919,34 +967,59 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
 static size_t tc8f_smem() { return (size_t)tc8f::B_STAGES * tc8f::B_STAGE + (size_t)tc8f::RAW_STAGES * tc8::RAW_BYTES + 1024; }   // the larger raw stage (Q8_0)
 
 // The folded-scale GEMM for either weight format (the Q4_K planner and launcher in k_mmq_tc.cu call it for more than 64 columns)
-uint64_t mm_fold_blob_unit() { return (uint64_t)4 * tc8f::B_STAGE; }
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
-cudaError_t launch_mm_fold_f16(bool q4k, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y, int64_t ldy, int *err,
-                               cudaStream_t st) {
-    CUtensorMap map;
-    cudaError_t e = q4k ? tc_encode_2d(&map, W, (uint64_t)(K / 256 * 144), (uint64_t)M, 144, tc8::ROWS, 2)
-                        : tc_encode_2d(&map, W, (uint64_t)(K / 32 * 34), (uint64_t)M, tc8::ROW_CHUNK, tc8::ROWS, 2);
-    if (e != cudaSuccess) return e;
+// Columns of a tile, a multiple of 16: of the even splits of N into tiles of at most 256 columns, the one whose slowest SM has the
+// least to do. A unit of K was measured at 1.3 us up to 100 columns (the expansion of its weights), 1.47 at 128, 1.86 at 192 and 2.15
+// at 256; draining a wide tile, which has no second accumulator, at about 1 us.
+static int fold_cols(int64_t N, int row_tiles, int nst, int sms) {
+    double best = 0;
+    int cols = 0;
+    for (int64_t ct = (N + tc8f::NW - 1) / tc8f::NW, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
+        const int nw = (int)(((N + ct - 1) / ct + 15) / 16 * 16);
+        const int64_t tiles = (int64_t)row_tiles * ((N + nw - 1) / nw), waves = (tiles + sms - 1) / sms;
+        const double t = (double)waves * (nst * std::max(1.3, 0.65 + 0.0059 * nw) + (nw > 128 ? 1.0 : 0.2));
+        if (cols == 0 || t < best * 0.98) {
+            best = t;
+            cols = nw;
+        }
+    }
+    return cols;
+}
+cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
+                               int64_t ldy, int *err, cudaStream_t st) {
+    if (n_mats < 1 || n_mats > tc8f::MAX_MATS) return cudaErrorInvalidValue;
     static int sm_of[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!sm_of[dev]) cudaDeviceGetAttribute(&sm_of[dev], cudaDevAttrMultiProcessorCount, dev);
+    Tc8fMaps maps;
     Tc8fParams p{};
+    for (int j = 0; j < tc8f::MAX_MATS; j++) {
+        if (j >= n_mats) {
+            maps.m[j] = maps.m[0];
+            p.tile0[j] = 1 << 30;
+            continue;
+        }
+        const cudaError_t e = tc_encode_2d(&maps.m[j], W[j], (uint64_t)tlb_row_size(q4k ? TLB_TYPE_Q4_K : TLB_TYPE_Q8_0, K), (uint64_t)M[j], q4k ? 144 : tc8::ROW_CHUNK, tc8::ROWS, 2);
+        if (e != cudaSuccess) return e;
+        p.out[j] = y[j];
+        p.M[j] = M[j];
+        p.ldy[j] = n_mats > 1 ? M[j] : ldy;
+        p.tile0[j] = p.row_tiles;
+        p.row_tiles += (int)((M[j] + tc8::ROWS - 1) / tc8::ROWS);
+    }
     p.act = (const uint8_t *)blobs;
-    p.out = y;
-    p.M = M;
-    p.ldy = ldy;
     p.N = (int)N;
     p.nst = (int)(K / 256);
-    p.row_tiles = (int)((M + tc8::ROWS - 1) / tc8::ROWS);
-    p.col_tiles = (int)((N + tc8f::NW - 1) / tc8f::NW);
+    p.nw = fold_cols(N, p.row_tiles, p.nst, sm_of[dev]);
+    p.groups = mm_fold_groups(N);
+    p.col_tiles = (int)((N + p.nw - 1) / p.nw);
     p.err = err;
-    const int tiles = p.row_tiles * p.col_tiles;
-    const dim3 grid((unsigned)std::min(tiles, sm_of[dev]));
-    return q4k ? launch_pdl(k_mm_q80_f16<true>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, map, p)
-               : launch_pdl(k_mm_q80_f16<false>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, map, p);
+    const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sm_of[dev]));
+    return q4k ? launch_pdl(k_mm_q80_f16<true>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, maps, p)
+               : launch_pdl(k_mm_q80_f16<false>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, maps, p);
 }
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st) {
     const char *ab = (const char *)act;
@@ -986,9 +1059,9 @@ TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
         t.n_split = 1;
         t.sb_per_split = t.nsb;
         t.streamk = 0;
-        t.n_col_chunks = (int)((N + t.npad - 1) / t.npad);
-        t.blob_unit = (uint64_t)4 * tc8f::B_STAGE;   // one unit of 256 elements of K = four stages of 64
-        t.blob_bytes = (uint64_t)t.n_col_chunks * t.nsb * t.blob_unit;
+        t.n_col_chunks = 1;
+        t.blob_unit = 0;
+        t.blob_bytes = mm_fold_bytes(K, N);
         t.partial_bytes = 0;
         return t;
     }
@@ -1051,7 +1124,7 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
     // described in 16-bit elements: a 272-byte box is 136 of them (the limit is 256 elements per dimension)
     cudaError_t e = tc_encode_2d(&map, W, (uint64_t)(K / 32 * 34), (uint64_t)M, tc8::ROW_CHUNK, tc8::ROWS, 2);
     if (e != cudaSuccess) return e;
-    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, W, K, M, N, blobs, y, ldy, err, st);
+    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, err, st);
     if (t.npad == tc8w::NW) {
         Tc8Params p{};
         p.act = (const uint8_t *)blobs;

@@ -72,11 +72,17 @@ cudaError_t launch_act_pack_tc8(const ActLayout &a, const void *act, int npad, v
 cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
                            int64_t ldy, void *partial, int *err, cudaStream_t st);
 void mmq_tc8_configure();
-// the folded-scale prompt GEMM (k_mm_q80_f16) for Q8_0 or Q4_K weights: blobs of 256 columns x 64 elements, f16(code x scale)
-constexpr int MM_FOLD_NPAD = 256;
-uint64_t mm_fold_blob_unit();   // bytes of the blobs of one 256-element unit of K (four stages)
-cudaError_t launch_mm_fold_f16(bool q4k, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y, int64_t ldy, int *err,
-                               cudaStream_t st);
+// the folded-scale prompt GEMM (k_mm_q80_f16) for Q8_0 or Q4_K weights; its activation operand is f16(code x scale), laid out by
+// stages of 64 elements of K, in a stage by groups of eight columns of 1 KB each (any run of groups is a column tile)
+constexpr int MM_FOLD_NPAD = 256;   // marks the operand in the plans (and is the widest column tile)
+inline __host__ __device__ int mm_fold_groups(int64_t N) { return (int)((N + 15) / 16) * 2; }   // the matrix instruction takes 16 columns at a time
+inline __host__ __device__ size_t mm_fold_at(int n, int64_t k, int groups) {   // bytes; k a multiple of 8
+    return ((size_t)(k >> 6) * groups + (n >> 3)) * 1024 + (size_t)((k & 63) >> 3) * 128 + (size_t)(n & 7) * 16;
+}
+inline uint64_t mm_fold_bytes(int64_t K, int64_t N) { return (uint64_t)(K / 64) * mm_fold_groups(N) * 1024; }
+// n_mats matrices of one type that share the activations (y[j]: [column][M[j]]; of a single one [column][ldy])
+cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
+                               int64_t ldy, int *err, cudaStream_t st);
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_mm_plain.cu

@@ -533,7 +533,7 @@ void lower_gemv(L &l) {
     });
 }
 
-// MUL_MAT_GROUP (pseudo-op made by fuse_mul_mat_groups): up to three Q4_K mul_mats over the same
+// MUL_MAT_GROUP (pseudo-op made by fuse_mul_mat_groups): up to three mul_mats of one weight type over the same
 // activations (wq / wk / wv) in one tensor-core launch. src = w0, x, quantized x, w1, y1, w2, y2; the
 // node's own tensor is y0.
 void lower_mul_mat_group(L &l) {
@@ -541,6 +541,7 @@ void lower_mul_mat_group(L &l) {
     const int32_t x = l.src(1), qa = l.src(2);
     const Tensor &tx = l.T(x);
     const int64_t K = tx.ne[0], N = tx.ne[1];
+    const uint32_t wty = l.T(l.src(0)).ty;
     int n_mats = 0;
     Place pw[3], py[3];
     int64_t Ms[3] = {0, 0, 0}, Msum = 0;
@@ -549,7 +550,7 @@ void lower_mul_mat_group(L &l) {
         if (t.src[wslot[j]] < 0) break;
         const int32_t w = t.src[wslot[j]], y = j == 0 ? l.id : l.src(yslot[j]);
         const Tensor &tw = l.T(w), &ty = l.T(y);
-        if (tw.ty != TLB_TYPE_Q4_K || tw.ne[0] != K || tw.nb[1] != tw.row_size() || ty.ty != TLB_TYPE_F32 || !ty.is_contiguous() ||
+        if (tw.ty != wty || tw.ne[0] != K || tw.nb[1] != tw.row_size() || ty.ty != TLB_TYPE_F32 || !ty.is_contiguous() ||
             ty.ne[0] != tw.ne[1] || ty.ne[1] != N)
             throw std::string("a grouped mul_mat lost its shape invariants");
         pw[j] = l.place(w);
@@ -559,9 +560,9 @@ void lower_mul_mat_group(L &l) {
         n_mats++;
     }
     const int sm = l.c.dev->prop.multiProcessorCount;
-    const TcPlan tp = mmq_tc_plan(K, Msum, N, sm);
+    const TcPlan tp = tc_plan(wty, K, Msum, N, sm);
     if (tp.npad != l.T(qa).op_params[1] || tp.n_col_chunks != 1) throw std::string("activation blobs were packed for another column count");
-    const ActLayout a = act_layout(ACT_Q8_K, K, tx.nrows());
+    const ActLayout a = act_layout(act_kind_for(wty), K, tx.nrows());
     const int64_t sc = l.c.layout->scratch[l.pos];
     if (tp.partial_bytes > 0 && sc < 0) throw std::string("split-K scratch was not planned");
     Place ps;
@@ -576,6 +577,7 @@ void lower_mul_mat_group(L &l) {
             W[j] = r.at(pw[j]);
             Y[j] = (float *)r.at(py[j]);
         }
+        if (wty == TLB_TYPE_Q8_0) return launch_mm_fold_f16(false, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.err, r.stream);
         return launch_mmq_tc_group(tp, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.at(ps), r.err, r.stream);
     });
 }
@@ -1688,10 +1690,11 @@ void fuse_mul_mat_groups(Graph &g) {
         if (t.op_params[GEMV_MARK] && (t.op == "MUL_MAT" || t.op == "MUL_MAT_GROUP")) return false;
         if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || t.src[2] < 0) return false;
         const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]], &q = g.tensors[t.src[2]];
-        if (!is_qact(q.op) || q.op_params[1] <= 0 || tw.ty != TLB_TYPE_Q4_K) return false;
+        if (!is_qact(q.op) || q.op_params[1] <= 0) return false;
         if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1 || tw.nb[1] != tw.row_size() || !t.is_contiguous() || t.view_src >= 0) return false;
-        if (tx.ne[1] > 64 || !mmq_tc_supported(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1]) || getenv("TLB_NO_TC") || getenv("TLB_MM_GENERIC")) return false;
-        return true;
+        if (!tc_supported(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1]) || getenv("TLB_NO_TC") || getenv("TLB_MM_GENERIC")) return false;
+        // up to 64 columns the Q4_K kernel takes groups; above, the folded-scale kernel of either type
+        return q.op_params[1] == MM_FOLD_NPAD || (tw.ty == TLB_TYPE_Q4_K && tx.ne[1] <= 64);
     };
     for (size_t i = 0; i < nn; i++) {
         if (dead[i]) continue;
@@ -1702,10 +1705,10 @@ void fuse_mul_mat_groups(Graph &g) {
         const int wslot[3] = {0, 3, 5}, yslot[3] = {-1, 4, 6};
         for (size_t j = i + 1; j < nn && members < 3; j++) {
             const Tensor &B = g.tensors[g.nodes[j]];
-            if (!eligible(B) || B.src[1] != A.src[1] || B.src[2] != A.src[2]) break;
+            if (!eligible(B) || B.src[1] != A.src[1] || B.src[2] != A.src[2] || g.tensors[B.src[0]].ty != g.tensors[A.src[0]].ty) break;
             const int64_t tb = (B.ne[0] + 127) / 128;
             // a group stays within one wave of CTAs, or is big enough for the stream-K schedule (gate + up)
-            if (tiles + tb > 148 && !mmq_tc_plan(g.tensors[A.src[1]].ne[0], (tiles + tb) * 128, g.tensors[A.src[1]].ne[1], 148).streamk) break;
+            if (tiles + tb > 148 && g.tensors[A.src[2]].op_params[1] != MM_FOLD_NPAD && !mmq_tc_plan(g.tensors[A.src[1]].ne[0], (tiles + tb) * 128, g.tensors[A.src[1]].ne[1], 148).streamk) break;
             tiles += tb;
             A.src[wslot[members]] = B.src[0];
             A.src[yslot[members]] = g.nodes[j];

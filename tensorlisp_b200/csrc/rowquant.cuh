@@ -87,10 +87,9 @@ __device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int
     if ((lane & 1) == 0) bsums[(size_t)n * (K / 16) + sb * 16 + (lane >> 1)] = (int16_t)s16;
     if (lane == 0) ds[(size_t)n * (K / 256) + sb] = d;
     if (p.npad == MM_FOLD_NPAD) {
-        // operand of the folded-scale prompt GEMM: f16(code x scale), blobs of 256 columns x 64 elements of K, natural order
+        // operand of the folded-scale prompt GEMM: f16(code x scale) in natural order
         const int64_t kk = (int64_t)sb * 256 + lane * 8;
-        uint8_t *o = (uint8_t *)ob + p.blob_off + ((size_t)(n >> 8) * (size_t)(K / 64) + (size_t)(kk >> 6)) * 32768 + (size_t)((n & 255) >> 3) * 1024 +
-                     (size_t)((kk & 63) >> 3) * 128 + (size_t)(n & 7) * 16;
+        uint8_t *o = (uint8_t *)ob + p.blob_off + mm_fold_at(n, kk, mm_fold_groups(p.N));
         uint32_t h[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
