@@ -591,26 +591,27 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // Each product carries two f16 roundings (2^-12 relative each, independent across k), so y differs from the reference's
 // integer arithmetic by about 1e-4 of max|y| at K = 4096: inside the 1e-3 bar of mul_mat, not bit-comparable. The exact
 // kernel above stays reachable (TLB_PROMPT_EXACT=1).
-// A persistent CTA walks (row tile, column tile) pairs, 128 weight rows x up to 256 activation columns each. Per 256 elements
-// of K: TMA brings 128 x 272 raw bytes; eight warps strip the scales, turn the codes into scaled f16 and store them into
-// tensor memory (A operand, 128 columns); the packed B arrives as four bulk copies (64 elements of K each, core
-// matrix layout, 32 KB for 256 columns); one warp issues 16 MMAs of 128 x columns x 16. Eight warps drain the accumulator
-// once per tile; tiles of at most 128 columns have two, so that the next tile's MMAs do not wait for that.
+// A persistent CTA walks (row tile, column tile) pairs, 128 weight rows x up to 256 (or 2 x 192) activation columns each. Per 256
+// elements of K: TMA brings 128 x 272 raw bytes; sixteen warps strip the scales, turn the codes into scaled f16 and store them into
+// tensor memory (A operand, 32 columns per 64 elements of K); the packed B arrives in bulk copies of 64 elements of K (core
+// matrix layout, 32 KB for 256 columns); one thread issues four MMAs of 128 x columns x 16 for each. Eight warps drain the
+// accumulator once per tile; tiles of at most 128 columns have two, so that the next tile's MMAs do not wait for that.
 //
-// What bounds it: the way of B into shared memory, or below about 110 columns the expansion of the weights. So the tile's width is
-// chosen for the number of columns and row tiles at hand (fold_cols): 333 columns as 2 x 256 wasted a third of the MMAs,
+// What bounds it: at 256 columns the tensor pipe with the copies of B (1.55 us per 256 elements of K; 2.15 while a whole warp probed
+// the barriers and issued), at narrow tiles the chain of waits per 64 elements of K (1.2 us). So the tile's width is
+// chosen for the number of columns and row tiles at hand (fold_tile): 333 columns as 2 x 256 wasted a third of the MMAs,
 // and 8 row tiles x 2 left 132 SMs idle. Matrices that share the activations are one launch. Measured for 333 columns, Q4_K:
-// [14336 x 4096] 67 -> 56 us, [4096 x 14336] 100 -> 56, [4096 x 4096] 34 -> 16, [1024 x 4096] 33 -> 9.
+// gate and up (14336 x 4096) 134 -> 75 us, [4096 x 14336] 100 -> 70, [4096 x 4096] 34 -> 23.
 namespace tc8f {
 constexpr int NW = MM_FOLD_NPAD;                         // widest column tile
 constexpr int MAX_MATS = 3;
 constexpr int KS = 64;                                   // elements of K per B stage
-constexpr int B_STAGE = NW * KS * 2;                     // 32 KB
-constexpr int B_STAGES = 4, RAW_STAGES = 2, A_RING = 2;
+constexpr int HALF_NW = 192;                             // and of one of two that share their weights
+constexpr int MAX_STAGES = 8;
+constexpr int SMEM = 226 * 1024;
 constexpr int TMA_RAW_WARP = 0, TMA_B_WARP = 1, MMA_WARP = 2;   // warp 3 idles (keeps the quadrant numbering of the rest aligned)
-constexpr int DEQ_WARP0 = 4, DEQ_WARPS = 8, EPI_WARP0 = 12, EPI_WARPS = 8;
-constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;    // 640
-constexpr uint32_t ACC_COL0 = 0, A_COL0 = 256;           // accumulator [0, 256), A ring 2 x 128 columns behind it
+constexpr int DEQ_WARP0 = 4, DEQ_WARPS = 16, EPI_WARP0 = 20, EPI_WARPS = 8;
+constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;    // 896
 // 4 int8 codes of a word -> two f16x2 of code * scale (exact integer first: (1024 + u) - 1152 with u = code + 128)
 __device__ __forceinline__ void codes_to_f16(uint32_t w, uint32_t dd, uint32_t &lo, uint32_t &hi) {
     const uint32_t x = w ^ 0x80808080u;
@@ -670,7 +671,8 @@ struct Tc8fParams {
     float *out[tc8f::MAX_MATS];
     int64_t M[tc8f::MAX_MATS], ldy[tc8f::MAX_MATS];
     int tile0[tc8f::MAX_MATS];   // first row tile of each matrix (past the end: not there)
-    int N, nst, row_tiles, col_tiles, nw, groups;   // nw: columns of a tile
+    int N, nst, row_tiles, col_tiles, nw, groups;   // nw: columns of a tile or of half of one
+    int raw_stages, b_stages;
     int *err;
     // Tile t: column tiles in bands of eight, the eight of a row tile one after the other. A band's share of B stays in L2 and the
     // weights come past it once per band (gate and up of a layer, 125 MB in Q8_0, do not fit into L2 beside it).
@@ -701,23 +703,105 @@ __device__ __forceinline__ uint64_t twice(float x) {
     return r;
 }
 
-// WQ4K = false: Q8_0 weights (raw rows of 8 x 34 bytes per unit); true: Q4_K weights (one 144-byte super-block per unit:
-// f16 d, dmin, twelve bytes of 6-bit scales and mins, 128 bytes of nibbles), expanded to f16(d * sc * q - dmin * m), the f32
-// value that ggml's dequantizer produces (dequantize_row_q4_K, ggml-quants.c) rounded once.
+// the phase's state now, without waiting: a probe takes 100 to 300 cycles to answer, so the next one's goes out ahead of other work
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(tc::su32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// four MMAs over 64 elements of K: A 8 columns apart in tensor memory, B 16 (x 16 bytes) apart in shared memory; more = 0: the
+// first one starts the sum
+__device__ __forceinline__ void umma4_f16_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+        "add.u64 b1, %2, 16;\n\tadd.u64 b2, %2, 32;\n\tadd.u64 b3, %2, 48;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, q;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more)
+        : "memory");
+}
+
+// 64 weights (group j of a unit of 256) of one row as f16 into 32 tensor-memory columns.
+// Q8_0: two blocks of 34 bytes. Q4_K (one 144-byte super-block: f16 d, dmin, twelve bytes of 6-bit scales and mins, 128 bytes of
+// nibbles): f16(d * sc * q - dmin * m), dequantize_row_q4_K (ggml-quants.c); low nibbles are the first 32 values, high ones the rest.
 template <bool WQ4K>
+__device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t taddr) {
+    if constexpr (WQ4K) {
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(rrow);   // d, dmin, scales[12]
+        // get_scale_min_k4 (ggml-quants.c:880-887), four sub-blocks at a time
+        const uint32_t sc4 = j < 2 ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
+        const uint32_t mn4 = j < 2 ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
+        const int sh = (j & 1) * 16;
+        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu)));
+        const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
+        const uint64_t a0 = twice(__fmul_rn(d, (float)((sc4 >> sh) & 0xff))), b0 = twice(-__fmul_rn(dmin, (float)((mn4 >> sh) & 0xff)));
+        const uint64_t a1 = twice(__fmul_rn(d, (float)((sc4 >> (sh + 8)) & 0xff))), b1 = twice(-__fmul_rn(dmin, (float)((mn4 >> (sh + 8)) & 0xff)));
+        uint32_t lo[16], hi[16];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint4 qv = *reinterpret_cast<const uint4 *>(rrow + 16 + j * 32 + u * 16);
+            const uint32_t w4[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int wi = 0; wi < 4; wi++) {
+                const uint32_t x = w4[wi] & 0x0f0f0f0fu, y = (w4[wi] >> 4) & 0x0f0f0f0fu;
+                lo[(u * 4 + wi) * 2] = fold_pair(__byte_perm(x, 0x64646464u, 0x4140), a0, b0);
+                lo[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(x, 0x64646464u, 0x4342), a0, b0);
+                hi[(u * 4 + wi) * 2] = fold_pair(__byte_perm(y, 0x64646464u, 0x4140), a1, b1);
+                hi[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(y, 0x64646464u, 0x4342), a1, b1);
+            }
+        }
+        tc::tmem_st16(taddr, lo);
+        tc::tmem_st16(taddr + 16, hi);
+    } else {
+        uint32_t qa[8], qb[8], h[16];
+        float da, db;
+        if (j == 0) tc8::split_blocks<0>(rrow, qa, qb, da, db);
+        else if (j == 1) tc8::split_blocks<1>(rrow, qa, qb, da, db);
+        else if (j == 2) tc8::split_blocks<2>(rrow, qa, qb, da, db);
+        else tc8::split_blocks<3>(rrow, qa, qb, da, db);
+        uint32_t dd = (uint32_t)__half_as_ushort(__float2half_rn(da));   // the block's own f16 scale, back from f32 unchanged
+        dd |= dd << 16;
+#pragma unroll
+        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qa[i], dd, h[2 * i], h[2 * i + 1]);
+        tc::tmem_st16(taddr, h);
+        dd = (uint32_t)__half_as_ushort(__float2half_rn(db));
+        dd |= dd << 16;
+#pragma unroll
+        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qb[i], dd, h[2 * i], h[2 * i + 1]);
+        tc::tmem_st16(taddr + 16, h);
+    }
+}
+
+// CT column halves of nw columns per tile, which share the expanded weights. Tensor memory: accumulators [0, 256), or of the halves
+// [0, 192) and [192, 384); behind them eight or four A slots of 64 elements of K.
+template <bool WQ4K, int CT>
 __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
     using namespace tc;
     using namespace tc8f;
     constexpr int ROWS = tc8::ROWS;
+    constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
+    constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
+    constexpr uint32_t ACOLS = CT == 1 ? 256 : 2 * HALF_NW;   // first A column
+    constexpr int A_RING = (512 - (int)ACOLS) / 32;
     const uint32_t IDESC = (1u << 4) | ((uint32_t)(p.nw >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
-    constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
-    constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
-    uint8_t *bst = smem;                                   // tc8f::B_STAGES x tc8f::B_STAGE
-    uint8_t *raw = bst + tc8f::B_STAGES * tc8f::B_STAGE;               // tc8f::RAW_STAGES x RAW_BYTES
-    __shared__ uint64_t bar_raw[tc8f::RAW_STAGES], bar_rawfree[tc8f::RAW_STAGES], bar_b[tc8f::B_STAGES], bar_bfree[tc8f::B_STAGES];
-    __shared__ uint64_t bar_aready[tc8f::A_RING], bar_afree[tc8f::A_RING], bar_accfull[2], bar_accfree[2];
+    const int b_stage = p.nw * KS * 2;
+    uint8_t *bst = smem;                                   // b_stages x b_stage
+    uint8_t *raw = bst + p.b_stages * b_stage;             // raw_stages x RAW_BYTES
+    __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[MAX_STAGES], bar_bfree[MAX_STAGES];
+    __shared__ uint64_t bar_aready[A_RING], bar_afree[A_RING], bar_accfull[2], bar_accfree[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_fail;
     volatile int *fail = &s_fail;
@@ -725,18 +809,16 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nst = p.nst;   // units of 256 elements of K
     const int n_tiles = p.row_tiles * p.col_tiles;
-    const uint32_t accs = p.nw <= 128 ? 2 : 1;   // accumulators, 128 columns apart
+    const uint32_t accs = CT == 1 && p.nw <= 128 ? 2 : 1;   // accumulators in turn, 128 columns apart
     if (tid == 0) {
-        for (int i = 0; i < tc8f::RAW_STAGES; i++) {
+        for (int i = 0; i < MAX_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
             mbar_init(&bar_rawfree[i], tc8f::DEQ_WARPS);
-        }
-        for (int i = 0; i < tc8f::B_STAGES; i++) {
             mbar_init(&bar_b[i], 1);
             mbar_init(&bar_bfree[i], 1);
         }
-        for (int i = 0; i < tc8f::A_RING; i++) {
-            mbar_init(&bar_aready[i], tc8f::DEQ_WARPS);
+        for (int i = 0; i < A_RING; i++) {
+            mbar_init(&bar_aready[i], 4);
             mbar_init(&bar_afree[i], 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -752,200 +834,163 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     griddep_launch();
+    // Every ring: slot s, parity ph of its current round; whoever fills it waits for the parity before (true of a fresh barrier).
 
     if (warp == tc8f::TMA_RAW_WARP) {
-        // ---- raw weights: one 128-row x 272-byte box per unit (they do not depend on the kernel in front)
+        // ---- raw weights: one box of 128 rows per unit (they do not depend on the kernel in front)
         if (lane == 0) {
-            uint32_t g = 0;
+            int s = 0;
+            uint32_t ph = 0;
             for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
                 int row_tile, col_tile;
                 p.at(t, row_tile, col_tile);
                 const int mat = p.mat_of(row_tile);
                 const CUtensorMap *wmap = mat == 0 ? &maps.m[0] : (mat == 1 ? &maps.m[1] : &maps.m[2]);
                 const int row0 = (row_tile - p.tile0[mat]) * ROWS;
-                for (int i = 0; i < nst; i++, g++) {
-                    const int s = g % tc8f::RAW_STAGES;
-                    if (g >= tc8f::RAW_STAGES) mbar_wait_nap(&bar_rawfree[s], ((g / tc8f::RAW_STAGES) - 1) & 1, fail, 64);
+                for (int i = 0; i < nst; i++) {
+                    mbar_wait_nap(&bar_rawfree[s], ph ^ 1u, fail, 64);
                     mbar_expect_tx(&bar_raw[s], RAW_BYTES);
                     tma_2d(raw + s * RAW_BYTES, wmap, i * (ROW_CHUNK / 2), row0, &bar_raw[s]);   // x in 16-bit elements
+                    if (++s == p.raw_stages) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
         }
     } else if (warp == tc8f::TMA_B_WARP) {
-        // ---- packed activations: four stages per unit (of the last column tile only what there is: columns do not mix)
+        // ---- packed activations: four stages per unit and half (at the end only what there is: columns do not mix; a half
+        // that is not there at all gets the last columns once more)
         if (lane == 0) {
             griddep_wait();
-            uint32_t g = 0;
+            int s = 0;
+            uint32_t ph = 0;
             for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
                 int row_tile, col_tile;
                 p.at(t, row_tile, col_tile);
-                const int g0 = col_tile * (p.nw / 8);
-                const uint32_t bytes = (uint32_t)min(p.nw / 8, p.groups - g0) * 1024u;
-                const uint8_t *src = p.act + (size_t)g0 * 1024;
-                for (int i = 0; i < nst * 4; i++, g++) {
-                    const int s = g % tc8f::B_STAGES;
-                    if (g >= tc8f::B_STAGES) mbar_wait_nap(&bar_bfree[s], ((g / tc8f::B_STAGES) - 1) & 1, fail, 32);
-                    mbar_expect_tx(&bar_b[s], bytes);
-                    bulk_g2s(bst + s * tc8f::B_STAGE, src + (size_t)i * p.groups * 1024, bytes, &bar_b[s]);
-                }
+                for (int i = 0; i < nst * 4; i++)
+#pragma unroll
+                    for (int ct = 0; ct < CT; ct++) {
+                        const int g0 = min((col_tile * CT + ct) * (p.nw / 8), p.groups - 1);
+                        const uint32_t bytes = (uint32_t)min(p.nw / 8, p.groups - g0) * 1024u;
+                        mbar_wait_nap(&bar_bfree[s], ph ^ 1u, fail, 32);
+                        mbar_expect_tx(&bar_b[s], bytes);
+                        bulk_g2s(bst + s * b_stage, p.act + ((size_t)i * p.groups + g0) * 1024, bytes, &bar_b[s]);
+                        if (++s == p.b_stages) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
+                    }
             }
         }
     } else if (warp == tc8f::MMA_WARP) {
-        // ---- MMA issuer: the whole warp runs the loop (converged), one elected lane issues
-        const bool leader = elect_one();
-        uint32_t g = 0, gb = 0, it = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
-            const uint32_t ai = it % accs, acc = tmem_base + tc8f::ACC_COL0 + ai * 128u;
-            if (it >= accs) {
-                mbar_wait_nap(&bar_accfree[ai], (it / accs - 1) & 1, fail, 32);   // the tile before in this accumulator has been drained
-                tc_fence_after();
-            }
-            for (int i = 0; i < nst; i++, g++) {
-                const int slot = g % tc8f::A_RING;
-                mbar_wait_nap(&bar_aready[slot], (g / tc8f::A_RING) & 1, fail, 32);
-                tc_fence_after();
-                const uint32_t a0 = tmem_base + tc8f::A_COL0 + (uint32_t)(slot * 128);
+        // ---- MMA issuer: one thread. Its own instructions are what bounds tiles of any width (a warp that probed and issued with all
+        // lanes: 750 cycles per 64 elements of K, of which the four MMAs of 256 columns need 512).
+        if (elect_one()) {
+            int bs = 0, as = 0;
+            uint32_t bph = 0, aph = 0, it = 0;
+            const uint64_t b_desc0 = smem_desc(su32(bst), 128, 1024);
+            const uint32_t b_step = (uint32_t)b_stage >> 4;
+            uint32_t b_at = 0;
+            bool b_here = false, a_here = false;
+            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
+                const uint32_t ai = it % accs;
+                mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
+                uint32_t more = 0;
 #pragma unroll 1
-                for (int s4 = 0; s4 < 4; s4++, gb++) {
-                    const int bs = gb % tc8f::B_STAGES;
-                    mbar_wait_nap(&bar_b[bs], (gb / tc8f::B_STAGES) & 1, fail, 32);
-                    tc_fence_after();
-                    if (leader) {
-                        const uint64_t b_desc0 = smem_desc(su32(bst + bs * tc8f::B_STAGE), 128, 1024);
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            umma_f16_ta(acc, a0 + (uint32_t)((s4 * 4 + k) * 8), b_desc0 + (uint64_t)(k * 16), IDESC,
-                                        (i | s4 | k) ? 1u : 0u);
-                        umma_commit(&bar_bfree[bs]);
-                        if (s4 == 3) {
-                            umma_commit(&bar_afree[slot]);
-                            if (i == nst - 1) umma_commit(&bar_accfull[ai]);
-                        }
+                for (int i = nst * 4; i > 0; i--) {
+                    if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
+                    const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * 32u;
+                    uint64_t *const afree = &bar_afree[as];
+                    if (++as == A_RING) {
+                        as = 0;
+                        aph ^= 1u;
                     }
-                    __syncwarp();
+#pragma unroll
+                    for (int ct = 0; ct < CT; ct++) {
+                        if (!b_here) mbar_wait_nap(&bar_b[bs], bph, fail, 0);
+                        if (ct == 0) tc_fence_after();
+                        uint64_t *const bfree = &bar_bfree[bs];
+                        const uint64_t desc = b_desc0 + b_at;
+                        b_at += b_step;
+                        if (++bs == p.b_stages) {
+                            bs = 0;
+                            b_at = 0;
+                            bph ^= 1u;
+                        }
+                        if (ct == CT - 1) a_here = mbar_test(&bar_aready[as], aph);
+                        b_here = mbar_test(&bar_b[bs], bph);
+                        umma4_f16_ta(tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ct * HALF_NW)), a0, desc, IDESC, more);
+                        umma_commit(bfree);
+                    }
+                    umma_commit(afree);
+                    more = 1;
                 }
+                umma_commit(&bar_accfull[ai]);
             }
         }
+        __syncwarp();
     } else if (warp >= tc8f::DEQ_WARP0 && warp < tc8f::EPI_WARP0) {
-        // ---- expanders: lane quadrant warp % 4 fixes the rows; the two warps of a quadrant take four blocks each
-        const int q = warp & 3, half = (warp - tc8f::DEQ_WARP0) >> 2;
+        // ---- expanders: lane quadrant warp % 4 fixes the rows; of the four warps of a quadrant each takes 64 elements of a unit, a
+        // slot of its own. (A slot's waits, loads and stores are a chain of about 1000 cycles whatever its size: eight warps
+        // with 128 elements each took 1.3 us per unit.)
+        const int q = warp & 3, j = (warp - tc8f::DEQ_WARP0) >> 2;
         const int r = q * 32 + lane;
-        const uint32_t a_lane = tmem_base + tc8f::A_COL0 + ((uint32_t)(q * 32) << 16);
-        uint32_t g = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            for (int i = 0; i < nst; i++, g++) {
-                const int rs = g % tc8f::RAW_STAGES, slot = g % tc8f::A_RING;
-                mbar_wait_nap(&bar_raw[rs], (g / tc8f::RAW_STAGES) & 1, fail, 64);
-                if (g >= tc8f::A_RING) {
-                    mbar_wait_nap(&bar_afree[slot], ((g / tc8f::A_RING) - 1) & 1, fail, 64);   // the MMAs that read this slot are done
-                    tc_fence_after();
-                }
-                const uint8_t *rrow = raw + rs * RAW_BYTES + r * ROW_CHUNK;
-                if constexpr (WQ4K) {
-                    // this warp's half of the super-block: the 64-value groups 2 * half and 2 * half + 1 (the low nibbles of
-                    // a group's 32 bytes are one sub-block, the high nibbles the next)
-                    const uint4 hdr = *reinterpret_cast<const uint4 *>(rrow);   // d, dmin, scales[12]
-                    const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu)));
-                    const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-                    // byte i of scales[12], taken out of the three words with shifts (no byte array in local memory)
-                    auto sb = [&](int i) -> int { return (int)(((i < 4 ? hdr.y : (i < 8 ? hdr.z : hdr.w)) >> ((i & 3) * 8)) & 0xffu); };
-                    auto scale_min = [&](int jj, int &sc, int &mn) {   // get_scale_min_k4 (ggml-quants.c:880-887)
-                        if (jj < 4) {
-                            sc = sb(jj) & 63;
-                            mn = sb(jj + 4) & 63;
-                        } else {
-                            sc = (sb(jj + 4) & 0xF) | ((sb(jj - 4) >> 6) << 4);
-                            mn = (sb(jj + 4) >> 4) | ((sb(jj) >> 6) << 4);
-                        }
-                    };
-#pragma unroll
-                    for (int gg = 0; gg < 2; gg++) {
-                        const int j = half * 2 + gg;
-                        int sc0, mn0, sc1, mn1;
-                        scale_min(2 * j, sc0, mn0);
-                        scale_min(2 * j + 1, sc1, mn1);
-                        const uint64_t a0 = twice(__fmul_rn(d, (float)sc0)), b0 = twice(-__fmul_rn(dmin, (float)mn0));
-                        const uint64_t a1 = twice(__fmul_rn(d, (float)sc1)), b1 = twice(-__fmul_rn(dmin, (float)mn1));
-                        uint32_t lo[16], hi[16];
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            const uint4 qv = *reinterpret_cast<const uint4 *>(rrow + 16 + j * 32 + u * 16);
-                            const uint32_t w4[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-                            for (int wi = 0; wi < 4; wi++) {
-                                const uint32_t w = w4[wi];
-                                const uint32_t x = w & 0x0f0f0f0fu, y = (w >> 4) & 0x0f0f0f0fu;
-                                lo[(u * 4 + wi) * 2] = fold_pair(__byte_perm(x, 0x64646464u, 0x4140), a0, b0);
-                                lo[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(x, 0x64646464u, 0x4342), a0, b0);
-                                hi[(u * 4 + wi) * 2] = fold_pair(__byte_perm(y, 0x64646464u, 0x4140), a1, b1);
-                                hi[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(y, 0x64646464u, 0x4342), a1, b1);
-                            }
-                        }
-                        tmem_st16(a_lane + (uint32_t)(slot * 128 + j * 32), lo);
-                        tmem_st16(a_lane + (uint32_t)(slot * 128 + j * 32 + 16), hi);
-                    }
-                } else {
-#pragma unroll
-                for (int gg = 0; gg < 2; gg++) {
-                    uint32_t qa[8], qb[8];
-                    float da, db;
-                    if (half == 0) {
-                        if (gg == 0) tc8::split_blocks<0>(rrow, qa, qb, da, db);
-                        else tc8::split_blocks<1>(rrow, qa, qb, da, db);
-                    } else {
-                        if (gg == 0) tc8::split_blocks<2>(rrow, qa, qb, da, db);
-                        else tc8::split_blocks<3>(rrow, qa, qb, da, db);
-                    }
-                    const int blk = (half * 2 + gg) * 2;
-                    uint32_t h[16];
-                    uint32_t dd = (uint32_t)__half_as_ushort(__float2half_rn(da));   // the block's own f16 scale, back from f32 unchanged
-                    dd |= dd << 16;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) codes_to_f16(qa[j], dd, h[2 * j], h[2 * j + 1]);
-                    tmem_st16(a_lane + (uint32_t)(slot * 128 + blk * 16), h);
-                    dd = (uint32_t)__half_as_ushort(__float2half_rn(db));
-                    dd |= dd << 16;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) codes_to_f16(qb[j], dd, h[2 * j], h[2 * j + 1]);
-                    tmem_st16(a_lane + (uint32_t)(slot * 128 + (blk + 1) * 16), h);
-                }
-                }
+        const uint32_t a_lane = tmem_base + ACOLS + ((uint32_t)(q * 32) << 16);
+        int s = 0, as = j;
+        uint32_t ph = 0, aph = 0;
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x)
+            for (int i = 0; i < nst; i++) {
+                mbar_wait_nap(&bar_raw[s], ph, fail, 64);
+                mbar_wait_nap(&bar_afree[as], aph ^ 1u, fail, 64);   // the MMAs that read this slot are done
+                tc_fence_after();
+                expand64<WQ4K>(raw + s * RAW_BYTES + r * ROW_CHUNK, j, a_lane + (uint32_t)as * 32u);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&bar_aready[slot]);
-                    mbar_arrive(&bar_rawfree[rs]);
+                    mbar_arrive(&bar_aready[as]);
+                    mbar_arrive(&bar_rawfree[s]);
+                }
+                as += 4;
+                if (as >= A_RING) {
+                    as -= A_RING;
+                    aph ^= 1u;
+                }
+                if (++s == p.raw_stages) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
-        }
     } else if (warp >= tc8f::EPI_WARP0) {
-        // ---- draining warps: lane quadrant warp % 4, every other 32 columns from (warp - tc8f::EPI_WARP0) / 4 on; once per tile
+        // ---- draining warps, once per tile: lane quadrant warp % 4; of the two warps of a quadrant each takes every other 32
+        // columns (CT = 1) or one of the halves (CT = 2)
         const int q = warp & 3, ch = (warp - tc8f::EPI_WARP0) >> 2;
         const int row_in_tile = q * 32 + lane, chunks = (p.nw + 31) / 32;
+        const int c0 = CT == 1 ? ch : 0, step = CT == 1 ? 2 : 1;
         uint32_t it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
             int row_tile, col_tile;
             p.at(t, row_tile, col_tile);
-            const int col0 = col_tile * p.nw, mat = p.mat_of(row_tile);
+            const int col0 = (CT == 1 ? col_tile : 2 * col_tile + ch) * p.nw, mat = p.mat_of(row_tile);
             const uint32_t ai = it % accs;
-            const uint32_t lane_addr = tmem_base + tc8f::ACC_COL0 + ai * 128u + ((uint32_t)(q * 32) << 16);
+            const uint32_t lane_addr = tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ch * HALF_NW)) + ((uint32_t)(q * 32) << 16);
             mbar_wait_nap(&bar_accfull[ai], (it / accs) & 1, fail, 128);
             tc_fence_after();
             const int64_t row = (int64_t)(row_tile - p.tile0[mat]) * ROWS + row_in_tile, M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]);
             const int64_t ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
             float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + (size_t)col0 * ldy + row;
-            if (ch >= chunks) {
+            if (c0 >= chunks) {
                 if (lane == 0) mbar_arrive(&bar_accfree[ai]);
                 continue;
             }
             const int cols = min(p.nw, p.N - col0);
 #pragma unroll 1
-            for (int c = ch; c < chunks; c += 2) {
+            for (int c = c0; c < chunks; c += step) {
                 uint32_t v[32];
                 tmem_ld32(lane_addr + (uint32_t)(c * 32), v);   // (past the tile's last column: other columns of the same 512, not used)
                 tmem_ld_wait();
-                if (c + 2 >= chunks) {   // everything of this warp's part is in registers: the accumulator may be overwritten
+                if (c + step >= chunks) {   // everything of this warp's part is in registers: the accumulator may be overwritten
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bar_accfree[ai]);
@@ -964,27 +1009,32 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
-static size_t tc8f_smem() { return (size_t)tc8f::B_STAGES * tc8f::B_STAGE + (size_t)tc8f::RAW_STAGES * tc8::RAW_BYTES + 1024; }   // the larger raw stage (Q8_0)
-
-// The folded-scale GEMM for either weight format (the Q4_K planner and launcher in k_mmq_tc.cu call it for more than 64 columns)
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
-// Columns of a tile, a multiple of 16: of the even splits of N into tiles of at most 256 columns, the one whose slowest SM has the
-// least to do. A unit of K was measured at 1.3 us up to 100 columns (the expansion of its weights), 1.47 at 128, 1.86 at 192 and 2.15
-// at 256; draining a wide tile, which has no second accumulator, at about 1 us.
-static int fold_cols(int64_t N, int row_tiles, int nst, int sms) {
+struct FoldTile {
+    int halves, nw;
+};
+// Halves of a tile and columns of each (a multiple of 16): of the even splits of N, the one whose slowest SM has the least to do.
+// Measured per unit of K: 1.2 us at 64 columns, 1.3 at 128, 1.55 at 256; in halves 1.75 at 192 and 2.4 at 384, which pays where it
+// saves a wave (224 row tiles x 333 columns). Draining a tile without a second accumulator is about 1.2 us.
+static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
+    FoldTile f{1, 0};
     double best = 0;
-    int cols = 0;
-    for (int64_t ct = (N + tc8f::NW - 1) / tc8f::NW, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
-        const int nw = (int)(((N + ct - 1) / ct + 15) / 16 * 16);
-        const int64_t tiles = (int64_t)row_tiles * ((N + nw - 1) / nw), waves = (tiles + sms - 1) / sms;
-        const double t = (double)waves * (nst * std::max(1.3, 0.65 + 0.0059 * nw) + (nw > 128 ? 1.0 : 0.2));
-        if (cols == 0 || t < best * 0.98) {
-            best = t;
-            cols = nw;
+    for (int halves = 1; halves <= 2; halves++) {
+        const int widest = halves == 1 ? tc8f::NW : 2 * tc8f::HALF_NW;
+        for (int64_t ct = (N + widest - 1) / widest, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
+            const int nw = (int)(((N + ct * halves - 1) / (ct * halves) + 15) / 16 * 16);
+            const int64_t tiles = (int64_t)row_tiles * ((N + halves * nw - 1) / (halves * nw)), waves = (tiles + sms - 1) / sms;
+            const double unit = halves == 1 ? std::max(1.2, 1.07 + 0.00185 * nw) : std::max(1.75, 0.65 + 0.0046 * 2 * nw);
+            const double t = (double)waves * (nst * unit + (halves == 1 && nw <= 128 ? 0.3 : 1.2));
+            if (f.nw == 0 || t < best * 0.98) {
+                best = t;
+                f.halves = halves;
+                f.nw = nw;
+            }
         }
     }
-    return cols;
+    return f;
 }
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
                                int64_t ldy, int *err, cudaStream_t st) {
@@ -1013,13 +1063,20 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.act = (const uint8_t *)blobs;
     p.N = (int)N;
     p.nst = (int)(K / 256);
-    p.nw = fold_cols(N, p.row_tiles, p.nst, sm_of[dev]);
+    const FoldTile tile = fold_tile(N, p.row_tiles, p.nst, sm_of[dev]);
+    p.nw = tile.nw;
+    // raw stages: 128 rows x 256 elements (18 or 34 KB); what they leave goes to B
+    const int raw_bytes = tc8::ROWS * (q4k ? 144 : tc8::ROW_CHUNK);
+    p.raw_stages = q4k ? 4 : (tile.halves == 1 && p.nw <= 192 ? 3 : 2);
+    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * 2));
+    if (p.b_stages < 2) return cudaErrorInvalidValue;
     p.groups = mm_fold_groups(N);
-    p.col_tiles = (int)((N + p.nw - 1) / p.nw);
+    p.col_tiles = (int)((N + tile.halves * p.nw - 1) / (tile.halves * p.nw));
     p.err = err;
     const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sm_of[dev]));
-    return q4k ? launch_pdl(k_mm_q80_f16<true>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, maps, p)
-               : launch_pdl(k_mm_q80_f16<false>, grid, dim3(tc8f::THREADS), tc8f_smem(), st, maps, p);
+    auto go = [&](auto *k) { return launch_pdl(k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
+    if (tile.halves == 2) return q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
+    return q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
 }
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st) {
     const char *ab = (const char *)act;
@@ -1042,8 +1099,11 @@ void mmq_tc8_configure() {
     cudaFuncSetAttribute(k_mmq_tc_q80<16, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<16, 4, 4>());
     cudaFuncSetAttribute(k_mmq_tc_q80<32, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<32, 4, 4>());
     cudaFuncSetAttribute(k_mmq_tc_q80_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
-    cudaFuncSetAttribute(k_mm_q80_f16<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8f_smem());
-    cudaFuncSetAttribute(k_mm_q80_f16<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8f_smem());
+    auto fold = [](auto *k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc8f::SMEM); };
+    fold(k_mm_q80_f16<false, 1>);
+    fold(k_mm_q80_f16<true, 1>);
+    fold(k_mm_q80_f16<false, 2>);
+    fold(k_mm_q80_f16<true, 2>);
 }
 
 bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N) {
