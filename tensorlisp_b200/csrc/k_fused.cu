@@ -215,7 +215,6 @@ __device__ __forceinline__ void xr_body(const ArRank &a, const RowQuantArgs &p, 
     const bool live = warp < nblk;
     const int64_t e0 = (int64_t)n * K + warp * 256 + lane * 8;   // this lane's 8 elements of the [rows][K] matrix
     if (tid == 0) s_fail = 0;
-    float b[8];
     if (live) {
         const float *src = (a.n_split > 0 ? a.partial : a.data) + e0;
         float4 b0 = *reinterpret_cast<const float4 *>(src), b1 = *reinterpret_cast<const float4 *>(src + 4);

@@ -182,6 +182,9 @@ struct RopeKvArgs {
 };
 cudaError_t launch_rope_kv(const RopeKvArgs &p, const void *q, const void *k, const void *v, const int32_t *pos, const float *ff,
                            void *q16, void *kpool, void *vpool, const int64_t *slots, int *err, cudaStream_t st);
+// the same for a prompt: q -> f32 (rope.d: dense), k and v -> f16 [hs, kv_heads, tokens] and into the pools
+cudaError_t launch_rope_kv_prompt(const RopeKvArgs &p, const void *q, const void *k, const void *v, const int32_t *pos, float *q32, void *k16,
+                                  void *v16, void *kpool, void *vpool, const int64_t *slots, int *err, cudaStream_t st);
 struct SoftmaxArgs { TView a, m, d; float scale, max_bias, m0, m1; int n_head_log2; int has_mask; uint32_t mty; };
 cudaError_t launch_soft_max(const SoftmaxArgs &p, const void *a, const void *m, void *d, cudaStream_t st);
 struct RowsArgs { TView a, ids, d; uint32_t aty, idty, dty; };

@@ -234,11 +234,13 @@ void lower_rope(L &l) {
 
 // ROPE_KV_WRITE (pseudo-op made by fuse_rope_cache): src = q, k, v (f32), pos, freq factors or -1,
 // key pool, value pool, slots, and the f16 query it produces. op_params: the rope's, with the
-// kv-head count and block size in [12], [13].
+// kv-head count and block size in [12], [13]. ROPE_KV_PROMPT: no freq factors, src[4] = the f16 value, src[8] = the f32 query,
+// src[9] = the f16 key that it produces.
 void lower_rope_kv(L &l) {
     const Tensor &t = l.t();
     const int32_t q = l.src(0), k = l.src(1), v = l.src(2), pos = l.src(3), kc = l.src(5), vc = l.src(6), slots = l.src(7), q16 = l.src(8);
-    const int32_t ff = t.src[4];
+    const bool prompt = t.op == "ROPE_KV_PROMPT";
+    const int32_t ff = prompt ? -1 : t.src[4];
     const Tensor &tq = l.T(q), &tk = l.T(k), &tv = l.T(v);
     RopeKvArgs p{};
     p.rope = rope_params(t, tq.ne[0]);
@@ -251,13 +253,21 @@ void lower_rope_kv(L &l) {
     p.kv_heads = t.op_params[12];
     p.block_size = t.op_params[13];
     if (p.block_size < 1) unsupported(t, "the block size of a cache write must be at least 1");
-    p.pool_slots = l.T(kc).nelements() / ((int64_t)p.kv_heads * p.hs);
+    p.pool_slots = (prompt ? std::min(l.T(kc).nelements(), l.T(vc).nelements()) : l.T(kc).nelements()) / ((int64_t)p.kv_heads * p.hs);
     // v arrives as [hs * kv_heads, tokens]
     p.v = view_of(tv);
     p.v.nb[2] = (int64_t)tv.nb[1];
     p.v.nb[1] = (int64_t)p.hs * 4;
     const Place pq = l.place(q), pk = l.place(k), pv = l.place(v), pp = l.place(pos), pkc = l.place(kc), pvc = l.place(vc),
                 psl = l.place(slots), pq16 = l.place(q16);
+    if (prompt) {
+        const Place pk16 = l.place(l.src(9)), pv16 = l.place(l.src(4));
+        l.push([=](const RunCtx &r) {
+            return launch_rope_kv_prompt(p, r.at(pq), r.at(pk), r.at(pv), (const int32_t *)r.at(pp), (float *)r.at(pq16), r.at(pk16), r.at(pv16), r.at(pkc),
+                                         r.at(pvc), (const int64_t *)r.at(psl), r.err, r.stream);
+        });
+        return;
+    }
     Place pf;
     if (ff >= 0) pf = l.place(ff);
     const bool hf = ff >= 0;
@@ -1113,7 +1123,7 @@ void lower_node(const LowerCtx &c, int32_t id, int pos, std::vector<Dispatch> &o
     if (op == "NORM" || op == "RMS_NORM") return lower_norm(l, false);
     if (op == "RMS_NORM_MUL") return lower_norm(l, true);
     if (op == "ROPE") return lower_rope(l);
-    if (op == "ROPE_KV_WRITE") return lower_rope_kv(l);
+    if (op == "ROPE_KV_WRITE" || op == "ROPE_KV_PROMPT") return lower_rope_kv(l);
     if (op == "SOFT_MAX") return lower_soft_max(l);
     if (op == "GET_ROWS") return lower_get_rows(l);
     if (op == "SET_ROWS") return lower_set_rows(l);
@@ -1438,7 +1448,8 @@ void fuse_row_producers(Graph &g) {
 // rope(q) -> cast, rope(k) -> cast, v -> cast, cache write: one ROPE_KV_WRITE node in place of the
 // cache write (decode-step shape of scheme/core.ss:222-271 callers). Legality as for the other
 // fusions: every folded intermediate has exactly one reader, is not kept, and is a plain f32/f16
-// tensor of the expected shape; both ropes share position tensor and parameters.
+// tensor of the expected shape; both ropes share position tensor and parameters. In a prompt pass the dense attention
+// reads the f32 rope(q) and the f16 keys and values themselves: ROPE_KV_PROMPT writes those too (whoever reads them comes later).
 void fuse_rope_cache(Graph &g) {
     const size_t nn = g.nodes.size();
     std::vector<int> pos_of(g.tensors.size(), -1);
@@ -1470,6 +1481,64 @@ void fuse_rope_cache(Graph &g) {
         return src;
     };
     std::vector<char> dead(nn, 0);
+    // does a node between positions a and b (exclusive) read or write a root?
+    auto touched = [&](int32_t root, int a, int b) {
+        for (int i = a + 1; i < b; i++) {
+            const Tensor &t = g.tensors[g.nodes[i]];
+            if (dead[i] || t.is_view_op()) continue;
+            if (g.root(g.nodes[i]) == root) return true;
+            for (int s = 0; s < 10; s++)
+                if (t.src[s] >= 0 && g.root(t.src[s]) == root) return true;
+        }
+        return false;
+    };
+    auto written = [&](int32_t root, int a, int b) {
+        for (int i = a + 1; i < b; i++)
+            if (!dead[i] && !g.tensors[g.nodes[i]].is_view_op() && g.root(g.nodes[i]) == root) return true;
+        return false;
+    };
+    auto fuse_rope_prompt = [&](size_t ci, int32_t k16, int32_t v16, int32_t rk, int32_t vsrc) {
+        Tensor &Cw = g.tensors[g.nodes[ci]];
+        const PagedUd u = paged_ud(Cw);
+        const Tensor RK = g.tensors[rk];
+        if (RK.src[2] >= 0 || RK.src[0] < 0 || u.block_size < 1 || u.kv_heads < 1) return;
+        // the query's rope: the same positions and parameters, right in front of the key's or somewhere between it and here
+        int qi = -1;
+        for (int i = (int)ci - 1; i >= 0 && qi < 0; i--) {
+            const Tensor &R = g.tensors[g.nodes[i]];
+            if (dead[i] || g.nodes[i] == rk || R.op != "ROPE" || R.src[1] != RK.src[1] || R.src[2] >= 0 || R.ty != TLB_TYPE_F32 || R.view_src >= 0) continue;
+            bool same = R.ne[0] == RK.ne[0] && R.ne[2] == RK.ne[2];
+            for (int x = 0; x < 16; x++) same = same && R.op_params[x] == RK.op_params[x];
+            if (same) qi = i;
+            else return;
+        }
+        if (qi < 0) return;
+        const int32_t rq = g.nodes[qi];
+        const Tensor RQ = g.tensors[rq];
+        const Tensor &QI = g.tensors[RQ.src[0]], &KI = g.tensors[RK.src[0]], &VI = g.tensors[g.tensors[v16].src[0]];
+        const int64_t hs = QI.ne[0], tokens = QI.ne[2];
+        const int at = (int)ci;
+        bool ok = QI.ty == 0 && KI.ty == 0 && VI.ty == 0 && QI.nb[0] == 4 && KI.nb[0] == 4 && VI.nb[0] == 4 && QI.ne[3] == 1 && KI.ne[3] == 1 &&
+                  KI.ne[0] == hs && KI.ne[1] == u.kv_heads && KI.ne[2] == tokens && VI.ne[0] == hs * u.kv_heads && VI.nrows() == tokens && VI.ne[2] == 1 &&
+                  hs % 8 == 0 && hs <= 512 && VI.nb[1] % 8 == 0 && g.tensors[RQ.src[1]].ty == TLB_TYPE_I32 && g.tensors[RQ.src[1]].ne[0] == tokens &&
+                  RQ.is_contiguous() && g.tensors[k16].nelements() == hs * u.kv_heads * tokens && g.tensors[Cw.src[2]].ty == TLB_TYPE_F16 &&
+                  g.tensors[Cw.src[3]].ty == TLB_TYPE_F16 && g.tensors[Cw.src[4]].nelements() == 2 * tokens && n_readers(rk, pos_of[rk]) == 1;
+        uint64_t vo = 0;
+        g.root(g.tensors[v16].src[0], &vo);
+        ok = ok && vo % 8 == 0;
+        // nobody needs the results before the new place of the node, and its sources still hold their values there
+        ok = ok && !touched(rq, qi, at) && !touched(k16, pos_of[k16], at) && !touched(v16, pos_of[v16], at) && !written(g.root(RQ.src[0]), qi, at) &&
+             !written(g.root(RK.src[0]), pos_of[rk], at) && !written(vsrc, pos_of[v16], at) && !written(g.root(RQ.src[1]), std::min(qi, pos_of[rk]), at);
+        if (!ok) return;
+        const int32_t pools[2] = {Cw.src[2], Cw.src[3]}, slots = Cw.src[4], vin = g.tensors[v16].src[0];
+        Cw.op = "ROPE_KV_PROMPT";
+        for (int i = 0; i < 16; i++) Cw.op_params[i] = RQ.op_params[i];
+        Cw.op_params[12] = u.kv_heads;
+        Cw.op_params[13] = u.block_size;
+        const int32_t src[10] = {RQ.src[0], RK.src[0], vin, RQ.src[1], v16, pools[0], pools[1], slots, rq, k16};
+        for (int i = 0; i < 10; i++) Cw.src[i] = src[i];
+        dead[qi] = dead[pos_of[rk]] = dead[pos_of[k16]] = dead[pos_of[v16]] = 1;
+    };
     for (size_t ci = 0; ci < nn; ci++) {
         const int32_t cid = g.nodes[ci];
         Tensor &Cw = g.tensors[cid];
@@ -1485,7 +1554,10 @@ void fuse_rope_cache(Graph &g) {
             const Tensor &A = g.tensors[g.nodes[i]];
             if (A.op == "CUSTOM" && paged_ud(A).kind == 1 && A.src[1] == Cw.src[2] && A.src[2] == Cw.src[3]) ai = (int)i;
         }
-        if (ai < 0) continue;
+        if (ai < 0) {
+            fuse_rope_prompt(ci, k16, v16, rk, vsrc);
+            continue;
+        }
         const int32_t q16 = g.tensors[g.nodes[ai]].src[0];
         const int32_t rq = cast_of(q16, "ROPE");
         if (rq < 0) continue;
