@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
         h[e] = *reinterpret_cast<const uint32_t *>(&t);
     }
     if (p.npad) *reinterpret_cast<uint4 *>(blob) = make_uint4(h[0], h[1], h[2], h[3]);
+    if (p.operand_only) return;
     // the Q8_0 block itself (int8 codes and f32 scales): the few-column mul_mat reads it (npad 0: nothing else is wanted), and any
     // consumer that is not a prompt-sized 2-D product
     uint2 packed;
@@ -175,6 +176,84 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
     packed.y = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
     *reinterpret_cast<uint2 *>((int8_t *)p.out + p.qs_off + (size_t)n * K + k0) = packed;
     if ((lane & 3) == 0) reinterpret_cast<float *>((char *)p.out + p.d_off)[(size_t)n * (K / 32) + (k0 >> 5)] = dh;
+}
+
+// ---------------------------------------------------------------- many plain rows: eight columns per CTA
+// f32 (or f16) rows as they are into the prompt's operand. What bounds it is memory; the kernels above reach half of that, because a
+// row leaves 16 bytes in each 128-byte line of the operand and one block per warp is little in flight. Here a warp holds four
+// blocks of one column, and the eight columns of a group meet in shared memory, from where whole kilobytes leave.
+// 16384 rows of 4096: 118 -> 92 us. (Behind a norm or a gate the same split gained nothing: arithmetic bounds those.)
+template <bool Q80>
+__global__ void __launch_bounds__(256) k_row_quant_plain(RowQuantArgs p) {
+    __shared__ __align__(16) uint8_t tile[4 * 4096];   // [block][stage of 64][chunk of 8][column ^ chunk][16 bytes]
+    griddep_launch();
+    griddep_wait();
+    const int lane = threadIdx.x & 31, col = threadIdx.x >> 5;
+    const int n = (int)blockIdx.x * 8 + col;
+    const int64_t K = p.K;
+    const int sb0 = (int)blockIdx.y * 4, here = min(4, (int)(K / 256) - sb0);
+    const bool row = n < p.N;
+    char *ob = (char *)p.out;
+    float v[4][8];
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[b][e] = 0.f;   // padding columns of the operand are zero
+        if (row && b < here) rq_load8(p, n, (int64_t)(sb0 + b) * 256 + lane * 8, v[b]);
+    }
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        if (b >= here) break;
+        const int64_t k0 = (int64_t)(sb0 + b) * 256 + lane * 8;
+        int q[8];
+        float d;
+        if (Q80) {   // quantize_row_q8_0_ref (ggml-quants.c:276-299)
+            float amax = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[b][e]));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            d = __fdiv_rn(amax, 127.f);
+            const float id = d != 0.f ? __fdiv_rn(1.0f, d) : 0.0f;
+            d = __half2float(__float2half_rn(d));   // the block's scale as the dot product reads it
+#pragma unroll
+            for (int e = 0; e < 8; e++) q[e] = (int)roundf(__fmul_rn(v[b][e], id));
+        } else {
+            rq_q8k(lane, v[b], q, d);
+        }
+        uint32_t h[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const __half2 t = __floats2half2_rn(__fmul_rn((float)q[2 * e], d), __fmul_rn((float)q[2 * e + 1], d));
+            h[e] = *reinterpret_cast<const uint32_t *>(&t);
+        }
+        const int chunk = lane & 7;
+        *reinterpret_cast<uint4 *>(tile + b * 4096 + (lane >> 3) * 1024 + chunk * 128 + ((col ^ chunk) * 16)) = make_uint4(h[0], h[1], h[2], h[3]);
+        if (p.operand_only || !row) continue;
+        uint2 packed;
+        packed.x = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+        packed.y = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
+        *reinterpret_cast<uint2 *>((int8_t *)ob + p.qs_off + (size_t)n * K + k0) = packed;
+        float *ds = reinterpret_cast<float *>(ob + p.d_off);
+        if (Q80) {
+            if ((lane & 3) == 0) ds[(size_t)n * (K / 32) + (k0 >> 5)] = d;
+        } else {
+            int s8 = 0;
+#pragma unroll
+            for (int e = 0; e < 8; e++) s8 += q[e];
+            s8 += __shfl_xor_sync(0xffffffffu, s8, 1);
+            if ((lane & 1) == 0) reinterpret_cast<int16_t *>(ob + p.bsum_off)[(size_t)n * (K / 16) + (sb0 + b) * 16 + (lane >> 1)] = (int16_t)s8;
+            if (lane == 0) ds[(size_t)n * (K / 256) + sb0 + b] = d;
+        }
+    }
+    __syncthreads();
+    const int groups = mm_fold_groups(p.N);
+    uint8_t *o = (uint8_t *)ob + p.blob_off + ((size_t)sb0 * 4 * groups + blockIdx.x) * 1024;
+    for (int u = threadIdx.x; u < here * 256; u += 256) {
+        const int stage = u >> 6, chunk = (u >> 3) & 7, c = u & 7;
+        const uint4 t = *reinterpret_cast<const uint4 *>(tile + stage * 1024 + chunk * 128 + ((c ^ chunk) * 16));
+        *reinterpret_cast<uint4 *>(o + (size_t)stage * groups * 1024 + (u & 63) * 16) = t;
+    }
 }
 
 bool row_quant_q80_supported(int64_t K, int mode) { return K % 256 == 0 && K >= 256 && (mode != RQ_NORM || K <= 8192); }
@@ -405,6 +484,12 @@ bool row_quant_supported(int64_t K) { return K % 256 == 0 && K / 256 <= 65535 * 
 
 cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st) {
     if (p.N == 0 || p.K == 0) return cudaSuccess;
+    // eight columns per CTA: from two CTAs per SM on
+    const int64_t eights = mm_fold_groups(p.N), strips = (p.K / 256 + 3) / 4;
+    if (p.npad == MM_FOLD_NPAD && (p.mode == RQ_PLAIN || p.mode == RQ_F16) && !p.b && !p.y_out && eights * strips >= 296 && strips <= 65535) {
+        const dim3 grid((unsigned)eights, (unsigned)strips);
+        return p.q80 ? launch_pdl(k_row_quant_plain<true>, grid, dim3(256), 0, st, p) : launch_pdl(k_row_quant_plain<false>, grid, dim3(256), 0, st, p);
+    }
     if (p.q80) {
         if ((p.npad != 256 && p.npad != 0) || !row_quant_q80_supported(p.K, p.mode)) return cudaErrorInvalidValue;
         const int nb = (int)(p.K / 256);

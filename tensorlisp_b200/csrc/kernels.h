@@ -115,6 +115,7 @@ struct RowQuantArgs {
     int64_t wn;
     float eps;
     float *y_out;        // optional f32 copy of the produced row
+    int operand_only;    // every reader takes the folded-scale operand: codes, scales and sums are not written
     int64_t ld_y;
     void *out;           // ActLayout block (ACT_Q8_K) for N columns
     uint64_t qs_off, d_off, bsum_off;

@@ -62,6 +62,23 @@ bool gemv_node(const Graph &g, const Tensor &t) {
 bool gemv_self_quant(const Graph &g, const Tensor &t) { return t.ne[1] <= 2 || g.tensors[t.src[0]].ty == TLB_TYPE_Q6_K; }
 constexpr int GEMV_MARK = 8, GEMV_MODE = 9, GEMV_GLU = 10;   // op_params of such a node once fuse_gemv has seen it; eps in 15
 
+// Whether the readers of quantized activations all are products that take the folded-scale operand behind the block (lower_mul_mat
+// and lower_mul_mat_group choose by the same conditions), so that the block itself need not be written.
+bool operand_only(const Graph &g, int32_t q) {
+    if (g.tensors[q].op_params[1] != MM_FOLD_NPAD || getenv("TLB_MM_GENERIC") || getenv("TLB_NO_TC")) return false;
+    for (int32_t id : g.nodes) {
+        const Tensor &t = g.tensors[id];
+        for (int s = 0; s < 10; s++) {
+            if (t.src[s] < 0 || g.root(t.src[s]) != q) continue;
+            if (s != 2 || (t.op != "MUL_MAT" && t.op != "MUL_MAT_GROUP") || t.src[2] != q) return false;
+            if (t.op == "MUL_MAT_GROUP") continue;
+            const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
+            if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1 || tw.nb[1] != tw.row_size() || !t.is_contiguous() || !tc_supported(tw.ty, tw.ne[0], tw.ne[1], tx.nrows())) return false;
+        }
+    }
+    return true;
+}
+
 int act_kind_for(uint32_t wty) { return wty == TLB_TYPE_Q4_K ? ACT_Q8_K : ACT_Q8_0; }
 bool is_qact(const std::string &op) { return op == "QUANT_ACT" || op == "ROW_QUANT"; }
 
@@ -600,18 +617,21 @@ void lower_quant_act(L &l) {
     const int64_t ldx = tx.nrows() > 1 ? (int64_t)tx.nb[1] / 4 : tx.ne[0];
     const Place px = l.place(x), pd = l.place(l.id);
     const int npad = t.op_params[1];   // > 0: also pack the blobs of the tensor-core path behind the Q8_K block
-    if (a.kind == ACT_Q8_0 && npad == 256 && row_quant_q80_supported(a.K, RQ_PLAIN) && tx.nb[0] == 4 && ldx % 4 == 0) {
-        // the prompt mul_mat reads the packed f16 operand only: one launch from the f32 rows straight to it
+    if (npad > 0 && (a.kind == ACT_Q8_0 ? npad == MM_FOLD_NPAD && row_quant_q80_supported(a.K, RQ_PLAIN) : row_quant_supported(a.K)) && tx.nb[0] == 4 && ldx % 4 == 0) {
+        // one launch from the f32 rows straight to the packed operand of the tensor-core kernels
         RowQuantArgs p{};
         p.mode = RQ_PLAIN;
         p.K = a.K;
         p.N = a.N;
         p.lda = ldx;
         p.npad = npad;
-        p.q80 = 1;
+        p.q80 = a.kind == ACT_Q8_0;
         p.qs_off = a.qs_off;
         p.d_off = a.d_off;
+        p.bsum_off = a.bsum_off;
         p.blob_off = a.bytes;
+        p.blob_bytes = p.q80 ? 0 : mmq_tc_plan(p.K, 128, p.N, 148).blob_unit;
+        p.operand_only = operand_only(*l.c.g, l.id);
         l.push([=](const RunCtx &r) {
             RowQuantArgs q = p;
             q.a = (const float *)r.at(px);
@@ -650,6 +670,7 @@ void lower_row_quant(L &l) {
     p.blob_off = al.bytes;
     p.blob_bytes = p.npad > 0 ? mmq_tc_plan(p.K, 128, p.N, 148).blob_unit : 0;
     p.q80 = t.op_params[0] == ACT_Q8_0;
+    p.operand_only = operand_only(*l.c.g, l.id);
     p.eps = t.param_f32(15);
     p.lda = mode == RQ_F16 ? p.K : (p.N > 1 ? (int64_t)l.T(a).nb[1] / 4 : p.K);
     const int32_t b = t.src[1], w = t.src[3], sum = t.src[4];

@@ -41,19 +41,8 @@ __device__ __forceinline__ void rq_load8(const RowQuantArgs &p, int n, int64_t k
     }
 }
 
-// Q8_K quantization of one 256-value block held by a warp (lane l: values l*8 .. l*8+7), its optional f32
-// copy, and its slice of the tensor-core operand blob (quantize_row_q8_K_ref, ggml-quants.c:2768-2805)
-__device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int sb, int nblk, int lane, float (&v)[8]) {
-    char *ob = (char *)p.out;
-    const int64_t K = p.K;
-    const int64_t k0 = (int64_t)sb * 256 + lane * 8;
-    int8_t *qs = (int8_t *)(ob + p.qs_off);
-    float *ds = (float *)(ob + p.d_off);
-    int16_t *bsums = (int16_t *)(ob + p.bsum_off);
-    if (p.y_out) {
-        *reinterpret_cast<float4 *>(p.y_out + n * p.ld_y + k0) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4 *>(p.y_out + n * p.ld_y + k0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    }
+// Codes and scale of one 256-value block held by a warp (lane l: values l*8 .. l*8+7; quantize_row_q8_K_ref, ggml-quants.c:2768-2805)
+__device__ __forceinline__ void rq_q8k(int lane, const float (&v)[8], int (&q)[8], float &d) {
     float amax = 0.f, mx = 0.f;
     int idx = 512;
 #pragma unroll
@@ -65,8 +54,7 @@ __device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int
         const int oi = __shfl_xor_sync(0xffffffffu, idx, s);
         if (oa > amax || (oa == amax && oi < idx)) { amax = oa; mx = om; idx = oi; }
     }
-    int q[8];
-    float d = 0.f;
+    d = 0.f;
     if (amax == 0.f) {
 #pragma unroll
         for (int e = 0; e < 8; e++) q[e] = 0;
@@ -76,6 +64,24 @@ __device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int
         for (int e = 0; e < 8; e++) q[e] = min(127, nearest_int_f(__fmul_rn(iscale, v[e])));
         d = __fdiv_rn(1.f, iscale);
     }
+}
+
+// Q8_K quantization of one 256-value block held by a warp (lane l: values l*8 .. l*8+7), its optional f32
+// copy, and its slice of the tensor-core operand blob
+__device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int sb, int nblk, int lane, float (&v)[8]) {
+    char *ob = (char *)p.out;
+    const int64_t K = p.K;
+    const int64_t k0 = (int64_t)sb * 256 + lane * 8;
+    int8_t *qs = (int8_t *)(ob + p.qs_off);
+    float *ds = (float *)(ob + p.d_off);
+    int16_t *bsums = (int16_t *)(ob + p.bsum_off);
+    if (p.y_out) {
+        *reinterpret_cast<float4 *>(p.y_out + n * p.ld_y + k0) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(p.y_out + n * p.ld_y + k0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    int q[8];
+    float d;
+    rq_q8k(lane, v, q, d);
     int s8 = 0;
 #pragma unroll
     for (int e = 0; e < 8; e++) s8 += q[e];
@@ -83,9 +89,11 @@ __device__ __forceinline__ void rq_quant_block(const RowQuantArgs &p, int n, int
     uint2 packed;
     packed.x = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
     packed.y = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
-    *reinterpret_cast<uint2 *>(qs + (size_t)n * K + k0) = packed;
-    if ((lane & 1) == 0) bsums[(size_t)n * (K / 16) + sb * 16 + (lane >> 1)] = (int16_t)s16;
-    if (lane == 0) ds[(size_t)n * (K / 256) + sb] = d;
+    if (!p.operand_only) {
+        *reinterpret_cast<uint2 *>(qs + (size_t)n * K + k0) = packed;
+        if ((lane & 1) == 0) bsums[(size_t)n * (K / 16) + sb * 16 + (lane >> 1)] = (int16_t)s16;
+        if (lane == 0) ds[(size_t)n * (K / 256) + sb] = d;
+    }
     if (p.npad == MM_FOLD_NPAD) {
         // operand of the folded-scale prompt GEMM: f16(code x scale) in natural order
         const int64_t kk = (int64_t)sb * 256 + lane * 8;
