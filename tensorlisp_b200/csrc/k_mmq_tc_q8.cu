@@ -598,7 +598,8 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // accumulator once per tile; tiles of at most 128 columns have two, so that the next tile's MMAs do not wait for that.
 //
 // What bounds it: at 256 columns the tensor pipe with the copies of B (1.55 us per 256 elements of K; 2.15 while a whole warp probed
-// the barriers and issued), at narrow tiles the chain of waits per 64 elements of K (1.2 us). So the tile's width is
+// the barriers and issued), at narrow tiles the instructions and waits per step (1.03 us with
+// steps of 128 elements of K, which fit up to 192 columns; 1.2 with 64). So the tile's width is
 // chosen for the number of columns and row tiles at hand (fold_tile): 333 columns as 2 x 256 wasted a third of the MMAs,
 // and 8 row tiles x 2 left 132 SMs idle. Matrices that share the activations are one launch. Measured for 333 columns, Q4_K:
 // gate and up (14336 x 4096) 134 -> 75 us, [4096 x 14336] 100 -> 70, [4096 x 4096] 34 -> 23.
@@ -783,21 +784,23 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t ta
     }
 }
 
-// CT column halves of nw columns per tile, which share the expanded weights. Tensor memory: accumulators [0, 256), or of the halves
-// [0, 192) and [192, 384); behind them eight or four A slots of 64 elements of K.
-template <bool WQ4K, int CT>
+// SHAPE 0: up to 192 columns, one accumulator or (up to 128) two in turn, steps of 128 elements of K; 1: up to 256 columns, steps of 64;
+// 2: two halves of nw columns, which share the expanded weights, accumulators [0, 192) and [192, 384), steps of 64. Behind the
+// accumulators lie four, eight or four A slots of a step each.
+template <bool WQ4K, int SHAPE>
 __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
     using namespace tc;
     using namespace tc8f;
     constexpr int ROWS = tc8::ROWS;
     constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
     constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
+    constexpr int CT = SHAPE == 2 ? 2 : 1, STEP = SHAPE == 0 ? 2 : 1;   // halves; 64s of K in a step
     constexpr uint32_t ACOLS = CT == 1 ? 256 : 2 * HALF_NW;   // first A column
-    constexpr int A_RING = (512 - (int)ACOLS) / 32;
+    constexpr int A_RING = (512 - (int)ACOLS) / (32 * STEP);
     const uint32_t IDESC = (1u << 4) | ((uint32_t)(p.nw >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
-    const int b_stage = p.nw * KS * 2;
+    const int b_half = p.nw * KS * 2, b_stage = b_half * STEP;
     uint8_t *bst = smem;                                   // b_stages x b_stage
     uint8_t *raw = bst + p.b_stages * b_stage;             // raw_stages x RAW_BYTES
     __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[MAX_STAGES], bar_bfree[MAX_STAGES];
@@ -809,7 +812,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nst = p.nst;   // units of 256 elements of K
     const int n_tiles = p.row_tiles * p.col_tiles;
-    const uint32_t accs = CT == 1 && p.nw <= 128 ? 2 : 1;   // accumulators in turn, 128 columns apart
+    const uint32_t accs = SHAPE == 0 && p.nw <= 128 ? 2 : 1;   // accumulators in turn, 128 columns apart
     if (tid == 0) {
         for (int i = 0; i < MAX_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
@@ -818,7 +821,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             mbar_init(&bar_bfree[i], 1);
         }
         for (int i = 0; i < A_RING; i++) {
-            mbar_init(&bar_aready[i], 4);
+            mbar_init(&bar_aready[i], 4 * STEP);
             mbar_init(&bar_afree[i], 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -868,14 +871,16 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
                 int row_tile, col_tile;
                 p.at(t, row_tile, col_tile);
-                for (int i = 0; i < nst * 4; i++)
+                for (int i = 0; i < nst * 4; i += STEP)
 #pragma unroll
                     for (int ct = 0; ct < CT; ct++) {
                         const int g0 = min((col_tile * CT + ct) * (p.nw / 8), p.groups - 1);
                         const uint32_t bytes = (uint32_t)min(p.nw / 8, p.groups - g0) * 1024u;
                         mbar_wait_nap(&bar_bfree[s], ph ^ 1u, fail, 32);
-                        mbar_expect_tx(&bar_b[s], bytes);
-                        bulk_g2s(bst + s * b_stage, p.act + ((size_t)i * p.groups + g0) * 1024, bytes, &bar_b[s]);
+                        mbar_expect_tx(&bar_b[s], bytes * STEP);
+#pragma unroll
+                        for (int k = 0; k < STEP; k++)
+                            bulk_g2s(bst + s * b_stage + k * b_half, p.act + ((size_t)(i + k) * p.groups + g0) * 1024, bytes, &bar_b[s]);
                         if (++s == p.b_stages) {
                             s = 0;
                             ph ^= 1u;
@@ -898,9 +903,9 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                 mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
                 uint32_t more = 0;
 #pragma unroll 1
-                for (int i = nst * 4; i > 0; i--) {
+                for (int i = nst * 4 / STEP; i > 0; i--) {
                     if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
-                    const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * 32u;
+                    const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * (32u * STEP);
                     uint64_t *const afree = &bar_afree[as];
                     if (++as == A_RING) {
                         as = 0;
@@ -920,7 +925,9 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                         }
                         if (ct == CT - 1) a_here = mbar_test(&bar_aready[as], aph);
                         b_here = mbar_test(&bar_b[bs], bph);
-                        umma4_f16_ta(tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ct * HALF_NW)), a0, desc, IDESC, more);
+#pragma unroll
+                        for (int k = 0; k < STEP; k++)
+                            umma4_f16_ta(tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ct * HALF_NW)), a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), IDESC, k ? 1u : more);
                         umma_commit(bfree);
                     }
                     umma_commit(afree);
@@ -937,14 +944,14 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         const int q = warp & 3, j = (warp - tc8f::DEQ_WARP0) >> 2;
         const int r = q * 32 + lane;
         const uint32_t a_lane = tmem_base + ACOLS + ((uint32_t)(q * 32) << 16);
-        int s = 0, as = j;
+        int s = 0, as = j / STEP;
         uint32_t ph = 0, aph = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x)
             for (int i = 0; i < nst; i++) {
                 mbar_wait_nap(&bar_raw[s], ph, fail, 64);
                 mbar_wait_nap(&bar_afree[as], aph ^ 1u, fail, 64);   // the MMAs that read this slot are done
                 tc_fence_after();
-                expand64<WQ4K>(raw + s * RAW_BYTES + r * ROW_CHUNK, j, a_lane + (uint32_t)as * 32u);
+                expand64<WQ4K>(raw + s * RAW_BYTES + r * ROW_CHUNK, j, a_lane + (uint32_t)as * (32u * STEP) + (uint32_t)(j % STEP) * 32u);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
@@ -952,7 +959,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                     mbar_arrive(&bar_aready[as]);
                     mbar_arrive(&bar_rawfree[s]);
                 }
-                as += 4;
+                as += 4 / STEP;
                 if (as >= A_RING) {
                     as -= A_RING;
                     aph ^= 1u;
@@ -1015,7 +1022,7 @@ struct FoldTile {
     int halves, nw;
 };
 // Halves of a tile and columns of each (a multiple of 16): of the even splits of N, the one whose slowest SM has the least to do.
-// Measured per unit of K: 1.2 us at 64 columns, 1.3 at 128, 1.55 at 256; in halves 1.75 at 192 and 2.4 at 384, which pays where it
+// Measured per unit of K: 1.03 us at 64 columns, 1.24 at 128, 1.3 at 192, 1.55 at 256; in halves 1.75 at 192 and 2.4 at 384, which pays where it
 // saves a wave (224 row tiles x 333 columns). Draining a tile without a second accumulator is about 1.2 us.
 static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
     FoldTile f{1, 0};
@@ -1025,7 +1032,7 @@ static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
         for (int64_t ct = (N + widest - 1) / widest, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
             const int nw = (int)(((N + ct * halves - 1) / (ct * halves) + 15) / 16 * 16);
             const int64_t tiles = (int64_t)row_tiles * ((N + halves * nw - 1) / (halves * nw)), waves = (tiles + sms - 1) / sms;
-            const double unit = halves == 1 ? std::max(1.2, 1.07 + 0.00185 * nw) : std::max(1.75, 0.65 + 0.0046 * 2 * nw);
+            const double unit = halves == 2 ? std::max(1.75, 0.65 + 0.0046 * 2 * nw) : (nw <= 192 ? std::max(1.03, 0.88 + 0.0025 * nw) : 1.07 + 0.00185 * nw);
             const double t = (double)waves * (nst * unit + (halves == 1 && nw <= 128 ? 0.3 : 1.2));
             if (f.nw == 0 || t < best * 0.98) {
                 best = t;
@@ -1067,8 +1074,9 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.nw = tile.nw;
     // raw stages: 128 rows x 256 elements (18 or 34 KB); what they leave goes to B
     const int raw_bytes = tc8::ROWS * (q4k ? 144 : tc8::ROW_CHUNK);
-    p.raw_stages = q4k ? 4 : (tile.halves == 1 && p.nw <= 192 ? 3 : 2);
-    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * 2));
+    p.raw_stages = q4k ? 4 : (tile.halves == 1 && p.nw <= 128 ? 3 : 2);
+    const bool narrow = tile.halves == 1 && p.nw <= 192;
+    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * (narrow ? 4 : 2)));
     if (p.b_stages < 2) return cudaErrorInvalidValue;
     p.groups = mm_fold_groups(N);
     p.col_tiles = (int)((N + tile.halves * p.nw - 1) / (tile.halves * p.nw));
@@ -1076,6 +1084,7 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sm_of[dev]));
     auto go = [&](auto *k) { return launch_pdl(k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
     if (tile.halves == 2) return q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
+    if (narrow) return q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);
     return q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
 }
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st) {
@@ -1100,6 +1109,8 @@ void mmq_tc8_configure() {
     cudaFuncSetAttribute(k_mmq_tc_q80<32, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<32, 4, 4>());
     cudaFuncSetAttribute(k_mmq_tc_q80_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
     auto fold = [](auto *k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc8f::SMEM); };
+    fold(k_mm_q80_f16<false, 0>);
+    fold(k_mm_q80_f16<true, 0>);
     fold(k_mm_q80_f16<false, 1>);
     fold(k_mm_q80_f16<true, 1>);
     fold(k_mm_q80_f16<false, 2>);
