@@ -328,6 +328,7 @@ cudaError_t copy_d2h(int ordinal, void *dst, const void *src, uint64_t n, cudaSt
     // half the ring is on the link while the other half is copied out
     const int wave = RING_SLOTS / 2;
     auto issue = [&](int w) {
+        r.next = base + std::min(chunks, (w + 1) * wave);   // behind an error no further wave is sent: the numbers of its chunks stay free
         for (int c = w * wave; c < std::min(chunks, (w + 1) * wave); c++) {
             const uint64_t k = base + c;
             const int s = (int)(k % RING_SLOTS);
@@ -354,7 +355,6 @@ cudaError_t copy_d2h(int ordinal, void *dst, const void *src, uint64_t n, cudaSt
             stream_copy((char *)dst + off, r.mem + s * RING_CHUNK, std::min(chunk, n - off));
         });
     }
-    r.next = base + chunks;
     const cudaError_t e = cudaStreamSynchronize(st);   // also behind an error: nothing writes the ring any more
     return err != cudaSuccess ? (cudaError_t)err.load() : e;
 }

@@ -1,0 +1,97 @@
+// The staged copies of csrc/hostio.cu against a CUDA runtime that fails on demand: the linker sends the calls below here
+// (--wrap), device memory is ordinary memory, and copies happen at once. One scenario per run, named on the command line;
+// exit code 0 means that it held.
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "hostio.h"
+
+namespace {
+constexpr int ORDINAL = 3;
+std::atomic<int> copies{0}, waits{0}, fail_copy{-1}, fail_wait{-1}, stray{0};
+thread_local int device = 0;
+void on_device() {
+    if (device != ORDINAL) stray++;
+}
+}  // namespace
+
+extern "C" {
+cudaError_t __wrap_cudaSetDevice(int d) {
+    device = d;
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaHostAlloc(void **p, size_t n, unsigned) {
+    *p = std::aligned_alloc(4096, (n + 4095) / 4096 * 4096);
+    return *p ? cudaSuccess : cudaErrorMemoryAllocation;
+}
+cudaError_t __wrap_cudaFreeHost(void *p) {
+    std::free(p);
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
+    std::memset(a, 0, sizeof(*a));
+    a->type = cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaGetLastError() { return cudaSuccess; }
+cudaError_t __wrap_cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    *e = (cudaEvent_t)1;
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaEventRecord(cudaEvent_t, cudaStream_t) {
+    on_device();
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaEventSynchronize(cudaEvent_t) {
+    on_device();
+    return waits++ == fail_wait ? cudaErrorUnknown : cudaSuccess;
+}
+cudaError_t __wrap_cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    on_device();
+    if (copies++ == fail_copy) return cudaErrorUnknown;
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t __wrap_cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+}
+
+#define HOLDS(x)                                      \
+    do {                                              \
+        if (!(x)) {                                   \
+            std::printf("does not hold: %s\n", #x);   \
+            return 1;                                 \
+        }                                             \
+    } while (0)
+
+int main(int argc, char **argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    const size_t n = (40u << 20) + 12345;   // 41 chunks, six half rings
+    std::vector<char> host(n), dev(n), back(n);
+    for (size_t i = 0; i < n; i++) host[i] = (char)(i * 2654435761u >> 13);
+    cudaSetDevice(ORDINAL);
+    auto up = [&] { return tlb::copy_h2d(ORDINAL, dev.data(), host.data(), n, nullptr); };
+    auto down = [&] {
+        std::memset(back.data(), 0, n);
+        return tlb::copy_d2h(ORDINAL, back.data(), dev.data(), n, nullptr);
+    };
+    auto same = [&] { return std::memcmp(host.data(), dev.data(), n) == 0 && std::memcmp(host.data(), back.data(), n) == 0; };
+    HOLDS(up() == cudaSuccess && down() == cudaSuccess && same());
+    if (what == "device") {   // every call is made for the copy's device, on whichever thread
+        for (int i = 0; i < 20; i++) HOLDS(up() == cudaSuccess && down() == cudaSuccess);
+        HOLDS(stray == 0);
+        return 0;
+    }
+    // a failing call is reported, and the copies after it are whole again
+    const int at = argc > 2 ? std::atoi(argv[2]) : 0;
+    const bool upload = what == "h2d_copy" || what == "h2d_wait", copy = what == "h2d_copy" || what == "d2h_copy";
+    (copy ? fail_copy : fail_wait) = (copy ? copies : waits) + at;
+    HOLDS((upload ? up() : down()) == cudaErrorUnknown);
+    fail_copy = fail_wait = -1;
+    std::memset(dev.data(), 0, n);
+    for (int i = 0; i < 3; i++) HOLDS(up() == cudaSuccess && down() == cudaSuccess && same());
+    return 0;
+}
