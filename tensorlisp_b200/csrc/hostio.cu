@@ -283,18 +283,19 @@ cudaError_t copy_h2d(int ordinal, void *dst, const void *src, uint64_t n, cudaSt
     const uint64_t base = r.next;
     std::atomic<int> err{cudaSuccess};
     host_parallel(chunks, threads_of(n), [&](int c) {
+        cudaError_t e = cudaSetDevice(ordinal);   // a helper thread begins with device 0
+        if (e != cudaSuccess) err = e;
         const uint64_t k = base + c;
         const int s = (int)(k % RING_SLOTS);
         if (k >= RING_SLOTS) {   // the chunk that used the slot before: enqueued (perhaps by another thread), then read by the link
             while (r.issued[s].load(std::memory_order_acquire) < k - RING_SLOTS + 1) std::this_thread::yield();
-            const cudaError_t e = cudaEventSynchronize(r.ev[s]);
+            e = cudaEventSynchronize(r.ev[s]);
             if (e != cudaSuccess) err = e;
         }
         const uint64_t off = (uint64_t)c * chunk, m = std::min(chunk, n - off);
         char *slot = r.mem + s * RING_CHUNK;
         stream_copy(slot, (const char *)src + off, m);
-        cudaError_t e = cudaSetDevice(ordinal);
-        if (e == cudaSuccess) e = cudaMemcpyAsync((char *)dst + off, slot, m, cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync((char *)dst + off, slot, m, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(r.ev[s], st);
         if (e != cudaSuccess) err = e;
         r.issued[s].store(k + 1, std::memory_order_release);
@@ -346,7 +347,8 @@ cudaError_t copy_d2h(int ordinal, void *dst, const void *src, uint64_t n, cudaSt
         const int c0 = w * wave, c1 = std::min(chunks, (w + 1) * wave);
         host_parallel(c1 - c0, threads_of(n), [&](int i) {
             const int c = c0 + i, s = (int)((base + c) % RING_SLOTS);
-            const cudaError_t e = cudaEventSynchronize(r.ev[s]);
+            cudaError_t e = cudaSetDevice(ordinal);
+            if (e == cudaSuccess) e = cudaEventSynchronize(r.ev[s]);
             if (e != cudaSuccess) {
                 err = e;
                 return;

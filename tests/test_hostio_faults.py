@@ -29,3 +29,9 @@ def program(tmp_path_factory):
 def test_an_error_is_reported_and_the_ring_goes_on(program, what, at):
     r = subprocess.run([str(program), what, str(at)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("what", ["device_up", "device_down"])
+def test_helper_threads_call_for_the_device_of_the_copy(program, what):
+    r = subprocess.run([str(program), what], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
