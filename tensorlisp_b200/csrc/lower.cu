@@ -1162,6 +1162,32 @@ void lower_node(const LowerCtx &c, int32_t id, int pos, std::vector<Dispatch> &o
 }
 
 // ---------------------------------------------------------------------------- IR rewrites
+// Whether a node writes to the storage of `root`: its own tensor, or what cache writes and the fused nodes below write besides it.
+static bool writes_root(const Graph &g, int32_t id, int32_t root) {
+    const Tensor &t = g.tensors[id];
+    auto same = [&](int32_t a) {
+        if (a < 0) return false;
+        a = g.root(a);
+        // leaves of one kind may lie on the same bytes (two tensors of one state, states that the caller laid out to overlap)
+        return a == root || (g.tensors[a].storage_kind != TEMP && g.tensors[a].storage_kind == g.tensors[root].storage_kind);
+    };
+    if (t.is_view_op()) return false;
+    if (same(id)) return true;
+    const auto &s = t.src;
+    if (t.op == "CUSTOM") return paged_ud(t).kind == 2 ? same(s[2]) || same(s[3]) : same(s[9]);
+    if (t.op == "ROPE_KV_WRITE") return same(s[5]) || same(s[6]) || same(s[8]);
+    if (t.op == "ROPE_KV_PROMPT") return same(s[4]) || same(s[5]) || same(s[6]) || same(s[8]) || same(s[9]);
+    if (t.op == "ROW_QUANT") return same(s[4]);
+    if (t.op == "MUL_MAT_GROUP") return same(s[4]) || same(s[6]) || same(s[9]);
+    return t.op == "MUL_MAT" && same(s[9]);
+}
+// Whether a node at a position in (after, before) writes to the storage of `id`: a read of it must not move across.
+static bool written_between(const Graph &g, const std::vector<char> &dead, int32_t id, int after, int before) {
+    if (id < 0) return false;
+    for (int i = after + 1; i < before; i++)
+        if (!dead[i] && writes_root(g, g.nodes[i], g.root(id))) return true;
+    return false;
+}
 void fuse_row_producers(Graph &g);
 void fuse_rope_cache(Graph &g);
 void fuse_mul_mat_groups(Graph &g);
@@ -1206,7 +1232,9 @@ void rewrite_graph(Graph &g) {
             if (!same || tw.ne[0] == 0 || n.ne[0] % tw.ne[0] != 0) continue;
             bool bc = true;
             for (int k = 1; k < 4; k++) bc = bc && tw.ne[k] != 0 && t.ne[k] % tw.ne[k] == 0;
-            if (!bc || n.src[0] < 0 || g.tensors[n.src[0]].nb[0] != 4) continue;
+            if (!bc || n.src[0] < 0 || g.tensors[n.src[0]].nb[0] != 4 || written_between(g, dead, n.src[0], pos_of[a], (int)i) ||
+                written_between(g, dead, a, pos_of[a], (int)i))
+                continue;
             t.op = "RMS_NORM_MUL";
             t.op_params[15] = n.op_params[0];  // eps moves to slot 15
             t.src[0] = n.src[0];
@@ -1235,7 +1263,7 @@ void rewrite_graph(Graph &g) {
             if (t.ty != 0 || tg.ty != 0 || tu.ty != 0 || !t.is_contiguous() || !tg.is_contiguous() || !tu.is_contiguous()) continue;
             bool same = true;
             for (int k = 0; k < 4; k++) same = same && t.ne[k] == tg.ne[k] && t.ne[k] == tu.ne[k];
-            if (!same) continue;
+            if (!same || written_between(g, dead, gsrc, pos_of[a], (int)i) || written_between(g, dead, a, pos_of[a], (int)i)) continue;
             t.op = "GLU";
             for (int k = 0; k < 16; k++) t.op_params[k] = 0;
             t.op_params[0] = glu;
@@ -1255,9 +1283,8 @@ void rewrite_graph(Graph &g) {
         const int32_t id = g.nodes[i];
         {
             // a node that writes into storage an activation lives in invalidates its quantized copy
-            const int32_t root = g.root(id);
             for (auto it = cache.begin(); it != cache.end();) {
-                if (g.root(it->first.first) == root && !g.tensors[id].is_view_op()) it = cache.erase(it);
+                if (writes_root(g, id, g.root(it->first.first))) it = cache.erase(it);
                 else ++it;
             }
         }
@@ -1409,6 +1436,9 @@ void fuse_row_producers(Graph &g) {
         // (a cast lists itself as src[1], ggml.c:3549-3563, so the producer shows up as its own reader)
         for (int r : rd) only_q = only_q && (r == (int)qi || r == xp || g.tensors[g.nodes[r]].is_view_op());
         if (!only_q) continue;
+        // the producer's sources are read here from now on, and nothing adds to its result in place
+        auto moves = [&](int32_t s, int from) { return !written_between(g, dead, s, from, (int)qi); };
+        if (!moves(x, xp) || !moves(P.src[0], xp) || ((P.op == "RMS_NORM_MUL" || P.op == "GLU") && !moves(P.src[1], xp))) continue;
         Tensor &Q = g.tensors[qid];
         if (P.op == "RMS_NORM_MUL" && xroot == x) {
             const int32_t a = P.src[0], w = P.src[1];
@@ -1434,6 +1464,7 @@ void fuse_row_producers(Graph &g) {
                 // nobody may read the sum between the ADD's old position and the fused node
                 readers(aroot, rd);
                 for (int r : rd) ok = ok && (r >= (int)qi || r == xp);
+                ok = ok && moves(a, ap) && moves(s0, ap) && moves(s1, ap);
                 if (ok) {
                     Q.src[0] = s0;
                     Q.src[1] = s1;
@@ -1507,17 +1538,13 @@ void fuse_rope_cache(Graph &g) {
         for (int i = a + 1; i < b; i++) {
             const Tensor &t = g.tensors[g.nodes[i]];
             if (dead[i] || t.is_view_op()) continue;
-            if (g.root(g.nodes[i]) == root) return true;
+            if (writes_root(g, g.nodes[i], root)) return true;
             for (int s = 0; s < 10; s++)
                 if (t.src[s] >= 0 && g.root(t.src[s]) == root) return true;
         }
         return false;
     };
-    auto written = [&](int32_t root, int a, int b) {
-        for (int i = a + 1; i < b; i++)
-            if (!dead[i] && !g.tensors[g.nodes[i]].is_view_op() && g.root(g.nodes[i]) == root) return true;
-        return false;
-    };
+    auto written = [&](int32_t id, int a, int b) { return written_between(g, dead, id, a, b); };
     auto fuse_rope_prompt = [&](size_t ci, int32_t k16, int32_t v16, int32_t rk, int32_t vsrc) {
         Tensor &Cw = g.tensors[g.nodes[ci]];
         const PagedUd u = paged_ud(Cw);
@@ -1598,6 +1625,12 @@ void fuse_rope_cache(Graph &g) {
              n_readers(v16, pos_of[v16]) == 1 && n_readers(q16, pos_of[q16]) == 1;
         // the folded nodes all sit before the attention; the fused node takes the cache write's place
         ok = ok && pos_of[rq] < (int)ci && pos_of[rk] < (int)ci && pos_of[k16] < (int)ci && pos_of[v16] < (int)ci && pos_of[q16] < ai;
+        // what they read still holds its values there, and their results are what the attention and the cache write got
+        const int at = (int)ci;
+        ok = ok && !written(RQ.src[0], pos_of[rq], at) && !written(RK.src[0], pos_of[rk], at) && !written(vsrc, pos_of[v16], at) &&
+             !written(RQ.src[1], std::min(pos_of[rq], pos_of[rk]), at) && !written(RQ.src[2], std::min(pos_of[rq], pos_of[rk]), at) &&
+             !written(rq, pos_of[rq], ai) && !written(rk, pos_of[rk], at) && !written(k16, pos_of[k16], at) && !written(v16, pos_of[v16], at) &&
+             !written(q16, pos_of[q16], ai);
         if (!ok) continue;
         const int32_t pools[2] = {Cw.src[2], Cw.src[3]};
         const int32_t slots = Cw.src[4];
@@ -1689,6 +1722,12 @@ void fuse_gemv(Graph &g, bool groups, bool producers) {
             if (!dead[k] && g.nodes[k] == xroot) xp = (int)k;
         bool only = self && xp >= 0 && !kept[xroot] && g.tensors[xroot].view_src < 0 && W0.ty != TLB_TYPE_Q6_K;
         for (int r : rd) only = only && (r == (int)i || r == xp);   // (a cast lists itself as a source)
+        // the producer's sources are read here from now on, and nothing adds to its result in place
+        auto moves = [&](int32_t s, int from) { return !written_between(g, dead, s, from, (int)i); };
+        if (only) {
+            const Tensor &P = g.tensors[xroot];
+            only = moves(x, xp) && moves(P.src[0], xp) && ((P.op != "RMS_NORM_MUL" && P.op != "GLU") || moves(P.src[1], xp));
+        }
         if (only) {
             const Tensor P = g.tensors[xroot];
             if (P.op == "RMS_NORM_MUL" && xroot == x) {
@@ -1710,9 +1749,7 @@ void fuse_gemv(Graph &g, bool groups, bool producers) {
                         for (int k = 0; ok && k < 4; k++) ok = g.tensors[s0].ne[k] == R.ne[k] && g.tensors[s1].ne[k] == R.ne[k];
                         live_readers(a, rd);   // nobody may read the sum between the add's old place and this node
                         for (int r : rd) ok = ok && (r >= (int)i || r == ap);
-                        // the operands keep their values until here: nothing in between writes to them in place
-                        for (int k = ap + 1; ok && k < (int)i; k++)
-                            if (!dead[k] && !g.tensors[g.nodes[k]].is_view_op()) ok = g.root(g.nodes[k]) != g.root(s0) && g.root(g.nodes[k]) != g.root(s1);
+                        ok = ok && moves(a, ap) && moves(s0, ap) && moves(s1, ap);
                         if (ok) {
                             A.src[1] = s0;
                             A.src[7] = s1;
