@@ -701,9 +701,9 @@ cudaError_t launch_gemv(const GemvArgs &g, int sm_count, int *err, cudaStream_t 
             e = tc_encode_2d_bytes(&maps.m[j], g.W[j < g.n_mats ? j : 0], tlb_row_size(g.type, g.K), (uint64_t)g.M[j < g.n_mats ? j : 0], (uint32_t)p.row_stride, 16);
         if (e != cudaSuccess) return e;
         switch (g.type) {
-            case TLB_TYPE_Q4_K: e = nc == 1 ? launch_pdl(k_gemv<TLB_TYPE_Q4_K, true>, grid, block, smem, st, maps, p) : launch_pdl(k_gemv<TLB_TYPE_Q4_K, false>, grid, block, smem, st, maps, p); break;
-            case TLB_TYPE_Q8_0: e = nc == 1 ? launch_pdl(k_gemv<TLB_TYPE_Q8_0, true>, grid, block, smem, st, maps, p) : launch_pdl(k_gemv<TLB_TYPE_Q8_0, false>, grid, block, smem, st, maps, p); break;
-            case TLB_TYPE_Q4_0: e = nc == 1 ? launch_pdl(k_gemv<TLB_TYPE_Q4_0, true>, grid, block, smem, st, maps, p) : launch_pdl(k_gemv<TLB_TYPE_Q4_0, false>, grid, block, smem, st, maps, p); break;
+            case TLB_TYPE_Q4_K: e = nc == 1 ? launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q4_K, true>, grid, block, smem, st, maps, p) : launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q4_K, false>, grid, block, smem, st, maps, p); break;
+            case TLB_TYPE_Q8_0: e = nc == 1 ? launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q8_0, true>, grid, block, smem, st, maps, p) : launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q8_0, false>, grid, block, smem, st, maps, p); break;
+            case TLB_TYPE_Q4_0: e = nc == 1 ? launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q4_0, true>, grid, block, smem, st, maps, p) : launch_pdl_if(g.early, k_gemv<TLB_TYPE_Q4_0, false>, grid, block, smem, st, maps, p); break;
             default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;

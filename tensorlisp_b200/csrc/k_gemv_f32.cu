@@ -373,10 +373,10 @@ cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStrea
         const dim3 grid((unsigned)sm_count), block(gemvf::THREADS);
         cudaError_t e;
         switch (nc) {
-            case 1: e = launch_pdl(k_gemv_f32<1>, grid, block, smem, st, p); break;
-            case 2: e = launch_pdl(k_gemv_f32<2>, grid, block, smem, st, p); break;
-            case 3: e = launch_pdl(k_gemv_f32<3>, grid, block, smem, st, p); break;
-            default: e = launch_pdl(k_gemv_f32<4>, grid, block, smem, st, p); break;
+            case 1: e = launch_pdl_if(g.early, k_gemv_f32<1>, grid, block, smem, st, p); break;
+            case 2: e = launch_pdl_if(g.early, k_gemv_f32<2>, grid, block, smem, st, p); break;
+            case 3: e = launch_pdl_if(g.early, k_gemv_f32<3>, grid, block, smem, st, p); break;
+            default: e = launch_pdl_if(g.early, k_gemv_f32<4>, grid, block, smem, st, p); break;
         }
         if (e != cudaSuccess) return e;
         n0 += nc;

@@ -366,23 +366,23 @@ PlainPlan mm_plain_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
 }
 
 template <bool BF16>
-static cudaError_t launch_plain_pass(const PlainPlan &t, const CUtensorMap &map, PlainParams p, cudaStream_t st) {
+static cudaError_t launch_plain_pass(const PlainPlan &t, const CUtensorMap &map, PlainParams p, cudaStream_t st, bool early) {
     const int nc = p.N <= 8 ? 8 : (p.N <= 16 ? 16 : (p.N <= 24 ? 24 : (p.N <= 48 ? 48 : 80)));
     const int b_bytes = 2 * plain::chunk_steps(nc) * p.n_mma * plain::KS * 2;
     p.stages = std::min(plain::MAX_STAGES, (plain::SMEM - b_bytes) / plain::A_STAGE);
     const size_t smem = (size_t)b_bytes + (size_t)p.stages * plain::A_STAGE + 1024;
     const dim3 grid((unsigned)t.ctas), block(plain::THREADS);
     switch (nc) {
-        case 8: return launch_pdl(k_mm_plain<BF16, 8>, grid, block, smem, st, map, p);
-        case 16: return launch_pdl(k_mm_plain<BF16, 16>, grid, block, smem, st, map, p);
-        case 24: return launch_pdl(k_mm_plain<BF16, 24>, grid, block, smem, st, map, p);
-        case 48: return launch_pdl(k_mm_plain<BF16, 48>, grid, block, smem, st, map, p);
-        default: return launch_pdl(k_mm_plain<BF16, 80>, grid, block, smem, st, map, p);
+        case 8: return launch_pdl_if(early, k_mm_plain<BF16, 8>, grid, block, smem, st, map, p);
+        case 16: return launch_pdl_if(early, k_mm_plain<BF16, 16>, grid, block, smem, st, map, p);
+        case 24: return launch_pdl_if(early, k_mm_plain<BF16, 24>, grid, block, smem, st, map, p);
+        case 48: return launch_pdl_if(early, k_mm_plain<BF16, 48>, grid, block, smem, st, map, p);
+        default: return launch_pdl_if(early, k_mm_plain<BF16, 80>, grid, block, smem, st, map, p);
     }
 }
 
 cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64_t w_row_bytes, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx, float *y, int64_t ldy,
-                            void *scratch, int *err, cudaStream_t st) {
+                            void *scratch, int *err, cudaStream_t st, bool early) {
     CUtensorMap map;
     cudaError_t e = tc_encode_2d_sw128(&map, W, w_row_bytes, (uint64_t)K, (uint64_t)M, plain::KB, tc::ROWS, bf16);
     for (int pass = 0; pass < t.passes && e == cudaSuccess; pass++) {
@@ -404,7 +404,7 @@ cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64
         p.tiles = t.tiles;
         p.idesc = (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(p.n_mma >> 3) << 17) | ((uint32_t)(tc::ROWS >> 4) << 24);
         p.err = err;
-        e = bf16 ? launch_plain_pass<true>(t, map, p, st) : launch_plain_pass<false>(t, map, p, st);
+        e = bf16 ? launch_plain_pass<true>(t, map, p, st, early) : launch_plain_pass<false>(t, map, p, st, early);
         if (e == cudaSuccess && t.tiles % t.ctas != 0)
             e = launch_pdl(k_mm_plain_fixup, dim3((unsigned)t.tiles, (unsigned)((n * tc::ROWS + 255) / 256)), dim3(256), 0, st, (const float *)p.partial, p.out, M, ldy, n, t.steps, t.tiles,
                            t.ctas);

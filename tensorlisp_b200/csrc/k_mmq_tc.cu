@@ -742,9 +742,9 @@ cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsi
 
 // n_mats weight matrices [M[j] x K] sharing the activations; y[j] dense [N][M[j]] when n_mats > 1 or K is split
 cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs,
-                                float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool leave_partial) {
+                                float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool early, bool leave_partial) {
     if (t.npad == MM_FOLD_NPAD) {
-        return launch_mm_fold_f16(true, n_mats, W, K, M, N, blobs, y, ldy, err, st);
+        return launch_mm_fold_f16(true, n_mats, W, K, M, N, blobs, y, ldy, err, st, early);
     }
     if (n_mats < 1 || n_mats > TC_MAX_MATS || (n_mats > 1 && t.n_col_chunks != 1)) return cudaErrorInvalidValue;
     if (t.n_split > 16) return cudaErrorInvalidValue;
@@ -795,9 +795,9 @@ cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *
             }
         }
         switch (t.npad) {
-            case 16: e = launch_pdl(k_mmq_tc_q4k<16, 6, 4>, grid, dim3(Q4K_THREADS), tc_smem<16, 6, 4>(), st, maps, p); break;
-            case 32: e = launch_pdl(k_mmq_tc_q4k<32, 6, 4>, grid, dim3(Q4K_THREADS), tc_smem<32, 6, 4>(), st, maps, p); break;
-            default: e = launch_pdl(k_mmq_tc_q4k<64, 5, 2>, grid, dim3(Q4K_THREADS), tc_smem<64, 5, 2>(), st, maps, p); break;
+            case 16: e = launch_pdl_if(early, k_mmq_tc_q4k<16, 6, 4>, grid, dim3(Q4K_THREADS), tc_smem<16, 6, 4>(), st, maps, p); break;
+            case 32: e = launch_pdl_if(early, k_mmq_tc_q4k<32, 6, 4>, grid, dim3(Q4K_THREADS), tc_smem<32, 6, 4>(), st, maps, p); break;
+            default: e = launch_pdl_if(early, k_mmq_tc_q4k<64, 5, 2>, grid, dim3(Q4K_THREADS), tc_smem<64, 5, 2>(), st, maps, p); break;
         }
         if (e != cudaSuccess) return e;
         if (t.streamk) {
@@ -828,10 +828,10 @@ cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *
 }
 
 cudaError_t launch_mmq_tc(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
-                          int64_t ldy, void *partial, int *err, cudaStream_t st, bool leave_partial) {
+                          int64_t ldy, void *partial, int *err, cudaStream_t st, bool early, bool leave_partial) {
     const void *Ws[1] = {W};
     float *ys[1] = {y};
-    return launch_mmq_tc_group(t, 1, Ws, K, &M, N, blobs, ys, ldy, partial, err, st, leave_partial);
+    return launch_mmq_tc_group(t, 1, Ws, K, &M, N, blobs, ys, ldy, partial, err, st, early, leave_partial);
 }
 
 }  // namespace tlb

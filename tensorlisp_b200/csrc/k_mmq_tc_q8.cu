@@ -1044,7 +1044,7 @@ static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
     return f;
 }
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
-                               int64_t ldy, int *err, cudaStream_t st) {
+                               int64_t ldy, int *err, cudaStream_t st, bool early) {
     if (n_mats < 1 || n_mats > tc8f::MAX_MATS) return cudaErrorInvalidValue;
     static int sm_of[64] = {0};
     int dev = 0;
@@ -1082,7 +1082,7 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.col_tiles = (int)((N + tile.halves * p.nw - 1) / (tile.halves * p.nw));
     p.err = err;
     const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sm_of[dev]));
-    auto go = [&](auto *k) { return launch_pdl(k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
+    auto go = [&](auto *k) { return launch_pdl_if(early, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
     if (tile.halves == 2) return q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
     if (narrow) return q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);
     return q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
@@ -1190,12 +1190,12 @@ cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes,
 void launch_mmq_reduce(const float *partial, float *y, int64_t total, int n_split, cudaStream_t st);
 
 cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y, int64_t ldy,
-                           void *partial, int *err, cudaStream_t st) {
+                           void *partial, int *err, cudaStream_t st, bool early) {
     CUtensorMap map;
     // described in 16-bit elements: a 272-byte box is 136 of them (the limit is 256 elements per dimension)
     cudaError_t e = tc_encode_2d(&map, W, (uint64_t)(K / 32 * 34), (uint64_t)M, tc8::ROW_CHUNK, tc8::ROWS, 2);
     if (e != cudaSuccess) return e;
-    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, err, st);
+    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, err, st, early);
     if (t.npad == tc8w::NW) {
         Tc8Params p{};
         p.act = (const uint8_t *)blobs;
@@ -1207,7 +1207,7 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
         p.n_split = 1;
         p.ldy = ldy;
         p.err = err;
-        return launch_pdl(k_mmq_tc_q80_wide, dim3((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_col_chunks), dim3(tc8w::THREADS),
+        return launch_pdl_if(early, k_mmq_tc_q80_wide, dim3((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_col_chunks), dim3(tc8w::THREADS),
                           tc8w_smem(), st, map, p);
     }
     dim3 grid((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_split);
@@ -1230,8 +1230,8 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
             p.out = yc;
             p.ldy = ldy;
         }
-        if (t.npad == 16) e = launch_pdl(k_mmq_tc_q80<16, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<16, 4, 4>(), st, map, p);
-        else e = launch_pdl(k_mmq_tc_q80<32, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<32, 4, 4>(), st, map, p);
+        if (t.npad == 16) e = launch_pdl_if(early, k_mmq_tc_q80<16, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<16, 4, 4>(), st, map, p);
+        else e = launch_pdl_if(early, k_mmq_tc_q80<32, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<32, 4, 4>(), st, map, p);
         if (e != cudaSuccess) return e;
         if (t.n_split > 1) {
             if (ldy != M) return cudaErrorInvalidValue;

@@ -54,12 +54,13 @@ struct TcPlan {
 bool mmq_tc_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 TcPlan mmq_tc_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_act_pack_tc(const ActLayout &a, const void *act, int npad, void *blobs, cudaStream_t st);
+// early (here and below): the weights may be copied while the kernel in front is still running (weights_settled, lower.cu).
 // leave_partial: with a K split, do not add the partial sums [split][N][M] up (the caller's next kernel does)
 cudaError_t launch_mmq_tc(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
-                          int64_t ldy, void *partial, int *err, cudaStream_t st, bool leave_partial = false);
+                          int64_t ldy, void *partial, int *err, cudaStream_t st, bool early, bool leave_partial = false);
 // up to 3 matrices [M[j] x K] that share the activations in one launch; outputs dense [N][M[j]]
 cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs,
-                                float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool leave_partial = false);
+                                float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool early, bool leave_partial = false);
 void mmq_tc_configure();
 bool tc_available();
 cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsigned long long *ns, cudaStream_t st);   // the driver offers cuTensorMapEncodeTiled
@@ -70,7 +71,7 @@ bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N);
 TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_act_pack_tc8(const ActLayout &a, const void *act, int npad, void *blobs, cudaStream_t st);
 cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
-                           int64_t ldy, void *partial, int *err, cudaStream_t st);
+                           int64_t ldy, void *partial, int *err, cudaStream_t st, bool early);
 void mmq_tc8_configure();
 // the folded-scale prompt GEMM (k_mm_q80_f16) for Q8_0 or Q4_K weights; its activation operand is f16(code x scale), laid out by
 // stages of 64 elements of K, in a stage by groups of eight columns of 1 KB each (any run of groups is a column tile)
@@ -82,7 +83,7 @@ inline __host__ __device__ size_t mm_fold_at(int n, int64_t k, int groups) {   /
 inline uint64_t mm_fold_bytes(int64_t K, int64_t N) { return (uint64_t)(K / 64) * mm_fold_groups(N) * 1024; }
 // n_mats matrices of one type that share the activations (y[j]: [column][M[j]]; of a single one [column][ldy])
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
-                               int64_t ldy, int *err, cudaStream_t st);
+                               int64_t ldy, int *err, cudaStream_t st, bool early);
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_mm_plain.cu
@@ -95,7 +96,7 @@ struct PlainPlan {
 bool mm_plain_supported(uint32_t type, int64_t K, int64_t M, int64_t N, uint64_t w_row_bytes);
 PlainPlan mm_plain_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64_t w_row_bytes, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx,
-                            float *y, int64_t ldy, void *scratch, int *err, cudaStream_t st);
+                            float *y, int64_t ldy, void *scratch, int *err, cudaStream_t st, bool early);
 void mm_plain_configure();
 
 // ---------------------------------------------------------------- k_fused.cu
@@ -139,6 +140,7 @@ struct GemvArgs {
     int64_t K, N;
     RowQuantArgs act;
     const void *ready;
+    bool early;                  // the weights may be copied while the kernel in front is still running
 };
 bool gemv_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 cudaError_t launch_gemv(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);

@@ -10,7 +10,19 @@
 
 namespace tlb {
 
+static bool writes_root(const Graph &g, int32_t id, int32_t root);
+
 namespace {
+
+// Whether the weights of a product may be copied while the kernel in front of it is still running: a weight leaf that no node of the
+// program writes to. (The kernel in front may be the one that makes any other operand: most release their dependents at their first line.)
+bool weights_settled(const Graph &g, int32_t w) {
+    w = g.root(w);
+    if (g.tensors[w].storage_kind != WEIGHT) return false;
+    for (int32_t id : g.nodes)
+        if (writes_root(g, id, w)) return false;
+    return true;
+}
 
 [[noreturn]] void unsupported(const Tensor &t, const std::string &why) { throw Unsupported{t.op, t.name, why}; }
 
@@ -437,6 +449,7 @@ void lower_mul_mat(L &l) {
     const Place pw = l.place(w), px = l.place(x), pd = l.place(l.id);
     const int64_t K = tw.ne[0], M = tw.ne[1], N = tx.ne[1];
     const int sm = l.c.dev->prop.multiProcessorCount;
+    const bool early = weights_settled(*l.c.g, w);
     MMGeneric g{};
     g.wtype = tw.ty;
     g.w = view_of(tw);
@@ -456,7 +469,7 @@ void lower_mul_mat(L &l) {
         const int64_t ldx = N > 1 ? (int64_t)tx.nb[1] / 4 : K;
         l.push([=](const RunCtx &r) {
             if (((uintptr_t)r.at(pw) | (uintptr_t)r.at(px)) & 15) return launch_mm_generic(g, r.at(pw), r.at(px), r.at(pd), r.stream);   // a state block laid out by the caller
-            return launch_mm_plain(pp, bf16, r.at(pw), wrow, K, M, N, (const float *)r.at(px), ldx, (float *)r.at(pd), M, r.at(ps), r.err, r.stream);
+            return launch_mm_plain(pp, bf16, r.at(pw), wrow, K, M, N, (const float *)r.at(px), ldx, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early);
         });
         return;
     }
@@ -490,8 +503,8 @@ void lower_mul_mat(L &l) {
         const size_t n_out = (size_t)(N * M);
         l.push([=](const RunCtx &r) {
             const bool leave = ar_next && comm_p2p_takes(dev, n_out);
-            return q8 ? launch_mmq_tc8(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream)
-                      : launch_mmq_tc(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, leave);
+            return q8 ? launch_mmq_tc8(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early)
+                      : launch_mmq_tc(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early, leave);
         });
         return;
     }
@@ -514,11 +527,13 @@ void lower_gemv(L &l) {
     p.K = tw0.ne[0];
     p.N = t.ne[1];
     p.glu = t.op_params[GEMV_GLU];
+    p.early = true;
     Place pw[3], py[3];
     const int wslot[3] = {0, 3, 5}, yslot[3] = {-1, 4, 6};
     for (int j = 0; j < 3 && t.src[wslot[j]] >= 0; j++) {
         const int32_t y = j == 0 || p.glu ? l.id : l.src(yslot[j]);
         pw[j] = l.place(t.src[wslot[j]]);
+        p.early = p.early && weights_settled(*l.c.g, t.src[wslot[j]]);
         py[j] = l.place(y);
         p.M[j] = p.ldy[j] = l.T(t.src[wslot[j]]).ne[1];
         p.n_mats++;
@@ -572,6 +587,7 @@ void lower_mul_mat_group(L &l) {
     int n_mats = 0;
     Place pw[3], py[3];
     int64_t Ms[3] = {0, 0, 0}, Msum = 0;
+    bool early = true;
     const int wslot[3] = {0, 3, 5}, yslot[3] = {-1, 4, 6};
     for (int j = 0; j < 3; j++) {
         if (t.src[wslot[j]] < 0) break;
@@ -580,6 +596,7 @@ void lower_mul_mat_group(L &l) {
         if (tw.ty != wty || tw.ne[0] != K || tw.nb[1] != tw.row_size() || ty.ty != TLB_TYPE_F32 || !ty.is_contiguous() ||
             ty.ne[0] != tw.ne[1] || ty.ne[1] != N)
             throw std::string("a grouped mul_mat lost its shape invariants");
+        early = early && weights_settled(*l.c.g, w);
         pw[j] = l.place(w);
         py[j] = l.place(y);
         Ms[j] = tw.ne[1];
@@ -604,8 +621,8 @@ void lower_mul_mat_group(L &l) {
             W[j] = r.at(pw[j]);
             Y[j] = (float *)r.at(py[j]);
         }
-        if (wty == TLB_TYPE_Q8_0) return launch_mm_fold_f16(false, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.err, r.stream);
-        return launch_mmq_tc_group(tp, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.at(ps), r.err, r.stream);
+        if (wty == TLB_TYPE_Q8_0) return launch_mm_fold_f16(false, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.err, r.stream, early);
+        return launch_mmq_tc_group(tp, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.at(ps), r.err, r.stream, early);
     });
 }
 

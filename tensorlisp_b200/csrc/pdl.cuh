@@ -4,7 +4,8 @@
 // an earlier kernel wrote or writes anything an earlier kernel may still read. griddep_launch() at
 // its top lets the kernel after it do the same. Kernels launched the ordinary way keep the ordinary
 // stream order on both sides. TLB_NO_PDL=1 turns the attribute off (the device-side calls are then
-// no-ops).
+// no-ops). A product's weights may be copied in front of the wait only if no kernel writes them (weights_settled in
+// lower.cu): launch_pdl_if(false, ...) is the ordinary launch that other operands take.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdlib>
@@ -24,7 +25,7 @@ inline bool pdl_enabled() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+inline cudaError_t launch_pdl_if(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -34,8 +35,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    return launch_pdl_if(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace tlb
