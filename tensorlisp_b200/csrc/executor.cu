@@ -623,10 +623,16 @@ static void push_table(tlb_program *p) {
         p->page->out[n++] = {p->layout.place[o.tensor].off, o.host_off, (uint32_t)((o.bytes + 15) / 16)};
     p->page->n_out = n;
 }
+// whether two tensors of the arena lie on common bytes: views of one tensor, or one that takes over another's place
+static bool share_bytes(const tlb_program *p, uint32_t a, uint32_t b) {
+    if (p->graph.root((int32_t)a) == p->graph.root((int32_t)b)) return true;
+    const Place pa = p->layout.place[a], pb = p->layout.place[b];
+    return pa.off < pb.off + p->graph.tensors[b].nbytes() && pb.off < pa.off + p->graph.tensors[a].nbytes();
+}
 static void push_add(tlb_program *p, uint32_t tensor, uint64_t bytes) {
     if (!p->out_host_off || bytes != p->graph.tensors[tensor].nbytes() || !is_small_out(p, tensor) || p->pushed.size() >= IO_MAX_OUT) return;
     for (uint32_t t : p->no_push)
-        if (t == tensor) return;
+        if (share_bytes(p, t, tensor)) return;
     uint32_t at = p->out_host_off;   // first gap that holds it
     for (bool moved = true; moved;) {
         moved = false;
@@ -1039,13 +1045,13 @@ void *tlb_program_tensor_ptr(tlb_program *prog, uint32_t tensor_id, uint64_t *by
     const Place pl = prog->layout.place[tensor_id];
     if (bytes) *bytes = prog->graph.tensors[tensor_id].nbytes();
     if (pl.buf == BUF_ARENA) {
-        // the caller may write there: what read() returns comes from the tensor itself from now on
+        // the caller may write there: what read() returns of any tensor on those bytes comes from the tensor itself from now on
         cudaSetDevice(prog->ordinal);
         if (page_idle(prog) == cudaSuccess) {
-            prog->pushed.erase(std::remove_if(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; }), prog->pushed.end());
+            prog->pushed.erase(std::remove_if(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return share_bytes(prog, o.tensor, tensor_id); }), prog->pushed.end());
             push_table(prog);
         }
-        prog->no_push.push_back(tensor_id);
+        if (std::find(prog->no_push.begin(), prog->no_push.end(), tensor_id) == prog->no_push.end()) prog->no_push.push_back(tensor_id);
         return (char *)prog->arena + pl.off;
     }
     if (pl.buf == BUF_IO) {

@@ -102,6 +102,46 @@ def test_a_known_device_address_sees_every_input_and_every_result():
     native.close()
 
 
+@pytest.mark.parametrize("held", ["a view", "the tensor of a view", "the tensor itself"])
+def test_an_address_into_a_result_through_another_tensor_of_its_storage(held):
+    """Who holds the address of a view writes into the root's memory (and the other way round): what read() returns then comes from
+    there, not from the copy that runs push to the host."""
+    import torch
+
+    class At:
+        def __init__(self, ptr, n):
+            self.__cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(ptr, False), version=3, strides=None)
+
+    native = Native.load([])
+    g = G.Graph()
+    x = g.input(G.F32, [16], "x")
+    y = g.output(g.scale(x, 2.0))
+    v = g.output(g.view(y, [8], offset=16))
+    other = g.output(g.scale(x, 3.0))
+    prog = NativeProgram.compile(native, g)
+    a = np.arange(16, dtype=np.float32)
+    prog.set_input(0, a)
+    for _ in range(2):      # from the second run on the results are pushed
+        prog.run()
+        prog.read(y), prog.read(v), prog.read(other)
+    first, t = (4, v) if held == "a view" else (0, y)
+    ptr, nbytes = prog.tensor_ptr(t)
+    at = torch.as_tensor(At(ptr, nbytes // 4), device="cuda")
+    watched = {"a view": y, "the tensor of a view": v, "the tensor itself": y}[held]
+    for i in range(3):
+        prog.run()
+        want = 2 * a
+        assert np.array_equal(prog.read(watched).reshape(-1), want if watched == y else want[4:12])
+        at.fill_(9 + i)
+        torch.cuda.synchronize()
+        want[first:first + nbytes // 4] = 9 + i
+        assert np.array_equal(prog.read(y).reshape(-1), want)
+        assert np.array_equal(prog.read(v).reshape(-1), want[4:12])
+        assert np.array_equal(prog.read(other).reshape(-1), 3 * a)
+    prog.free()
+    native.close()
+
+
 @pytest.mark.parametrize("ty,name", [(G.Q8_0, "q8_0"), (G.Q4_K, "q4_K")])
 @pytest.mark.parametrize("rows,n", [(1, 256), (300, 256), (1025, 4096), (5000, 4096), (7, 1 << 20)])
 def test_quantize_rows_in_pieces(oracle, ty, name, rows, n):
