@@ -139,6 +139,9 @@ void       tlb_buffer_free(tlb_buffer *b);
  * between it and the device run at the link's rate and need no staging. Blocks come from a bounded pool that keeps up to 256 MB for
  * reuse; TLB_ALLOC when 1 GB is handed out (use ordinary memory then). Any thread may free. */
 tlb_status tlb_host_alloc(uint64_t bytes, void **out);
+/* A block for a result that is read many times: TLB_ALLOC also while the blocks of that size handed out so far do not come back
+ * (pinning a fresh one costs more than the copy into ordinary memory). Freed with tlb_host_free. */
+tlb_status tlb_result_alloc(uint64_t bytes, void **out);
 void       tlb_host_free(void *p);
 
 /* ------------------------------------------------------------------ programs

@@ -99,6 +99,7 @@ SYMBOLS = {
     "tlb_program_arena_bytes": (C.c_uint64, [_P]),
     "tlb_program_profile": (C.c_int, [_P, C.POINTER(_P), C.c_uint32, _P, C.POINTER(C.c_float), C.c_uint32]),
     "tlb_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(_P)]),
+    "tlb_result_alloc": (C.c_int, [C.c_uint64, C.POINTER(_P)]),
     "tlb_host_free": (None, [_P]),
     "tlb_quantize_rows": (C.c_int, [_P, C.c_uint32, _P, C.c_int64, C.c_int64, _P]),
     "tlb_quantize_rows_device": (C.c_int, [_P, C.c_uint32, _P, C.c_int64, C.c_int64, _P]),

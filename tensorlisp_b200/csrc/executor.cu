@@ -294,6 +294,7 @@ tlb_status tlb_device_open(int ordinal, tlb_device **dev) {
     }
     d->name = std::string("native ") + d->prop.name;
     configure_kernels_once(ordinal);   // cudaSetDevice(ordinal) above made it current
+    pinned_device(ordinal);
     *dev = d;
     return TLB_OK;
 }
@@ -513,8 +514,13 @@ void tlb_buffer_free(tlb_buffer *b) {
 
 tlb_status tlb_host_alloc(uint64_t bytes, void **out) {
     if (!out) return fail(TLB_INVALID, "tlb_host_alloc: null output");
-    *out = pinned_alloc(std::max<uint64_t>(bytes, 1));
+    *out = pinned_alloc(std::max<uint64_t>(bytes, 1), PIN_CALLER);
     return *out ? TLB_OK : fail(TLB_ALLOC, "no " + std::to_string(bytes) + " bytes of pinned host memory");
+}
+tlb_status tlb_result_alloc(uint64_t bytes, void **out) {
+    if (!out) return fail(TLB_INVALID, "tlb_result_alloc: null output");
+    *out = pinned_alloc(std::max<uint64_t>(bytes, 1), PIN_RESULT);
+    return *out ? TLB_OK : fail(TLB_ALLOC, "no pinned block of " + std::to_string(bytes) + " bytes for a result");
 }
 void tlb_host_free(void *p) { pinned_free(p); }
 
@@ -600,7 +606,7 @@ static bool page_create(tlb_program *p) {
     for (int32_t k : p->graph.keep)
         if ((uint32_t)k < p->n_user_tensors && is_small_out(p, (uint32_t)k)) p->out_host_off = (uint32_t)at;
     if (p->out_host_off) at += IO_OUT_TOTAL;
-    p->page = (IoPage *)pinned_alloc(at, true);
+    p->page = (IoPage *)pinned_alloc(at, PIN_LIBRARY);
     if (!p->page) return false;
     std::memset((void *)p->page, 0, sizeof(IoPage));
     return true;
@@ -776,6 +782,7 @@ void tlb_program_free(tlb_program *prog) {
         cudaDeviceSynchronize();   // the page goes back to the pool: no kernel may still write to it
         pinned_free(prog->page);
     }
+    pinned_trim();
     delete prog;
 }
 

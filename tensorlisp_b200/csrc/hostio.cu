@@ -26,20 +26,27 @@ namespace {
 
 constexpr uint64_t HOST_CACHE_LIMIT = 256ull << 20;   // bytes kept for reuse
 constexpr uint64_t HOST_LIVE_LIMIT = 1024ull << 20;   // bytes handed out at any time
+// Fresh result blocks per size: two (the caller lets go of one result when it has the next), and one more for every eight times that
+// a block was used again. Pinning is slow: a call whose result went into a fresh block took 0.6 to 2.5 ms at 1 MB and 6.5 to 9 ms at
+// 16 MB, into ordinary memory 0.45 and 2 to 3.5 ms (most of it the first touch of its pages), into a block that came back 0.06 and
+// 0.39 ms. A caller that keeps its results would pay for a fresh block every time.
+constexpr uint64_t RESULT_FRESH = 2, RESULT_HITS = 8;
 
 struct PinnedPool {
     std::mutex m;
     std::map<uintptr_t, uint64_t> live;                    // handed out: address -> block size
     std::multimap<uint64_t, void *> idle;                  // by block size
     uint64_t live_bytes = 0, idle_bytes = 0;
+    struct Use { uint64_t fresh = 0, hits = 0; };
+    std::map<uint64_t, Use> results;                       // by block size
+    std::atomic<int> device{0};
 };
 // never destroyed: blocks may be given back while the process ends
 PinnedPool &pool() {
     static PinnedPool *p = new PinnedPool;
     return *p;
 }
-// block sizes: powers of two and their halfway points, 64 KB at least (pinning works in pages and is slow: about 0.1 ms
-// and 0.2 ms per MB)
+// block sizes: powers of two and their halfway points, 64 KB at least
 uint64_t block_size(uint64_t bytes) {
     uint64_t b = 64 << 10;
     while (b < bytes) {
@@ -51,13 +58,38 @@ uint64_t block_size(uint64_t bytes) {
 
 }  // namespace
 
-void *pinned_alloc(uint64_t bytes, bool always) {
-    const uint64_t b = block_size(bytes);
+void pinned_device(int ordinal) { pool().device = ordinal; }
+
+void pinned_trim() {
     PinnedPool &p = pool();
+    std::vector<void *> drop;
     {
         std::lock_guard<std::mutex> lock(p.m);
-        if (!always && p.live_bytes + b > HOST_LIVE_LIMIT) return nullptr;
+        while (p.idle_bytes > HOST_CACHE_LIMIT) {   // the largest go first
+            auto last = std::prev(p.idle.end());
+            p.idle_bytes -= last->first;
+            drop.push_back(last->second);
+            p.idle.erase(last);
+        }
+    }
+    if (!drop.empty()) cudaSetDevice(p.device);
+    for (void *d : drop) cudaFreeHost(d);
+}
+
+void *pinned_alloc(uint64_t bytes, PinFor what) {
+    const uint64_t b = block_size(bytes);
+    PinnedPool &p = pool();
+    pinned_trim();
+    {
+        std::lock_guard<std::mutex> lock(p.m);
+        if (what != PIN_LIBRARY && p.live_bytes + b > HOST_LIVE_LIMIT) return nullptr;
         auto it = p.idle.find(b);
+        if (what == PIN_RESULT) {
+            PinnedPool::Use &use = p.results[b];
+            if (it != p.idle.end()) use.hits++;
+            else if (use.fresh >= RESULT_FRESH + use.hits / RESULT_HITS) return nullptr;
+            else use.fresh++;
+        }
         if (it != p.idle.end()) {
             void *q = it->second;
             p.idle.erase(it);
@@ -68,6 +100,7 @@ void *pinned_alloc(uint64_t bytes, bool always) {
         }
     }
     void *q = nullptr;
+    if (what != PIN_LIBRARY) cudaSetDevice(p.device);   // (the library's own calls have set theirs)
     if (cudaHostAlloc(&q, b, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
@@ -81,24 +114,14 @@ void *pinned_alloc(uint64_t bytes, bool always) {
 void pinned_free(void *q) {
     if (!q) return;
     PinnedPool &p = pool();
-    std::vector<void *> drop;
-    {
-        std::lock_guard<std::mutex> lock(p.m);
-        auto it = p.live.find((uintptr_t)q);
-        if (it == p.live.end()) return;
-        const uint64_t b = it->second;
-        p.live.erase(it);
-        p.live_bytes -= b;
-        p.idle.emplace(b, q);
-        p.idle_bytes += b;
-        while (p.idle_bytes > HOST_CACHE_LIMIT) {   // the largest go first
-            auto last = std::prev(p.idle.end());
-            p.idle_bytes -= last->first;
-            drop.push_back(last->second);
-            p.idle.erase(last);
-        }
-    }
-    for (void *d : drop) cudaFreeHost(d);
+    std::lock_guard<std::mutex> lock(p.m);
+    auto it = p.live.find((uintptr_t)q);
+    if (it == p.live.end()) return;
+    const uint64_t b = it->second;
+    p.live.erase(it);
+    p.live_bytes -= b;
+    p.idle.emplace(b, q);
+    p.idle_bytes += b;
 }
 
 bool pinned_owns(const void *q, uint64_t bytes) {
@@ -242,7 +265,7 @@ Ring &ring(int ordinal) {
 }
 bool ring_ready(Ring &r) {
     if (r.ok) return true;
-    if (!r.mem) r.mem = (char *)pinned_alloc(RING_SLOTS * RING_CHUNK, true);
+    if (!r.mem) r.mem = (char *)pinned_alloc(RING_SLOTS * RING_CHUNK, PIN_LIBRARY);
     if (!r.mem) return false;
     for (int s = 0; s < RING_SLOTS; s++) {
         r.issued[s] = 0;

@@ -12,10 +12,16 @@ namespace tlb {
 
 // ---- pinned host memory. Blocks are kept for reuse up to a bound (HOST_CACHE_LIMIT); what is handed out at any time
 // is bounded too (HOST_LIVE_LIMIT): beyond it, and when pinning fails, pinned_alloc returns null and the caller uses
-// pageable memory (`always`: a block the library itself cannot do without, whatever is handed out). Safe to use from
-// several threads.
-void *pinned_alloc(uint64_t bytes, bool always = false);
+// pageable memory. Safe to use from several threads.
+// PIN_RESULT: a fresh block only while the blocks of its size come back (a caller that keeps its results gets null).
+// PIN_LIBRARY: a block the library itself cannot do without, whatever is handed out.
+enum PinFor { PIN_CALLER, PIN_RESULT, PIN_LIBRARY };
+void *pinned_alloc(uint64_t bytes, PinFor what);
+// Makes no CUDA call (it runs wherever an array goes away): what the cache cannot hold is unpinned by the next pinned_alloc or
+// pinned_trim.
 void pinned_free(void *p);
+void pinned_trim();
+void pinned_device(int ordinal);                   // the device that pinning is done for
 bool pinned_owns(const void *p, uint64_t bytes);   // [p, p + bytes) lies in a block that is handed out
 
 // ---- host threads: runs fn(0) .. fn(n - 1), on the calling thread and up to `threads` - 1 others. When another caller

@@ -45,10 +45,10 @@ _PINNED_FROM = 64 << 10     # smaller results come through the program's page: a
 
 def _result_bytes(nbytes: int) -> np.ndarray:
     """Uninitialised bytes for a result: pinned where that pays (the copy goes straight there, and no page of the array
-    is touched for the first time while the caller waits), ordinary memory when the pool has none."""
+    is touched for the first time while the caller waits), ordinary memory when the pool has none (results that are kept)."""
     if nbytes >= _PINNED_FROM:
         p = C.c_void_p()
-        if _lib.lib().tlb_host_alloc(nbytes, C.byref(p)) == 0:
+        if _lib.lib().tlb_result_alloc(nbytes, C.byref(p)) == 0:
             return np.asarray(_HostBlock(p.value, nbytes))
     return np.empty(nbytes, np.uint8)
 

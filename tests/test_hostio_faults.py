@@ -35,3 +35,8 @@ def test_an_error_is_reported_and_the_ring_goes_on(program, what, at):
 def test_helper_threads_call_for_the_device_of_the_copy(program, what):
     r = subprocess.run([str(program), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_results_that_are_kept_and_results_that_come_back(program):
+    r = subprocess.run([str(program), "results"], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
