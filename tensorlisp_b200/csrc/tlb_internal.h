@@ -205,6 +205,7 @@ struct tlb_program {
         cudaGraphExec_t exec = nullptr;
     };
     std::vector<Captured> captured;
+    std::vector<std::vector<void *>> ran_once;   // of a program of one launch: pointer sets it has run for (the last eight), captured at the next run
     uint32_t kernel_nodes = 0;   // kernel launches in the most recently captured graph
     bool use_graph = true;
     uint32_t need_weights = 0;   // weight buffers the graph reads, and whether it reads state

@@ -142,6 +142,31 @@ def test_an_address_into_a_result_through_another_tensor_of_its_storage(held):
     native.close()
 
 
+def test_a_single_launch_is_captured_when_it_runs_again():
+    native = Native.load([])
+    g = G.Graph()
+    s, x = g.state(G.F32, [64], "s"), g.input(G.F32, [64], "x")
+    y = g.output(g.add(s, x))
+    native.alloc_states([256])
+    prog = NativeProgram.compile(native, g)
+    blocks = [native.new_state_block() for _ in range(3)]
+    rng = np.random.default_rng(0)
+    held = rng.standard_normal((3, 64)).astype(np.float32)
+    for b, h in zip(blocks, held):
+        b.write(0, h)
+    for turn in range(4):
+        for i, (b, h) in enumerate(zip(blocks, held)):
+            a = rng.standard_normal(64).astype(np.float32)
+            prog.set_input(0, a)
+            prog.run(b)
+            assert np.array_equal(prog.read(y).reshape(-1), h + a)
+            assert native.L.tlb_program_graph_count(prog.h) == (0 if turn == 0 else (i + 1 if turn == 1 else 3))
+    prog.free()
+    for b in blocks:
+        b.free()
+    native.close()
+
+
 @pytest.mark.parametrize("ty,name", [(G.Q8_0, "q8_0"), (G.Q4_K, "q4_K")])
 @pytest.mark.parametrize("rows,n", [(1, 256), (300, 256), (1025, 4096), (5000, 4096), (7, 1 << 20)])
 def test_quantize_rows_in_pieces(oracle, ty, name, rows, n):
