@@ -19,6 +19,16 @@ tlb_status fail(tlb_status st, const std::string &msg) {
 }
 std::string cuda_msg(cudaError_t e) { return std::string(cudaGetErrorName(e)) + ": " + cudaGetErrorString(e); }
 
+int current_sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        n = known[dev].load(std::memory_order_relaxed);
+        if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n > 0 ? n : 148;
+}
+
 // ---------------------------------------------------------------------------- type table
 // crates/kernels/src/graph.rs:30-50
 const TypeTraits *type_traits(uint32_t ty) {
@@ -686,8 +696,8 @@ tlb_status tlb_program_compile(tlb_device *dev, const tlb_graph *graph, const tl
     p->ordinal = dev->ordinal;
     p->n_user_tensors = graph->n_tensors;
     p->graph = std::move(g);
-    rewrite_graph(p->graph);   // TL_NATIVE_NOFUSE turns the fusions off inside; the shared activation quantizers always go in
     const int sm = dev->prop.multiProcessorCount;
+    rewrite_graph(p->graph, sm);   // TL_NATIVE_NOFUSE turns the fusions off inside; the shared activation quantizers always go in
     const Graph &G = p->graph;
     p->layout = plan(G, lv, [&](int32_t id) { return node_scratch_bytes(G, id, sm); });
 

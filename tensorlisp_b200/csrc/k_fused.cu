@@ -485,8 +485,9 @@ bool row_quant_supported(int64_t K) { return K % 256 == 0 && K / 256 <= 65535 * 
 cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st) {
     if (p.N == 0 || p.K == 0) return cudaSuccess;
     // eight columns per CTA: from two CTAs per SM on
+    const int64_t two_per_sm = 2 * current_sm_count();
     const int64_t eights = mm_fold_groups(p.N), strips = (p.K / 256 + 3) / 4;
-    if (p.npad == MM_FOLD_NPAD && (p.mode == RQ_PLAIN || p.mode == RQ_F16) && !p.b && !p.y_out && eights * strips >= 296 && strips <= 65535) {
+    if (p.npad == MM_FOLD_NPAD && (p.mode == RQ_PLAIN || p.mode == RQ_F16) && !p.b && !p.y_out && eights * strips >= two_per_sm && strips <= 65535) {
         const dim3 grid((unsigned)eights, (unsigned)strips);
         return p.q80 ? launch_pdl(k_row_quant_plain<true>, grid, dim3(256), 0, st, p) : launch_pdl(k_row_quant_plain<false>, grid, dim3(256), 0, st, p);
     }

@@ -1046,11 +1046,7 @@ static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
                                int64_t ldy, int *err, cudaStream_t st, bool early) {
     if (n_mats < 1 || n_mats > tc8f::MAX_MATS) return cudaErrorInvalidValue;
-    static int sm_of[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!sm_of[dev]) cudaDeviceGetAttribute(&sm_of[dev], cudaDevAttrMultiProcessorCount, dev);
+    const int sms = current_sm_count();
     Tc8fMaps maps;
     Tc8fParams p{};
     for (int j = 0; j < tc8f::MAX_MATS; j++) {
@@ -1070,7 +1066,7 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.act = (const uint8_t *)blobs;
     p.N = (int)N;
     p.nst = (int)(K / 256);
-    const FoldTile tile = fold_tile(N, p.row_tiles, p.nst, sm_of[dev]);
+    const FoldTile tile = fold_tile(N, p.row_tiles, p.nst, sms);
     p.nw = tile.nw;
     // raw stages: 128 rows x 256 elements (18 or 34 KB); what they leave goes to B
     const int raw_bytes = tc8::ROWS * (q4k ? 144 : tc8::ROW_CHUNK);
@@ -1081,7 +1077,7 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.groups = mm_fold_groups(N);
     p.col_tiles = (int)((N + tile.halves * p.nw - 1) / (tile.halves * p.nw));
     p.err = err;
-    const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sm_of[dev]));
+    const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sms));
     auto go = [&](auto *k) { return launch_pdl_if(early, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
     if (tile.halves == 2) return q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
     if (narrow) return q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);

@@ -126,6 +126,7 @@ struct RowQuantArgs {
                          // operand (blobs of 256 columns x 64 elements, value = code x f16 scale) is produced
 };
 bool row_quant_supported(int64_t K);
+int current_sm_count();   // SMs of the current device (148 where there is none to ask)
 
 // ---------------------------------------------------------------- k_gemv.cu
 // Up to three matrices of one block type and row length against a few activation columns (eight per launch). act: mode, sources,

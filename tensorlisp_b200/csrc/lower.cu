@@ -647,7 +647,7 @@ void lower_quant_act(L &l) {
         p.d_off = a.d_off;
         p.bsum_off = a.bsum_off;
         p.blob_off = a.bytes;
-        p.blob_bytes = p.q80 ? 0 : mmq_tc_plan(p.K, 128, p.N, 148).blob_unit;
+        p.blob_bytes = p.q80 ? 0 : mmq_tc_plan(p.K, 128, p.N, l.c.dev->prop.multiProcessorCount).blob_unit;
         p.operand_only = operand_only(*l.c.g, l.id);
         l.push([=](const RunCtx &r) {
             RowQuantArgs q = p;
@@ -685,7 +685,7 @@ void lower_row_quant(L &l) {
     p.bsum_off = al.bsum_off;
     p.npad = t.op_params[1];
     p.blob_off = al.bytes;
-    p.blob_bytes = p.npad > 0 ? mmq_tc_plan(p.K, 128, p.N, 148).blob_unit : 0;
+    p.blob_bytes = p.npad > 0 ? mmq_tc_plan(p.K, 128, p.N, l.c.dev->prop.multiProcessorCount).blob_unit : 0;
     p.q80 = t.op_params[0] == ACT_Q8_0;
     p.operand_only = operand_only(*l.c.g, l.id);
     p.eps = t.param_f32(15);
@@ -800,7 +800,7 @@ void lower_custom(L &l) {
             rq.bsum_off = al.bsum_off;
             rq.npad = l.T(qid).op_params[1];
             rq.blob_off = al.bytes;
-            rq.blob_bytes = rq.npad > 0 ? mmq_tc_plan(rq.K, 128, rq.N, 148).blob_unit : 0;
+            rq.blob_bytes = rq.npad > 0 ? mmq_tc_plan(rq.K, 128, rq.N, l.c.dev->prop.multiProcessorCount).blob_unit : 0;
             prq = l.place(qid);
         }
         l.push([=](const RunCtx &r) {
@@ -1207,11 +1207,11 @@ static bool written_between(const Graph &g, const std::vector<char> &dead, int32
 }
 void fuse_row_producers(Graph &g);
 void fuse_rope_cache(Graph &g);
-void fuse_mul_mat_groups(Graph &g);
-void fuse_attn_quant(Graph &g);
+void fuse_mul_mat_groups(Graph &g, int sm_count);
+void fuse_attn_quant(Graph &g, int sm_count);
 void fuse_gemv(Graph &g, bool groups, bool producers);
 // Readers of every root (views of a tensor count for the root), as fuse.rs:56-63 requires.
-void rewrite_graph(Graph &g) {
+void rewrite_graph(Graph &g, int sm_count) {
     const size_t nt0 = g.tensors.size();
     auto readers_of = [&](std::vector<int> &readers) {
         readers.assign(g.tensors.size(), 0);
@@ -1344,7 +1344,7 @@ void rewrite_graph(Graph &g) {
                 const Tensor &mm = g.tensors[id];
                 const bool plain2d = tw.ne[2] * tw.ne[3] * mm.ne[2] * mm.ne[3] == 1 && tw.nb[1] == tw.row_size();
                 if (plain2d && tc_supported(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1]) && !getenv("TLB_NO_TC")) {
-                    const TcPlan tp = tc_plan(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1], 148);
+                    const TcPlan tp = tc_plan(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1], sm_count);
                     Tensor &q = g.tensors[qa];
                     q.op_params[1] = tp.npad;
                     q.opaque_bytes = act_layout(kind, tx.ne[0], tx.nrows()).bytes + tp.blob_bytes;
@@ -1358,16 +1358,16 @@ void rewrite_graph(Graph &g) {
     g.nodes.swap(nodes);
     fuse_gemv(g, enabled("MUL_MAT_GROUP"), enabled("ROW_QUANT"));
     if (enabled("ROW_QUANT")) fuse_row_producers(g);
-    if (enabled("ROW_QUANT") && enabled("ATTN_QUANT")) fuse_attn_quant(g);
+    if (enabled("ROW_QUANT") && enabled("ATTN_QUANT")) fuse_attn_quant(g, sm_count);
     if (enabled("ROPE_KV_WRITE")) fuse_rope_cache(g);
-    if (enabled("MUL_MAT_GROUP")) fuse_mul_mat_groups(g);
+    if (enabled("MUL_MAT_GROUP")) fuse_mul_mat_groups(g, sm_count);
 }
 
 // The f16 output of paged attention, cast and quantized for the output projection (a ROW_QUANT node in RQ_F16 mode right
 // behind the attention): the attention kernel quantizes its rows itself when it runs without a context split (one
 // launch less per layer). The ROW_QUANT node leaves the node list; its tensor becomes src[9] of the attention node, which
 // also makes the planner keep it alive from that position on.
-void fuse_attn_quant(Graph &g) {
+void fuse_attn_quant(Graph &g, int sm_count) {
     const size_t nn = g.nodes.size();
     std::vector<int> pos_of(g.tensors.size(), -1);
     for (size_t i = 0; i < nn; i++) pos_of[g.nodes[i]] = (int)i;
@@ -1389,7 +1389,7 @@ void fuse_attn_quant(Graph &g) {
         if (S.ty != TLB_TYPE_F16 || !S.is_contiguous() || S.view_offs != 0 || S.nelements() != A.nelements()) continue;
         if (shape.ne[0] != A.ne[0] * A.ne[1] || shape.nrows() != A.ne[2]) continue;
         PagedGeom pg{};
-        if (!paged_geom(g, A, 148, pg) || pg.n_chunks != 1 || !paged_quant_fusable(pg)) continue;
+        if (!paged_geom(g, A, sm_count, pg) || pg.n_chunks != 1 || !paged_quant_fusable(pg)) continue;
         A.src[9] = qid;
         dead[qi] = 1;
     }
@@ -1830,7 +1830,7 @@ void fuse_gemv(Graph &g, bool groups, bool producers) {
 // 148 SMs), and gate + up (2 x 112 tiles) together are enough work for the stream-K schedule, which gives
 // every SM the same number of super-blocks instead of one wave of 112 tiles twice. Nothing reads a member's result before the
 // last member, because the members are adjacent in node order.
-void fuse_mul_mat_groups(Graph &g) {
+void fuse_mul_mat_groups(Graph &g, int sm_count) {
     const size_t nn = g.nodes.size();
     std::vector<char> dead(nn, 0);
     auto eligible = [&](const Tensor &t) {
@@ -1855,7 +1855,7 @@ void fuse_mul_mat_groups(Graph &g) {
             if (!eligible(B) || B.src[1] != A.src[1] || B.src[2] != A.src[2] || g.tensors[B.src[0]].ty != g.tensors[A.src[0]].ty) break;
             const int64_t tb = (B.ne[0] + 127) / 128;
             // a group stays within one wave of CTAs, or is big enough for the stream-K schedule (gate + up)
-            if (tiles + tb > 148 && g.tensors[A.src[2]].op_params[1] != MM_FOLD_NPAD && !mmq_tc_plan(g.tensors[A.src[1]].ne[0], (tiles + tb) * 128, g.tensors[A.src[1]].ne[1], 148).streamk) break;
+            if (tiles + tb > sm_count && g.tensors[A.src[2]].op_params[1] != MM_FOLD_NPAD && !mmq_tc_plan(g.tensors[A.src[1]].ne[0], (tiles + tb) * 128, g.tensors[A.src[1]].ne[1], sm_count).streamk) break;
             tiles += tb;
             A.src[wslot[members]] = B.src[0];
             A.src[yslot[members]] = g.nodes[j];

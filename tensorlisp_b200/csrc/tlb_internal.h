@@ -186,7 +186,7 @@ cudaError_t comm_exchange_row_quant(tlb_device *dev, float *data, const float *p
                                     int *err);
 int comm_ranks(tlb_device *dev);
 // IR rewrites before planning (fusion, shared activation quantization); fuse.cpp
-void rewrite_graph(Graph &g);
+void rewrite_graph(Graph &g, int sm_count);
 
 }  // namespace tlb
 
