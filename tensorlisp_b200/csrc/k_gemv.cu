@@ -38,7 +38,7 @@ cudaError_t tc_encode_2d_bytes(CUtensorMap *map, const void *base, uint64_t row_
 
 namespace gemv {
 
-using tc::tma_2d;
+using namespace tc;   // mbarriers and copies
 
 constexpr int WARPS = 8;                      // consumers
 constexpr int THREADS = 32 * (WARPS + 1);     // and the producer
@@ -46,40 +46,6 @@ constexpr int MAX_STAGES = 16;
 constexpr int MAX_COLS = (int)GEMV_MAX_COLS;
 constexpr int PART_BYTES = 8 * 1024;          // partial sums before they are added up
 
-__device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(bar)), "r"(count)); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(bar)) : "memory"); }
-// Bounded wait: gives up after about two seconds (a probe of an incomplete phase takes about 4 us) and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit = (1u << 19)) {
-    const uint32_t a = su32(bar);
-    for (uint32_t i = 0; i < limit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-// whether the phase has completed
-__device__ __forceinline__ bool mbar_probe(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(su32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory"); }
 // 16 rows x 32 codes times 32 codes x 8 columns; A as unsigned or signed bytes. (The zero addend is an operand of its own, so that
 // it costs no register moves.)
@@ -495,7 +461,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv(const __grid_constant__ Map
             for (int x = 0, seg = 0; seg < p.segs && ok; seg++, turn++, x += p.seg_units * p.unit_bytes / 8) {   // x in 8-byte elements
                 for (int set = 0; set < p.sets && slot0 + set < slots; set++) {
                     const int st = set * p.stages_per_set + s;
-                    if (turn >= p.stages_per_set && !(ok = mbar_wait(&empty[st], ph ^ 1u))) break;
+                    if (turn >= p.stages_per_set && !(ok = mbar_wait_limit(&empty[st], ph ^ 1u))) break;
                     mbar_expect_tx(&full[st], bytes);
                     // a box is 16 rows whatever is left of the range: rows past it are another CTA's, or zeros past the matrix
                     for (int gr = 0; gr < p.groups; gr++) {
@@ -514,7 +480,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv(const __grid_constant__ Map
             // the consumers stopped releasing stages: record it, then wait (bounded) for the copies still in flight
             report_error(p.err, 1);
             for (int st = 0; st < p.sets * p.stages_per_set; st++)
-                if (mbar_wait(&full[st], 0, 1u << 12)) mbar_wait(&full[st], 1, 1u << 12);   // one of the two phases has passed
+                if (mbar_wait_limit(&full[st], 0, 1u << 12)) mbar_wait_limit(&full[st], 1, 1u << 12);   // one of the two phases has passed
         }
         return;
     }
@@ -536,7 +502,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv(const __grid_constant__ Map
                 float f[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int seg = 0; seg < p.segs; seg++) {
                     const int st = set * p.stages_per_set + s;
-                    if (ok && !ready && !mbar_wait(&full[st], ph)) {
+                    if (ok && !ready && !mbar_wait_limit(&full[st], ph)) {
                         if (lane == 0) report_error(p.err, 1);
                         ok = false;   // this warp stops releasing stages; the producer's bounded wait ends the copies
                     }
@@ -545,7 +511,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv(const __grid_constant__ Map
                         ph ^= 1u;
                     }
                     // a probe takes 100 to 300 cycles to answer: the next stage's goes out before this one's weights are worked on
-                    ready = mbar_probe(&full[set * p.stages_per_set + s], ph);
+                    ready = mbar_test(su32(&full[set * p.stages_per_set + s]), ph);
                     const int unit = seg * p.seg_units + u;
                     if (unit < p.units) {
                         // rows past a matrix's end hold what the stage held before; their sums are not used

@@ -13,10 +13,13 @@
 
 #include "kernels.h"
 #include "pdl.cuh"
+#include "tc_common.cuh"
 
 namespace tlb {
 
 namespace gemvf {
+
+using namespace tc;   // mbarriers and copies
 
 constexpr int WARPS = 8;                      // consumers
 constexpr int THREADS = 32 * (WARPS + 1);     // and the producer
@@ -25,31 +28,6 @@ constexpr int PAD = 16;                       // word reads may run 2 bytes past
 constexpr int OUT_BYTES = 8 * 1024;           // partial sums before they are added up
 constexpr int RU = 2;                         // rows (or groups of short rows) of a unit
 
-__device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(bar)), "r"(count)); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(bar)) : "memory"); }
-// Bounded wait: gives up after about two seconds (a probe of an incomplete phase takes about 4 us) and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit = (1u << 19)) {
-    const uint32_t a = su32(bar);
-    for (uint32_t i = 0; i < limit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(su32(dst)), "l"(src), "r"(bytes), "r"(su32(bar)) : "memory");
-}
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory"); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     float2 d;
@@ -188,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, NC <= 2 ? 2 : 1) k_gemv_f32(const __g
         uint32_t ph = 0;
         bool ok = true;
         for (int t = 0; t < n_tiles; t++) {
-            if (t >= p.stages && !(ok = mbar_wait(&empty[s], ph ^ 1u))) break;
+            if (t >= p.stages && !(ok = mbar_wait_limit(&empty[s], ph ^ 1u))) break;
             const int64_t row0 = r0 + (int64_t)t * p.tile_rows;
             const int rows = (int)min((int64_t)p.tile_rows, r1 - row0);
             const uint32_t bytes = (uint32_t)(rows * p.row_bytes + 15) & ~15u;   // the last rows of a matrix may end between two 16-byte boundaries
@@ -203,7 +181,7 @@ __global__ void __launch_bounds__(THREADS, NC <= 2 ? 2 : 1) k_gemv_f32(const __g
         if (!ok) {
             // the consumers stopped releasing stages: record it, then wait (bounded) for the copies still in flight
             report_error(p.err, 1);
-            for (int t = max(0, issued - p.stages); t < issued; t++) mbar_wait(&full[t % p.stages], (uint32_t)((t / p.stages) & 1));
+            for (int t = max(0, issued - p.stages); t < issued; t++) mbar_wait_limit(&full[t % p.stages], (uint32_t)((t / p.stages) & 1));
         }
         return;
     }
@@ -221,7 +199,7 @@ __global__ void __launch_bounds__(THREADS, NC <= 2 ? 2 : 1) k_gemv_f32(const __g
     for (int e0 = 0; e0 < n_tiles; e0 += p.epoch_tiles) {
         const int e1 = min(n_tiles, e0 + p.epoch_tiles);
         for (; t < e1; t += p.sets) {
-            if (ok && !mbar_wait(&full[s], ph)) {
+            if (ok && !mbar_wait_limit(&full[s], ph)) {
                 if (lane == 0) report_error(p.err, 1);
                 ok = false;   // this warp stops releasing stages; the producer's bounded wait ends the copies
             }

@@ -1,5 +1,4 @@
-// mbarrier, TMA and tcgen05 wrappers shared by the tensor-core mul_mat kernels (k_mmq_tc.cu for Q4_K,
-// k_mmq_tc_q8.cu for Q8_0).
+// mbarrier, TMA and tcgen05 wrappers shared by the mul_mat and attention kernels.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -75,6 +74,13 @@ __device__ __forceinline__ void mbar_wait_nap(uint64_t *bar, uint32_t parity, vo
             return;
         }
     }
+}
+// For roles that end their own work when a wait gives up (k_gemv.cu, k_gemv_f32.cu): false after `limit` probes.
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t *bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
+    const uint32_t a = su32(bar);
+    for (uint32_t i = 0; i < limit; i++)
+        if (mbar_try(a, parity)) return true;
+    return false;
 }
 __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, volatile int *fail) { mbar_wait_nap(bar, parity, fail, 0); }
 __device__ __forceinline__ void mbar_wait_relaxed(uint64_t *bar, uint32_t parity, volatile int *fail) { mbar_wait_nap(bar, parity, fail, 64); }
