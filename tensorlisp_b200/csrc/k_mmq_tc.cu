@@ -593,7 +593,7 @@ void mmq_tc_configure() {
 }
 
 bool mmq_tc_supported(uint32_t type, int64_t K, int64_t M, int64_t N) {
-    return type == TLB_TYPE_Q4_K && K % 256 == 0 && K >= 256 && M >= 1 && N > GEMV_MAX_COLS && N <= (int64_t)MM_FOLD_NPAD * 65535 && encode_tiled() != nullptr;
+    return type == TLB_TYPE_Q4_K && K % 256 == 0 && K >= 256 && M >= 1 && !few_column_faster(type, K, M, N) && N <= (int64_t)MM_FOLD_NPAD * 65535 && encode_tiled() != nullptr;
 }
 
 TcPlan mmq_tc_plan(int64_t K, int64_t M, int64_t N, int sm_count) {

@@ -1114,7 +1114,7 @@ void mmq_tc8_configure() {
 }
 
 bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N) {
-    return K % 256 == 0 && K >= 256 && M >= 1 && N > GEMV_MAX_COLS && N <= (int64_t)tc8w::NW * 65535;   // column tiles are grid.y
+    return K % 256 == 0 && K >= 256 && M >= 1 && !few_column_faster(TLB_TYPE_Q8_0, K, M, N) && N <= (int64_t)tc8w::NW * 65535;   // column tiles are grid.y
 }
 
 TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count) {

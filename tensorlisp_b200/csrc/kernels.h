@@ -26,8 +26,21 @@ ActLayout act_layout(int kind, int64_t K, int64_t N);
 cudaError_t launch_quantize_rows(uint32_t type, const float *x, int64_t rows, int64_t n_per_row, void *y, cudaStream_t st);
 cudaError_t launch_act_quantize(const ActLayout &a, const float *x, int64_t ldx, void *out, cudaStream_t st);
 
-// Up to this many activation columns the few-column kernel (k_gemv.cu) is the faster one: its matrix instruction takes eight.
+// Columns that one launch of the few-column kernel (k_gemv.cu) takes: those of its matrix instruction.
 constexpr int64_t GEMV_MAX_COLS = 8;
+// Whether it is the faster one of a type that the tcgen05 kernels read too. Up to two columns: it quantizes its rows itself and takes
+// in the nodes around it. From three on a launch in front quantizes for both, and what remains is the time of a column more (0.7 us at 4096
+// weights a row) against that of a 16-column tile whatever is in it. Quantizer + product in us, k_gemv against k_mmq_tc_q4k / k_mmq_tc_q80:
+//   Q4_K [4096 x 4096]   3 columns 10.8 / 9.0, 5: 12.1 / 9.1, 8: 15.3 / 9.4     Q8_0   3: 11.3 / 12.8, 5: 12.2 / 12.6, 8: 14.5 / 13.0
+//   Q4_K [14336 x 4096]  3 columns 17.3 / 15.5, 5: 18.5 / 15.1, 8: 22.8 / 15.3  Q8_0   3: 21.7 / 21.3, 5: 22.6 / 20.6, 8: 24.0 / 20.6
+//   Q4_K [32000 x 4096]  3 columns 26.8 / 30.3, 5: 28.8 / 29.7, 8: 32.8 / 29.8
+//   Q4_K [128256 x 4096] 3 columns 63.0 / 88.3, 5: 64.7 / 87.2, 8: 70.9 / 88.3  Q8_0   3: 92.6 / 115, 5: 93.8 / 113, 8: 100 / 114
+//   eight decoder layers (4096 / 14336) and a vocabulary of 32000: Q4_K 3: 762 / 714, 5: 841 / 727, 8: 966 / 736; Q8_0 3: 748 / 1092, 8: 916 / 1103
+// Q4_K: a long stream hides the columns' cost, and the line moves with their number. Q8_0: k_mmq_tc_q80 has no groups and no gated or normed
+// quantizer in front, which costs a layer more than its products gain.
+inline bool few_column_faster(uint32_t type, int64_t K, int64_t M, int64_t N) {
+    return N <= 2 || (N <= GEMV_MAX_COLS && (type != TLB_TYPE_Q4_K || K * M >= 25000000 * (N + 1)));
+}
 
 // ---------------------------------------------------------------- k_mm.cu
 // Generic strided / batched product (any supported weight type, f32 activations or a quantized
@@ -42,7 +55,7 @@ struct MMGeneric {
 cudaError_t launch_mm_generic(const MMGeneric &p, const void *W, const void *X, void *Y, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_mmq_tc.cu
-// Q4_K weights x 5..64 activation columns on tcgen05 (f16 operands built from the integer codes).
+// Q4_K weights x activation columns on tcgen05, up to 64 of them (f16 operands built from the integer codes); more: k_mmq_tc_q8.cu.
 struct TcPlan {
     int npad, nsb, n_split, sb_per_split;
     int streamk;             // > 0: that many CTAs share all (row tile, super-block) units equally (k_mmq_tc.cu)
@@ -66,7 +79,7 @@ bool tc_available();
 cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsigned long long *ns, cudaStream_t st);   // the driver offers cuTensorMapEncodeTiled
 
 // ---------------------------------------------------------------- k_mmq_tc_q8.cu
-// Q8_0 weights x 5..32 activation columns on tcgen05 (kind::i8, one accumulator per 32-element block).
+// Q8_0 weights x activation columns on tcgen05 (kind::i8, one accumulator per 32-element block).
 bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N);
 TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_act_pack_tc8(const ActLayout &a, const void *act, int npad, void *blobs, cudaStream_t st);

@@ -55,8 +55,8 @@ TcPlan tc_plan(uint32_t wty, int64_t K, int64_t M, int64_t N, int sm) {
     return wty == TLB_TYPE_Q8_0 ? mmq_tc8_plan(K, M, N, sm) : mmq_tc_plan(K, M, N, sm);
 }
 
-// A product that the few-column kernel takes (k_gemv.cu): a 2-D matrix of whole super-blocks, at most eight columns, or any
-// number of them where no tensor-core kernel reads the type.
+// A product that the few-column kernel takes (k_gemv.cu): a 2-D matrix of whole super-blocks and the columns for which it is the faster
+// one (few_column_faster), or any number of them where no tensor-core kernel reads the type.
 bool gemv_node(const Graph &g, const Tensor &t) {
     if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || getenv("TLB_MM_GENERIC")) return false;
     const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];

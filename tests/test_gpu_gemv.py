@@ -59,3 +59,22 @@ def test_folded_nodes(oracle, ty, d, f, n):
     for y, w in zip(got[1:], ws[3:]):
         close(y.reshape(n, -1), oracle.mul_mat(ty, w, d, C), 2e-5)
     m.close()
+
+
+@pytest.mark.parametrize("K,M,N", [(28672, 3601, 3), (256, 488289, 4), (4096, 54945, 8)])
+def test_several_columns_of_a_long_stream(oracle, K, M, N):
+    """Q4_K from three columns on: the smallest matrices that few_column_faster leaves to this kernel."""
+    rng = np.random.default_rng(K + M + N)
+    assert 25_000_000 * (N + 1) <= K * M < 26_000_000 * (N + 1)
+    from tensorlisp_b200.native import Native, quantize_rows
+    native = Native(0)
+    Wq = quantize_rows(native, Q4_K, (rng.standard_normal((M, K), np.float32) * np.float32(0.02)))
+    native.close()
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q4_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    (got,) = m.run(X)
+    rows = np.unique(np.concatenate([[0, 15, 16, M - 1], rng.integers(0, M, 400)]))
+    close(got.reshape(N, M)[:, rows], oracle.mul_mat(Q4_K, np.ascontiguousarray(Wq.reshape(M, -1)[rows]), K, X), 2e-5)
+    m.close()
