@@ -176,8 +176,9 @@ __device__ __forceinline__ void store_blocks(const Params &p, uint8_t *act, int 
 }
 
 // The rows of this pass. RQ_READY: codes, scales and sums another launch has left in an ActLayout block. Otherwise they are
-// produced and quantized here: sums of squares in the order of k_row_quant_q8k (256 threads, stretches of 2048), so that the
-// fused and the separate launches agree in every bit.
+// produced and quantized here: sums of squares in the order of k_row_quant_q8k (256 threads, stretches of 2048), so that rows from
+// here and from the row quantizers agree in every bit. (k_norm, for a norm that is not folded, adds in another order: its scale may
+// differ by an ulp.)
 template <int TYPE>
 __device__ __forceinline__ void load_activations(const Params &p, uint8_t *act, float *red) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -19,7 +19,7 @@ import numpy as np
 import pytest
 
 from helpers import Model, NoisyOracle, close, make_decoder_weights, oracle_decoder_step
-from oracle.bindings import Q4_K
+from oracle.bindings import Q4_K, Q8_0
 from tensorlisp_b200 import graph as G
 from tensorlisp_b200.programs import DecoderConfig, decoder_step, swiglu_ffn
 
@@ -198,6 +198,41 @@ def _decode_step_case(oracle, cfg, ctx_before, max_ctx, noise_seeds):
     assert np.array_equal(out["logits"].argmax(axis=1)[decided], want.argmax(axis=1)[decided])
     m.close()
 
+
+
+@pytest.mark.parametrize("ty", [Q4_K, Q8_0])
+def test_a_deep_decoder_stays_at_f32_rounding_from_the_oracle(oracle, ty):
+    """32 layers for one sequence. The products are the oracle's integers, so the logits differ by the order of f32 additions only (1e-7),
+    unless that flips a code of some activation on the way: then by up to a few 1e-3, as the oracle's own logits do under 1e-7 noise on its
+    products. Most draws have no such flip; less precision anywhere would show in all of them."""
+    L, ctx = 32, 40
+    cfg = DecoderConfig(n_layers=L, d_model=512, n_heads=4, n_kv_heads=2, head_dim=128, d_ffn=1024, vocab=1000, wtype=ty)
+    dg = decoder_step(cfg, 1, 64, 4)
+    ids, pos = np.array([7], np.int32), np.array([ctx], np.int32)
+    far = []
+    for seed in range(5):
+        rng = np.random.default_rng(seed)
+        ws = []
+        for s in dg.weights:
+            if len(s.ne) == 1:
+                ws.append((1 + 0.1 * rng.standard_normal(s.ne[0])).astype(np.float32))
+                continue
+            # a residual stream that the layers change little, as a trained decoder's
+            std = 3.0 if s.name in ("token_embd", "output") else (0.02 / np.sqrt(2 * L) if s.name.endswith(("wo", "ffn_down")) else 0.02)
+            ws.append(oracle.quantize(s.ty, (rng.standard_normal((s.ne[1], s.ne[0])) * std).astype(np.float32)))
+        ks, vs = ([[rng.standard_normal((ctx + 1, 2, 128)).astype(np.float16)] for _ in range(L)] for _ in range(2))
+        m = Model(dg.graph, ws, dg.state_bytes, [("logits", dg.logits)])
+        for off, kv in zip(m.native.state_offsets, [x[0] for pair in zip(ks, vs) for x in pair]):
+            pool = np.zeros((4, 2, 16, 128), np.float16)
+            for i in range(ctx):
+                pool[i // 16, :, i % 16] = kv[i]
+            m.native.state.write(off, pool)
+        (got,) = m.run(ids, pos, np.arange(4, dtype=np.int32).reshape(1, 4), pos + 1, pos.astype(np.int64).view(np.int32))
+        m.close()
+        want = oracle_decoder_step(oracle, cfg, dg.weights, ws, ids, pos, ks, vs)
+        far.append(float(np.linalg.norm(got.reshape(want.shape) - want) / np.linalg.norm(want)))
+    print("deep decoder, relative distances from the oracle:", " ".join("%.1e" % f for f in far))
+    assert sorted(far)[2] <= 1e-6 and max(far) <= 1e-2, far
 
 
 def test_attention_quantizes_its_own_output(oracle):

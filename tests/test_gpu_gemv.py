@@ -78,3 +78,40 @@ def test_several_columns_of_a_long_stream(oracle, K, M, N):
     rows = np.unique(np.concatenate([[0, 15, 16, M - 1], rng.integers(0, M, 400)]))
     close(got.reshape(N, M)[:, rows], oracle.mul_mat(Q4_K, np.ascontiguousarray(Wq.reshape(M, -1)[rows]), K, X), 2e-5)
     m.close()
+
+
+def folded_block(ty, d, f, n, ws, wn):
+    g = G.Graph()
+    x, r = g.input(G.F32, [d, n], "x"), g.input(G.F32, [d, n], "r")
+    norm = g.weight(G.F32, [d], "norm")
+    gate, up, down, q, k, v = [g.weight(ty, [a, b], s) for s, a, b in (("gate", d, f), ("up", d, f), ("down", f, d), ("q", d, 96), ("k", d, 40), ("v", d, 24))]
+    h = g.add(x, r, "h")
+    t = g.mul(g.rms_norm(h, 1e-5), norm, "t")
+    y = g.mul_mat(down, g.glu(g.mul_mat(gate, t, "g"), b=g.mul_mat(up, t, "u"), name="a"), "y")
+    o = g.output(g.add(h, y, "o"))
+    c = g.cast(g.cast(o, G.F16), G.F32)
+    for w, s in ((q, "yq"), (k, "yk"), (v, "yv")):
+        g.output(g.mul_mat(w, c, s))
+    return Model(g, [wn] + ws)
+
+
+@pytest.mark.parametrize("ty", [Q4_K, Q8_0, Q4_0])
+@pytest.mark.parametrize("d,f", [(512, 768), (2048, 4864), (8448, 256), (4096, 2560)])
+def test_rows_quantized_in_the_launch_or_in_front_of_it(oracle, monkeypatch, ty, d, f):
+    """One and two columns produce and quantize their rows in the product's own launch, three get them from the row quantizers; the rows
+    they share come out the same to the last bit."""
+    rng = np.random.default_rng(d + f)
+    mk = lambda k, m: (rng.standard_normal((m, k)) * 0.02).astype(np.float32)
+    ws = [oracle.quantize(ty, mk(k, m)) for k, m in ((d, f), (d, f), (f, d), (d, 96), (d, 40), (d, 24))]
+    wn = (1 + 0.1 * rng.standard_normal(d)).astype(np.float32)
+    X, R = rng.standard_normal((2, 3, d)).astype(np.float32)
+    monkeypatch.setenv("TLB_NO_TC", "1")        # three columns stay on this kernel
+    seen = []
+    for n in (3, 1, 2):
+        m = folded_block(ty, d, f, n, ws, wn)
+        seen.append((n, m.program.dispatch_count(), [a.reshape(n, -1).copy() for a in m.run(X[:n], R[:n])]))
+        m.close()
+    assert seen[1][1] == seen[2][1] == 5 < seen[0][1]
+    for n, _, got in seen[1:]:
+        for a, b in zip(got, seen[0][2]):
+            assert a.tobytes() == b[:n].tobytes()
