@@ -505,7 +505,7 @@ def run_ours(args) -> dict:
     result = {
         "metric": METRIC, "value": BATCH / (ms_dev * 1e-3), "unit": "tok/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_dev, "higher_is_better": True, "scaling": "strong",
-        "vs_baseline": None, "dtype": "int8 codes: f16 / int8 tcgen05 mma and dp4a, f32 scales and accumulate", "data": "synthetic",
+        "vs_baseline": None, "dtype": "int8 codes: f16 / int8 tcgen05 mma, f32 scales and accumulate", "data": "synthetic",
         "config": {"workload": WORKLOAD, "kv": "paged f16 KV (16-token pages)",
                    "parallelism": "tp%d" % world, **({"allreduce": allreduce} if world > 1 else {}), "l2": "inputs larger than L2: %.2f GB weights + %.2f GB KV read per step per GPU"
                                                         % (ab["weights"] / 1e9, ab["kv"] / 1e9)},
@@ -692,9 +692,9 @@ def run_kernel(args) -> dict:
         rs = G.row_size(ty, K)
         copies = args.copies or max(2, int(300e6 // (rs * M)))
         ws = [g.weight(ty, [K, M], "W%d" % i) for i in range(copies)]
-        x = g.input(G.F32, [K, N], "x")
+        xs = [g.input(G.F32, [K, N], s) for s in ("x", "z")]     # in turn: products over one input share a launch
         for i, w in enumerate(ws):
-            g.output(g.mul_mat(w, x, "y%d" % i))
+            g.output(g.mul_mat(w, xs[i % 2], "y%d" % i))
         per = G.align256(rs * M)
         h = C.c_void_p()
         check(n.L.tlb_weights_create(n.dev, per * copies, C.byref(h)))
@@ -708,7 +708,8 @@ def run_kernel(args) -> dict:
             n.sync()
         n.alloc_states([])
         prog = NativeProgram.compile(n, g)
-        prog.set_input(0, rng.standard_normal((N, K)).astype(np.float32))
+        for i in range(2):
+            prog.set_input(i, rng.standard_normal((N, K)).astype(np.float32))
         bytes_per_launch = rs * M
         what = "%s weights [%d x %d], %d activation column(s)" % (spec[1], M, K, N)
     elif spec[0] == "ffn":
