@@ -1,10 +1,10 @@
-// MUL_MAT with block-quantized weights and up to eight activation columns (token generation for one or a few users):
+// MUL_MAT with Q8_0, Q4_0 or Q4_K weights and up to eight activation columns (token generation for one or a few users; k_gemv_f32.cu
+// has Q6_K, few_column_faster the line to the tcgen05 kernels):
 // every weight byte is read once, everything else hides behind that or is fixed cost.
 //
 // Arithmetic follows the reference's CPU backend (ggml-cpu.c:1272-1357): activations become int8 blocks, every output is an
 // integer dot product per block scaled in f32 (ggml-cpu/quants.c:451-479 for Q8_0, :225-260 for Q4_0, :696-770 for Q4_K); only
-// the order of the f32 additions differs. Q6_K weights meet the f32 activations themselves, decoded
-// (crates/kernels/src/cuda/native/mm.cu:16-42).
+// the order of the f32 additions differs.
 //
 // One kernel does what used to be three to six launches: the producer of the activation (residual add + RMS norm, gate, f16
 // cast), its quantizer, up to three matrices that read it, and SiLU(gate) * up behind a gate / up pair. At one column a

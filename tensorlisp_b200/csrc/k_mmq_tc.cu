@@ -1,4 +1,4 @@
-// Batched MUL_MAT (9..64 activation columns) with Q4_K weights on the 5th-generation tensor cores.
+// Batched MUL_MAT (up to 64 activation columns; few_column_faster says from how many on) with Q4_K weights on the 5th-generation tensor cores.
 //
 // Arithmetic (same integers as the reference's ggml-cpu path, vendor/ggml/src/ggml-cpu/quants.c:696-770):
 // the activations are the Q8_K codes q8 (k_quant.cu), the weights the 4-bit codes q with their 6-bit

@@ -1,4 +1,4 @@
-// Batched MUL_MAT (5 activation columns and up) with Q8_0 weights on the 5th-generation tensor cores:
+// Batched MUL_MAT (more than eight activation columns) with Q8_0 weights on the 5th-generation tensor cores:
 // the output projection of a decode step (vocab x d_model, Q8_0) is the largest matrix of the model.
 //
 // Arithmetic (same integers as the reference's ggml-cpu path, vendor/ggml/src/ggml-cpu/quants.c:451-479):
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // steps of 128 elements of K, which fit up to 192 columns; 1.2 with 64). So the tile's width is
 // chosen for the number of columns and row tiles at hand (fold_tile): 333 columns as 2 x 256 wasted a third of the MMAs,
 // and 8 row tiles x 2 left 132 SMs idle. Matrices that share the activations are one launch. Measured for 333 columns, Q4_K:
-// gate and up (14336 x 4096) 134 -> 75 us, [4096 x 14336] 100 -> 70, [4096 x 4096] 34 -> 23.
+// gate and up (14336 x 4096) 134 -> 75 us, [4096 x 14336] 100 -> 64, [4096 x 4096] 34 -> 22.
 namespace tc8f {
 constexpr int NW = MM_FOLD_NPAD;                         // widest column tile
 constexpr int MAX_MATS = 3;
