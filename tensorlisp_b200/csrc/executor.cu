@@ -708,7 +708,7 @@ tlb_status tlb_program_compile(tlb_device *dev, const tlb_graph *graph, const tl
         std::string detail;
     };
     std::vector<Missing> missing;
-    LowerCtx lc{dev, &p->graph, &p->layout};
+    LowerCtx lc{dev, &p->graph, &p->layout, writes_weights(p->graph)};
     for (size_t pos = 0; pos < G.nodes.size(); pos++) {
         try {
             lower_node(lc, G.nodes[pos], (int)pos, p->dispatches);

@@ -10,19 +10,11 @@
 
 namespace tlb {
 
-static bool writes_root(const Graph &g, int32_t id, int32_t root);
-
 namespace {
 
-// Whether the weights of a product may be copied while the kernel in front of it is still running: a weight leaf that no node of the
-// program writes to. (The kernel in front may be the one that makes any other operand: most release their dependents at their first line.)
-bool weights_settled(const Graph &g, int32_t w) {
-    w = g.root(w);
-    if (g.tensors[w].storage_kind != WEIGHT) return false;
-    for (int32_t id : g.nodes)
-        if (writes_root(g, id, w)) return false;
-    return true;
-}
+// Whether the weights of a product may be copied while the kernel in front of it is still running: a weight leaf, in a program of which no
+// node writes to one. (The kernel in front may be the one that makes any other operand: most release their dependents at their first line.)
+bool weights_settled(const LowerCtx &c, int32_t w) { return c.g->tensors[c.g->root(w)].storage_kind == WEIGHT && !c.weights_written; }
 
 [[noreturn]] void unsupported(const Tensor &t, const std::string &why) { throw Unsupported{t.op, t.name, why}; }
 
@@ -449,7 +441,7 @@ void lower_mul_mat(L &l) {
     const Place pw = l.place(w), px = l.place(x), pd = l.place(l.id);
     const int64_t K = tw.ne[0], M = tw.ne[1], N = tx.ne[1];
     const int sm = l.c.dev->prop.multiProcessorCount;
-    const bool early = weights_settled(*l.c.g, w);
+    const bool early = weights_settled(l.c, w);
     MMGeneric g{};
     g.wtype = tw.ty;
     g.w = view_of(tw);
@@ -533,7 +525,7 @@ void lower_gemv(L &l) {
     for (int j = 0; j < 3 && t.src[wslot[j]] >= 0; j++) {
         const int32_t y = j == 0 || p.glu ? l.id : l.src(yslot[j]);
         pw[j] = l.place(t.src[wslot[j]]);
-        p.early = p.early && weights_settled(*l.c.g, t.src[wslot[j]]);
+        p.early = p.early && weights_settled(l.c, t.src[wslot[j]]);
         py[j] = l.place(y);
         p.M[j] = p.ldy[j] = l.T(t.src[wslot[j]]).ne[1];
         p.n_mats++;
@@ -596,7 +588,7 @@ void lower_mul_mat_group(L &l) {
         if (tw.ty != wty || tw.ne[0] != K || tw.nb[1] != tw.row_size() || ty.ty != TLB_TYPE_F32 || !ty.is_contiguous() ||
             ty.ne[0] != tw.ne[1] || ty.ne[1] != N)
             throw std::string("a grouped mul_mat lost its shape invariants");
-        early = early && weights_settled(*l.c.g, w);
+        early = early && weights_settled(l.c, w);
         pw[j] = l.place(w);
         py[j] = l.place(y);
         Ms[j] = tw.ne[1];
@@ -1197,6 +1189,14 @@ static bool writes_root(const Graph &g, int32_t id, int32_t root) {
     if (t.op == "ROW_QUANT") return same(s[4]);
     if (t.op == "MUL_MAT_GROUP") return same(s[4]) || same(s[6]) || same(s[9]);
     return t.op == "MUL_MAT" && same(s[9]);
+}
+bool writes_weights(const Graph &g) {
+    int32_t leaf = -1;
+    for (size_t i = 0; i < g.tensors.size() && leaf < 0; i++)
+        if (g.tensors[i].storage_kind == WEIGHT && g.tensors[i].view_src < 0) leaf = (int32_t)i;
+    for (int32_t id : g.nodes)
+        if (leaf >= 0 && writes_root(g, id, leaf)) return true;
+    return false;
 }
 // Whether a node at a position in (after, before) writes to the storage of `id`: a read of it must not move across.
 static bool written_between(const Graph &g, const std::vector<char> &dead, int32_t id, int after, int before) {

@@ -172,7 +172,9 @@ struct LowerCtx {
     tlb_device *dev;
     const Graph *g;
     const Layout *layout;
+    bool weights_written;   // a node writes to a weight leaf (writes_weights)
 };
+bool writes_weights(const Graph &g);
 void lower_node(const LowerCtx &c, int32_t id, int pos, std::vector<Dispatch> &out);
 uint64_t node_scratch_bytes(const Graph &g, int32_t id, int sm_count);
 // comm.cu: sum over the ranks of the device's communicator, in place (no-op without one)
