@@ -601,7 +601,7 @@ TcPlan mmq_tc_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
     t.nsb = (int)(K / 256);
     if (N > 64 && !getenv("TLB_PROMPT_EXACT")) {
         // prompt-sized batches: the folded-scale GEMM of k_mmq_tc_q8.cu (weights dequantized to f16 in the kernel, one
-        // accumulator per 128 x 256 tile) instead of 64-column chunks with the reference's integer sums
+        // accumulator per tile) instead of 64-column chunks with the reference's integer sums
         t.npad = MM_FOLD_NPAD;
         t.n_split = 1;
         t.sb_per_split = t.nsb;
@@ -744,7 +744,7 @@ cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsi
 cudaError_t launch_mmq_tc_group(const TcPlan &t, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs,
                                 float *const *y, int64_t ldy, void *partial, int *err, cudaStream_t st, bool early, bool leave_partial) {
     if (t.npad == MM_FOLD_NPAD) {
-        return launch_mm_fold_f16(true, n_mats, W, K, M, N, blobs, y, ldy, err, st, early);
+        return launch_mm_fold_f16(true, n_mats, W, K, M, N, blobs, y, ldy, partial, err, st, early);
     }
     if (n_mats < 1 || n_mats > TC_MAX_MATS || (n_mats > 1 && t.n_col_chunks != 1)) return cudaErrorInvalidValue;
     if (t.n_split > 16) return cudaErrorInvalidValue;

@@ -591,24 +591,29 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // Each product carries two f16 roundings (2^-12 relative each, independent across k), so y differs from the reference's
 // integer arithmetic by about 1e-4 of max|y| at K = 4096: inside the 1e-3 bar of mul_mat, not bit-comparable. The exact
 // kernel above stays reachable (TLB_PROMPT_EXACT=1).
-// A persistent CTA walks (row tile, column tile) pairs, 128 weight rows x up to 256 (or 2 x 192) activation columns each. Per 256
-// elements of K: TMA brings 128 x 272 raw bytes; sixteen warps strip the scales, turn the codes into scaled f16 and store them into
-// tensor memory (A operand, 32 columns per 64 elements of K); the packed B arrives in bulk copies of 64 elements of K (core
-// matrix layout, 32 KB for 256 columns); one thread issues four MMAs of 128 x columns x 16 for each. Eight warps drain the
-// accumulator once per tile; tiles of at most 128 columns have two, so that the next tile's MMAs do not wait for that.
+// A pair of CTAs (the two SMs of a cluster, tcgen05 cta_group::2) walks items: a tile of 256 weight rows x up to 256 (or 2 x 192) activation
+// columns, or a stretch of its K. Per 256 elements of K each CTA brings its 128 rows of raw weights by TMA; sixteen warps strip the
+// scales, turn the codes into scaled f16 and store them into its tensor memory (A operand, 32 columns per 64 elements of K); each
+// CTA brings half of the tile's columns of the packed B (core matrix layout) and the matrix instruction reads both halves. One
+// thread of the pair issues four MMAs of 256 x columns x 16 per 64 elements of K. Eight warps per CTA drain its accumulator once
+// per item; tiles of at most 192 columns have two, so that the next item's MMAs do not wait for that.
 //
-// What bounds it: at 256 columns the tensor pipe with the copies of B (1.55 us per 256 elements of K; 2.15 while a whole warp probed
-// the barriers and issued), at narrow tiles the instructions and waits per step (1.03 us with
-// steps of 128 elements of K, which fit up to 192 columns; 1.2 with 64). So the tile's width is
-// chosen for the number of columns and row tiles at hand (fold_tile): 333 columns as 2 x 256 wasted a third of the MMAs,
-// and 8 row tiles x 2 left 132 SMs idle. Matrices that share the activations are one launch. Measured for 333 columns, Q4_K:
-// gate and up (14336 x 4096) 134 -> 75 us, [4096 x 14336] 100 -> 64, [4096 x 4096] 34 -> 22.
+// Why pairs: the copies of B bound wide tiles of single CTAs. 148 of them, each with the B of its own 128 rows, read 11 to 12.5 TB/s out
+// of L2 (2.4 us per unit of 256 elements of K at 336 columns, 1.55 at 256, whose MMAs take 1.45 and 1.1); the pair reads each
+// column once for 256 rows. Arrivals on the leader's barriers must not be of cluster scope: nothing but tensor memory and
+// copied shared memory passes between the CTAs, and a release of that scope made a unit 2.0 us instead of 1.15 at 64 columns.
+// The expanding warps fetch and expand before they wait for their slot (the wait, fetch, expansion and store as one chain took
+// 1000 cycles of a slot's round). Narrow tiles are bound by the expansion's instructions (404 per warp and unit for Q4_K, 268 for Q8_0, four
+// warps per scheduler); wide ones by the tensor pipe: 16384 columns run at 1400 to 1456 TFLOP/s (1253 to 1346 before).
+// The tile's width follows from rows, columns and the measured time of a unit; tiles that leave SMs idle are cut along K and their
+// parts added up by a second launch (mm_fold_plan). Matrices that share the activations are one launch. 333 columns, Q4_K, cold:
+// [4096 x 14336] 70 -> 50 us, gate and up (14336 x 4096) 86 -> 82, [4096 x 4096] 31 either way; 65 columns of [4096 x 14336] 68 -> 32.
 namespace tc8f {
 constexpr int NW = MM_FOLD_NPAD;                         // widest column tile
 constexpr int MAX_MATS = 3;
 constexpr int KS = 64;                                   // elements of K per B stage
 constexpr int HALF_NW = 192;                             // and of one of two that share their weights
-constexpr int MAX_STAGES = 8;
+constexpr int MAX_STAGES = 8, MAX_CUTS = 8;
 constexpr int SMEM = 226 * 1024;
 constexpr int TMA_RAW_WARP = 0, TMA_B_WARP = 1, MMA_WARP = 2;   // warp 3 idles (keeps the quadrant numbering of the rest aligned)
 constexpr int DEQ_WARP0 = 4, DEQ_WARPS = 16, EPI_WARP0 = 20, EPI_WARPS = 8;
@@ -667,12 +672,19 @@ __global__ void __launch_bounds__(256) k_act_pack_q80_f16(const int8_t *__restri
 struct Tc8fMaps {
     CUtensorMap m[tc8f::MAX_MATS];
 };
+// One pass of a pair: a tile's rows and columns and its stretch of K; part >= 0: the tile's sum is cut, this is its part's number.
+struct FoldItem {
+    int row_tile, col_tile, k0, k1, part;
+};
 struct Tc8fParams {
     const uint8_t *act;   // packed B operand
     float *out[tc8f::MAX_MATS];
+    float *part;          // [part][column of the tile][256 rows]
     int64_t M[tc8f::MAX_MATS], ldy[tc8f::MAX_MATS];
     int tile0[tc8f::MAX_MATS];   // first row tile of each matrix (past the end: not there)
-    int N, nst, row_tiles, col_tiles, nw, groups;   // nw: columns of a tile or of half of one
+    int N, nst, row_tiles, col_tiles, groups;
+    int nw, width;               // columns of a tile or of its first half; of a tile
+    int whole, cuts, items;      // tiles [whole, row_tiles * col_tiles) are cut into `cuts` stretches of K
     int raw_stages, b_stages;
     int *err;
     // Tile t: column tiles in bands of eight, the eight of a row tile one after the other. A band's share of B stays in L2 and the
@@ -681,6 +693,19 @@ struct Tc8fParams {
         const int per = row_tiles * 8, band = t / per, in = t - band * per, width = min(8, col_tiles - band * 8);
         row_tile = in / width;
         col_tile = band * 8 + in - row_tile * width;
+    }
+    __device__ __forceinline__ FoldItem item(int i) const {
+        FoldItem f{0, 0, 0, nst, -1};
+        int t = i;
+        if (i >= whole) {
+            f.part = i - whole;
+            const int c = f.part / cuts, s = f.part - c * cuts;
+            t = whole + c;
+            f.k0 = nst * s / cuts;
+            f.k1 = nst * (s + 1) / cuts;
+        }
+        at(t, f.row_tile, f.col_tile);
+        return f;
     }
     __device__ __forceinline__ int mat_of(int row_tile) const { return row_tile >= tile0[2] ? 2 : (row_tile >= tile0[1] ? 1 : 0); }
 };
@@ -704,40 +729,57 @@ __device__ __forceinline__ uint64_t twice(float x) {
     return r;
 }
 
-// the phase's state now, without waiting: a probe takes 100 to 300 cycles to answer, so the next one's goes out ahead of other work
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(tc::su32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
+// ---- what the two CTAs of a pair need of each other (rank 0 leads)
+__device__ __forceinline__ uint32_t pair_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
 }
-
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the shared-memory address of the leader's copy of `p`
+__device__ __forceinline__ uint32_t of_leader(const void *p) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(tc::su32(p)));
+    return r;
+}
+__device__ __forceinline__ void arrive_at(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t *dst_smem, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::su32(dst_smem)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t addr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+}
+// arrives on both CTAs' barrier at this offset once the MMAs issued so far are done
+__device__ __forceinline__ void pair_commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(tc::su32(bar)), "h"((uint16_t)3) : "memory");
+}
 // four MMAs over 64 elements of K: A 8 columns apart in tensor memory, B 16 (x 16 bytes) apart in shared memory; more = 0: the
-// first one starts the sum
-__device__ __forceinline__ void umma4_f16_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
+// first one starts the sum. 256 rows, 128 of each CTA; each CTA holds half of the columns of B.
+__device__ __forceinline__ void umma4_f16_pair(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\tsetp.eq.b32 q, 0, 0;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
         "add.u64 b1, %2, 16;\n\tadd.u64 b2, %2, 32;\n\tadd.u64 b3, %2, 48;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, q;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, q;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], b2, %3, q;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], b3, %3, q;\n\t}"
         ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more)
         : "memory");
 }
 
-// 64 weights (group j of a unit of 256) of one row as f16 into 32 tensor-memory columns.
+// 64 weights (group j of a unit of 256) of one row as f16 pairs, in the order of K.
 // Q8_0: two blocks of 34 bytes. Q4_K (one 144-byte super-block: f16 d, dmin, twelve bytes of 6-bit scales and mins, 128 bytes of
 // nibbles): f16(d * sc * q - dmin * m), dequantize_row_q4_K (ggml-quants.c); low nibbles are the first 32 values, high ones the rest.
 template <bool WQ4K>
-__device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t taddr) {
+__device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
     if constexpr (WQ4K) {
         const uint4 hdr = *reinterpret_cast<const uint4 *>(rrow);   // d, dmin, scales[12]
         // get_scale_min_k4 (ggml-quants.c:880-887), four sub-blocks at a time
@@ -748,7 +790,6 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t ta
         const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
         const uint64_t a0 = twice(__fmul_rn(d, (float)((sc4 >> sh) & 0xff))), b0 = twice(-__fmul_rn(dmin, (float)((mn4 >> sh) & 0xff)));
         const uint64_t a1 = twice(__fmul_rn(d, (float)((sc4 >> (sh + 8)) & 0xff))), b1 = twice(-__fmul_rn(dmin, (float)((mn4 >> (sh + 8)) & 0xff)));
-        uint32_t lo[16], hi[16];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const uint4 qv = *reinterpret_cast<const uint4 *>(rrow + 16 + j * 32 + u * 16);
@@ -762,10 +803,8 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t ta
                 hi[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(y, 0x64646464u, 0x4342), a1, b1);
             }
         }
-        tc::tmem_st16(taddr, lo);
-        tc::tmem_st16(taddr + 16, hi);
     } else {
-        uint32_t qa[8], qb[8], h[16];
+        uint32_t qa[8], qb[8];
         float da, db;
         if (j == 0) tc8::split_blocks<0>(rrow, qa, qb, da, db);
         else if (j == 1) tc8::split_blocks<1>(rrow, qa, qb, da, db);
@@ -774,33 +813,33 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t ta
         uint32_t dd = (uint32_t)__half_as_ushort(__float2half_rn(da));   // the block's own f16 scale, back from f32 unchanged
         dd |= dd << 16;
 #pragma unroll
-        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qa[i], dd, h[2 * i], h[2 * i + 1]);
-        tc::tmem_st16(taddr, h);
+        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qa[i], dd, lo[2 * i], lo[2 * i + 1]);
         dd = (uint32_t)__half_as_ushort(__float2half_rn(db));
         dd |= dd << 16;
 #pragma unroll
-        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qb[i], dd, h[2 * i], h[2 * i + 1]);
-        tc::tmem_st16(taddr + 16, h);
+        for (int i = 0; i < 8; i++) tc8f::codes_to_f16(qb[i], dd, hi[2 * i], hi[2 * i + 1]);
     }
 }
 
-// SHAPE 0: up to 192 columns, one accumulator or (up to 128) two in turn, steps of 128 elements of K; 1: up to 256 columns, steps of 64;
-// 2: two halves of nw columns, which share the expanded weights, accumulators [0, 192) and [192, 384), steps of 64. Behind the
-// accumulators lie four, eight or four A slots of a step each.
+// SHAPE 0: one accumulator of up to 256 columns or (up to 128) two in turn, steps of 128 elements of K; 1: two accumulators of up to 192
+// columns in turn, steps of 64; 2: two halves of up to 192 columns, which share the expanded weights, steps of 64. Behind the
+// accumulators lie four A slots of a step each.
 template <bool WQ4K, int SHAPE>
-__global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
     using namespace tc;
     using namespace tc8f;
     constexpr int ROWS = tc8::ROWS;
     constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
     constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
     constexpr int CT = SHAPE == 2 ? 2 : 1, STEP = SHAPE == 0 ? 2 : 1;   // halves; 64s of K in a step
-    constexpr uint32_t ACOLS = CT == 1 ? 256 : 2 * HALF_NW;   // first A column
+    constexpr uint32_t ACOLS = SHAPE == 0 ? 256 : 2 * HALF_NW;   // first A column
+    constexpr uint32_t ACC2 = SHAPE == 0 ? 128 : HALF_NW;        // second accumulator
     constexpr int A_RING = (512 - (int)ACOLS) / (32 * STEP);
-    const uint32_t IDESC = (1u << 4) | ((uint32_t)(p.nw >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B
+    constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(2 * ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B; columns / 8 at bit 17
+    const uint32_t idesc[2] = {IDESC0 | ((uint32_t)(p.nw >> 3) << 17), IDESC0 | ((uint32_t)((p.width - p.nw) >> 3) << 17)};
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
-    const int b_half = p.nw * KS * 2, b_stage = b_half * STEP;
+    const int b_half = p.nw / 2 * KS * 2, b_stage = b_half * STEP;   // this CTA's columns
     uint8_t *bst = smem;                                   // b_stages x b_stage
     uint8_t *raw = bst + p.b_stages * b_stage;             // raw_stages x RAW_BYTES
     __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[MAX_STAGES], bar_bfree[MAX_STAGES];
@@ -810,30 +849,30 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
     volatile int *fail = &s_fail;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nst = p.nst;   // units of 256 elements of K
-    const int n_tiles = p.row_tiles * p.col_tiles;
-    const uint32_t accs = SHAPE == 0 && p.nw <= 128 ? 2 : 1;   // accumulators in turn, 128 columns apart
+    const uint32_t rank = pair_rank();
+    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const uint32_t accs = SHAPE == 1 || (SHAPE == 0 && p.nw <= 128) ? 2 : 1;   // accumulators in turn
     if (tid == 0) {
         for (int i = 0; i < MAX_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
             mbar_init(&bar_rawfree[i], tc8f::DEQ_WARPS);
-            mbar_init(&bar_b[i], 1);
+            mbar_init(&bar_b[i], rank == 0 ? 2 : 1);   // the leader's: its own copy and word from the other CTA
             mbar_init(&bar_bfree[i], 1);
         }
         for (int i = 0; i < A_RING; i++) {
-            mbar_init(&bar_aready[i], 4 * STEP);
+            mbar_init(&bar_aready[i], 2 * 4 * STEP);
             mbar_init(&bar_afree[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&bar_accfull[i], 1);
-            mbar_init(&bar_accfree[i], tc8f::EPI_WARPS);
+            mbar_init(&bar_accfree[i], 2 * tc8f::EPI_WARPS);
         }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(&tmem_base_s, 512);
+    if (warp == 0) pair_tmem_alloc(&tmem_base_s, 512);
     tc_fence_before();
-    __syncthreads();
+    pair_sync();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     griddep_launch();
@@ -844,13 +883,12 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         if (lane == 0) {
             int s = 0;
             uint32_t ph = 0;
-            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-                int row_tile, col_tile;
-                p.at(t, row_tile, col_tile);
-                const int mat = p.mat_of(row_tile);
+            for (int t = pair; t < p.items; t += pairs) {
+                const FoldItem f = p.item(t);
+                const int mat = p.mat_of(f.row_tile);
                 const CUtensorMap *wmap = mat == 0 ? &maps.m[0] : (mat == 1 ? &maps.m[1] : &maps.m[2]);
-                const int row0 = (row_tile - p.tile0[mat]) * ROWS;
-                for (int i = 0; i < nst; i++) {
+                const int row0 = (f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 2 * ROWS + (int)rank * ROWS;
+                for (int i = f.k0; i < f.k1; i++) {
                     mbar_wait_nap(&bar_rawfree[s], ph ^ 1u, fail, 64);
                     mbar_expect_tx(&bar_raw[s], RAW_BYTES);
                     tma_2d(raw + s * RAW_BYTES, wmap, i * (ROW_CHUNK / 2), row0, &bar_raw[s]);   // x in 16-bit elements
@@ -862,20 +900,20 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             }
         }
     } else if (warp == tc8f::TMA_B_WARP) {
-        // ---- packed activations: four stages per unit and half (at the end only what there is: columns do not mix; a half
+        // ---- packed activations: this CTA's columns of each half (at the end only what there is: columns do not mix; a part
         // that is not there at all gets the last columns once more)
         if (lane == 0) {
             griddep_wait();
             int s = 0;
             uint32_t ph = 0;
-            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-                int row_tile, col_tile;
-                p.at(t, row_tile, col_tile);
-                for (int i = 0; i < nst * 4; i += STEP)
+            for (int t = pair; t < p.items; t += pairs) {
+                const FoldItem f = p.item(t);
+                for (int i = f.k0 * 4; i < f.k1 * 4; i += STEP)
 #pragma unroll
                     for (int ct = 0; ct < CT; ct++) {
-                        const int g0 = min((col_tile * CT + ct) * (p.nw / 8), p.groups - 1);
-                        const uint32_t bytes = (uint32_t)min(p.nw / 8, p.groups - g0) * 1024u;
+                        const int mine = (ct == 0 ? p.nw : p.width - p.nw) / 16;   // groups of eight columns
+                        const int g0 = min((f.col_tile * p.width + ct * p.nw) / 8 + (int)rank * mine, p.groups - 1);
+                        const uint32_t bytes = (uint32_t)min(mine, p.groups - g0) * 1024u;
                         mbar_wait_nap(&bar_bfree[s], ph ^ 1u, fail, 32);
                         mbar_expect_tx(&bar_b[s], bytes * STEP);
 #pragma unroll
@@ -889,51 +927,68 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             }
         }
     } else if (warp == tc8f::MMA_WARP) {
-        // ---- MMA issuer: one thread. Its own instructions are what bounds tiles of any width (a warp that probed and issued with all
-        // lanes: 750 cycles per 64 elements of K, of which the four MMAs of 256 columns need 512).
+        // ---- MMA issuer: one thread of the pair. Its own instructions are what bounds tiles of any width (a warp that probed and issued
+        // with all lanes: 750 cycles per 64 elements of K, of which the four MMAs of 256 columns need 512). The other CTA's thread
+        // passes on that its columns have arrived.
         if (elect_one()) {
             int bs = 0, as = 0;
             uint32_t bph = 0, aph = 0, it = 0;
-            const uint64_t b_desc0 = smem_desc(su32(bst), 128, 1024);
-            const uint32_t b_step = (uint32_t)b_stage >> 4;
-            uint32_t b_at = 0;
-            bool b_here = false, a_here = false;
-            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
-                const uint32_t ai = it % accs;
-                mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
-                uint32_t more = 0;
-#pragma unroll 1
-                for (int i = nst * 4 / STEP; i > 0; i--) {
-                    if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
-                    const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * (32u * STEP);
-                    uint64_t *const afree = &bar_afree[as];
-                    if (++as == A_RING) {
-                        as = 0;
-                        aph ^= 1u;
-                    }
-#pragma unroll
-                    for (int ct = 0; ct < CT; ct++) {
-                        if (!b_here) mbar_wait_nap(&bar_b[bs], bph, fail, 0);
-                        if (ct == 0) tc_fence_after();
-                        uint64_t *const bfree = &bar_bfree[bs];
-                        const uint64_t desc = b_desc0 + b_at;
-                        b_at += b_step;
+            if (rank != 0) {
+                const uint32_t lead = of_leader(bar_b);
+                for (int t = pair; t < p.items; t += pairs) {
+                    const FoldItem f = p.item(t);
+                    for (int i = (f.k1 - f.k0) * 4 / STEP * CT; i > 0; i--) {
+                        mbar_wait_nap(&bar_b[bs], bph, fail, 0);
+                        arrive_at(lead + (uint32_t)bs * 8u);
                         if (++bs == p.b_stages) {
                             bs = 0;
-                            b_at = 0;
                             bph ^= 1u;
                         }
-                        if (ct == CT - 1) a_here = mbar_test(&bar_aready[as], aph);
-                        b_here = mbar_test(&bar_b[bs], bph);
-#pragma unroll
-                        for (int k = 0; k < STEP; k++)
-                            umma4_f16_ta(tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ct * HALF_NW)), a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), IDESC, k ? 1u : more);
-                        umma_commit(bfree);
                     }
-                    umma_commit(afree);
-                    more = 1;
                 }
-                umma_commit(&bar_accfull[ai]);
+            } else {
+                const uint64_t b_desc0 = smem_desc(su32(bst), 128, 1024);
+                const uint32_t b_step = (uint32_t)b_stage >> 4;
+                uint32_t b_at = 0;
+                bool b_here = false, a_here = false;
+                for (int t = pair; t < p.items; t += pairs, it++) {
+                    const FoldItem f = p.item(t);
+                    const uint32_t ai = it % accs;
+                    mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
+                    uint32_t more = 0;
+#pragma unroll 1
+                    for (int i = (f.k1 - f.k0) * 4 / STEP; i > 0; i--) {
+                        if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
+                        const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * (32u * STEP);
+                        uint64_t *const afree = &bar_afree[as];
+                        if (++as == A_RING) {
+                            as = 0;
+                            aph ^= 1u;
+                        }
+#pragma unroll
+                        for (int ct = 0; ct < CT; ct++) {
+                            if (!b_here) mbar_wait_nap(&bar_b[bs], bph, fail, 0);
+                            if (ct == 0) tc_fence_after();
+                            uint64_t *const bfree = &bar_bfree[bs];
+                            const uint64_t desc = b_desc0 + b_at;
+                            b_at += b_step;
+                            if (++bs == p.b_stages) {
+                                bs = 0;
+                                b_at = 0;
+                                bph ^= 1u;
+                            }
+                            if (ct == CT - 1) a_here = mbar_test(su32(&bar_aready[as]), aph);
+                            b_here = mbar_test(su32(&bar_b[bs]), bph);
+#pragma unroll
+                            for (int k = 0; k < STEP; k++)
+                                umma4_f16_pair(tmem_base + (CT == 1 ? ai : (uint32_t)ct) * ACC2, a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), idesc[ct], k ? 1u : more);
+                            pair_commit(bfree);
+                        }
+                        pair_commit(afree);
+                        more = 1;
+                    }
+                    pair_commit(&bar_accfull[ai]);
+                }
             }
         }
         __syncwarp();
@@ -944,21 +999,26 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         const int q = warp & 3, j = (warp - tc8f::DEQ_WARP0) >> 2;
         const int r = q * 32 + lane;
         const uint32_t a_lane = tmem_base + ACOLS + ((uint32_t)(q * 32) << 16);
+        const uint32_t aready = of_leader(bar_aready);
         int s = 0, as = j / STEP;
         uint32_t ph = 0, aph = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x)
-            for (int i = 0; i < nst; i++) {
+        for (int t = pair; t < p.items; t += pairs) {
+            const FoldItem f = p.item(t);
+            for (int i = f.k1 - f.k0; i > 0; i--) {
                 mbar_wait_nap(&bar_raw[s], ph, fail, 64);
-                mbar_wait_nap(&bar_afree[as], aph ^ 1u, fail, 64);   // the MMAs that read this slot are done
+                uint32_t lo[16], hi[16];
+                expand64<WQ4K>(raw + s * RAW_BYTES + r * ROW_CHUNK, j, lo, hi);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_rawfree[s]);
+                mbar_wait_nap(&bar_afree[as], aph ^ 1u, fail, 0);   // the MMAs that read this slot are done
                 tc_fence_after();
-                expand64<WQ4K>(raw + s * RAW_BYTES + r * ROW_CHUNK, j, a_lane + (uint32_t)as * (32u * STEP) + (uint32_t)(j % STEP) * 32u);
+                const uint32_t to = a_lane + (uint32_t)as * (32u * STEP) + (uint32_t)(j % STEP) * 32u;
+                tmem_st16(to, lo);
+                tmem_st16(to + 16, hi);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&bar_aready[as]);
-                    mbar_arrive(&bar_rawfree[s]);
-                }
+                if (lane == 0) arrive_at(aready + (uint32_t)as * 8u);
                 as += 4 / STEP;
                 if (as >= A_RING) {
                     as -= A_RING;
@@ -969,29 +1029,34 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                     ph ^= 1u;
                 }
             }
+        }
     } else if (warp >= tc8f::EPI_WARP0) {
         // ---- draining warps, once per tile: lane quadrant warp % 4; of the two warps of a quadrant each takes every other 32
         // columns (CT = 1) or one of the halves (CT = 2)
         const int q = warp & 3, ch = (warp - tc8f::EPI_WARP0) >> 2;
-        const int row_in_tile = q * 32 + lane, chunks = (p.nw + 31) / 32;
+        const int row_in_tile = q * 32 + lane, nw = CT == 2 && ch ? p.width - p.nw : p.nw, chunks = nw / 32;
         const int c0 = CT == 1 ? ch : 0, step = CT == 1 ? 2 : 1;
+        const uint32_t accfree = of_leader(bar_accfree);
         uint32_t it = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, it++) {
-            int row_tile, col_tile;
-            p.at(t, row_tile, col_tile);
-            const int col0 = (CT == 1 ? col_tile : 2 * col_tile + ch) * p.nw, mat = p.mat_of(row_tile);
+        for (int t = pair; t < p.items; t += pairs, it++) {
+            const FoldItem f = p.item(t);
+            const int in_tile = CT == 1 ? 0 : ch * p.nw, col0 = f.col_tile * p.width + in_tile, mat = p.mat_of(f.row_tile);
             const uint32_t ai = it % accs;
-            const uint32_t lane_addr = tmem_base + (CT == 1 ? ai * 128u : (uint32_t)(ch * HALF_NW)) + ((uint32_t)(q * 32) << 16);
+            const uint32_t lane_addr = tmem_base + (CT == 1 ? ai : (uint32_t)ch) * ACC2 + ((uint32_t)(q * 32) << 16);
             mbar_wait_nap(&bar_accfull[ai], (it / accs) & 1, fail, 128);
             tc_fence_after();
-            const int64_t row = (int64_t)(row_tile - p.tile0[mat]) * ROWS + row_in_tile, M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]);
-            const int64_t ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
+            int64_t row = (int64_t)(f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 2 * ROWS + rank * ROWS + row_in_tile;
+            int64_t M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]), ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
             float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + (size_t)col0 * ldy + row;
+            if (f.part >= 0) {
+                ldy = 2 * ROWS;
+                o = p.part + ((size_t)f.part * p.width + in_tile) * ldy + rank * ROWS + row_in_tile;
+            }
             if (c0 >= chunks) {
-                if (lane == 0) mbar_arrive(&bar_accfree[ai]);
+                if (lane == 0) arrive_at(accfree + ai * 8u);
                 continue;
             }
-            const int cols = min(p.nw, p.N - col0);
+            const int cols = min(nw, p.N - col0);
 #pragma unroll 1
             for (int c = c0; c < chunks; c += step) {
                 uint32_t v[32];
@@ -1000,9 +1065,9 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                 if (c + step >= chunks) {   // everything of this warp's part is in registers: the accumulator may be overwritten
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_accfree[ai]);
+                    if (lane == 0) arrive_at(accfree + ai * 8u);
                 }
-                if (row < M) {
+                if (f.part >= 0 || row < M) {
 #pragma unroll
                     for (int j = 0; j < 32; j++)
                         if (c * 32 + j < cols) o[(size_t)(c * 32 + j) * ldy] = __uint_as_float(v[j]);
@@ -1010,41 +1075,88 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_base, 512);
+    pair_sync();   // neither CTA ends while the other one may still arrive on its barriers or read its columns
+    if (warp == 0) pair_tmem_dealloc(tmem_base, 512);
     if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
+// The parts of cut tiles, in the order of K. A thread: four rows of a column.
+__global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fParams p) {
+    griddep_launch();
+    griddep_wait();
+    const int r4 = threadIdx.x & 63, c = blockIdx.y * 4 + (threadIdx.x >> 6);
+    int row_tile, col_tile;
+    p.at(p.whole + (int)blockIdx.x, row_tile, col_tile);
+    const int64_t col = (int64_t)col_tile * p.width + c;
+    if (c >= p.width || col >= p.N) return;
+    const float4 *q = reinterpret_cast<const float4 *>(p.part) + ((size_t)blockIdx.x * p.cuts * p.width + c) * 64 + r4;
+    float4 v[tc8f::MAX_CUTS];
+#pragma unroll
+    for (int s = 0; s < tc8f::MAX_CUTS; s++) v[s] = s < p.cuts ? q[(size_t)s * p.width * 64] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+    for (int s = 1; s < tc8f::MAX_CUTS; s++) {
+        if (s >= p.cuts) break;
+        y[0] += v[s].x;
+        y[1] += v[s].y;
+        y[2] += v[s].z;
+        y[3] += v[s].w;
+    }
+    const int mat = p.mat_of(row_tile);
+    const int64_t row = (int64_t)(row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 256 + r4 * 4;
+    const int64_t M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]), ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
+    float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + col * ldy + row;
+    if (row + 4 <= M && ((uintptr_t)o & 15) == 0) {
+        *reinterpret_cast<float4 *>(o) = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (row + i < M) o[i] = y[i];
+    }
+}
+
+
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
-struct FoldTile {
-    int halves, nw;
-};
-// Halves of a tile and columns of each (a multiple of 16): of the even splits of N, the one whose slowest SM has the least to do.
-// Measured per unit of K: 1.03 us at 64 columns, 1.24 at 128, 1.3 at 192, 1.55 at 256; in halves 1.75 at 192 and 2.4 at 384, which pays where it
-// saves a wave (224 row tiles x 333 columns). Draining a tile without a second accumulator is about 1.2 us.
-static FoldTile fold_tile(int64_t N, int row_tiles, int nst, int sms) {
-    FoldTile f{1, 0};
+// Time of a unit (256 elements of K) of a tile in us. Measured, Q4_K / Q8_0: 1.15 / 0.90 at 64 columns, 1.23 / 1.00 at 128, 1.45 / 1.28 at 192,
+// 1.72 / 1.70 at 256, in halves 2.23 / 2.10 at 352.
+static double fold_unit_us(bool q4k, int width) { return q4k ? std::max(1.15, 0.55 + 0.0047 * width) : std::max(0.9, 0.35 + 0.005 * width); }
+// How a product is laid out over the pairs of SMs. Of the even splits of the columns into tiles, and of the cuts of the K of those tiles that
+// do not fill a wave, the one whose slowest pair has the least to do.
+FoldPlan mm_fold_plan(bool q4k, int n_mats, const int64_t *M, int64_t K, int64_t N, int sms) {
+    FoldPlan f{};
+    const int pairs = std::max(1, sms / 2), nst = (int)(K / 256);
+    int64_t row_tiles = 0;
+    for (int j = 0; j < n_mats; j++) row_tiles += (M[j] + 255) / 256;
     double best = 0;
     for (int halves = 1; halves <= 2; halves++) {
         const int widest = halves == 1 ? tc8f::NW : 2 * tc8f::HALF_NW;
         for (int64_t ct = (N + widest - 1) / widest, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
-            const int nw = (int)(((N + ct * halves - 1) / (ct * halves) + 15) / 16 * 16);
-            const int64_t tiles = (int64_t)row_tiles * ((N + halves * nw - 1) / (halves * nw)), waves = (tiles + sms - 1) / sms;
-            const double unit = halves == 2 ? std::max(1.75, 0.65 + 0.0046 * 2 * nw) : (nw <= 192 ? std::max(1.03, 0.88 + 0.0025 * nw) : 1.07 + 0.00185 * nw);
-            const double t = (double)waves * (nst * unit + (halves == 1 && nw <= 128 ? 0.3 : 1.2));
-            if (f.nw == 0 || t < best * 0.98) {
-                best = t;
-                f.halves = halves;
-                f.nw = nw;
+            const int width = (int)(((N + ct - 1) / ct + 31) / 32 * 32), nw = halves == 1 ? width : (width / 2 + 31) / 32 * 32;
+            if (nw == width && halves == 2) continue;
+            const int64_t tiles = row_tiles * ((N + width - 1) / width), full = tiles / pairs, rest = tiles % pairs;
+            const double unit = fold_unit_us(q4k, width), drain = halves == 1 && nw <= 192 ? 0.4 : 1.3;
+            for (int cuts = 1; cuts <= tc8f::MAX_CUTS && (cuts == 1 || (rest > 0 && cuts <= nst)); cuts++) {
+                const int64_t waves = (rest * cuts + pairs - 1) / pairs;
+                const double t = (double)full * (nst * unit + drain) + (double)waves * ((nst + cuts - 1) / cuts * unit + drain) +
+                                 (cuts > 1 ? 2.5 + (double)(rest * cuts) * width * 256 * 8 / 6.5e6 : 0);
+                if (f.width == 0 || t < best * 0.98) {
+                    best = t;
+                    f.nw = nw;
+                    f.width = width;
+                    f.cuts = cuts;
+                    f.whole = tiles - (cuts > 1 ? rest : 0);
+                    f.partial_bytes = cuts > 1 ? (uint64_t)(rest * cuts) * width * 256 * 4 : 0;
+                }
             }
         }
     }
     return f;
 }
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
-                               int64_t ldy, int *err, cudaStream_t st, bool early) {
+                               int64_t ldy, void *partial, int *err, cudaStream_t st, bool early) {
     if (n_mats < 1 || n_mats > tc8f::MAX_MATS) return cudaErrorInvalidValue;
     const int sms = current_sm_count();
     Tc8fMaps maps;
@@ -1061,27 +1173,37 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
         p.M[j] = M[j];
         p.ldy[j] = n_mats > 1 ? M[j] : ldy;
         p.tile0[j] = p.row_tiles;
-        p.row_tiles += (int)((M[j] + tc8::ROWS - 1) / tc8::ROWS);
+        p.row_tiles += (int)((M[j] + 255) / 256);
     }
     p.act = (const uint8_t *)blobs;
+    p.part = (float *)partial;
     p.N = (int)N;
     p.nst = (int)(K / 256);
-    const FoldTile tile = fold_tile(N, p.row_tiles, p.nst, sms);
-    p.nw = tile.nw;
+    const FoldPlan plan = mm_fold_plan(q4k, n_mats, M, K, N, sms);
+    if (plan.partial_bytes > 0 && partial == nullptr) return cudaErrorInvalidValue;
+    p.nw = plan.nw;
+    p.width = plan.width;
+    p.col_tiles = (int)((N + p.width - 1) / p.width);
+    const int tiles = p.row_tiles * p.col_tiles;
+    p.whole = (int)plan.whole;
+    p.cuts = plan.cuts;
+    p.items = p.whole + (tiles - p.whole) * p.cuts;
     // raw stages: 128 rows x 256 elements (18 or 34 KB); what they leave goes to B
     const int raw_bytes = tc8::ROWS * (q4k ? 144 : tc8::ROW_CHUNK);
-    p.raw_stages = q4k ? 4 : (tile.halves == 1 && p.nw <= 128 ? 3 : 2);
-    const bool narrow = tile.halves == 1 && p.nw <= 192;
-    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * (narrow ? 4 : 2)));
+    const int shape = p.width > p.nw ? 2 : (p.nw > 128 && p.nw <= tc8f::HALF_NW ? 1 : 0);
+    p.raw_stages = q4k ? 4 : 3;
+    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * (shape == 0 ? 2 : 1)));
     if (p.b_stages < 2) return cudaErrorInvalidValue;
     p.groups = mm_fold_groups(N);
-    p.col_tiles = (int)((N + tile.halves * p.nw - 1) / (tile.halves * p.nw));
     p.err = err;
-    const dim3 grid((unsigned)std::min(p.row_tiles * p.col_tiles, sms));
+    const dim3 grid((unsigned)(2 * std::min(p.items, std::max(1, sms / 2))));
     auto go = [&](auto *k) { return launch_pdl_if(early, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
-    if (tile.halves == 2) return q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
-    if (narrow) return q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);
-    return q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
+    cudaError_t e;
+    if (shape == 2) e = q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
+    else if (shape == 1) e = q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
+    else e = q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);
+    if (e != cudaSuccess || p.cuts == 1) return e;
+    return launch_pdl(k_fold_sum, dim3((unsigned)(tiles - p.whole), (unsigned)((p.width + 3) / 4)), dim3(256), 0, st, p);
 }
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st) {
     const char *ab = (const char *)act;
@@ -1191,7 +1313,7 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
     // described in 16-bit elements: a 272-byte box is 136 of them (the limit is 256 elements per dimension)
     cudaError_t e = tc_encode_2d(&map, W, (uint64_t)(K / 32 * 34), (uint64_t)M, tc8::ROW_CHUNK, tc8::ROWS, 2);
     if (e != cudaSuccess) return e;
-    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, err, st, early);
+    if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, partial, err, st, early);
     if (t.npad == tc8w::NW) {
         Tc8Params p{};
         p.act = (const uint8_t *)blobs;

@@ -96,7 +96,15 @@ inline __host__ __device__ size_t mm_fold_at(int n, int64_t k, int groups) {   /
 inline uint64_t mm_fold_bytes(int64_t K, int64_t N) { return (uint64_t)(K / 64) * mm_fold_groups(N) * 1024; }
 // n_mats matrices of one type that share the activations (y[j]: [column][M[j]]; of a single one [column][ldy])
 cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64_t K, const int64_t *M, int64_t N, const void *blobs, float *const *y,
-                               int64_t ldy, int *err, cudaStream_t st, bool early);
+                               int64_t ldy, void *partial, int *err, cudaStream_t st, bool early);
+// width: columns of a tile, nw: of its first half (all of them: one accumulator); tiles from `whole` on are cut into `cuts` stretches of K,
+// whose sums go to partial_bytes of scratch
+struct FoldPlan {
+    int nw, width, cuts;
+    int64_t whole;
+    uint64_t partial_bytes;
+};
+FoldPlan mm_fold_plan(bool q4k, int n_mats, const int64_t *M, int64_t K, int64_t N, int sm_count);
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_mm_plain.cu

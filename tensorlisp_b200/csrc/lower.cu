@@ -482,7 +482,7 @@ void lower_mul_mat(L &l) {
         const TcPlan tp = tc_plan(tw.ty, K, M, N, sm);
         if (tp.npad != l.T(qa).op_params[1]) throw std::string("activation blobs were packed for another column count");
         const int64_t sc = l.c.layout->scratch[l.pos];
-        if (tp.partial_bytes > 0 && sc < 0) throw std::string("split-K scratch was not planned");
+        if (node_scratch_bytes(*l.c.g, l.id, sm) > 0 && sc < 0) throw std::string("split-K scratch was not planned");
         Place ps;
         ps.buf = BUF_ARENA;
         ps.off = sc < 0 ? 0 : (uint64_t)sc;
@@ -600,7 +600,7 @@ void lower_mul_mat_group(L &l) {
     if (tp.npad != l.T(qa).op_params[1] || tp.n_col_chunks != 1) throw std::string("activation blobs were packed for another column count");
     const ActLayout a = act_layout(act_kind_for(wty), K, tx.nrows());
     const int64_t sc = l.c.layout->scratch[l.pos];
-    if (tp.partial_bytes > 0 && sc < 0) throw std::string("split-K scratch was not planned");
+    if (node_scratch_bytes(*l.c.g, l.id, sm) > 0 && sc < 0) throw std::string("split-K scratch was not planned");
     Place ps;
     ps.buf = BUF_ARENA;
     ps.off = sc < 0 ? 0 : (uint64_t)sc;
@@ -613,7 +613,7 @@ void lower_mul_mat_group(L &l) {
             W[j] = r.at(pw[j]);
             Y[j] = (float *)r.at(py[j]);
         }
-        if (wty == TLB_TYPE_Q8_0) return launch_mm_fold_f16(false, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.err, r.stream, early);
+        if (wty == TLB_TYPE_Q8_0) return launch_mm_fold_f16(false, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.at(ps), r.err, r.stream, early);
         return launch_mmq_tc_group(tp, n_mats, W, K, Ms, N, r.at(pq) + blob_off, Y, Ms[0], r.at(ps), r.err, r.stream, early);
     });
 }
@@ -1007,9 +1007,12 @@ uint64_t node_scratch_bytes(const Graph &g, int32_t id, int sm_count) {
     }
     if (t.op == "MUL_MAT_GROUP") {
         const Tensor &tx = g.tensors[t.src[1]];
-        int64_t Msum = 0;
+        int64_t Ms[3], Msum = 0;
+        int n_mats = 0;
         for (int s : {0, 3, 5})
-            if (t.src[s] >= 0) Msum += g.tensors[t.src[s]].ne[1];
+            if (t.src[s] >= 0) Msum += Ms[n_mats++] = g.tensors[t.src[s]].ne[1];
+        const uint32_t wty = g.tensors[t.src[0]].ty;
+        if (tc_plan(wty, tx.ne[0], Msum, tx.ne[1], sm_count).npad == MM_FOLD_NPAD) return mm_fold_plan(wty == TLB_TYPE_Q4_K, n_mats, Ms, tx.ne[0], tx.ne[1], sm_count).partial_bytes;
         return mmq_tc_plan(tx.ne[0], Msum, tx.ne[1], sm_count).partial_bytes;
     }
     if (plain_tc(g, t)) {
@@ -1020,8 +1023,10 @@ uint64_t node_scratch_bytes(const Graph &g, int32_t id, int sm_count) {
         g.tensors[t.src[2]].op_params[1] > 0) {
         // split-K partial sums of the tensor-core path
         const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
-        if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] == 1 && tc_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1]))
-            return tc_plan(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1], sm_count).partial_bytes;
+        if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] == 1 && tc_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1])) {
+            const TcPlan p = tc_plan(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1], sm_count);
+            return p.npad == MM_FOLD_NPAD ? mm_fold_plan(tw.ty == TLB_TYPE_Q4_K, 1, &tw.ne[1], tw.ne[0], tx.ne[1], sm_count).partial_bytes : p.partial_bytes;
+        }
     }
     return 0;
 }

@@ -26,3 +26,10 @@ def test_tiles(oracle, ty, K, M, N):
     for y, w, rows in zip(got, ws, M):
         close(y.reshape(N, rows), oracle.mul_mat(ty, w, K, X), 1e-3)
     m.close()
+
+
+# Few row tiles: their K is cut (into stretches of unequal length where it does not divide), a ragged last row tile and column tile among the parts.
+@pytest.mark.parametrize("ty", [Q4_K, Q8_0])
+@pytest.mark.parametrize("K,M,N", [(1792, [100], 65), (2816, [300, 40], 130), (5120, [257], 333), (4096, [513, 256, 31], 200), (3328, [1000], 390)])
+def test_cut_tiles(oracle, ty, K, M, N):
+    test_tiles(oracle, ty, K, M, N)
