@@ -603,8 +603,8 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 // column once for 256 rows. Arrivals on the leader's barriers must not be of cluster scope: nothing but tensor memory and
 // copied shared memory passes between the CTAs, and a release of that scope made a unit 2.0 us instead of 1.15 at 64 columns.
 // The expanding warps fetch and expand before they wait for their slot (the wait, fetch, expansion and store as one chain took
-// 1000 cycles of a slot's round). Narrow tiles are bound by the expansion's instructions (404 per warp and unit for Q4_K, 268 for Q8_0, four
-// warps per scheduler); wide ones by the tensor pipe: 16384 columns run at 1400 to 1456 TFLOP/s (1253 to 1346 before).
+// 1000 cycles of a slot's round). Narrow tiles are bound by the expansion's instructions (326 per warp and unit for Q4_K, 268 for Q8_0, four
+// warps per scheduler; 404 and 52 -> 47 us for gate and up of 14336 x 4096 at 128 columns while codes went through f32 one by one); wide ones by the tensor pipe: 16384 columns run at 1400 to 1456 TFLOP/s (1253 to 1346 before).
 // The tile's width follows from rows, columns and the measured time of a unit; tiles that leave SMs idle are cut along K and their
 // parts added up by a second launch (mm_fold_plan). Matrices that share the activations are one launch. 333 columns, Q4_K, cold:
 // [4096 x 14336] 70 -> 50 us, gate and up (14336 x 4096) 86 -> 82, [4096 x 4096] 31 either way; 65 columns of [4096 x 14336] 68 -> 32.
@@ -709,24 +709,26 @@ struct Tc8fParams {
     }
     __device__ __forceinline__ int mat_of(int row_tile) const { return row_tile >= tile0[2] ? 2 : (row_tile >= tile0[1] ? 1 : 0); }
 };
-// two weights: q * a - b in f32 (one rounding), then f16; q as the f16 1024 + q
-__device__ __forceinline__ uint32_t fold_pair(uint32_t q, uint64_t a, uint64_t nb) {
+// (v & mask) | 0x64006400: two codes of a word as the f16 pair 1024 + code (x 16 for high nibbles in place)
+__device__ __forceinline__ uint32_t code_pair(uint32_t v, uint32_t mask) {
     uint32_t r;
-    asm("{\n\t.reg .b16 l, h;\n\t.reg .f32 x, y;\n\t.reg .b64 p;\n\t"
-        "mov.b32 {l, h}, %1;\n\t"
-        "add.rn.f32.f16 x, l, 0fC4800000;\n\t"
-        "add.rn.f32.f16 y, h, 0fC4800000;\n\t"
-        "mov.b64 p, {x, y};\n\t"
-        "fma.rn.f32x2 p, p, %2, %3;\n\t"
-        "mov.b64 {x, y}, p;\n\t"
-        "cvt.rn.f16x2.f32 %0, y, x;\n\t}"
-        : "=r"(r) : "r"(q), "l"(a), "l"(nb));
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(r) : "r"(v), "r"(mask), "r"(0x64006400u));
     return r;
 }
-__device__ __forceinline__ uint64_t twice(float x) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
+// Four weights d * sc * q - b of the f16 pairs 1024 + (q0, q2) and 1024 + (q1, q3) in the order of K: sc * q is a whole number below
+// 946, exact in f16; the rest is one f32 rounding, then f16. (s, s0: sc and -1024 sc as pairs.)
+__device__ __forceinline__ void fold_four(uint32_t q02, uint32_t q13, uint32_t s, uint32_t s0, uint16_t d, float nb, uint32_t &w01, uint32_t &w23) {
+    asm("{\n\t.reg .b32 t, u;\n\t.reg .b16 t0, t1, t2, t3;\n\t.reg .f32 x0, x1, x2, x3;\n\t"
+        "fma.rn.f16x2 t, %2, %4, %5;\n\t"
+        "fma.rn.f16x2 u, %3, %4, %5;\n\t"
+        "mov.b32 {t0, t2}, t;\n\tmov.b32 {t1, t3}, u;\n\t"
+        "fma.rn.f32.f16 x0, t0, %6, %7;\n\t"
+        "fma.rn.f32.f16 x1, t1, %6, %7;\n\t"
+        "fma.rn.f32.f16 x2, t2, %6, %7;\n\t"
+        "fma.rn.f32.f16 x3, t3, %6, %7;\n\t"
+        "cvt.rn.f16x2.f32 %0, x1, x0;\n\t"
+        "cvt.rn.f16x2.f32 %1, x3, x2;\n\t}"
+        : "=r"(w01), "=r"(w23) : "r"(q02), "r"(q13), "r"(s), "r"(s0), "h"(d), "f"(nb));
 }
 
 // ---- what the two CTAs of a pair need of each other (rank 0 leads)
@@ -786,21 +788,33 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t (&
         const uint32_t sc4 = j < 2 ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
         const uint32_t mn4 = j < 2 ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
         const int sh = (j & 1) * 16;
-        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu)));
+        const uint16_t d = (uint16_t)hdr.x;
         const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        const uint64_t a0 = twice(__fmul_rn(d, (float)((sc4 >> sh) & 0xff))), b0 = twice(-__fmul_rn(dmin, (float)((mn4 >> sh) & 0xff)));
-        const uint64_t a1 = twice(__fmul_rn(d, (float)((sc4 >> (sh + 8)) & 0xff))), b1 = twice(-__fmul_rn(dmin, (float)((mn4 >> (sh + 8)) & 0xff)));
+        const float b0 = -__fmul_rn(dmin, (float)((mn4 >> sh) & 0xff)), b1 = -__fmul_rn(dmin, (float)((mn4 >> (sh + 8)) & 0xff));
+        // the scales as f16 pairs: 1024 + sc, less 1024; of the high nibbles (16 x code) a sixteenth
+        auto scale = [](uint32_t sc) {
+            const uint32_t v = (sc & 0xffu) | 0x6400u;
+            uint32_t r;
+            asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v | v << 16), "r"(0x64006400u));
+            return r;
+        };
+        auto times = [](uint32_t a, uint32_t f) {
+            uint32_t r;
+            asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(f));
+            return r;
+        };
+        const uint32_t s = scale(sc4 >> sh), s0 = times(s, 0xe400e400u);                             // x -1024
+        const uint32_t t16 = scale(sc4 >> (sh + 8)), t = times(t16, 0x2c002c00u), t0 = times(t16, 0xd400d400u);   // / 16, x -64
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const uint4 qv = *reinterpret_cast<const uint4 *>(rrow + 16 + j * 32 + u * 16);
             const uint32_t w4[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
             for (int wi = 0; wi < 4; wi++) {
-                const uint32_t x = w4[wi] & 0x0f0f0f0fu, y = (w4[wi] >> 4) & 0x0f0f0f0fu;
-                lo[(u * 4 + wi) * 2] = fold_pair(__byte_perm(x, 0x64646464u, 0x4140), a0, b0);
-                lo[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(x, 0x64646464u, 0x4342), a0, b0);
-                hi[(u * 4 + wi) * 2] = fold_pair(__byte_perm(y, 0x64646464u, 0x4140), a1, b1);
-                hi[(u * 4 + wi) * 2 + 1] = fold_pair(__byte_perm(y, 0x64646464u, 0x4342), a1, b1);
+                const uint32_t x = w4[wi], y = x >> 8;
+                const int at = (u * 4 + wi) * 2;
+                fold_four(code_pair(x, 0x000f000fu), code_pair(y, 0x000f000fu), s, s0, d, b0, lo[at], lo[at + 1]);
+                fold_four(code_pair(x, 0x00f000f0u), code_pair(y, 0x00f000f0u), t, t0, d, b1, hi[at], hi[at + 1]);
             }
         }
     } else {
@@ -1120,9 +1134,9 @@ __global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fPa
 
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
-// Time of a unit (256 elements of K) of a tile in us. Measured, Q4_K / Q8_0: 1.15 / 0.90 at 64 columns, 1.23 / 1.00 at 128, 1.45 / 1.28 at 192,
-// 1.72 / 1.70 at 256, in halves 2.23 / 2.10 at 352.
-static double fold_unit_us(bool q4k, int width) { return q4k ? std::max(1.15, 0.55 + 0.0047 * width) : std::max(0.9, 0.35 + 0.005 * width); }
+// Time of a unit (256 elements of K) of a tile in us. Measured, Q4_K / Q8_0: 1.02 / 0.90 at 64 columns, 1.10 / 1.00 at 128, 1.42 / 1.28 at 192,
+// 1.72 / 1.70 at 256, in halves 2.20 / 2.10 at 352.
+static double fold_unit_us(bool q4k, int width) { return q4k ? std::max(1.02, 0.50 + 0.0048 * width) : std::max(0.9, 0.35 + 0.005 * width); }
 // How a product is laid out over the pairs of SMs. Of the even splits of the columns into tiles, and of the cuts of the K of those tiles that
 // do not fill a wave, the one whose slowest pair has the least to do.
 FoldPlan mm_fold_plan(bool q4k, int n_mats, const int64_t *M, int64_t K, int64_t N, int sms) {
