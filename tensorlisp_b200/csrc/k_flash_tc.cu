@@ -2,13 +2,13 @@
 // optional f16 mask, no soft cap, no ALiBi; everything else takes k_flash.cu). Same arithmetic as k_flash.cu:
 // softmax(scale * f16(Q) K^T + mask) V with f16 operands, f32 scores, f32 running sums, P rounded to f16.
 //
-// Three launches per node:
-//   1. k_fa_pack_*: Q (f32 -> f16), K and V^T go into 32 KB blobs of 128 rows x 128 columns in the K-major core-matrix
+// Two launches per node:
+//   1. k_fa_pack: Q (f32 -> f16), K and V^T go into 32 KB blobs of 128 rows x 128 columns in the K-major core-matrix
 //      layout that tcgen05.mma reads from shared memory ([row / 8][16 chunks of 8 elements][row % 8][16 bytes]),
-//      so that the main kernel moves whole tiles with one bulk copy each and needs no transposition.
-//   2. k_fa_tile_flags: one byte per (query tile, key tile) of the mask: all -inf (the tile is skipped, the upper
-//      triangle of a causal mask), all zero (no mask values are read), or mixed.
-//   3. k_fa_tc: a CTA owns 128 queries of one (head, batch). Tensor memory holds two score accumulators S (128 columns
+//      so that the main kernel moves whole tiles with one bulk copy each and needs no transposition. Of the mask one byte per
+//      (query tile, key tile): all -inf (the tile is skipped, the upper triangle of a causal mask), all zero (no mask values are
+//      read), or mixed; where its rows do not start on 16 bytes, the mixed tiles once more with rows that do.
+//   2. k_fa_tc: a CTA owns 128 queries of one (head, batch). Tensor memory holds two score accumulators S (128 columns
 //      each), the output accumulator O (128 columns) and two P operands (f16, 64 columns each). One warp copies tiles,
 //      one issues MMAs (S = Q K^T: 8 x 128x128x16 from shared memory; O += P V: 8 x 128x128x16 with P read from tensor
 //      memory), eight warps do the softmax, two threads per query row with 64 score columns each: they pull their half
@@ -68,78 +68,145 @@ __device__ __forceinline__ int blob_off(int row, int c) { return (row >> 3) * 20
 }  // namespace fat
 
 // ---------------------------------------------------------------- operand packing
-// grid (query tile, head, batch): q f32 [D, nq, nh, nb] (strided) -> f16 blob; rows past nq are zero
-__global__ void __launch_bounds__(256) k_fa_pack_q(FlashArgs p, const uint8_t *__restrict__ q, uint8_t *__restrict__ out, int n_qt) {
-    griddep_launch();
-    griddep_wait();
-    const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-    uint8_t *o = out + (((size_t)b * p.nh + h) * n_qt + qt) * fat::TILE_BYTES;
-    const uint8_t *qb = q + (int64_t)h * p.q.nb[2] + (int64_t)b * p.q.nb[3];
-    for (int u = threadIdx.x; u < fat::T * 16; u += blockDim.x) {
-        const int row = u >> 4, c = u & 15, qr = qt * fat::T + row;
+// One launch: blocks [0, q_blocks) pack queries, the next kv_blocks keys and values, the rest look at the mask. (Three launches
+// cost a prompt of 333 tokens 6 us per node more.)
+struct FaPackParams {
+    FlashArgs f;
+    const uint8_t *q, *k, *v, *mask;
+    uint8_t *qp, *kp, *vt, *flags;
+    __half *mask_copy;   // null: the mask's own rows can be read by 16 bytes
+    int n_qt, n_kt, q_blocks, kv_blocks;
+};
+// A block packs 32 rows of a tile: two loads per thread and operand, all in flight at once (whole tiles: 9.6 us for 333 tokens of 32 + 8
+// heads, most of it the latency of a block's turns).
+constexpr int FA_PACK_ROWS = 32, FA_PACK_PARTS = fat::T / FA_PACK_ROWS;
+// (part, query tile, head, batch): q f32 [D, nq, nh, nb] (strided) -> f16 blob; rows past nq are zero
+__device__ __forceinline__ void fa_pack_q(const FaPackParams &a, int block) {
+    const FlashArgs &p = a.f;
+    const int row0 = block % FA_PACK_PARTS * FA_PACK_ROWS;
+    block /= FA_PACK_PARTS;
+    const int qt = block % a.n_qt, h = block / a.n_qt % p.nh, b = block / a.n_qt / p.nh;
+    uint8_t *o = a.qp + (size_t)((b * p.nh + h) * (int64_t)a.n_qt + qt) * fat::TILE_BYTES;
+    const uint8_t *qb = a.q + (int64_t)h * p.q.nb[2] + (int64_t)b * p.q.nb[3];
+#pragma unroll
+    for (int i = 0; i < FA_PACK_ROWS / 16; i++) {
+        const int row = row0 + i * 16 + (threadIdx.x >> 4), c = threadIdx.x & 15, qr = qt * fat::T + row;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (qr < p.nq) {
             const float *src = reinterpret_cast<const float *>(qb + (int64_t)qr * p.q.nb[1]) + c * 8;
-            const float4 a = *reinterpret_cast<const float4 *>(src), d = *reinterpret_cast<const float4 *>(src + 4);
-            v = make_uint4(fat::pack_h2(a.x, a.y), fat::pack_h2(a.z, a.w), fat::pack_h2(d.x, d.y), fat::pack_h2(d.z, d.w));
+            const float4 x = *reinterpret_cast<const float4 *>(src), y = *reinterpret_cast<const float4 *>(src + 4);
+            v = make_uint4(fat::pack_h2(x.x, x.y), fat::pack_h2(x.z, x.w), fat::pack_h2(y.x, y.y), fat::pack_h2(y.z, y.w));
         }
         *reinterpret_cast<uint4 *>(o + fat::blob_off(row, c)) = v;
     }
 }
-// grid (key tile, kv head, batch): k f16 [D, nkv, nhkv, nb] -> blob (rows = keys); v -> blob of V^T (rows = head
+// (part, key tile, kv head, batch): k f16 [D, nkv, nhkv, nb] -> blob (rows = keys); v -> blob of V^T (rows = head
 // dimensions, columns = keys). Keys past nkv are zero.
-__global__ void __launch_bounds__(256) k_fa_pack_kv(FlashArgs p, const uint8_t *__restrict__ k, const uint8_t *__restrict__ v,
-                                                     uint8_t *__restrict__ kout, uint8_t *__restrict__ vout, int n_kt) {
-    griddep_launch();
-    griddep_wait();
-    __shared__ __align__(16) __half vs[fat::T][fat::T + 8];
-    const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-    const size_t tile = (((size_t)b * p.nhkv + hk) * n_kt + kt) * fat::TILE_BYTES;
-    const uint8_t *kb = k + (int64_t)hk * p.k.nb[2] + (int64_t)b * p.k.nb[3];
-    const uint8_t *vb = v + (int64_t)hk * p.v.nb[2] + (int64_t)b * p.v.nb[3];
-    for (int u = threadIdx.x; u < fat::T * 16; u += blockDim.x) {
-        const int row = u >> 4, c = u & 15, key = kt * fat::T + row;
+__device__ __forceinline__ void fa_pack_kv(const FaPackParams &a, int block) {
+    const FlashArgs &p = a.f;
+    __shared__ __align__(16) __half vs[FA_PACK_ROWS][fat::T + 8];
+    const int row0 = block % FA_PACK_PARTS * FA_PACK_ROWS;
+    block /= FA_PACK_PARTS;
+    const int kt = block % a.n_kt, hk = block / a.n_kt % p.nhkv, b = block / a.n_kt / p.nhkv;
+    const size_t tile = (size_t)((b * p.nhkv + hk) * (int64_t)a.n_kt + kt) * fat::TILE_BYTES;
+    const uint8_t *kb = a.k + (int64_t)hk * p.k.nb[2] + (int64_t)b * p.k.nb[3];
+    const uint8_t *vb = a.v + (int64_t)hk * p.v.nb[2] + (int64_t)b * p.v.nb[3];
+#pragma unroll
+    for (int i = 0; i < FA_PACK_ROWS / 16; i++) {
+        const int row = row0 + i * 16 + (threadIdx.x >> 4), c = threadIdx.x & 15, key = kt * fat::T + row;
         uint4 kv = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
         if (key < p.nkv) {
             kv = *reinterpret_cast<const uint4 *>(kb + (int64_t)key * p.k.nb[1] + c * 16);
             vv = *reinterpret_cast<const uint4 *>(vb + (int64_t)key * p.v.nb[1] + c * 16);
         }
-        *reinterpret_cast<uint4 *>(kout + tile + fat::blob_off(row, c)) = kv;
-        *reinterpret_cast<uint4 *>(&vs[row][c * 8]) = vv;
+        *reinterpret_cast<uint4 *>(a.kp + tile + fat::blob_off(row, c)) = kv;
+        *reinterpret_cast<uint4 *>(&vs[row - row0][c * 8]) = vv;
     }
     __syncthreads();
-    for (int u = threadIdx.x; u < fat::T * 16; u += blockDim.x) {
-        const int d = u & 127, kc = u >> 7;   // consecutive threads take consecutive head dimensions of the same 8 keys
+#pragma unroll
+    for (int i = 0; i < FA_PACK_ROWS / 16; i++) {
+        const int d = threadIdx.x & 127, kc = i * 2 + (threadIdx.x >> 7);   // consecutive threads take consecutive head dimensions of the same 8 keys
         __half h[8];
 #pragma unroll
         for (int e = 0; e < 8; e++) h[e] = vs[kc * 8 + e][d];
-        *reinterpret_cast<uint4 *>(vout + tile + fat::blob_off(d, kc)) = *reinterpret_cast<const uint4 *>(h);
+        *reinterpret_cast<uint4 *>(a.vt + tile + fat::blob_off(d, row0 / 8 + kc)) = *reinterpret_cast<const uint4 *>(h);
     }
 }
-// grid (key tile, query tile, mask plane): 0 = every mask value of the tile is -inf, 1 = every one is zero, 2 = mixed
-__global__ void __launch_bounds__(256) k_fa_tile_flags(FlashArgs p, const uint8_t *__restrict__ mask, uint8_t *__restrict__ flags, int n_qt, int n_kt) {
-    griddep_launch();
-    griddep_wait();
-    const int kt = blockIdx.x, qt = blockIdx.y, plane = blockIdx.z;
+// (key tile, query tile, mask plane): 0 = every mask value of the tile is -inf, 1 = every one is zero, 2 = mixed. A thread takes eight
+// keys at a time, for all its rows before it looks at the first (15 us for 2048 x 2048 with a load of 2 bytes per turn).
+// Rows that do not start on 16 bytes (a number of keys that is no multiple of eight) are read by words here, once, and tiles that the
+// attention kernel reads again are left in rows that do.
+__device__ __forceinline__ void fa_mask_tile(const FaPackParams &a, int block) {
+    const FlashArgs &p = a.f;
+    const int kt = block % a.n_kt, qt = block / a.n_kt % a.n_qt, plane = block / a.n_kt / a.n_qt;
     const int m2 = plane % p.m_ne2, m3 = plane / p.m_ne2;
-    const uint8_t *mb = mask + (int64_t)m2 * p.m.nb[2] + (int64_t)m3 * p.m.nb[3];
+    const int c = threadIdx.x & 15, key = kt * fat::T + c * 8, row0 = threadIdx.x >> 4;
+    const uint8_t *mb = a.mask + (int64_t)m2 * p.m.nb[2] + (int64_t)m3 * p.m.nb[3] + (int64_t)key * 2;
+    const int have = min(8, p.nkv - key);   // keys of this thread
+    uint4 x[8];
+    // (no branches between the loads: with one per row and alignment this block took 10 us)
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uintptr_t r = (uintptr_t)mb + (int64_t)min(qt * fat::T + row0 + i * 16, p.nq - 1) * p.m.nb[1];
+        if (!a.mask_copy) {
+            x[i] = have >= 8 ? *reinterpret_cast<const uint4 *>(r) : make_uint4(0, 0, 0, 0);
+        } else {
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(r & ~(uintptr_t)3);
+            const uint32_t sh = (uint32_t)(r & 2) * 8;
+            uint32_t v[5];
+#pragma unroll
+            for (int e = 0; e < 5; e++) v[e] = have >= 8 && (e < 4 || sh) ? w[e] : 0u;   // whole words that hold a value of the row
+            x[i] = make_uint4(__funnelshift_r(v[0], v[1], sh), __funnelshift_r(v[1], v[2], sh), __funnelshift_r(v[2], v[3], sh), __funnelshift_r(v[3], v[4], sh));
+        }
+    }
+    if (have > 0 && have < 8) {   // the last keys of a row
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const __half *r = reinterpret_cast<const __half *>(mb + (int64_t)min(qt * fat::T + row0 + i * 16, p.nq - 1) * p.m.nb[1]);
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint32_t l = 2 * e < have ? __half_as_ushort(r[2 * e]) : 0u, h = 2 * e + 1 < have ? __half_as_ushort(r[2 * e + 1]) : 0u;
+                w[e] = l | h << 16;
+            }
+            x[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
     bool not_dead = false, not_plain = false;
-    for (int u = threadIdx.x; u < fat::T * fat::T; u += blockDim.x) {
-        const int row = u >> 7, col = u & 127, qr = qt * fat::T + row, key = kt * fat::T + col;
-        if (qr < p.nq && key < p.nkv) {
-            const unsigned short bits = __half_as_ushort(reinterpret_cast<const __half *>(mb + (int64_t)qr * p.m.nb[1])[key]);
-            not_dead |= bits != 0xfc00;
-            not_plain |= (bits & 0x7fff) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        if (qt * fat::T + row0 + i * 16 >= p.nq) continue;
+        const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const uint32_t bits = e & 1 ? w[e / 2] >> 16 : w[e / 2] & 0xffffu;
+            not_dead |= e < have && bits != 0xfc00u;
+            not_plain |= e < have && (bits & 0x7fffu) != 0;
         }
     }
     const int nd = __syncthreads_or(not_dead), np = __syncthreads_or(not_plain);
-    if (threadIdx.x == 0) flags[((size_t)plane * n_qt + qt) * n_kt + kt] = !nd ? 0 : (np ? 2 : 1);
+    if (threadIdx.x == 0) a.flags[((size_t)plane * a.n_qt + qt) * a.n_kt + kt] = !nd ? 0 : (np ? 2 : 1);
+    if (a.mask_copy && nd && np) {
+        const int64_t row_keys = (int64_t)a.n_kt * fat::T;
+        __half *o = a.mask_copy + ((int64_t)plane * a.n_qt + qt) * fat::T * row_keys + key;
+#pragma unroll
+        for (int i = 0; i < 8; i++) *reinterpret_cast<uint4 *>(o + (row0 + i * 16) * row_keys) = x[i];
+    }
+}
+__global__ void __launch_bounds__(256) k_fa_pack(const __grid_constant__ FaPackParams a) {
+    griddep_launch();
+    griddep_wait();
+    const int block = (int)blockIdx.x;
+    if (block < a.q_blocks) fa_pack_q(a, block);
+    else if (block < a.q_blocks + a.kv_blocks) fa_pack_kv(a, block - a.q_blocks);
+    else fa_mask_tile(a, block - a.q_blocks - a.kv_blocks);
 }
 
 // ---------------------------------------------------------------- the attention kernel
 struct FaTcParams {
     const uint8_t *qp, *kp, *vt, *flags, *mask;   // flags and mask null without a mask
-    TView m;
+    TView m;              // rows on 16-byte boundaries
+    int m_keys;           // keys that a mask row holds
     int m_ne2, m_ne3;
     float *out;
     int nq, nkv, nh, nhkv, nb, n_qt, n_kt;
@@ -288,7 +355,7 @@ __global__ void __launch_bounds__(fat::THREADS, 1) k_fa_tc(FaTcParams p) {
 #pragma unroll
             for (int i = 0; i < 64; i++) x[i] *= p.scale_log2;
             if (flag & 2) {
-                const bool full = key0 + 64 <= p.nkv;
+                const bool full = key0 + 64 <= p.m_keys;
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
                     uint4 v = make_uint4(0, 0, 0, 0);
@@ -404,18 +471,28 @@ __global__ void __launch_bounds__(fat::THREADS, 1) k_fa_tc(FaTcParams p) {
 static size_t fa_tc_smem() { return 5 * (size_t)fat::TILE_BYTES + 1024; }
 void flash_tc_configure() { cudaFuncSetAttribute(k_fa_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fa_tc_smem()); }
 
+// The mask with rows of whole key tiles, for masks whose rows do not start on 16-byte boundaries (333 keys, say). More than MASK_COPY_MAX (one
+// plane of 11585 x 11585) is left to k_flash.cu.
+constexpr uint64_t MASK_COPY_MAX = 256ull << 20;
+static bool mask_needs_copy(const FlashArgs &p) { return p.m.nb[1] % 16 || p.m.nb[2] % 16 || p.m.nb[3] % 16 || p.m_offset % 16; }
+static uint64_t mask_copy_bytes(const FlashArgs &p) {
+    const uint64_t qt = (p.nq + fat::T - 1) / fat::T, kt = (p.nkv + fat::T - 1) / fat::T;
+    return (uint64_t)p.m_ne2 * p.m_ne3 * qt * kt * fat::T * fat::T * 2;
+}
 bool flash_tc_supported(const FlashArgs &p, bool has_mask) {
     if (getenv("TLB_NO_FLASH_TC") || !tc_available()) return false;
     if (p.d != fat::T || p.dv != fat::T || p.k_ty != TLB_TYPE_F16 || p.v_ty != TLB_TYPE_F16 || p.softcap != 0.f || p.max_bias != 0.f) return false;
-    if (p.nq < 64 || p.nkv < 1 || (p.nkv + fat::T - 1) / fat::T > 512 || p.nh % p.nhkv != 0) return false;
+    // Few keys: the packing launch costs more than these tiles save. One node of 32 + 8 heads in us, this against k_flash.cu: 128 causal tokens
+    // 21.6 / 17.0, 160: 20.0 / 18.9, 192: 19.6 / 20.5, 333: 23.3 / 30.9, 1001: 47 / 116, 2041: 103 / 354; eight prompts of 160: 49.6 / 43.9, of 192:
+    // 50.7 / 51.3, of 256: 55.6 / 74.9.
+    if (p.nq < 64 || p.nkv <= 160 || (p.nkv + fat::T - 1) / fat::T > 512 || p.nh % p.nhkv != 0) return false;
     if (p.q.nb[1] % 16 || p.q.nb[2] % 16 || p.q.nb[3] % 16) return false;
-    if (has_mask && (p.m.nb[1] % 16 || p.m.nb[2] % 16 || p.m.nb[3] % 16)) return false;
-    return true;
+    return !has_mask || !mask_needs_copy(p) || mask_copy_bytes(p) <= MASK_COPY_MAX;
 }
 
 struct FaTcLayout {
     int n_qt, n_kt;
-    uint64_t q_off, k_off, v_off, f_off, bytes;
+    uint64_t q_off, k_off, v_off, f_off, m_off, bytes;
 };
 static FaTcLayout fa_tc_layout(const FlashArgs &p, bool has_mask) {
     FaTcLayout L;
@@ -425,7 +502,8 @@ static FaTcLayout fa_tc_layout(const FlashArgs &p, bool has_mask) {
     L.k_off = L.q_off + (uint64_t)p.nb * p.nh * L.n_qt * fat::TILE_BYTES;
     L.v_off = L.k_off + (uint64_t)p.nb * p.nhkv * L.n_kt * fat::TILE_BYTES;
     L.f_off = L.v_off + (uint64_t)p.nb * p.nhkv * L.n_kt * fat::TILE_BYTES;
-    L.bytes = L.f_off + (has_mask ? ((uint64_t)p.m_ne2 * p.m_ne3 * L.n_qt * L.n_kt + 255) / 256 * 256 : 0);
+    L.m_off = L.f_off + (has_mask ? ((uint64_t)p.m_ne2 * p.m_ne3 * L.n_qt * L.n_kt + 255) / 256 * 256 : 0);
+    L.bytes = L.m_off + (has_mask && mask_needs_copy(p) ? mask_copy_bytes(p) : 0);
     return L;
 }
 uint64_t flash_tc_scratch_bytes(const FlashArgs &p, bool has_mask) { return fa_tc_layout(p, has_mask).bytes; }
@@ -435,23 +513,41 @@ cudaError_t launch_flash_attn_tc(const FlashArgs &p, const void *q, const void *
     if (p.nq == 0 || p.nh == 0 || p.nb == 0) return cudaSuccess;
     const FaTcLayout L = fa_tc_layout(p, mask != nullptr);
     uint8_t *sc = (uint8_t *)scratch;
-    cudaError_t e = launch_pdl(k_fa_pack_q, dim3((unsigned)L.n_qt, (unsigned)p.nh, (unsigned)p.nb), dim3(256), 0, st, p, (const uint8_t *)q, sc + L.q_off, L.n_qt);
+    const bool copy = mask && mask_needs_copy(p);
+    FaPackParams k_args{};
+    k_args.f = p;
+    k_args.q = (const uint8_t *)q;
+    k_args.k = (const uint8_t *)k;
+    k_args.v = (const uint8_t *)v;
+    k_args.mask = (const uint8_t *)mask;
+    k_args.qp = sc + L.q_off;
+    k_args.kp = sc + L.k_off;
+    k_args.vt = sc + L.v_off;
+    k_args.flags = sc + L.f_off;
+    k_args.mask_copy = copy ? (__half *)(sc + L.m_off) : nullptr;
+    k_args.n_qt = L.n_qt;
+    k_args.n_kt = L.n_kt;
+    const int64_t q_blocks = (int64_t)L.n_qt * p.nh * p.nb * FA_PACK_PARTS, kv_blocks = (int64_t)L.n_kt * p.nhkv * p.nb * FA_PACK_PARTS,
+                  m_blocks = mask ? (int64_t)L.n_qt * L.n_kt * p.m_ne2 * p.m_ne3 : 0;
+    if (q_blocks + kv_blocks + m_blocks > INT32_MAX) return cudaErrorInvalidValue;
+    k_args.q_blocks = (int)q_blocks;
+    k_args.kv_blocks = (int)kv_blocks;
+    const cudaError_t e = launch_pdl(k_fa_pack, dim3((unsigned)(q_blocks + kv_blocks + m_blocks)), dim3(256), 0, st, k_args);
     if (e != cudaSuccess) return e;
-    e = launch_pdl(k_fa_pack_kv, dim3((unsigned)L.n_kt, (unsigned)p.nhkv, (unsigned)p.nb), dim3(256), 0, st, p, (const uint8_t *)k, (const uint8_t *)v,
-                   sc + L.k_off, sc + L.v_off, L.n_kt);
-    if (e != cudaSuccess) return e;
-    if (mask) {
-        e = launch_pdl(k_fa_tile_flags, dim3((unsigned)L.n_kt, (unsigned)L.n_qt, (unsigned)(p.m_ne2 * p.m_ne3)), dim3(256), 0, st, p, (const uint8_t *)mask,
-                       sc + L.f_off, L.n_qt, L.n_kt);
-        if (e != cudaSuccess) return e;
-    }
     FaTcParams a{};
     a.qp = sc + L.q_off;
     a.kp = sc + L.k_off;
     a.vt = sc + L.v_off;
     a.flags = mask ? sc + L.f_off : nullptr;
-    a.mask = (const uint8_t *)mask;
+    a.mask = copy ? sc + L.m_off : (const uint8_t *)mask;
     a.m = p.m;
+    a.m_keys = p.nkv;
+    if (copy) {
+        a.m_keys = L.n_kt * fat::T;
+        a.m.nb[1] = (int64_t)a.m_keys * 2;
+        a.m.nb[2] = a.m.nb[1] * L.n_qt * fat::T;
+        a.m.nb[3] = a.m.nb[2] * p.m_ne2;
+    }
     a.m_ne2 = p.m_ne2;
     a.m_ne3 = p.m_ne3;
     a.out = out;

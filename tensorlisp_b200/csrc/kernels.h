@@ -241,6 +241,7 @@ cudaError_t launch_pad(const PadArgs &p, const void *a, void *d, cudaStream_t st
 struct FlashArgs {
     TView q, k, v, m;
     int nq, nkv, nh, nhkv, nb, d, dv, m_ne2, m_ne3, n_head_log2;   // d: head size of queries and keys, dv: of values
+    uint64_t m_offset;   // of the mask in its buffer (a view)
     float scale, softcap, max_bias, m0, m1;   // scale already divided by softcap when that is set
     bool k_f32, v_f32;
     uint32_t k_ty, v_ty;   // ggml types of keys and values: f16 / f32 everywhere, bf16 and the block types on the one-query-per-CTA kernel

@@ -876,6 +876,7 @@ static const char *flash_args(const Graph &g, const Tensor &t, FlashArgs &p) {
         if (tm.ty != TLB_TYPE_F16 || tm.nb[0] != 2 || tm.ne[0] < tk.ne[1] || tm.ne[1] < tq.ne[1] || tm.ne[2] < 1 || tm.ne[3] < 1)
             return "the mask must be f16 [keys, >= queries, ...]";
         p.m = view_of(tm);
+        g.root(m, &p.m_offset);
         p.m_ne2 = (int)tm.ne[2];
         p.m_ne3 = (int)tm.ne[3];
     }

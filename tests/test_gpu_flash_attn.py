@@ -255,3 +255,10 @@ def test_few_queries_over_a_long_cache_split_the_keys(nq, nkv, nh, nhkv, nb):
     want = closed_form(q.astype(np.float16), k, v, mask, scale, 0.0, 0.0)
     close(got, want, TOL)
     close(got, plain, 5e-4)     # P is rounded to f16 against a different running maximum in the two schedules
+
+
+# Key counts that are no multiple of eight: mask rows on any 2-byte boundary, one plane and one per head and batch, tiles that are mixed, plain and dead.
+@pytest.mark.parametrize("case", [(128, 333, 333, 8, 2, 1, "causal", 0.0, 0.0, G.F16), (128, 130, 257, 4, 4, 2, "per_head", 0.0, 0.0, G.F16),
+                                  (128, 64, 177, 2, 1, 1, "causal", 0.0, 0.0, G.F16), (128, 257, 401, 4, 2, 2, "causal", 0.0, 0.0, G.F16)], ids=lambda c: str(c[:7]))
+def test_mask_rows_of_any_alignment_on_the_tensor_cores(case):
+    test_flash_attn_closed_form(case)
