@@ -179,6 +179,9 @@ tlb_status tlb_program_run(tlb_program *prog, tlb_buffer *const *weights, uint32
 tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, uint32_t n_weights, tlb_buffer *state);
 /* Program::read (exec.rs:228-239): bytes of a tensor that lives in the arena or the io buffer. */
 tlb_status tlb_program_read(tlb_program *prog, uint32_t tensor_id, uint64_t bytes, void *out);
+/* A result that has been read after earlier runs is written into pinned memory by the run itself. If the last run has done so for this
+ * tensor (64 KB to 2 MB), *out is that block, which becomes the caller's (tlb_host_free); NULL: use tlb_program_read. */
+tlb_status tlb_program_take(tlb_program *p, uint32_t tensor_id, uint64_t bytes, void **out);
 /* Program::dispatch_count / labels (exec.rs:81-88) */
 uint32_t   tlb_program_dispatch_count(tlb_program *prog);
 const char *tlb_program_label(tlb_program *prog, uint32_t i);

@@ -589,14 +589,14 @@ static std::string import_graph(const tlb_graph *graph, const tlb_leaves *leaves
 }
 
 // ------------------------------------------------------------------ the pinned page of a program
-// Inputs of at most IO_SMALL bytes wait in the page until the program's launch sequence fetches them (k_io_page):
-// a blocking copy of the same bytes takes 10 to 12 us, most of it the wait. Kept results of at most IO_SMALL bytes that
-// the caller reads after its runs are pushed into the page by the sequence itself. The sequence's kernels also write
+// Inputs of at most IO_IN_MAX bytes wait in the page until the program's launch sequence fetches them (k_io_page):
+// a blocking copy of the same bytes takes 10 to 12 us, most of it the wait. Kept results of at most IO_OUT_MAX bytes that
+// the caller reads after its runs are pushed by the sequence itself, the small ones into the page. Its kernels also write
 // their error word there, so run() needs no copy to see it.
-static bool is_small_out(const tlb_program *p, uint32_t tensor) {
+static bool is_pushed_out(const tlb_program *p, uint32_t tensor) {
     const Place pl = p->layout.place[tensor];
     const uint64_t n = p->graph.tensors[tensor].nbytes();
-    if (pl.buf != BUF_ARENA || pl.off % 16 || n == 0 || n > IO_SMALL) return false;
+    if (pl.buf != BUF_ARENA || pl.off % 16 || n == 0 || n > IO_OUT_MAX) return false;
     for (int32_t k : p->graph.keep)
         if ((uint32_t)k == tensor) return true;
     return false;
@@ -608,13 +608,18 @@ static bool page_create(tlb_program *p) {
     int n = 0;
     for (size_t i = 0; i < p->layout.inputs.size(); i++) {
         const uint64_t bytes = align_up(p->layout.inputs[i].second);
-        if (bytes == 0 || p->layout.inputs[i].second > IO_SMALL || at + bytes > in_end || n == IO_MAX_IN) continue;
+        if (bytes == 0 || p->layout.inputs[i].second > IO_IN_MAX || at + bytes > in_end || n == IO_MAX_IN) continue;
         p->in_host_off[i] = (uint32_t)at;
+        p->in_bytes += bytes;
         at += bytes;
         n++;
     }
     for (int32_t k : p->graph.keep)
-        if ((uint32_t)k < p->n_user_tensors && is_small_out(p, (uint32_t)k)) p->out_host_off = (uint32_t)at;
+        if ((uint32_t)k < p->n_user_tensors && is_pushed_out(p, (uint32_t)k)) {
+            const uint64_t bytes = p->graph.tensors[k].nbytes();
+            p->out_bytes += bytes;
+            if (bytes <= IO_OUT_SMALL) p->out_host_off = (uint32_t)at;
+        }
     if (p->out_host_off) at += IO_OUT_TOTAL;
     p->page = (IoPage *)pinned_alloc(at, PIN_LIBRARY);
     if (!p->page) return false;
@@ -628,7 +633,7 @@ static void page_in_use(tlb_program *p) { p->page_seq = ++p->dev->work; }
 static cudaError_t flush_inputs(tlb_program *p) {
     if (!p->in_dirty) return cudaSuccess;
     p->in_dirty = false;
-    const cudaError_t e = launch_fetch_inputs(p->page, p->io, p->dev->stream);
+    const cudaError_t e = launch_fetch_inputs(p->page, p->io, p->io_sync, p->in_bytes, p->dev->stream);
     page_in_use(p);
     return e;
 }
@@ -636,7 +641,7 @@ static cudaError_t flush_inputs(tlb_program *p) {
 static void push_table(tlb_program *p) {
     int n = 0;
     for (const auto &o : p->pushed)
-        p->page->out[n++] = {p->layout.place[o.tensor].off, o.host_off, (uint32_t)((o.bytes + 15) / 16)};
+        p->page->out[n++] = {p->layout.place[o.tensor].off, o.block ? (uint64_t)o.block : (uint64_t)p->page + o.host_off, (o.bytes + 15) / 16, 0};
     p->page->n_out = n;
 }
 // whether two tensors of the arena lie on common bytes: views of one tensor, or one that takes over another's place
@@ -646,13 +651,21 @@ static bool share_bytes(const tlb_program *p, uint32_t a, uint32_t b) {
     return pa.off < pb.off + p->graph.tensors[b].nbytes() && pb.off < pa.off + p->graph.tensors[a].nbytes();
 }
 static void push_add(tlb_program *p, uint32_t tensor, uint64_t bytes) {
-    if (!p->out_host_off || bytes != p->graph.tensors[tensor].nbytes() || !is_small_out(p, tensor) || p->pushed.size() >= IO_MAX_OUT) return;
+    if (bytes != p->graph.tensors[tensor].nbytes() || !is_pushed_out(p, tensor) || p->pushed.size() >= IO_MAX_OUT) return;
     for (uint32_t t : p->no_push)
         if (share_bytes(p, t, tensor)) return;
+    if (bytes > IO_OUT_SMALL) {
+        if (void *block = pinned_alloc(bytes, PIN_RESULT)) {   // (null: the caller keeps its results)
+            p->pushed.push_back({tensor, 0, block, bytes, p->runs + 1, 0});
+            push_table(p);
+        }
+        return;
+    }
     uint32_t at = p->out_host_off;   // first gap that holds it
     for (bool moved = true; moved;) {
         moved = false;
         for (const auto &o : p->pushed) {
+            if (o.block) continue;
             const uint32_t end = o.host_off + (uint32_t)align_up(o.bytes);
             if (at < end && o.host_off < at + align_up(bytes)) {
                 at = end;
@@ -661,13 +674,18 @@ static void push_add(tlb_program *p, uint32_t tensor, uint64_t bytes) {
         }
     }
     if (at + align_up(bytes) > p->out_host_off + IO_OUT_TOTAL) return;
-    p->pushed.push_back({tensor, at, bytes, p->runs + 1, 0});
+    p->pushed.push_back({tensor, at, nullptr, bytes, p->runs + 1, 0});
     push_table(p);
 }
-static void push_drop_unread(tlb_program *p) {
+static void push_drop(tlb_program *p, const std::function<bool(const tlb_program::Pushed &)> &which) {
     const size_t before = p->pushed.size();
-    p->pushed.erase(std::remove_if(p->pushed.begin(), p->pushed.end(), [](const tlb_program::Pushed &o) { return o.unread > 64; }), p->pushed.end());
+    for (const auto &o : p->pushed)
+        if (o.block && which(o)) pinned_free(o.block);
+    p->pushed.erase(std::remove_if(p->pushed.begin(), p->pushed.end(), which), p->pushed.end());
     if (p->pushed.size() != before) push_table(p);
+}
+static void push_drop_unread(tlb_program *p) {
+    push_drop(p, [](const tlb_program::Pushed &o) { return o.unread > 64; });
 }
 
 // ------------------------------------------------------------------ programs
@@ -735,7 +753,11 @@ tlb_status tlb_program_compile(tlb_device *dev, const tlb_graph *graph, const tl
         return bad(TLB_UNSUPPORTED, m);
     }
     cudaSetDevice(dev->ordinal);
-    cudaError_t e = cudaMalloc(&p->arena, std::max<uint64_t>(p->layout.arena_size, 1) + 256);
+    cudaError_t e = cudaMalloc(&p->arena, align_up(std::max<uint64_t>(p->layout.arena_size, 1)) + 256 + align_up(sizeof(IoSync)));
+    if (e == cudaSuccess) {
+        p->io_sync = (IoSync *)((char *)p->arena + align_up(std::max<uint64_t>(p->layout.arena_size, 1)) + 256);
+        e = cudaMemsetAsync(p->io_sync, 0, sizeof(IoSync), dev->stream);
+    }
     if (e == cudaSuccess) e = cudaMalloc(&p->io, std::max<uint64_t>(p->layout.io_size, 1));
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -791,6 +813,7 @@ void tlb_program_free(tlb_program *prog) {
     if (prog->page) {
         cudaDeviceSynchronize();   // the page goes back to the pool: no kernel may still write to it
         pinned_free(prog->page);
+        for (const auto &o : prog->pushed) pinned_free(o.block);
     }
     pinned_trim();
     delete prog;
@@ -812,8 +835,8 @@ tlb_status tlb_program_set_input(tlb_program *prog, uint32_t i, const void *byte
         IoPage *pg = prog->page;
         std::memcpy((char *)pg + at, bytes, n);
         int e = 0;
-        while (e < pg->n_in && pg->in[e].host_off != at) e++;
-        pg->in[e] = {in.first, at, (uint32_t)((n + 15) / 16)};
+        while (e < pg->n_in && pg->in[e].host != (uint64_t)pg + at) e++;
+        pg->in[e] = {in.first, (uint64_t)pg + at, (n + 15) / 16, 0};
         if (e == pg->n_in) pg->n_in = e + 1;
         prog->in_dirty = true;
     }
@@ -886,14 +909,15 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     for (auto &o : prog->pushed) o.unread++;
     if (idle) push_drop_unread(prog);
     // Small inputs come in, the launches, results that are read after every run go out. A captured sequence always has
-    // the two page kernels (their tables say what moves), a direct one launches them when there is something to move.
+    // the two page kernels that it may need (their tables say what moves), a direct one launches them when there is something to move.
     auto sequence = [&](bool captured, bool prof) {
         cudaError_t e = cudaSuccess;
         const bool any_in = std::any_of(prog->in_host_off.begin(), prog->in_host_off.end(), [](uint32_t o) { return o != 0; });
-        if (captured ? any_in : prog->in_dirty) e = launch_fetch_inputs(prog->page, prog->io, rc.stream);
+        const bool out = captured ? prog->out_bytes != 0 : !prog->pushed.empty();
+        if (out || (captured ? any_in : prog->in_dirty)) e = launch_fetch_inputs(prog->page, prog->io, prog->io_sync, prog->in_bytes, rc.stream);
         tlb_status s = e == cudaSuccess ? launch_all(prog, rc, prof) : fail(TLB_EXECUTION, "fetching inputs: " + cuda_msg(e));
-        if (s == TLB_OK && (captured ? prog->out_host_off != 0 : !prog->pushed.empty())) {
-            e = launch_push_outputs(prog->page, prog->arena, rc.stream);
+        if (s == TLB_OK && out) {
+            e = launch_push_outputs(prog->arena, prog->io_sync, prog->out_bytes, rc.stream);
             if (e != cudaSuccess) s = fail(TLB_EXECUTION, "pushing results: " + cuda_msg(e));
         }
         return s;
@@ -1042,15 +1066,34 @@ tlb_status tlb_program_read(tlb_program *prog, uint32_t tensor_id, uint64_t byte
     for (auto &o : prog->pushed)
         if (o.tensor == tensor_id && o.bytes == bytes && prog->runs >= o.valid_from) {
             TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
-            std::memcpy(out, (const char *)prog->page + o.host_off, bytes);
+            std::memcpy(out, o.block ? o.block : (const char *)prog->page + o.host_off, bytes);
             o.unread = 0;
             return TLB_OK;
         }
     if (pl.buf == BUF_IO) TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
     TLB_TRY_CUDA(copy_d2h(prog->ordinal, out, base + pl.off, bytes, prog->dev->stream), TLB_EXECUTION);
-    if (prog->out_host_off && bytes <= IO_SMALL && std::none_of(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; })) {
+    if (bytes <= IO_OUT_MAX && std::none_of(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; })) {
         TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
         push_add(prog, tensor_id, bytes);
+    }
+    return TLB_OK;
+}
+
+// A result that the last run has pushed into a pinned block: the block becomes the caller's.
+tlb_status tlb_program_take(tlb_program *prog, uint32_t tensor_id, uint64_t bytes, void **out) {
+    if (!prog || !out) return fail(TLB_INVALID, "tlb_program_take: bad arguments");
+    *out = nullptr;
+    for (auto &o : prog->pushed) {
+        if (o.tensor != tensor_id || o.bytes != bytes || !o.block || prog->runs < o.valid_from) continue;
+        cudaSetDevice(prog->dev->ordinal);
+        TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
+        *out = o.block;
+        o.block = pinned_alloc(bytes, PIN_RESULT);
+        o.valid_from = prog->runs + 1;
+        o.unread = 0;
+        if (o.block) push_table(prog);
+        else push_drop(prog, [](const tlb_program::Pushed &x) { return !x.block && x.bytes > IO_OUT_SMALL; });
+        return TLB_OK;
     }
     return TLB_OK;
 }
@@ -1072,8 +1115,7 @@ void *tlb_program_tensor_ptr(tlb_program *prog, uint32_t tensor_id, uint64_t *by
         // the caller may write there: what read() returns of any tensor on those bytes comes from the tensor itself from now on
         cudaSetDevice(prog->ordinal);
         if (page_idle(prog) == cudaSuccess) {
-            prog->pushed.erase(std::remove_if(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return share_bytes(prog, o.tensor, tensor_id); }), prog->pushed.end());
-            push_table(prog);
+            push_drop(prog, [&](const tlb_program::Pushed &o) { return share_bytes(prog, o.tensor, tensor_id); });
         }
         if (std::find(prog->no_push.begin(), prog->no_push.end(), tensor_id) == prog->no_push.end()) prog->no_push.push_back(tensor_id);
         return (char *)prog->arena + pl.off;

@@ -4,8 +4,9 @@
 // the B200 host: 443 us for 8 MB, 19 GB/s, and a fresh result array pays a page fault per 4 KB on top), and every
 // blocking copy ends with a stream synchronisation of 8 to 10 us however small it is. So large copies are staged by
 // several host threads into a pinned ring while the earlier chunks are on the link, results are read straight into
-// pinned arrays, and tensors of at most 64 KB make no copy call at all: they wait in a pinned page that a kernel at
-// the head (tail) of the program's launch sequence reads (writes) over the link.
+// pinned arrays, and inputs of at most 256 KB and results of at most 2 MB make no copy call at all: a kernel at the head of
+// the program's launch sequence reads them over the link from a pinned page, one at its tail writes them into pinned memory that the
+// caller then takes over.
 #include <emmintrin.h>
 
 #include <algorithm>
@@ -18,6 +19,7 @@
 #include <vector>
 
 #include "hostio.h"
+#include "pdl.cuh"
 
 namespace tlb {
 
@@ -227,7 +229,7 @@ constexpr uint64_t RING_CHUNK = 1 << 20;
 // Bytes per chunk and threads for a copy of n bytes: a chunk costs about 5 us of driver calls, and the link idles
 // until the first one is staged.
 uint64_t chunk_of(uint64_t n) { return n >= (16 << 20) ? RING_CHUNK : (n >= (2 << 20) ? 512 << 10 : 256 << 10); }
-int threads_of(uint64_t n) { return n >= (2 << 20) ? 4 : 1; }
+int threads_of(uint64_t n) { return n >= (2 << 20) ? 4 : (n >= (512 << 10) ? 2 : 1); }
 
 // memcpy with stores that bypass the caches (x86-64 baseline instructions)
 void stream_copy(char *d, const char *s, uint64_t n) {
@@ -393,19 +395,25 @@ __device__ __forceinline__ uint4 ld_host(const void *p) {
     return v;
 }
 
-// One CTA: at most 128 KB, and what it costs is two round trips over the link (the table, then the data: about
-// 1.5 us each), not bandwidth. All pieces of all entries are spread over the threads, four loads in flight each.
-template <bool IN>
-__global__ void __launch_bounds__(1024) k_io_page(IoPage *page, char *dev) {
-    constexpr int MAXN = IN ? IO_MAX_IN : IO_MAX_OUT;
-    __shared__ uint4 ent[MAXN];
+// What these cost is round trips over the link (the table, then the data: about 1.5 us each) and reads by many CTAs: those of
+// pinned memory queue up, 1.6 us for every CTA that reads the table. So few CTAs fetch, and the first of them leaves the table of the
+// results in device memory, where the CTAs of the second kernel find it: 8 KB each, 1 MB of results in 24 us (one CTA wrote 10 GB/s). The
+// fetch does not let its successors start early: beside its CTA a product's came to lie two to an SM (a [32000 x 4096] Q6_K product with its
+// inputs and results 57 -> 76 us, the feed-forward block of one token 43 -> 51).
+__global__ void __launch_bounds__(1024) k_io_fetch(IoPage *page, char *dev, IoSync *sync) {
+    __shared__ uint4 ent[IO_MAX_IN][2];
     __shared__ int s_n;
-    __shared__ uint32_t first[MAXN + 1];
+    __shared__ uint32_t first[IO_MAX_IN + 1];
     const int tid = threadIdx.x;
-    if (tid < MAXN) ent[tid] = ld_host(IN ? &page->in[tid] : &page->out[tid]);
-    if (tid == MAXN) {
-        const int n = *(volatile int *)(IN ? &page->n_in : &page->n_out);
-        s_n = n < 0 ? 0 : (n > MAXN ? MAXN : n);
+    if (tid < 2 * IO_MAX_IN) ent[tid >> 1][tid & 1] = ld_host(reinterpret_cast<const uint4 *>(page->in) + tid);
+    if (tid == 2 * IO_MAX_IN) {
+        const int n = *(volatile int *)&page->n_in;
+        s_n = n < 0 ? 0 : (n > IO_MAX_IN ? IO_MAX_IN : n);
+    }
+    if (blockIdx.x == 0 && tid >= 128) {
+        const int i = tid - 128;
+        if (i < 2 * IO_MAX_OUT) reinterpret_cast<uint4 *>(sync->out)[i] = ld_host(reinterpret_cast<const uint4 *>(page->out) + i);
+        if (i == 2 * IO_MAX_OUT) sync->n_out = *(volatile int *)&page->n_out;
     }
     __syncthreads();
     const int n = s_n;
@@ -413,14 +421,17 @@ __global__ void __launch_bounds__(1024) k_io_page(IoPage *page, char *dev) {
         uint32_t at = 0;
         for (int i = 0; i < n; i++) {
             first[i] = at;
-            at += ent[i].w;
+            at += ent[i][1].x;
         }
         first[n] = at;
+        if (gridDim.x == 1 || atomicAdd(&sync->in_done, 1u) == gridDim.x - 1) {   // every CTA has read the table
+            sync->in_done = 0;
+            *(volatile int *)&page->n_in = 0;
+        }
     }
     __syncthreads();
     const uint32_t total = first[n];
-    char *host = reinterpret_cast<char *>(page);
-    for (uint32_t i0 = tid; i0 < total; i0 += 4096) {
+    for (uint32_t i0 = blockIdx.x * 4096 + tid; i0 < total; i0 += gridDim.x * 4096) {
         uint4 v[4];
         char *to[4];
 #pragma unroll
@@ -430,31 +441,36 @@ __global__ void __launch_bounds__(1024) k_io_page(IoPage *page, char *dev) {
             if (i >= total) continue;
             int e = 0;
             while (i >= first[e + 1]) e++;
-            char *d = dev + ((uint64_t)ent[e].x | ((uint64_t)ent[e].y << 32)) + (uint64_t)(i - first[e]) * 16;
-            char *h = host + ent[e].z + (uint64_t)(i - first[e]) * 16;
-            v[u] = IN ? ld_host(h) : *reinterpret_cast<const uint4 *>(d);
-            to[u] = IN ? d : h;
+            to[u] = dev + ((uint64_t)ent[e][0].x | ((uint64_t)ent[e][0].y << 32)) + (uint64_t)(i - first[e]) * 16;
+            v[u] = ld_host(reinterpret_cast<const char *>((uint64_t)ent[e][0].z | ((uint64_t)ent[e][0].w << 32)) + (uint64_t)(i - first[e]) * 16);
         }
 #pragma unroll
         for (int u = 0; u < 4; u++)
             if (to[u]) *reinterpret_cast<uint4 *>(to[u]) = v[u];
     }
-    if (IN) {
-        if (tid == 0) *(volatile int *)&page->n_in = 0;
+}
+__global__ void __launch_bounds__(512) k_io_push(const char *dev, const IoSync *sync) {
+    griddep_wait();
+    const int n = min(max(sync->n_out, 0), IO_MAX_OUT);
+    for (int e = 0; e < n; e++) {
+        const IoPiece p = sync->out[e];
+        const uint4 *from = reinterpret_cast<const uint4 *>(dev + p.dev_off);
+        uint4 *to = reinterpret_cast<uint4 *>(p.host);
+#pragma unroll 2
+        for (uint64_t i = blockIdx.x * 512 + threadIdx.x; i < p.n16; i += gridDim.x * 512) to[i] = from[i];
     }
 }
 
 }  // namespace
 
-static_assert(sizeof(IoPiece) == 16, "an entry is one 16-byte load");
+static_assert(sizeof(IoPiece) == 32, "an entry is two 16-byte loads");
 
-cudaError_t launch_fetch_inputs(IoPage *page, void *io, cudaStream_t st) {
-    k_io_page<true><<<1, 1024, 0, st>>>(page, (char *)io);
+cudaError_t launch_fetch_inputs(IoPage *page, void *io, IoSync *sync, uint64_t bytes, cudaStream_t st) {
+    k_io_fetch<<<bytes > (64 << 10) ? 4 : 1, 1024, 0, st>>>(page, (char *)io, sync);
     return cudaGetLastError();
 }
-cudaError_t launch_push_outputs(IoPage *page, const void *arena, cudaStream_t st) {
-    k_io_page<false><<<1, 1024, 0, st>>>(page, (char *)const_cast<void *>(arena));
-    return cudaGetLastError();
+cudaError_t launch_push_outputs(const void *arena, const IoSync *sync, uint64_t bytes, cudaStream_t st) {
+    return launch_pdl(k_io_push, dim3((unsigned)std::max<uint64_t>(1, std::min<uint64_t>(64, (bytes + (8 << 10) - 1) / (8 << 10)))), dim3(512), 0, st, (const char *)arena, sync);
 }
 
 }  // namespace tlb

@@ -36,12 +36,14 @@ cudaError_t copy_d2h(int ordinal, void *dst, const void *src, uint64_t n, cudaSt
 
 // ---- a program's pinned page
 constexpr int IO_MAX_IN = 32, IO_MAX_OUT = 8;          // entries of the two tables
-constexpr uint64_t IO_SMALL = 64 << 10;                // a tensor of at most this many bytes travels through the page
-constexpr uint64_t IO_IN_TOTAL = 128 << 10, IO_OUT_TOTAL = 64 << 10;
+constexpr uint64_t IO_IN_MAX = 256 << 10, IO_IN_TOTAL = 512 << 10;      // an input of at most IO_IN_MAX bytes waits in the page
+constexpr uint64_t IO_OUT_SMALL = 64 << 10, IO_OUT_TOTAL = 64 << 10;    // a result of at most IO_OUT_SMALL goes there,
+constexpr uint64_t IO_OUT_MAX = 2 << 20;                                // one of at most this into a pinned block of its own (4 MB: no gain)
 struct IoPiece {
     uint64_t dev_off;    // byte offset in the program's io buffer (inputs) or arena (outputs), a multiple of 16
-    uint32_t host_off;   // byte offset in the page, a multiple of 16
-    uint32_t n16;        // 16-byte pieces
+    uint64_t host;       // address in pinned memory, a multiple of 16
+    uint64_t n16;        // 16-byte pieces
+    uint64_t pad;
 };
 struct IoPage {
     int err;             // error word of the program's kernels (bounded waits, indices out of range)
@@ -50,9 +52,16 @@ struct IoPage {
     IoPiece in[IO_MAX_IN];
     IoPiece out[IO_MAX_OUT];
 };
-// moves the n_in listed inputs from the page to the io buffer and sets n_in to 0
-cudaError_t launch_fetch_inputs(IoPage *page, void *io, cudaStream_t st);
-// moves the n_out listed outputs from the arena to the page
-cudaError_t launch_push_outputs(IoPage *page, const void *arena, cudaStream_t st);
+// In device memory, zero at first: CTAs of a fetch that have read the table, and the table of results that it found.
+struct IoSync {
+    uint32_t in_done;
+    int n_out, pad[6];
+    IoPiece out[IO_MAX_OUT];
+};
+// moves the n_in listed inputs from the page to the io buffer and sets n_in to 0 (bytes: what they may come to); takes over the
+// table of results
+cudaError_t launch_fetch_inputs(IoPage *page, void *io, IoSync *sync, uint64_t bytes, cudaStream_t st);
+// moves the listed outputs from the arena to pinned memory, as the fetch in front of it in the sequence found them listed
+cudaError_t launch_push_outputs(const void *arena, const IoSync *sync, uint64_t bytes, cudaStream_t st);
 
 }  // namespace tlb

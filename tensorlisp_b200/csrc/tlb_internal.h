@@ -214,6 +214,8 @@ struct tlb_program {
     bool need_state = false;
     // ---- the pinned page: error word, and the small inputs and results (hostio.h)
     tlb::IoPage *page = nullptr;
+    tlb::IoSync *io_sync = nullptr;      // behind the arena
+    uint64_t in_bytes = 0, out_bytes = 0;   // of inputs that wait in the page; of results that may be pushed
     std::vector<uint32_t> in_host_off;   // per input: where it waits in the page, 0 = it is copied instead
     uint32_t out_host_off = 0;           // where results start in the page, 0 = none is small enough
     bool in_dirty = false;               // inputs wait in the page that no fetch has been enqueued for
@@ -221,7 +223,8 @@ struct tlb_program {
     bool io_exposed = false;             // the caller holds an address in the io buffer: set_input then waits for its copy
     // results the caller reads after every run: pushed into the page at the end of the sequence
     struct Pushed {
-        uint32_t tensor, host_off;
+        uint32_t tensor, host_off;       // where in the page, or
+        void *block;                     // the pinned block of a larger one, which tlb_program_take hands to the caller
         uint64_t bytes, valid_from;      // first run that pushes it
         int unread;                      // runs since it was last read
     };

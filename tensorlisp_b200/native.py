@@ -41,6 +41,7 @@ class _HostBlock:
 
 
 _PINNED_FROM = 64 << 10     # smaller results come through the program's page: an ordinary array is as good
+_TAKEN_UP_TO = 2 << 20      # results up to here may lie in a block that the run has written
 
 
 def _result_bytes(nbytes: int) -> np.ndarray:
@@ -305,8 +306,15 @@ class NativeProgram:
                 shape.pop(0)
             known = self._result[(tensor, dtype)] = (T.nbytes(), dtype or _NP_OF.get(T.ty), tuple(shape))
         n, dt, shape = known
-        out = _result_bytes(n)
-        check(self.native.L.tlb_program_read(self.h, tensor, n, _address(out)))
+        out = None
+        if _PINNED_FROM < n <= _TAKEN_UP_TO:
+            p = C.c_void_p()
+            check(self.native.L.tlb_program_take(self.h, tensor, n, C.byref(p)))
+            if p.value:
+                out = np.asarray(_HostBlock(p.value, n))
+        if out is None:
+            out = _result_bytes(n)
+            check(self.native.L.tlb_program_read(self.h, tensor, n, _address(out)))
         return out if dt is None else out.view(dt).reshape(shape)
 
     def outputs(self) -> list[tuple[str, np.ndarray]]:

@@ -102,6 +102,38 @@ def test_a_known_device_address_sees_every_input_and_every_result():
     native.close()
 
 
+@pytest.mark.parametrize("n", [16385, 65536, 524288])
+def test_a_result_that_the_run_has_written_is_handed_over_once(n):
+    """Above 64 KB a result comes in the block that the run has written: a second read() of the same run, reads behind runs that were not
+    waited for, and arrays that are kept (no block is left at some point) all see their own run's values."""
+    native = Native.load([])
+    g = G.Graph()
+    x, z = g.input(G.F32, [n], "x"), g.input(G.F32, [4], "z")
+    y, w = g.output(g.scale(x, 2.0)), g.output(g.scale(x, 3.0))
+    prog = NativeProgram.compile(native, g)
+    rng = np.random.default_rng(n)
+    kept = []
+    for i in range(12):
+        a = rng.standard_normal(n).astype(np.float32)
+        prog.set_input(0, a)
+        prog.enqueue()
+        if i % 3 == 0:
+            prog.enqueue()
+        got = [prog.read(y), prog.read(w), prog.read(y)]
+        for r, f in zip(got, (2, 3, 2)):
+            assert np.array_equal(r.reshape(-1), f * a)
+        got[2][...] = -1        # the caller's to write to
+        assert np.array_equal(prog.read(y).reshape(-1), 2 * a)
+        if i >= 4:
+            kept.append((got[:2], a))
+    for got, a in kept:
+        assert np.array_equal(got[0].reshape(-1), 2 * a) and np.array_equal(got[1].reshape(-1), 3 * a)
+    prog.free()
+    for got, a in kept:
+        assert np.array_equal(got[0].reshape(-1), 2 * a)
+    native.close()
+
+
 @pytest.mark.parametrize("held", ["a view", "the tensor of a view", "the tensor itself"])
 def test_an_address_into_a_result_through_another_tensor_of_its_storage(held):
     """Who holds the address of a view writes into the root's memory (and the other way round): what read() returns then comes from
