@@ -371,15 +371,41 @@ __global__ void __launch_bounds__(128) k_paged_reduce(PagedParams p) {
     const int ctx = paged_ctx(p, seq);
     const int valid = ctx > 0 ? min(p.n_chunks, (ctx + p.chunk_tokens - 1) / p.chunk_tokens) : 0;
     const float *pp = p.partial + ((size_t)seq * p.heads + head) * p.n_chunks * (HS + 2);
-    float m = -CUDART_INF_F;
-    for (int c = 0; c < valid; c++) m = fmaxf(m, pp[(size_t)c * (HS + 2)]);
-    const float mu = m == -CUDART_INF_F ? 0.f : m;
     for (int d = threadIdx.x; d < HS; d += blockDim.x) {
+        // sixteen chunks' (max, sum) and values on their way at once: a chunk at a time is a chain of trips to L2 (8 us for sixteen)
+        constexpr int B = 16;
+        float2 ml[B];
+        float o[B];
+        auto fetch = [&](int c0) {
+#pragma unroll
+            for (int u = 0; u < B; u++) {
+                const float *q = pp + (size_t)min(c0 + u, p.n_chunks - 1) * (HS + 2);
+                const bool live = c0 + u < valid;
+                ml[u] = live ? *reinterpret_cast<const float2 *>(q) : make_float2(-CUDART_INF_F, 0.f);
+                o[u] = live ? q[2 + d] : 0.f;
+            }
+        };
+        fetch(0);
+        float m = -CUDART_INF_F;
+#pragma unroll
+        for (int u = 0; u < B; u++) m = fmaxf(m, ml[u].x);
+        for (int c0 = B; c0 < valid; c0 += B) {
+            float x[B];
+#pragma unroll
+            for (int u = 0; u < B; u++) x[u] = c0 + u < valid ? pp[(size_t)(c0 + u) * (HS + 2)] : -CUDART_INF_F;
+#pragma unroll
+            for (int u = 0; u < B; u++) m = fmaxf(m, x[u]);
+        }
+        const float mu = m == -CUDART_INF_F ? 0.f : m;
         float l = 0.f, a = 0.f;
-        for (int c = 0; c < valid; c++) {
-            const float f = exp2f(pp[(size_t)c * (HS + 2)] - mu);
-            l += pp[(size_t)c * (HS + 2) + 1] * f;
-            a += pp[(size_t)c * (HS + 2) + 2 + d] * f;
+        for (int c0 = 0; c0 < valid; c0 += B) {
+            if (c0 > 0) fetch(c0);
+#pragma unroll
+            for (int u = 0; u < B; u++) {
+                const float f = exp2f(ml[u].x - mu);   // 0 past the last chunk
+                l += ml[u].y * f;
+                a += o[u] * f;
+            }
         }
         p.out[((size_t)seq * p.heads + head) * HS + d] = __float2half_rn(l > 0.f ? a / l : 0.f);
     }

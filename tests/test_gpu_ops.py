@@ -363,3 +363,39 @@ def test_entry_cache_compiles_per_shape_and_converts_i32_inputs():
         cache.run("lookup", [np.array([0.5, 1, 2], np.float32), np.zeros((2, 64), np.float32)])
     cache.free()
     n.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 4095, 4096, 4097, 9000])
+def test_norms_around_the_rows_that_stay_in_registers(n):
+    """Rows of up to 4096 values stay in registers; longer ones are read again. Weights of the row's length and of a divisor of it."""
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((3, n)) * 2 + 0.5).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(n)).astype(np.float32)
+    g = G.Graph()
+    tx, tw = g.input(G.F32, [n, 3], "x"), g.weight(G.F32, [n], "w")
+    outs = [g.output(g.rms_norm(tx, 1e-5)), g.output(g.norm(tx, 1e-5)), g.output(g.mul(g.rms_norm(tx, 1e-6), tw))]
+    m = Model(g, [w], outputs=[("a", outs[0]), ("b", outs[1]), ("c", outs[2])])
+    a, b, c = (v.reshape(3, n) for v in m.run(x))
+    d = x.astype(np.float64)
+    rms = lambda e: d / np.sqrt((d * d).mean(1, keepdims=True) + e)
+    mean = d.mean(1, keepdims=True)
+    # sums of n squares in f32: n / 256 additions per thread and 13 across them, a few units in the last place
+    for got, want in ((a, rms(1e-5)), (b, (d - mean) / np.sqrt(((d - mean) ** 2).mean(1, keepdims=True) + 1e-5)), (c, rms(1e-6) * w)):
+        close(got, want.astype(np.float32), 4e-6)
+    m.close()
+
+
+@pytest.mark.parametrize("ty,n,rows", [(G.F32, 1, 1), (G.F32, 1025, 3), (G.Q8_0, 4096, 1), (G.Q8_0, 1056, 255), (G.Q8_0, 2080, 256), (G.F16, 70000, 2)])
+def test_get_rows_in_slices(oracle, ty, n, rows):
+    """Below 256 rows a row is cut into slices of 1024 elements, one CTA each."""
+    rng = np.random.default_rng(n + rows)
+    t = rng.standard_normal((7, n)).astype(np.float32)
+    table = t if ty == G.F32 else t.astype(np.float16) if ty == G.F16 else oracle.quantize(ty, t)
+    ids = rng.integers(0, 7, rows).astype(np.int32)
+    g = G.Graph()
+    y = g.output(g.get_rows(g.weight(ty, [n, 7], "t"), g.input(G.I32, [rows], "ids")))
+    m = Model(g, [table], outputs=[("y", y)])
+    (got,) = m.run(ids)
+    want = t if ty == G.F32 else table.astype(np.float32) if ty == G.F16 else oracle.dequantize(ty, table, n)
+    assert np.array_equal(got.reshape(rows, n), want.reshape(7, n)[ids])
+    m.close()

@@ -238,3 +238,10 @@ def test_cache_write_with_block_size_zero_is_refused():
     with pytest.raises(TlbError) as e:
         Model(g, state_bytes=[8192, 8192])
     assert "block size" in str(e.value)
+
+
+@pytest.mark.parametrize("ctxs", [[2500], [64, 1024], [1025, 3000]])
+def test_more_chunks_than_are_merged_at_once(oracle, ctxs):
+    """Chunks of 64 tokens: 40, 16, and 47 beside 17 of them (the merge takes sixteen at a time)."""
+    got, want = paged_case(oracle, len(ctxs), 4, 1, 64, 16, ctxs, seed=len(ctxs))
+    close(got, want, 1e-3)
