@@ -679,10 +679,10 @@ struct FoldItem {
 struct Tc8fParams {
     const uint8_t *act;   // packed B operand
     float *out[tc8f::MAX_MATS];
-    float *part;          // [part][column of the tile][256 rows]
+    float *part;          // [part][column of the tile][tile_rows]
     int64_t M[tc8f::MAX_MATS], ldy[tc8f::MAX_MATS];
     int tile0[tc8f::MAX_MATS];   // first row tile of each matrix (past the end: not there)
-    int N, nst, row_tiles, col_tiles, groups;
+    int N, nst, tile_rows, row_tiles, col_tiles, groups;
     int nw, width;               // columns of a tile or of its first half; of a tile
     int whole, cuts, items;      // tiles [whole, row_tiles * col_tiles) are cut into `cuts` stretches of K
     int raw_stages, b_stages;
@@ -737,7 +737,12 @@ __device__ __forceinline__ uint32_t pair_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void pair_sync() {
+template <bool PAIR>
+__device__ __forceinline__ void all_sync() {   // of a CTA, or of both
+    if constexpr (!PAIR) {
+        __syncthreads();
+        return;
+    }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -747,35 +752,46 @@ __device__ __forceinline__ uint32_t of_leader(const void *p) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(tc::su32(p)));
     return r;
 }
+// on a barrier of this CTA, or at an address that of_leader gave
 __device__ __forceinline__ void arrive_at(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void pair_tmem_alloc(uint32_t *dst_smem, uint32_t cols) {
+template <bool PAIR>
+__device__ __forceinline__ void fold_tmem_alloc(uint32_t *dst_smem, uint32_t cols) {
+    if constexpr (!PAIR) return tc::tmem_alloc(dst_smem, cols);
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::su32(dst_smem)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void pair_tmem_dealloc(uint32_t addr, uint32_t cols) {
+template <bool PAIR>
+__device__ __forceinline__ void fold_tmem_dealloc(uint32_t addr, uint32_t cols) {
+    if constexpr (!PAIR) return tc::tmem_dealloc(addr, cols);
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
-// arrives on both CTAs' barrier at this offset once the MMAs issued so far are done
-__device__ __forceinline__ void pair_commit(uint64_t *bar) {
+// arrives on the barrier (of a pair: on both CTAs' at this offset) once the MMAs issued so far are done
+template <bool PAIR>
+__device__ __forceinline__ void fold_commit(uint64_t *bar) {
+    if constexpr (!PAIR) return tc::umma_commit(bar);
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(tc::su32(bar)), "h"((uint16_t)3) : "memory");
 }
 // four MMAs over 64 elements of K: A 8 columns apart in tensor memory, B 16 (x 16 bytes) apart in shared memory; more = 0: the
-// first one starts the sum. 256 rows, 128 of each CTA; each CTA holds half of the columns of B.
-__device__ __forceinline__ void umma4_f16_pair(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\tsetp.eq.b32 q, 0, 0;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-        "add.u64 b1, %2, 16;\n\tadd.u64 b2, %2, 32;\n\tadd.u64 b3, %2, 48;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, q;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], b2, %3, q;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], b3, %3, q;\n\t}"
-        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more)
-        : "memory");
+// first one starts the sum. Of a pair: 256 rows, 128 of each CTA; each CTA holds half of the columns of B.
+#define TLB_UMMA4(GROUP)                                                                                                            \
+    asm volatile(                                                                                                                   \
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\tsetp.eq.b32 q, 0, 0;\n\t"                        \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                                                                 \
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"                                                      \
+        "add.u64 b1, %2, 16;\n\tadd.u64 b2, %2, 32;\n\tadd.u64 b3, %2, 48;\n\t"                                                     \
+        "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [%1], %2, %3, p;\n\t"                                                     \
+        "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [a1], b1, %3, q;\n\t"                                                     \
+        "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [a2], b2, %3, q;\n\t"                                                     \
+        "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [a3], b3, %3, q;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more)     \
+        : "memory")
+template <bool PAIR>
+__device__ __forceinline__ void umma4_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
+    if constexpr (PAIR) TLB_UMMA4("2");
+    else TLB_UMMA4("1");
 }
+#undef TLB_UMMA4
 
 // 64 weights (group j of a unit of 256) of one row as f16 pairs, in the order of K.
 // Q8_0: two blocks of 34 bytes. Q4_K (one 144-byte super-block: f16 d, dmin, twelve bytes of 6-bit scales and mins, 128 bytes of
@@ -838,22 +854,23 @@ __device__ __forceinline__ void expand64(const uint8_t *rrow, int j, uint32_t (&
 // SHAPE 0: one accumulator of up to 256 columns or (up to 128) two in turn, steps of 128 elements of K; 1: two accumulators of up to 192
 // columns in turn, steps of 64; 2: two halves of up to 192 columns, which share the expanded weights, steps of 64. Behind the
 // accumulators lie four A slots of a step each.
-template <bool WQ4K, int SHAPE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
+// PAIR: launched as clusters of two.
+template <bool WQ4K, int SHAPE, bool PAIR>
+__global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_constant__ Tc8fMaps maps, const __grid_constant__ Tc8fParams p) {
     using namespace tc;
     using namespace tc8f;
-    constexpr int ROWS = tc8::ROWS;
+    constexpr int ROWS = tc8::ROWS, CTAS = PAIR ? 2 : 1;
     constexpr int ROW_CHUNK = WQ4K ? 144 : tc8::ROW_CHUNK;   // raw bytes of a row per unit of 256 elements
     constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
     constexpr int CT = SHAPE == 2 ? 2 : 1, STEP = SHAPE == 0 ? 2 : 1;   // halves; 64s of K in a step
     constexpr uint32_t ACOLS = SHAPE == 0 ? 256 : 2 * HALF_NW;   // first A column
     constexpr uint32_t ACC2 = SHAPE == 0 ? 128 : HALF_NW;        // second accumulator
     constexpr int A_RING = (512 - (int)ACOLS) / (32 * STEP);
-    constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(2 * ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B; columns / 8 at bit 17
+    constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(CTAS * ROWS >> 4) << 24);   // f16 x f16 -> f32, K-major A and B; columns / 8 at bit 17
     const uint32_t idesc[2] = {IDESC0 | ((uint32_t)(p.nw >> 3) << 17), IDESC0 | ((uint32_t)((p.width - p.nw) >> 3) << 17)};
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
-    const int b_half = p.nw / 2 * KS * 2, b_stage = b_half * STEP;   // this CTA's columns
+    const int b_half = p.nw / CTAS * KS * 2, b_stage = b_half * STEP;   // this CTA's columns
     uint8_t *bst = smem;                                   // b_stages x b_stage
     uint8_t *raw = bst + p.b_stages * b_stage;             // raw_stages x RAW_BYTES
     __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[MAX_STAGES], bar_bfree[MAX_STAGES];
@@ -863,30 +880,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
     volatile int *fail = &s_fail;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rank = pair_rank();
-    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const uint32_t rank = PAIR ? pair_rank() : 0u;
+    const int pair = (int)blockIdx.x / CTAS, pairs = (int)gridDim.x / CTAS;
     const uint32_t accs = SHAPE == 1 || (SHAPE == 0 && p.nw <= 128) ? 2 : 1;   // accumulators in turn
     if (tid == 0) {
         for (int i = 0; i < MAX_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
             mbar_init(&bar_rawfree[i], tc8f::DEQ_WARPS);
-            mbar_init(&bar_b[i], rank == 0 ? 2 : 1);   // the leader's: its own copy and word from the other CTA
+            mbar_init(&bar_b[i], PAIR && rank == 0 ? 2 : 1);   // the leader's: its own copy and word from the other CTA
             mbar_init(&bar_bfree[i], 1);
         }
         for (int i = 0; i < A_RING; i++) {
-            mbar_init(&bar_aready[i], 2 * 4 * STEP);
+            mbar_init(&bar_aready[i], CTAS * 4 * STEP);
             mbar_init(&bar_afree[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&bar_accfull[i], 1);
-            mbar_init(&bar_accfree[i], 2 * tc8f::EPI_WARPS);
+            mbar_init(&bar_accfree[i], CTAS * tc8f::EPI_WARPS);
         }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) pair_tmem_alloc(&tmem_base_s, 512);
+    if (warp == 0) fold_tmem_alloc<PAIR>(&tmem_base_s, 512);
     tc_fence_before();
-    pair_sync();
+    all_sync<PAIR>();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     griddep_launch();
@@ -901,7 +918,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
                 const FoldItem f = p.item(t);
                 const int mat = p.mat_of(f.row_tile);
                 const CUtensorMap *wmap = mat == 0 ? &maps.m[0] : (mat == 1 ? &maps.m[1] : &maps.m[2]);
-                const int row0 = (f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 2 * ROWS + (int)rank * ROWS;
+                const int row0 = (f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * CTAS * ROWS + (int)rank * ROWS;
                 for (int i = f.k0; i < f.k1; i++) {
                     mbar_wait_nap(&bar_rawfree[s], ph ^ 1u, fail, 64);
                     mbar_expect_tx(&bar_raw[s], RAW_BYTES);
@@ -925,7 +942,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
                 for (int i = f.k0 * 4; i < f.k1 * 4; i += STEP)
 #pragma unroll
                     for (int ct = 0; ct < CT; ct++) {
-                        const int mine = (ct == 0 ? p.nw : p.width - p.nw) / 16;   // groups of eight columns
+                        const int mine = (ct == 0 ? p.nw : p.width - p.nw) / (8 * CTAS);   // groups of eight columns
                         const int g0 = min((f.col_tile * p.width + ct * p.nw) / 8 + (int)rank * mine, p.groups - 1);
                         const uint32_t bytes = (uint32_t)min(mine, p.groups - g0) * 1024u;
                         mbar_wait_nap(&bar_bfree[s], ph ^ 1u, fail, 32);
@@ -947,7 +964,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
         if (elect_one()) {
             int bs = 0, as = 0;
             uint32_t bph = 0, aph = 0, it = 0;
-            if (rank != 0) {
+            if (PAIR && rank != 0) {
                 const uint32_t lead = of_leader(bar_b);
                 for (int t = pair; t < p.items; t += pairs) {
                     const FoldItem f = p.item(t);
@@ -995,13 +1012,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
                             b_here = mbar_test(su32(&bar_b[bs]), bph);
 #pragma unroll
                             for (int k = 0; k < STEP; k++)
-                                umma4_f16_pair(tmem_base + (CT == 1 ? ai : (uint32_t)ct) * ACC2, a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), idesc[ct], k ? 1u : more);
-                            pair_commit(bfree);
+                                umma4_f16<PAIR>(tmem_base + (CT == 1 ? ai : (uint32_t)ct) * ACC2, a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), idesc[ct], k ? 1u : more);
+                            fold_commit<PAIR>(bfree);
                         }
-                        pair_commit(afree);
+                        fold_commit<PAIR>(afree);
                         more = 1;
                     }
-                    pair_commit(&bar_accfull[ai]);
+                    fold_commit<PAIR>(&bar_accfull[ai]);
                 }
             }
         }
@@ -1013,7 +1030,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
         const int q = warp & 3, j = (warp - tc8f::DEQ_WARP0) >> 2;
         const int r = q * 32 + lane;
         const uint32_t a_lane = tmem_base + ACOLS + ((uint32_t)(q * 32) << 16);
-        const uint32_t aready = of_leader(bar_aready);
+        const uint32_t aready = PAIR ? of_leader(bar_aready) : su32(bar_aready);
         int s = 0, as = j / STEP;
         uint32_t ph = 0, aph = 0;
         for (int t = pair; t < p.items; t += pairs) {
@@ -1048,9 +1065,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
         // ---- draining warps, once per tile: lane quadrant warp % 4; of the two warps of a quadrant each takes every other 32
         // columns (CT = 1) or one of the halves (CT = 2)
         const int q = warp & 3, ch = (warp - tc8f::EPI_WARP0) >> 2;
-        const int row_in_tile = q * 32 + lane, nw = CT == 2 && ch ? p.width - p.nw : p.nw, chunks = nw / 32;
+        const int row_in_tile = q * 32 + lane, nw = CT == 2 && ch ? p.width - p.nw : p.nw, chunks = (nw + 31) / 32;
         const int c0 = CT == 1 ? ch : 0, step = CT == 1 ? 2 : 1;
-        const uint32_t accfree = of_leader(bar_accfree);
+        const uint32_t accfree = PAIR ? of_leader(bar_accfree) : su32(bar_accfree);
         uint32_t it = 0;
         for (int t = pair; t < p.items; t += pairs, it++) {
             const FoldItem f = p.item(t);
@@ -1059,11 +1076,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
             const uint32_t lane_addr = tmem_base + (CT == 1 ? ai : (uint32_t)ch) * ACC2 + ((uint32_t)(q * 32) << 16);
             mbar_wait_nap(&bar_accfull[ai], (it / accs) & 1, fail, 128);
             tc_fence_after();
-            int64_t row = (int64_t)(f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 2 * ROWS + rank * ROWS + row_in_tile;
+            int64_t row = (int64_t)(f.row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * CTAS * ROWS + rank * ROWS + row_in_tile;
             int64_t M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]), ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
             float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + (size_t)col0 * ldy + row;
             if (f.part >= 0) {
-                ldy = 2 * ROWS;
+                ldy = CTAS * ROWS;
                 o = p.part + ((size_t)f.part * p.width + in_tile) * ldy + rank * ROWS + row_in_tile;
             }
             if (c0 >= chunks) {
@@ -1091,8 +1108,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
     }
     __syncwarp();
     tc_fence_before();
-    pair_sync();   // neither CTA ends while the other one may still arrive on its barriers or read its columns
-    if (warp == 0) pair_tmem_dealloc(tmem_base, 512);
+    all_sync<PAIR>();   // neither CTA of a pair ends while the other one may still arrive on its barriers or read its columns
+    if (warp == 0) fold_tmem_dealloc<PAIR>(tmem_base, 512);
     if (tid == 0 && s_fail) report_error(p.err, 2);
 }
 
@@ -1100,15 +1117,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc8f::THREADS, 1) k_
 __global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fParams p) {
     griddep_launch();
     griddep_wait();
-    const int r4 = threadIdx.x & 63, c = blockIdx.y * 4 + (threadIdx.x >> 6);
+    const int quads = p.tile_rows / 4, r4 = (int)threadIdx.x % quads, c = (int)blockIdx.y * (256 / quads) + (int)threadIdx.x / quads;
     int row_tile, col_tile;
     p.at(p.whole + (int)blockIdx.x, row_tile, col_tile);
     const int64_t col = (int64_t)col_tile * p.width + c;
     if (c >= p.width || col >= p.N) return;
-    const float4 *q = reinterpret_cast<const float4 *>(p.part) + ((size_t)blockIdx.x * p.cuts * p.width + c) * 64 + r4;
+    const float4 *q = reinterpret_cast<const float4 *>(p.part) + ((size_t)blockIdx.x * p.cuts * p.width + c) * quads + r4;
     float4 v[tc8f::MAX_CUTS];
 #pragma unroll
-    for (int s = 0; s < tc8f::MAX_CUTS; s++) v[s] = s < p.cuts ? q[(size_t)s * p.width * 64] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < tc8f::MAX_CUTS; s++) v[s] = s < p.cuts ? q[(size_t)s * p.width * quads] : make_float4(0.f, 0.f, 0.f, 0.f);
     float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
 #pragma unroll
     for (int s = 1; s < tc8f::MAX_CUTS; s++) {
@@ -1119,7 +1136,7 @@ __global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fPa
         y[3] += v[s].w;
     }
     const int mat = p.mat_of(row_tile);
-    const int64_t row = (int64_t)(row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * 256 + r4 * 4;
+    const int64_t row = (int64_t)(row_tile - (mat == 0 ? p.tile0[0] : (mat == 1 ? p.tile0[1] : p.tile0[2]))) * p.tile_rows + r4 * 4;
     const int64_t M = mat == 0 ? p.M[0] : (mat == 1 ? p.M[1] : p.M[2]), ldy = mat == 0 ? p.ldy[0] : (mat == 1 ? p.ldy[1] : p.ldy[2]);
     float *o = (mat == 0 ? p.out[0] : (mat == 1 ? p.out[1] : p.out[2])) + col * ldy + row;
     if (row + 4 <= M && ((uintptr_t)o & 15) == 0) {
@@ -1134,35 +1151,41 @@ __global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fPa
 
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
-// Time of a unit (256 elements of K) of a tile in us. Measured, Q4_K / Q8_0: 1.02 / 0.90 at 64 columns, 1.10 / 1.00 at 128, 1.42 / 1.28 at 192,
-// 1.72 / 1.70 at 256, in halves 2.20 / 2.10 at 352.
-static double fold_unit_us(bool q4k, int width) { return q4k ? std::max(1.02, 0.50 + 0.0048 * width) : std::max(0.9, 0.35 + 0.005 * width); }
-// How a product is laid out over the pairs of SMs. Of the even splits of the columns into tiles, and of the cuts of the K of those tiles that
-// do not fill a wave, the one whose slowest pair has the least to do.
+// Time of a unit (256 elements of K) of a tile in us, all SMs at work. Measured, Q4_K / Q8_0: pairs 1.02 / 0.90 at 64 columns, 1.10 / 1.00 at 128,
+// 1.42 / 1.28 at 192, 1.72 / 1.70 at 256, in halves 2.20 / 2.10 at 352; single CTAs 1.15 at 80, 1.33 at 128, 2.1 at 256.
+static double fold_unit_us(bool q4k, int ctas, int width) {
+    if (ctas == 1) return (q4k ? 0.80 : 0.70) + 0.0048 * width;
+    return q4k ? std::max(1.02, 0.50 + 0.0048 * width) : std::max(0.9, 0.35 + 0.005 * width);
+}
+// How a product is laid out over pairs of SMs or single ones. Of the even splits of the columns into tiles, and of the cuts of the K of those
+// tiles that do not fill a wave, the one whose slowest SM has the least to do. A launch of pairs takes 2 to 3 us more than one of single CTAs
+// (two sets of barriers to agree on, arrivals across the pair): they are for products of several units per SM.
 FoldPlan mm_fold_plan(bool q4k, int n_mats, const int64_t *M, int64_t K, int64_t N, int sms) {
     FoldPlan f{};
-    const int pairs = std::max(1, sms / 2), nst = (int)(K / 256);
-    int64_t row_tiles = 0;
-    for (int j = 0; j < n_mats; j++) row_tiles += (M[j] + 255) / 256;
+    const int nst = (int)(K / 256);
     double best = 0;
-    for (int halves = 1; halves <= 2; halves++) {
-        const int widest = halves == 1 ? tc8f::NW : 2 * tc8f::HALF_NW;
+    for (int form = 0; form < 3; form++) {   // single CTAs, pairs, pairs with two halves
+        const int ctas = form == 0 ? 1 : 2, halves = form == 2 ? 2 : 1, workers = std::max(1, sms / ctas);
+        const int widest = halves == 1 ? tc8f::NW : 2 * tc8f::HALF_NW, step = ctas == 1 ? 16 : 32;
+        int64_t row_tiles = 0;
+        for (int j = 0; j < n_mats; j++) row_tiles += (M[j] + 128 * ctas - 1) / (128 * ctas);
         for (int64_t ct = (N + widest - 1) / widest, last = ct + 12; ct <= (N + 63) / 64 && ct <= last; ct++) {
-            const int width = (int)(((N + ct - 1) / ct + 31) / 32 * 32), nw = halves == 1 ? width : (width / 2 + 31) / 32 * 32;
+            const int width = (int)(((N + ct - 1) / ct + step - 1) / step * step), nw = halves == 1 ? width : (width / 2 + 31) / 32 * 32;
             if (nw == width && halves == 2) continue;
-            const int64_t tiles = row_tiles * ((N + width - 1) / width), full = tiles / pairs, rest = tiles % pairs;
-            const double unit = fold_unit_us(q4k, width), drain = halves == 1 && nw <= 192 ? 0.4 : 1.3;
+            const int64_t tiles = row_tiles * ((N + width - 1) / width), full = tiles / workers, rest = tiles % workers;
+            const double unit = fold_unit_us(q4k, ctas, width), drain = halves == 1 && nw <= 192 ? 0.4 : 1.3;
             for (int cuts = 1; cuts <= tc8f::MAX_CUTS && (cuts == 1 || (rest > 0 && cuts <= nst)); cuts++) {
-                const int64_t waves = (rest * cuts + pairs - 1) / pairs;
-                const double t = (double)full * (nst * unit + drain) + (double)waves * ((nst + cuts - 1) / cuts * unit + drain) +
-                                 (cuts > 1 ? 2.5 + (double)(rest * cuts) * width * 256 * 8 / 6.5e6 : 0);
+                const int64_t waves = (rest * cuts + workers - 1) / workers;
+                const double t = (ctas == 2 ? 2.8 : 0.0) + (double)full * (nst * unit + drain) + (double)waves * ((nst + cuts - 1) / cuts * unit + drain) +
+                                 (cuts > 1 ? 5.0 + (double)(rest * cuts) * width * (128 * ctas) * 8 / 6.5e6 : 0);
                 if (f.width == 0 || t < best * 0.98) {
                     best = t;
+                    f.ctas = ctas;
                     f.nw = nw;
                     f.width = width;
                     f.cuts = cuts;
                     f.whole = tiles - (cuts > 1 ? rest : 0);
-                    f.partial_bytes = cuts > 1 ? (uint64_t)(rest * cuts) * width * 256 * 4 : 0;
+                    f.partial_bytes = cuts > 1 ? (uint64_t)(rest * cuts) * width * (128 * ctas) * 4 : 0;
                 }
             }
         }
@@ -1173,6 +1196,8 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
                                int64_t ldy, void *partial, int *err, cudaStream_t st, bool early) {
     if (n_mats < 1 || n_mats > tc8f::MAX_MATS) return cudaErrorInvalidValue;
     const int sms = current_sm_count();
+    const FoldPlan plan = mm_fold_plan(q4k, n_mats, M, K, N, sms);
+    if (plan.partial_bytes > 0 && partial == nullptr) return cudaErrorInvalidValue;
     Tc8fMaps maps;
     Tc8fParams p{};
     for (int j = 0; j < tc8f::MAX_MATS; j++) {
@@ -1187,14 +1212,13 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
         p.M[j] = M[j];
         p.ldy[j] = n_mats > 1 ? M[j] : ldy;
         p.tile0[j] = p.row_tiles;
-        p.row_tiles += (int)((M[j] + 255) / 256);
+        p.row_tiles += (int)((M[j] + 128 * plan.ctas - 1) / (128 * plan.ctas));
     }
     p.act = (const uint8_t *)blobs;
     p.part = (float *)partial;
     p.N = (int)N;
     p.nst = (int)(K / 256);
-    const FoldPlan plan = mm_fold_plan(q4k, n_mats, M, K, N, sms);
-    if (plan.partial_bytes > 0 && partial == nullptr) return cudaErrorInvalidValue;
+    p.tile_rows = 128 * plan.ctas;
     p.nw = plan.nw;
     p.width = plan.width;
     p.col_tiles = (int)((N + p.width - 1) / p.width);
@@ -1205,19 +1229,22 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     // raw stages: 128 rows x 256 elements (18 or 34 KB); what they leave goes to B
     const int raw_bytes = tc8::ROWS * (q4k ? 144 : tc8::ROW_CHUNK);
     const int shape = p.width > p.nw ? 2 : (p.nw > 128 && p.nw <= tc8f::HALF_NW ? 1 : 0);
-    p.raw_stages = q4k ? 4 : 3;
-    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw * tc8f::KS * (shape == 0 ? 2 : 1)));
+    p.raw_stages = q4k ? 4 : (plan.ctas == 1 && p.nw > 128 ? 2 : 3);
+    p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw / plan.ctas * tc8f::KS * (shape == 0 ? 4 : 2)));
     if (p.b_stages < 2) return cudaErrorInvalidValue;
     p.groups = mm_fold_groups(N);
     p.err = err;
-    const dim3 grid((unsigned)(2 * std::min(p.items, std::max(1, sms / 2))));
-    auto go = [&](auto *k) { return launch_pdl_if(early, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
+    const dim3 grid((unsigned)(plan.ctas * std::min(p.items, std::max(1, sms / plan.ctas))));
+    auto go = [&](auto *k) { return launch_pdl_cluster(early, plan.ctas, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
     cudaError_t e;
-    if (shape == 2) e = q4k ? go(k_mm_q80_f16<true, 2>) : go(k_mm_q80_f16<false, 2>);
-    else if (shape == 1) e = q4k ? go(k_mm_q80_f16<true, 1>) : go(k_mm_q80_f16<false, 1>);
-    else e = q4k ? go(k_mm_q80_f16<true, 0>) : go(k_mm_q80_f16<false, 0>);
+    if (shape == 2) e = q4k ? go(k_mm_q80_f16<true, 2, true>) : go(k_mm_q80_f16<false, 2, true>);
+    else if (plan.ctas == 2 && shape == 1) e = q4k ? go(k_mm_q80_f16<true, 1, true>) : go(k_mm_q80_f16<false, 1, true>);
+    else if (plan.ctas == 2) e = q4k ? go(k_mm_q80_f16<true, 0, true>) : go(k_mm_q80_f16<false, 0, true>);
+    else if (shape == 1) e = q4k ? go(k_mm_q80_f16<true, 1, false>) : go(k_mm_q80_f16<false, 1, false>);
+    else e = q4k ? go(k_mm_q80_f16<true, 0, false>) : go(k_mm_q80_f16<false, 0, false>);
     if (e != cudaSuccess || p.cuts == 1) return e;
-    return launch_pdl(k_fold_sum, dim3((unsigned)(tiles - p.whole), (unsigned)((p.width + 3) / 4)), dim3(256), 0, st, p);
+    const int per = 1024 / p.tile_rows;   // columns of a CTA
+    return launch_pdl(k_fold_sum, dim3((unsigned)(tiles - p.whole), (unsigned)((p.width + per - 1) / per)), dim3(256), 0, st, p);
 }
 cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blobs, cudaStream_t st) {
     const char *ab = (const char *)act;
@@ -1241,12 +1268,16 @@ void mmq_tc8_configure() {
     cudaFuncSetAttribute(k_mmq_tc_q80<32, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<32, 4, 4>());
     cudaFuncSetAttribute(k_mmq_tc_q80_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
     auto fold = [](auto *k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc8f::SMEM); };
-    fold(k_mm_q80_f16<false, 0>);
-    fold(k_mm_q80_f16<true, 0>);
-    fold(k_mm_q80_f16<false, 1>);
-    fold(k_mm_q80_f16<true, 1>);
-    fold(k_mm_q80_f16<false, 2>);
-    fold(k_mm_q80_f16<true, 2>);
+    fold(k_mm_q80_f16<false, 0, false>);
+    fold(k_mm_q80_f16<true, 0, false>);
+    fold(k_mm_q80_f16<false, 1, false>);
+    fold(k_mm_q80_f16<true, 1, false>);
+    fold(k_mm_q80_f16<false, 0, true>);
+    fold(k_mm_q80_f16<true, 0, true>);
+    fold(k_mm_q80_f16<false, 1, true>);
+    fold(k_mm_q80_f16<true, 1, true>);
+    fold(k_mm_q80_f16<false, 2, true>);
+    fold(k_mm_q80_f16<true, 2, true>);
 }
 
 bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N) {

@@ -100,7 +100,7 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
 // width: columns of a tile, nw: of its first half (all of them: one accumulator); tiles from `whole` on are cut into `cuts` stretches of K,
 // whose sums go to partial_bytes of scratch
 struct FoldPlan {
-    int nw, width, cuts;
+    int ctas, nw, width, cuts;   // ctas: of a tile, each with 128 of its rows
     int64_t whole;
     uint64_t partial_bytes;
 };

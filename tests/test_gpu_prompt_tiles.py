@@ -30,6 +30,6 @@ def test_tiles(oracle, ty, K, M, N):
 
 # Few row tiles: their K is cut (into stretches of unequal length where it does not divide), a ragged last row tile and column tile among the parts.
 @pytest.mark.parametrize("ty", [Q4_K, Q8_0])
-@pytest.mark.parametrize("K,M,N", [(1792, [100], 65), (2816, [300, 40], 130), (5120, [257], 333), (4096, [513, 256, 31], 200), (3328, [1000], 390)])
+@pytest.mark.parametrize("K,M,N", [(1792, [100], 65), (2816, [300, 40], 130), (5120, [257], 333), (4096, [513, 256, 31], 200), (3328, [1000], 390), (14336, [4000], 70)])
 def test_cut_tiles(oracle, ty, K, M, N):
     test_tiles(oracle, ty, K, M, N)
