@@ -312,8 +312,9 @@ __device__ __forceinline__ void rope_cs(const RopeArgs &p, int64_t pr, float pos
         th = __fadd_rn(__fmul_rn(theta_interp, 1.f - ramp_mix), __fmul_rn(theta_extrap, ramp_mix));
         mscale *= 1.0f + 0.1f * logf(1.0f / p.freq_scale);
     }
-    cs = cosf(th) * mscale;
-    sn = sinf(th) * mscale;
+    sincosf(th, &sn, &cs);
+    cs *= mscale;
+    sn *= mscale;
 }
 
 // A thread owns one (pair, position) and walks `hc` heads with it: cos and sin depend on the position and the pair
@@ -359,6 +360,11 @@ __global__ void k_rope_kv(RopeKvArgs p, const uint8_t *q, const uint8_t *k, cons
     griddep_wait();
     const int tok = blockIdx.x, hsl = blockIdx.y, pr = threadIdx.x;
     const int hs = p.hs;
+    // (page and place in it with 32-bit arithmetic where the slot allows: a 64-bit division is a subroutine)
+    auto place = [&](int64_t slot, int h) {
+        const int64_t page = (slot >> 31) == 0 ? (int64_t)((uint32_t)slot / (uint32_t)p.block_size) : slot / p.block_size;
+        return (((size_t)page * p.kv_heads + h) * p.block_size + (size_t)(slot - page * p.block_size)) * hs;
+    };
     if (hsl < p.heads + p.kv_heads) {
         const bool is_q = hsl < p.heads;
         const int h = is_q ? hsl : hsl - p.heads;
@@ -375,7 +381,7 @@ __global__ void k_rope_kv(RopeKvArgs p, const uint8_t *q, const uint8_t *k, cons
                 return;
             }
             src = k + h * p.k.nb[1] + tok * p.k.nb[2];
-            dst = kpool + (((size_t)(slot / p.block_size) * p.kv_heads + h) * p.block_size + slot % p.block_size) * hs;
+            dst = kpool + place(slot, h);
         }
         const float *x = reinterpret_cast<const float *>(src);
         const int i0 = 2 * pr;
@@ -384,11 +390,11 @@ __global__ void k_rope_kv(RopeKvArgs p, const uint8_t *q, const uint8_t *k, cons
             dst[i0 + 1] = __float2half_rn(x[i0 + 1]);
             return;
         }
-        float cs, sn;
-        rope_cs(p.rope, pr, (float)pos[tok], ff, cs, sn);
         const int ic = p.rope.mode == 0 ? i0 : pr;
         const int off = p.rope.mode == 0 ? 1 : p.rope.n_dims / 2;
-        const float x0 = x[ic], x1 = x[ic + off];
+        const float x0 = x[ic], x1 = x[ic + off];   // on their way beside the position
+        float cs, sn;
+        rope_cs(p.rope, pr, (float)pos[tok], ff, cs, sn);
         dst[ic] = __float2half_rn(x0 * cs - x1 * sn);
         dst[ic + off] = __float2half_rn(x0 * sn + x1 * cs);
     } else {
@@ -396,8 +402,7 @@ __global__ void k_rope_kv(RopeKvArgs p, const uint8_t *q, const uint8_t *k, cons
         if (slot < 0 || slot >= p.pool_slots) return;   // reported by the key's CTA
         const int h = hsl - p.heads - p.kv_heads;
         const float2 x = *reinterpret_cast<const float2 *>(v + h * p.v.nb[1] + tok * p.v.nb[2] + pr * 8);
-        __half *dst = vpool + (((size_t)(slot / p.block_size) * p.kv_heads + h) * p.block_size + slot % p.block_size) * hs;
-        *reinterpret_cast<__half2 *>(dst + 2 * pr) = __floats2half2_rn(x.x, x.y);
+        *reinterpret_cast<__half2 *>(vpool + place(slot, h) + 2 * pr) = __floats2half2_rn(x.x, x.y);
     }
 }
 // One launch for the attention inputs of a prompt: rope(q) in f32, rope(k) and v as f16 for the attention and into the pools.
