@@ -170,6 +170,10 @@ void gemv_configure();
 bool gemv_f32_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
 void gemv_f32_configure();
+// Q6_K on the integer matrix instruction (k_gemv_q6.cu): rows whose tiles fit, any number of columns
+bool gemv_q6_supported(int64_t K);
+cudaError_t launch_gemv_q6(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
+void gemv_q6_configure();
 bool row_quant_q80_supported(int64_t K, int mode);
 cudaError_t launch_row_quant(const RowQuantArgs &p, cudaStream_t st);
 // the all-reduce in front of a residual add + RMS norm + quantizer fused into one kernel (tensor parallelism):

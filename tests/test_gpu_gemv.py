@@ -115,3 +115,44 @@ def test_rows_quantized_in_the_launch_or_in_front_of_it(oracle, monkeypatch, ty,
     for n, _, got in seen[1:]:
         for a, b in zip(got, seen[0][2]):
             assert a.tobytes() == b[:n].tobytes()
+
+
+@pytest.mark.parametrize("K,M", [(256, 130), (768, 45), (1792, 300), (2048, 17), (4096, 148 * 32 + 5), (7168, 33), (7424, 40), (14336, 20)])
+def test_q6_K_against_f64(oracle, K, M):
+    """Activations as four digits of eight bits: rows of less than eight super-blocks (several row groups per tile), whole rows, segments of eight,
+    and 7424 (29 super-blocks), whose rows do not fit and take the kernel that decodes. Whole numbers are exact, so the error is that of one f32 sum
+    over the super-blocks and the eight warps: a few units in the last place of the result's root mean square, whatever the spread of the values."""
+    rng = np.random.default_rng(K + M)
+    Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32))
+    W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
+    for N in (1, 2, 3, 4, 7):
+        X = (rng.standard_normal((N, K)) * np.exp(2 * rng.standard_normal((N, K)))).astype(np.float32)
+        g = G.Graph()
+        g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+        m = Model(g, [Wq])
+        for scale in (1.0, 2.0 ** 60, 2.0 ** -80):
+            (got,) = m.run((X * np.float32(scale)).astype(np.float32))
+            want = (X * np.float32(scale)).astype(np.float64) @ W.T
+            assert np.linalg.norm(got.reshape(N, M) - want) <= 2.5e-7 * np.linalg.norm(want)
+        m.close()
+
+
+@pytest.mark.parametrize("N", [1, 2])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_q6_K_values_that_are_not_finite(oracle, bad, N):
+    rng = np.random.default_rng(N)
+    K, M = 4096, 64
+    Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32))
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    X[0, 777] = bad
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    (got,) = m.run(X)
+    with np.errstate(invalid="ignore"):
+        want = X.astype(np.float64) @ oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64).T
+    got = got.reshape(N, M)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    inf, fin = np.isinf(want), np.isfinite(want)
+    assert np.array_equal(np.sign(got[inf]), np.sign(want[inf])) and np.allclose(got[fin], want[fin], atol=1e-5)
+    m.close()
