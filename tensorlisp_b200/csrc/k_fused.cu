@@ -17,6 +17,17 @@
 
 namespace tlb {
 
+// Eight norm weights from k0 on, beside the row's own values (behind the scale they are one more trip to L2, and eight loads)
+__device__ __forceinline__ void norm_weights(const RowQuantArgs &p, int64_t k0, float (&w)[8]) {
+    if (p.wn == p.K && ((uintptr_t)p.w & 15) == 0) {
+        const float4 a = *reinterpret_cast<const float4 *>(p.w + k0), b = *reinterpret_cast<const float4 *>(p.w + k0 + 4);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) w[e] = p.w[(uint32_t)(k0 + e) % (uint32_t)p.wn];
+}
+
 constexpr int RQ_THREADS = 256;
 constexpr int RQ_WARPS = RQ_THREADS / 32;
 
@@ -52,22 +63,29 @@ __global__ void __launch_bounds__(RQ_THREADS) k_row_quant_q8k(RowQuantArgs p) {
         return;
     }
     float scale = 1.f;
-    float v[8];
+    float v[8], w[8];
     bool have = false;   // v already holds this warp's block (met while the whole row was read for the norm)
     if (p.mode == RQ_NORM) {
+        if (sb < nblk) norm_weights(p, (int64_t)sb * 256 + lane * 8, w);
         // thread t reads elements t*8.. of every 2048-element stretch in turn: in stretch blockIdx.y those are the very
         // values of the block this warp quantizes below, so they are kept instead of being read a second time
+        // (two stretches in flight at a time)
         float ss = 0.f;
         int it = 0;
-        for (int64_t k0 = (int64_t)threadIdx.x * 8; k0 < K; k0 += RQ_THREADS * 8, it++) {
-            float x[8];
-            rq_load8(p, n, k0, x);
+        for (int64_t k0 = (int64_t)threadIdx.x * 8; k0 < K; k0 += 2 * RQ_THREADS * 8, it += 2) {
+            float x[2][8] = {};
+            rq_load8<true>(p, n, k0, x[0]);
+            const bool second = k0 + RQ_THREADS * 8 < K;
+            if (second) rq_load8<true>(p, n, k0 + RQ_THREADS * 8, x[1]);
 #pragma unroll
-            for (int e = 0; e < 8; e++) ss = __fadd_rn(ss, __fmul_rn(x[e], x[e]));
-            if (it == (int)blockIdx.y) {
-                have = true;
+            for (int h = 0; h < 2; h++) {
 #pragma unroll
-                for (int e = 0; e < 8; e++) v[e] = x[e];
+                for (int e = 0; e < 8; e++) ss = __fadd_rn(ss, __fmul_rn(x[h][e], x[h][e]));   // (zeros add nothing)
+                if (it + h == (int)blockIdx.y && (h == 0 || second)) {
+                    have = true;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) v[e] = x[h][e];
+                }
             }
         }
 #pragma unroll
@@ -89,10 +107,7 @@ __global__ void __launch_bounds__(RQ_THREADS) k_row_quant_q8k(RowQuantArgs p) {
     }
     if (p.mode == RQ_NORM) {
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int wi = p.wn == K ? (int)(k0 + e) : (int)((uint32_t)(k0 + e) % (uint32_t)p.wn);
-            v[e] = __fmul_rn(__fmul_rn(v[e], scale), p.w[wi]);
-        }
+        for (int e = 0; e < 8; e++) v[e] = __fmul_rn(__fmul_rn(v[e], scale), w[e]);
     }
     rq_quant_block(p, n, sb, nblk, lane, v);
 }
@@ -121,8 +136,9 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
         if (live) *reinterpret_cast<uint4 *>(blob) = make_uint4(0, 0, 0, 0);
         return;
     }
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, w[8];
     if (live) {
+        if (p.mode == RQ_NORM) norm_weights(p, k0, w);
         rq_load8(p, n, k0, v);
         if (p.mode != RQ_GLU && p.mode != RQ_F16 && p.b && p.sum_out) {   // the sum is the new residual stream
             *reinterpret_cast<float4 *>(p.sum_out + n * p.ld_sum + k0) = make_float4(v[0], v[1], v[2], v[3]);
@@ -142,10 +158,7 @@ __global__ void __launch_bounds__(1024) k_row_quant_q80(RowQuantArgs p) {
         const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)K), p.eps)));
         if (live) {
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const int wi = p.wn == K ? (int)(k0 + e) : (int)((uint32_t)(k0 + e) % (uint32_t)p.wn);
-                v[e] = __fmul_rn(__fmul_rn(v[e], scale), p.w[wi]);
-            }
+            for (int e = 0; e < 8; e++) v[e] = __fmul_rn(__fmul_rn(v[e], scale), w[e]);
         }
     }
     if (!live) return;

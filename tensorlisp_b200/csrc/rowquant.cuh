@@ -14,14 +14,17 @@ __device__ __forceinline__ int nearest_int_f(float v) {
 
 
 // The f32 value at (column n, element k) before any normalisation: a, a + b, act(a) * b or f16 a.
+// PLAIN: the caller knows the mode to be RQ_PLAIN or RQ_NORM (eight exponentials and divisions at every place that loads a row are most of
+// a kernel's code, and a kernel of a few microseconds waits for its code).
+template <bool PLAIN = false>
 __device__ __forceinline__ void rq_load8(const RowQuantArgs &p, int n, int64_t k0, float (&x)[8]) {
-    if (p.mode == RQ_GLU) {
+    if (!PLAIN && p.mode == RQ_GLU) {
         const float4 g0 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0), g1 = *reinterpret_cast<const float4 *>(p.a + n * p.lda + k0 + 4);
         const float4 u0 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0), u1 = *reinterpret_cast<const float4 *>(p.b + n * p.ldb + k0 + 4);
         const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
         for (int e = 0; e < 8; e++) x[e] = __fmul_rn(__fdiv_rn(g[e], __fadd_rn(1.0f, expf(-g[e]))), u[e]);   // SiLU(g)*u
-    } else if (p.mode == RQ_F16) {
+    } else if (!PLAIN && p.mode == RQ_F16) {
         const uint4 h = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p.a) + n * p.lda + k0);
         const __half2 *h2 = reinterpret_cast<const __half2 *>(&h);
 #pragma unroll
