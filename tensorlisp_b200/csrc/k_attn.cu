@@ -100,22 +100,27 @@ __global__ void __launch_bounds__(PA_WARPS * 32) k_paged_attn(PagedParams p) {
     const int g = lane >> 2, t = lane & 3;
     const int chunk = blockIdx.x, seq = blockIdx.z;
     const int kvh = blockIdx.y / p.groups_per_kv, grp = blockIdx.y % p.groups_per_kv;
-    const int ctx = paged_ctx(p, seq);
     const int c_begin = chunk * p.chunk_tokens;
+    const int32_t *table = p.tables + (size_t)seq * p.max_blocks;
+    // this thread's first block id, on its way beside the length
+    const int b0 = (c_begin >> p.block_shift) + (int)threadIdx.x;
+    const int32_t id0 = b0 < p.max_blocks ? table[b0] : 0;
+    const int ctx = paged_ctx(p, seq);
     if (c_begin >= ctx && !(chunk == 0)) return;  // nothing to do; the reduce skips this chunk
     const int c_end = min(ctx, c_begin + p.chunk_tokens);
     const int head0 = kvh * p.group + grp * 16;               // first query head of this CTA
     const int nrows = min(16, p.group - grp * 16);            // query heads served here
     const int n_tiles = c_end > c_begin ? (c_end - c_begin + PA_TILE - 1) / PA_TILE : 0;
-    const int32_t *table = p.tables + (size_t)seq * p.max_blocks;
     {
         // The block ids of this CTA's stretch of the context are checked here, once, and not in the copy loop below
         // (every instruction there is paid per 16 bytes moved): an id outside the pools never becomes an address,
         // the CTA reports it and leaves, and its part of the result stays unwritten.
         bool bad = false;
-        if (c_end > c_begin)
-            for (int b = (c_begin >> p.block_shift) + (int)threadIdx.x; b <= ((c_end - 1) >> p.block_shift); b += PA_WARPS * 32)
-                bad |= (uint32_t)table[b] >= p.pool_blocks;   // negative ids are large here
+        if (c_end > c_begin) {
+            const int last = (c_end - 1) >> p.block_shift;
+            bad = b0 <= last && (uint32_t)id0 >= p.pool_blocks;   // negative ids are large here
+            for (int b = b0 + PA_WARPS * 32; b <= last; b += PA_WARPS * 32) bad |= (uint32_t)table[b] >= p.pool_blocks;
+        }
         if (__syncthreads_or(bad)) {
             if (threadIdx.x == 0 && p.err) report_error(p.err, TLB_ERR_INDEX);
             return;
