@@ -1,4 +1,4 @@
-// Batched MUL_MAT (more than eight activation columns) with Q8_0 weights on the 5th-generation tensor cores:
+// Batched MUL_MAT (more than eight activation columns) with Q8_0 or Q4_0 weights on the 5th-generation tensor cores:
 // the output projection of a decode step (vocab x d_model, Q8_0) is the largest matrix of the model.
 //
 // Arithmetic (same integers as the reference's ggml-cpu path, vendor/ggml/src/ggml-cpu/quants.c:451-479):
@@ -14,6 +14,11 @@
 // tensor memory (tcgen05.st), where the MMA reads its A operand; B (the int8 activations, K-major core
 // matrices) stays in shared memory. Eight warps drain the accumulators, one warp issues the MMAs,
 // one the TMA copies; they meet only through mbarriers, every wait is bounded.
+//
+// Q4_0 has the same blocks in 18 bytes (a box is 144 bytes wide, 9 x 16: its 128-bit reads are conflict-free too) and the same
+// activations; the realigning warps turn a nibble into the code less 8 on the way, three instructions for four weights. In passes of
+// eight columns of the few-column kernel every eight cost another stream of the weights: [4096 x 4096] x 16 columns 27.6 -> 15.4 us,
+// [32000 x 4096] x 64 254 -> 97 (a launch timed alone, cold, about 8 us of which are not the kernel's).
 #include <algorithm>
 #include <cstdlib>
 #include <cuda.h>
@@ -32,6 +37,8 @@ constexpr int EPI_WARP0 = 1, DEQ_WARP0 = 9, MMA_WARP = 25;
 constexpr int STAGE_BLOCKS = 8;                       // Q8_0 blocks of a row per pipeline stage (256 elements of K)
 constexpr int ROW_CHUNK = STAGE_BLOCKS * 34;          // 272 bytes: 17 x 16, so 128-bit reads at row stride are conflict-free
 constexpr int RAW_BYTES = ROWS * ROW_CHUNK;
+__host__ __device__ constexpr int row_chunk(bool q4) { return STAGE_BLOCKS * (q4 ? 18 : 34); }   // bytes of a row per stage
+__host__ __device__ constexpr int raw_bytes(bool q4) { return ROWS * row_chunk(q4); }
 constexpr uint32_t TMEM_COLS = 512;                   // accumulators in [0, 256), the A ring in [256, 512)
 constexpr uint32_t A_COL0 = 256;
 constexpr int A_RING = 4;                             // stages of A (8 blocks x 8 columns of 4 int8) and of weight scales
@@ -115,21 +122,50 @@ __device__ __forceinline__ void split_blocks(const uint8_t *row, uint32_t (&qa)[
 #pragma unroll
     for (int j = 0; j < 8; j++) qb[j] = w[W0 + 9 + j];
 }
+
+// The same for a row's 144-byte chunk of Q4_0 blocks: bytes [36G, 36G + 36) = 9 words in three units. A word of codes has elements
+// 4j .. 4j + 3 in its low nibbles and 16 + 4j .. in its high ones; nibble - 8 as a signed byte is ((nibble | 0x80) - 8) ^ 0x80.
+__device__ __forceinline__ void nibbles_signed(uint32_t w, uint32_t &lo, uint32_t &hi) {
+    lo = (((w & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
+    hi = ((((w >> 4) & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
+}
+template <int G>
+__device__ __forceinline__ void split_blocks4(const uint8_t *row, uint32_t (&qa)[8], uint32_t (&qb)[8], float &da, float &db) {
+    constexpr int U0 = (36 * G) / 16, W0 = (36 * G) / 4 - 4 * U0;
+    uint32_t w[12];
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(row + (U0 + u) * 16);
+        w[4 * u] = v.x; w[4 * u + 1] = v.y; w[4 * u + 2] = v.z; w[4 * u + 3] = v.w;
+    }
+    da = __half2float(__ushort_as_half((unsigned short)(w[W0] & 0xffffu)));
+    db = __half2float(__ushort_as_half((unsigned short)(w[W0 + 4] >> 16)));
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        nibbles_signed(__funnelshift_r(w[W0 + j], w[W0 + j + 1], 16), qa[j], qa[4 + j]);
+        nibbles_signed(w[W0 + 5 + j], qb[j], qb[4 + j]);
+    }
+}
+template <bool Q4, int G>
+__device__ __forceinline__ void row_blocks(const uint8_t *row, uint32_t (&qa)[8], uint32_t (&qb)[8], float &da, float &db) {
+    if constexpr (Q4) split_blocks4<G>(row, qa, qb, da, db);
+    else split_blocks<G>(row, qa, qb, da, db);
+}
 }  // namespace tc8
 
-template <int NPAD, int RAW_STAGES, int ACT_STAGES>
+template <bool Q4, int NPAD, int RAW_STAGES, int ACT_STAGES>
 __global__ void __launch_bounds__(tc8::THREADS, 1) k_mmq_tc_q80(const __grid_constant__ CUtensorMap wmap, Tc8Params p) {
     using namespace tc;
     using namespace tc8;
     constexpr int ROWS = tc8::ROWS;
-    constexpr int BLOB = NPAD * 288;
+    constexpr int BLOB = NPAD * 288, ROW_CHUNK = tc8::row_chunk(Q4), RAW_BYTES = tc8::raw_bytes(Q4);
     // int8 x int8 -> int32, K-major A and B: c_format s32 (2) at bit 4, a/b format signed 8-bit (1) at bits 7 and 10
     constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NPAD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
     constexpr int GCOLS = 4 * NPAD;   // accumulator columns of one group of four blocks
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
     uint8_t *raw = smem;                                              // RAW_STAGES x RAW_BYTES
-    uint8_t *actb = raw + RAW_STAGES * tc8::RAW_BYTES;                // ACT_STAGES x BLOB
+    uint8_t *actb = raw + RAW_STAGES * RAW_BYTES;                // ACT_STAGES x BLOB
     float *dw = reinterpret_cast<float *>(actb + ACT_STAGES * BLOB);  // [A_RING][8][ROWS] weight scales
     __shared__ uint64_t bar_raw[RAW_STAGES], bar_rawfree[RAW_STAGES], bar_act[ACT_STAGES], bar_actfree[ACT_STAGES];
     __shared__ uint64_t bar_aready[tc8::A_RING], bar_afree[tc8::A_RING], bar_dwfree[tc8::A_RING], bar_mma[2], bar_epi[2];
@@ -170,8 +206,8 @@ __global__ void __launch_bounds__(tc8::THREADS, 1) k_mmq_tc_q80(const __grid_con
 
     auto load_raw = [&](int i) {
         const int s = i % RAW_STAGES;
-        mbar_expect_tx(&bar_raw[s], tc8::RAW_BYTES);
-        tma_2d(raw + s * tc8::RAW_BYTES, &wmap, (st0 + i) * (tc8::ROW_CHUNK / 2), row_tile * ROWS, &bar_raw[s]);   // x in 16-bit elements
+        mbar_expect_tx(&bar_raw[s], RAW_BYTES);
+        tma_2d(raw + s * RAW_BYTES, &wmap, (st0 + i) * (ROW_CHUNK / 2), row_tile * ROWS, &bar_raw[s]);   // x in 16-bit elements
     };
     auto load_act = [&](int i) {
         const int s = i % ACT_STAGES;
@@ -290,14 +326,14 @@ __global__ void __launch_bounds__(tc8::THREADS, 1) k_mmq_tc_q80(const __grid_con
         for (int i = 0; i < nst; i++) {
             const int rs = i % RAW_STAGES, slot = i % tc8::A_RING;
             mbar_wait(&bar_raw[rs], (uint32_t)((i / RAW_STAGES) & 1), fail);
-            const uint8_t *rrow = raw + rs * tc8::RAW_BYTES + r * tc8::ROW_CHUNK;
+            const uint8_t *rrow = raw + rs * RAW_BYTES + r * ROW_CHUNK;
             uint32_t qa[8], qb[8];
             float da, db;
             switch (g) {   // warp-uniform
-                case 0: split_blocks<0>(rrow, qa, qb, da, db); break;
-                case 1: split_blocks<1>(rrow, qa, qb, da, db); break;
-                case 2: split_blocks<2>(rrow, qa, qb, da, db); break;
-                default: split_blocks<3>(rrow, qa, qb, da, db); break;
+                case 0: row_blocks<Q4, 0>(rrow, qa, qb, da, db); break;
+                case 1: row_blocks<Q4, 1>(rrow, qa, qb, da, db); break;
+                case 2: row_blocks<Q4, 2>(rrow, qa, qb, da, db); break;
+                default: row_blocks<Q4, 3>(rrow, qa, qb, da, db); break;
             }
             if (i >= tc8::A_RING) {
                 // the MMAs that read this ring slot are done, and the epilogue has read its scales
@@ -372,16 +408,17 @@ __device__ __forceinline__ void drain16(uint64_t *y, const int (&D)[16], uint64_
 }
 }  // namespace tc8w
 
+template <bool Q4>
 __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __grid_constant__ CUtensorMap wmap, Tc8Params p) {
     using namespace tc;
     using namespace tc8w;
-    constexpr int ROWS = tc8::ROWS;
+    constexpr int ROWS = tc8::ROWS, ROW_CHUNK = tc8::row_chunk(Q4), RAW_BYTES = tc8::raw_bytes(Q4);
     constexpr int A_RING = tc8w::A_RING;
     constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NW >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
     uint8_t *raw = smem;                                              // RAW_STAGES x RAW_BYTES
-    uint8_t *actb = raw + RAW_STAGES * tc8::RAW_BYTES;                // ACT_STAGES x BLOB
+    uint8_t *actb = raw + RAW_STAGES * RAW_BYTES;                // ACT_STAGES x BLOB
     float *dw = reinterpret_cast<float *>(actb + ACT_STAGES * BLOB);  // [A_RING][8][ROWS] weight scales
     __shared__ uint64_t bar_raw[RAW_STAGES], bar_rawfree[RAW_STAGES], bar_act[ACT_STAGES], bar_actfree[ACT_STAGES];
     __shared__ uint64_t bar_aready[A_RING], bar_afree[A_RING], bar_dwfree[A_RING], bar_mma[N_ACC], bar_epi[N_ACC];
@@ -422,8 +459,8 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 
     auto load_raw = [&](int i) {
         const int s = i % RAW_STAGES;
-        mbar_expect_tx(&bar_raw[s], tc8::RAW_BYTES);
-        tma_2d(raw + s * tc8::RAW_BYTES, &wmap, i * (tc8::ROW_CHUNK / 2), row_tile * ROWS, &bar_raw[s]);   // x in 16-bit elements
+        mbar_expect_tx(&bar_raw[s], RAW_BYTES);
+        tma_2d(raw + s * RAW_BYTES, &wmap, i * (ROW_CHUNK / 2), row_tile * ROWS, &bar_raw[s]);   // x in 16-bit elements
     };
     auto load_act = [&](int i) {
         const int s = i % ACT_STAGES;
@@ -551,16 +588,16 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
                 mbar_wait_nap(&bar_dwfree[slot], (uint32_t)(((i / A_RING) - 1) & 1), fail, 128);
                 tc_fence_after();
             }
-            const uint8_t *rrow = raw + rs * tc8::RAW_BYTES + r * tc8::ROW_CHUNK;
+            const uint8_t *rrow = raw + rs * RAW_BYTES + r * ROW_CHUNK;
             float *dws = dw + (size_t)slot * 8 * ROWS + r;
 #pragma unroll
             for (int g = 0; g < 4; g++) {
                 uint32_t qa[8], qb[8];
                 float da, db;
-                if (g == 0) tc8::split_blocks<0>(rrow, qa, qb, da, db);
-                else if (g == 1) tc8::split_blocks<1>(rrow, qa, qb, da, db);
-                else if (g == 2) tc8::split_blocks<2>(rrow, qa, qb, da, db);
-                else tc8::split_blocks<3>(rrow, qa, qb, da, db);
+                if (g == 0) tc8::row_blocks<Q4, 0>(rrow, qa, qb, da, db);
+                else if (g == 1) tc8::row_blocks<Q4, 1>(rrow, qa, qb, da, db);
+                else if (g == 2) tc8::row_blocks<Q4, 2>(rrow, qa, qb, da, db);
+                else tc8::row_blocks<Q4, 3>(rrow, qa, qb, da, db);
                 tmem_st8(a_lane + (uint32_t)(slot * 64 + (2 * g) * 8), qa);
                 tmem_st8(a_lane + (uint32_t)(slot * 64 + (2 * g + 1) * 8), qb);
                 dws[(2 * g) * ROWS] = da;
@@ -1253,20 +1290,34 @@ cudaError_t launch_act_pack_fold(const ActLayout &a, const void *act, void *blob
     return cudaGetLastError();
 }
 
-static size_t tc8w_smem() {
+static size_t tc8w_smem() {   // Q4_0's raw stages are smaller
     return (size_t)tc8w::RAW_STAGES * tc8::RAW_BYTES + (size_t)tc8w::ACT_STAGES * tc8w::BLOB + (size_t)tc8w::A_RING * 8 * tc8::ROWS * sizeof(float) + 1024;
 }
 
 // ---------------------------------------------------------------- host side
-template <int NPAD, int RS, int AS>
+// stages of raw weights: as many bytes in flight for either type
+constexpr int tc8_raw_stages(bool q4) { return q4 ? 7 : 4; }
+template <bool Q4, int NPAD, int AS>
 static size_t tc8_smem() {
-    return (size_t)RS * tc8::RAW_BYTES + (size_t)AS * tc8_blob_bytes(NPAD) + (size_t)tc8::A_RING * 8 * tc8::ROWS * sizeof(float) + 1024;
+    return (size_t)tc8_raw_stages(Q4) * tc8::raw_bytes(Q4) + (size_t)AS * tc8_blob_bytes(NPAD) + (size_t)tc8::A_RING * 8 * tc8::ROWS * sizeof(float) + 1024;
+}
+
+template <bool Q4, int NPAD>
+static void tc8_attr() {
+    cudaFuncSetAttribute(k_mmq_tc_q80<Q4, NPAD, tc8_raw_stages(Q4), 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<Q4, NPAD, 4>());
+}
+template <bool Q4, int NPAD>
+static cudaError_t tc8_launch(bool early, dim3 grid, cudaStream_t st, const CUtensorMap &map, const Tc8Params &p) {
+    return launch_pdl_if(early, k_mmq_tc_q80<Q4, NPAD, tc8_raw_stages(Q4), 4>, grid, dim3(tc8::THREADS), tc8_smem<Q4, NPAD, 4>(), st, map, p);
 }
 
 void mmq_tc8_configure() {
-    cudaFuncSetAttribute(k_mmq_tc_q80<16, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<16, 4, 4>());
-    cudaFuncSetAttribute(k_mmq_tc_q80<32, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8_smem<32, 4, 4>());
-    cudaFuncSetAttribute(k_mmq_tc_q80_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
+    tc8_attr<false, 16>();
+    tc8_attr<false, 32>();
+    tc8_attr<true, 16>();
+    tc8_attr<true, 32>();
+    cudaFuncSetAttribute(k_mmq_tc_q80_wide<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
+    cudaFuncSetAttribute(k_mmq_tc_q80_wide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc8w_smem());
     auto fold = [](auto *k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc8f::SMEM); };
     fold(k_mm_q80_f16<false, 0, false>);
     fold(k_mm_q80_f16<true, 0, false>);
@@ -1280,14 +1331,14 @@ void mmq_tc8_configure() {
     fold(k_mm_q80_f16<true, 2, true>);
 }
 
-bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N) {
-    return K % 256 == 0 && K >= 256 && M >= 1 && !few_column_faster(TLB_TYPE_Q8_0, K, M, N) && N <= (int64_t)tc8w::NW * 65535;   // column tiles are grid.y
+bool mmq_tc8_supported(uint32_t type, int64_t K, int64_t M, int64_t N) {
+    return (type == TLB_TYPE_Q8_0 || type == TLB_TYPE_Q4_0) && K % 256 == 0 && K >= 256 && M >= 1 && !few_column_faster(type, K, M, N) && N <= (int64_t)tc8w::NW * 65535;   // column tiles are grid.y
 }
 
-TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
+TcPlan mmq_tc8_plan(uint32_t type, int64_t K, int64_t M, int64_t N, int sm_count) {
     TcPlan t;
     t.nsb = (int)(K / 256);
-    if (N > 64 && !getenv("TLB_NO_WIDE_TC") && !getenv("TLB_PROMPT_EXACT")) {
+    if (type == TLB_TYPE_Q8_0 && N > 64 && !getenv("TLB_NO_WIDE_TC") && !getenv("TLB_PROMPT_EXACT")) {
         // prompt-sized batches: 128 x 256 tiles, scales folded into f16 operands, one accumulator (k_mm_q80_f16)
         t.npad = tc8f::NW;
         t.n_split = 1;
@@ -1299,8 +1350,11 @@ TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
         t.partial_bytes = 0;
         return t;
     }
-    if (N > 64 && !getenv("TLB_NO_WIDE_TC")) {
-        // the same batches with the reference's integer arithmetic (TLB_PROMPT_EXACT=1): 128-column tiles, whole K per
+    // Q4_0 in 128-column tiles once they are a third of the SMs; fewer leave so much of the chip idle that passes of 32 columns with K cut
+    // over the SMs are faster ([4096 x 14336] x 128, 32 tiles: 205 us against 100; x 256: 207 against 200)
+    const bool wide = type == TLB_TYPE_Q8_0 || (M + tc8::ROWS - 1) / tc8::ROWS * ((N + tc8w::NW - 1) / tc8w::NW) >= sm_count / 3;
+    if (N > 64 && wide && !getenv("TLB_NO_WIDE_TC")) {
+        // the same batches with the reference's integer arithmetic (Q4_0, which has no other; TLB_PROMPT_EXACT=1): 128-column tiles, whole K per
         // CTA (k_mmq_tc_q80_wide), row tiles x column tiles fill the GPU
         t.npad = tc8w::NW;
         t.n_split = 1;
@@ -1352,11 +1406,12 @@ cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes,
                          uint32_t elem_bytes);
 void launch_mmq_reduce(const float *partial, float *y, int64_t total, int n_split, cudaStream_t st);
 
-cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y, int64_t ldy,
+cudaError_t launch_mmq_tc8(uint32_t type, const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y, int64_t ldy,
                            void *partial, int *err, cudaStream_t st, bool early) {
     CUtensorMap map;
+    const bool q4 = type == TLB_TYPE_Q4_0;
     // described in 16-bit elements: a 272-byte box is 136 of them (the limit is 256 elements per dimension)
-    cudaError_t e = tc_encode_2d(&map, W, (uint64_t)(K / 32 * 34), (uint64_t)M, tc8::ROW_CHUNK, tc8::ROWS, 2);
+    cudaError_t e = tc_encode_2d(&map, W, (uint64_t)tlb_row_size(type, K), (uint64_t)M, (uint32_t)tc8::row_chunk(q4), tc8::ROWS, 2);
     if (e != cudaSuccess) return e;
     if (t.npad == tc8f::NW) return launch_mm_fold_f16(false, 1, &W, K, &M, N, blobs, &y, ldy, partial, err, st, early);
     if (t.npad == tc8w::NW) {
@@ -1370,8 +1425,9 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
         p.n_split = 1;
         p.ldy = ldy;
         p.err = err;
-        return launch_pdl_if(early, k_mmq_tc_q80_wide, dim3((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_col_chunks), dim3(tc8w::THREADS),
-                          tc8w_smem(), st, map, p);
+        const dim3 grid((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_col_chunks);
+        return q4 ? launch_pdl_if(early, k_mmq_tc_q80_wide<true>, grid, dim3(tc8w::THREADS), tc8w_smem(), st, map, p)
+                  : launch_pdl_if(early, k_mmq_tc_q80_wide<false>, grid, dim3(tc8w::THREADS), tc8w_smem(), st, map, p);
     }
     dim3 grid((unsigned)((M + tc8::ROWS - 1) / tc8::ROWS), (unsigned)t.n_split);
     for (int c = 0; c < t.n_col_chunks; c++) {   // one launch per chunk of npad columns
@@ -1393,8 +1449,8 @@ cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M,
             p.out = yc;
             p.ldy = ldy;
         }
-        if (t.npad == 16) e = launch_pdl_if(early, k_mmq_tc_q80<16, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<16, 4, 4>(), st, map, p);
-        else e = launch_pdl_if(early, k_mmq_tc_q80<32, 4, 4>, grid, dim3(tc8::THREADS), tc8_smem<32, 4, 4>(), st, map, p);
+        if (t.npad == 16) e = q4 ? tc8_launch<true, 16>(early, grid, st, map, p) : tc8_launch<false, 16>(early, grid, st, map, p);
+        else e = q4 ? tc8_launch<true, 32>(early, grid, st, map, p) : tc8_launch<false, 32>(early, grid, st, map, p);
         if (e != cudaSuccess) return e;
         if (t.n_split > 1) {
             if (ldy != M) return cudaErrorInvalidValue;

@@ -79,11 +79,11 @@ bool tc_available();
 cudaError_t launch_wait_runs_out(uint32_t limit, unsigned nap_ns, int *err, unsigned long long *ns, cudaStream_t st);   // the driver offers cuTensorMapEncodeTiled
 
 // ---------------------------------------------------------------- k_mmq_tc_q8.cu
-// Q8_0 weights x activation columns on tcgen05 (kind::i8, one accumulator per 32-element block).
-bool mmq_tc8_supported(int64_t K, int64_t M, int64_t N);
-TcPlan mmq_tc8_plan(int64_t K, int64_t M, int64_t N, int sm_count);
+// Q8_0 or Q4_0 weights x activation columns on tcgen05 (kind::i8, one accumulator per 32-element block).
+bool mmq_tc8_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
+TcPlan mmq_tc8_plan(uint32_t type, int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_act_pack_tc8(const ActLayout &a, const void *act, int npad, void *blobs, cudaStream_t st);
-cudaError_t launch_mmq_tc8(const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
+cudaError_t launch_mmq_tc8(uint32_t type, const TcPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const void *blobs, float *y,
                            int64_t ldy, void *partial, int *err, cudaStream_t st, bool early);
 void mmq_tc8_configure();
 // the folded-scale prompt GEMM (k_mm_q80_f16) for Q8_0 or Q4_K weights; its activation operand is f16(code x scale), laid out by

@@ -40,11 +40,11 @@ TView view_of(const Tensor &t) {
 // tensor-core mul_mat kernels by weight type
 bool tc_supported(uint32_t wty, int64_t K, int64_t M, int64_t N) {
     if (wty == TLB_TYPE_Q4_K) return mmq_tc_supported(wty, K, M, N);
-    if (wty == TLB_TYPE_Q8_0) return tc_available() && mmq_tc8_supported(K, M, N);
+    if (wty == TLB_TYPE_Q8_0 || wty == TLB_TYPE_Q4_0) return tc_available() && mmq_tc8_supported(wty, K, M, N);
     return false;
 }
 TcPlan tc_plan(uint32_t wty, int64_t K, int64_t M, int64_t N, int sm) {
-    return wty == TLB_TYPE_Q8_0 ? mmq_tc8_plan(K, M, N, sm) : mmq_tc_plan(K, M, N, sm);
+    return wty == TLB_TYPE_Q4_K ? mmq_tc_plan(K, M, N, sm) : mmq_tc8_plan(wty, K, M, N, sm);
 }
 
 // A product that the few-column kernel takes (k_gemv.cu): a 2-D matrix of whole super-blocks and the columns for which it is the faster
@@ -472,7 +472,7 @@ void lower_mul_mat(L &l) {
     const int32_t qa = t.src[2];
     if (qa < 0 || !is_qact(l.T(qa).op)) unsupported(t, "activations could not be quantized (rows must be dense f32 with uniformly strided columns and a length that is a multiple of the block size)");
     const Place pq = l.place(qa);
-    const ActLayout a = act_layout(act_kind_for(tw.ty), K, tx.nrows());
+    const ActLayout a = g.a = act_layout(act_kind_for(tw.ty), K, tx.nrows());
     const bool batched = tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1;
     const bool dense_w = tw.nb[1] == tw.row_size();
     const bool dense_y = t.is_contiguous();
@@ -487,7 +487,8 @@ void lower_mul_mat(L &l) {
         ps.buf = BUF_ARENA;
         ps.off = sc < 0 ? 0 : (uint64_t)sc;
         const uint64_t blob_off = a.bytes;
-        const bool q8 = tw.ty == TLB_TYPE_Q8_0;
+        const uint32_t ty = tw.ty;
+        const bool q8 = ty != TLB_TYPE_Q4_K;   // the kernels with Q8_0 activations
         // a row-parallel projection: when the exchange that follows runs over peer memory, it adds the K-split
         // partial sums itself (decided at launch: the communicator may be set up after the program is compiled)
         const bool ar_next = !q8 && tp.n_split > 1 && tp.n_col_chunks == 1 && allreduce_follows(l);
@@ -495,12 +496,16 @@ void lower_mul_mat(L &l) {
         const size_t n_out = (size_t)(N * M);
         l.push([=](const RunCtx &r) {
             const bool leave = ar_next && comm_p2p_takes(dev, n_out);
-            return q8 ? launch_mmq_tc8(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early)
+            if (ty == TLB_TYPE_Q4_0 && ((uintptr_t)r.at(pw) & 15)) {   // a matrix that the copies cannot address
+                MMGeneric gg = g;
+                gg.act = r.at(pq);
+                return launch_mm_generic(gg, r.at(pw), r.at(px), r.at(pd), r.stream);
+            }
+            return q8 ? launch_mmq_tc8(ty, tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early)
                       : launch_mmq_tc(tp, r.at(pw), K, M, N, r.at(pq) + blob_off, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early, leave);
         });
         return;
     }
-    g.a = a;
     l.push([=](const RunCtx &r) {
         MMGeneric gg = g;
         gg.act = r.at(pq);
@@ -1300,7 +1305,10 @@ void rewrite_graph(Graph &g, int sm_count) {
     // Quantize each distinct activation once: a QUANT_ACT node in front of the first quantized
     // MUL_MAT that reads it, shared by later ones until something writes its storage again.
     std::vector<int32_t> nodes;
-    std::map<std::pair<int32_t, int>, int32_t> cache;  // (activation tensor, kind) -> QUANT_ACT tensor
+    // (activation tensor, kind) -> QUANT_ACT tensor. Q4_0 matrices and Q8_0 ones that read the same activation agree on the packed
+    // operand up to 64 columns; above, they take different ones, and the key says so.
+    std::map<std::pair<int32_t, int>, int32_t> cache;
+    constexpr int OTHER_OPERAND = 256;
     for (size_t i = 0; i < g.nodes.size(); i++) {
         if (dead[i]) continue;
         const int32_t id = g.nodes[i];
@@ -1324,7 +1332,7 @@ void rewrite_graph(Graph &g, int sm_count) {
             if (ok && tx.ne[2] > 1) ok = tx.nb[2] == tx.nb[1] * (uint64_t)tx.ne[1];
             if (ok && tx.ne[3] > 1) ok = tx.nb[3] == tx.nb[1] * (uint64_t)tx.ne[1] * (uint64_t)tx.ne[2];
             if (ok) {
-                auto key = std::make_pair(x, kind);
+                auto key = std::make_pair(x, tw.ty == TLB_TYPE_Q4_0 && tx.ne[1] > 64 ? kind | OTHER_OPERAND : kind);
                 auto it = cache.find(key);
                 int32_t qa;
                 if (it != cache.end()) {

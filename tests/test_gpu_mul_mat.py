@@ -168,3 +168,24 @@ def test_stream_k_schedule(oracle, N, monkeypatch):
     (y2,) = m.run(X)
     m.close()
     assert np.abs(y2 - y).max() <= 2e-5 * np.abs(want).max() + 1e-6
+
+
+@pytest.mark.parametrize("K,M,N", [(256, 300, 17), (512, 130, 100), (256, 6300, 70), (1024, 2100, 400)])
+def test_q4_0_beside_q8_0(oracle, K, M, N):
+    """A Q4_0 and a Q8_0 matrix that read one activation: up to 64 columns they share its packed blocks, above they take different
+    operands, Q4_0 in passes of 32 columns (few row tiles) or tiles of 128. Q4_0 keeps the integer sums of a block at every size, so only
+    the order of K / 32 f32 additions differs: their rounding is below K / 32 * 2^-24 of the sum of the terms' magnitudes, here at most
+    about sqrt(K / 32) times max|y|, 1e-5 of it at K = 1024."""
+    rng = np.random.default_rng(K + M + N)
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    Ws = [oracle.quantize(ty, (rng.standard_normal((M, K)) * 0.02).astype(np.float32)) for ty in (Q4_0, Q8_0)]
+    g = G.Graph()
+    w4, w8 = g.weight(Q4_0, [K, M], "W4"), g.weight(Q8_0, [K, M], "W8")
+    x = g.input(G.F32, [K, N], "x")
+    g.output(g.mul_mat(w4, x, "y4"))
+    g.output(g.mul_mat(w8, x, "y8"))
+    m = Model(g, Ws)
+    y4, y8 = m.run(X)
+    assert close(y4, oracle.mul_mat(Q4_0, Ws[0], K, X), TOL) <= 1e-5 * np.abs(y4).max()
+    close(y8, oracle.mul_mat(Q8_0, Ws[1], K, X), TOL)
+    m.close()
