@@ -225,6 +225,7 @@ static void configure_kernels_once(int ordinal) {
     mmq_tc_configure();
     mmq_tc8_configure();
     mm_plain_configure();
+    mm_q6_configure();
     flash_tc_configure();
     g_configured_ordinals |= bit;
 }

@@ -371,7 +371,6 @@ void gemv_q6_configure() {
     set(gemvq6::k_gemv_q6<1>);
     set(gemvq6::k_gemv_q6<2>);
 }
-// columns that the next pass takes (0: none); y[column][ldy]
 cudaError_t launch_gemv_q6(const GemvArgs &g, int sm_count, int *err, cudaStream_t st) {
     gemvq6::Params p{};
     p.W = (const uint8_t *)g.W[0];

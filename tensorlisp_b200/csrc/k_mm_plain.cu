@@ -22,6 +22,7 @@
 #include "kernels.h"
 #include "pdl.cuh"
 #include "tc_common.cuh"
+#include "mm_terms.cuh"
 
 namespace tlb {
 
@@ -30,12 +31,11 @@ cudaError_t tc_encode_2d_sw128(CUtensorMap *map, const void *base, uint64_t row_
 namespace plain {
 
 using namespace tc;
-constexpr int KB = 64;                  // weights of a row per box: one 128-byte swizzled line
 constexpr int KS = 2 * KB;              // and per step. A thread that waits for a barrier and starts a copy needs about 420
                                         // cycles for the pair, so a step of one 16 KB box would leave no slack (34 -> 29 us)
 constexpr int A_BOX = ROWS * KB * 2, A_STAGE = 2 * A_BOX;
 constexpr int MAX_COLS = 80;            // activation columns per pass: three terms each, 240 MMA columns
-constexpr int CONV_WARP0 = 6, CONV_WARPS = 8;
+constexpr int CONV_WARP0 = 6;
 constexpr int THREADS = 32 * (CONV_WARP0 + CONV_WARPS);   // TMA, MMA, four adding and eight splitting warps
 constexpr int SMEM = 208 * 1024;
 constexpr int MAX_STAGES = 6;
@@ -44,44 +44,7 @@ constexpr int MAX_STAGES = 6;
 // room for the weights in flight.
 __host__ __device__ constexpr int chunk_steps(int nc) { return nc <= 24 ? 2 : 1; }
 
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {   // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
-    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)64 << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
-// A value and what is left of it: pairs of terms as the weights' type, packed
-template <bool BF16>
-__device__ __forceinline__ uint32_t take_term(float &a, float &b) {
-    float2 back;
-    uint32_t bits;
-    if (BF16) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        bits = *reinterpret_cast<const uint32_t *>(&h);
-        back = __bfloat1622float2(h);
-    } else {
-        const __half2 h = __floats2half2_rn(a, b);
-        bits = *reinterpret_cast<const uint32_t *>(&h);
-        back = __half22float2(h);
-    }
-    // an infinite or undefined activation stays what it is in the first term and adds nothing in the others
-    a = fabsf(back.x) < __int_as_float(0x7f800000) ? a - back.x : 0.f;
-    b = fabsf(back.y) < __int_as_float(0x7f800000) ? b - back.y : 0.f;
-    return bits;
-}
-
 }  // namespace plain
-
-struct PlainParams {
-    const float *x;        // activations: column n at x + n * ldx
-    float *out;            // [N][ldy]
-    float *partial;        // [CTA][first / last segment][N][128]
-    int64_t K, M, ldx, ldy;
-    int N, n_mma, acc_stride, steps, tiles, stages, tmem_cols;
-    uint32_t idesc;
-    int *err;
-};
-
-// where a CTA's stretch of the tiles x steps sequence begins
-__device__ __forceinline__ int64_t plain_begin(int64_t c, int64_t total, int ctas) { return c * total / ctas; }
 
 // NC: columns the adding warps hold in registers, a multiple of 8 and at least N
 template <bool BF16, int NC>
@@ -121,19 +84,7 @@ __global__ void __launch_bounds__(plain::THREADS, 1) k_mm_plain(const __grid_con
     const int64_t total = (int64_t)p.tiles * p.steps;   // below 2^31 (mm_plain_supported)
     const int g0 = (int)plain_begin(blockIdx.x, total, gridDim.x), g1 = (int)plain_begin(blockIdx.x + 1, total, gridDim.x);
     const int tile_first = g0 / p.steps;
-    // A segment is the part of the stretch that lies in one tile, a chunk up to CS steps of a segment. Every role walks the
-    // same chunks: body(chunk number, first step, end, whether a segment begins / ends with it).
-    auto walk = [&](auto &&body) {
-        int c = 0, tile_end = (tile_first + 1) * p.steps;
-        for (int g = g0; g < g1; tile_end += p.steps) {
-            const int seg = g, seg_end = min(g1, tile_end);
-            for (; g < seg_end; c++) {
-                const int e = min(seg_end, g + CS);
-                body(c, g, e, g == seg, e == seg_end);
-                g = e;
-            }
-        }
-    };
+    auto walk = [&](auto &&body) { plain::walk<CS>(p.steps, g0, g1, tile_first, body); };
 
     if (warp == 0) {
         if (lane == 0) {   // the weights do not depend on the kernel in front
@@ -229,81 +180,8 @@ __global__ void __launch_bounds__(plain::THREADS, 1) k_mm_plain(const __grid_con
                 if (n < p.N) o[(size_t)n * ldo] = sum[n];
         });
     } else {
-        // ---- splitting warps: U columns of a chunk at a time, a lane holds V consecutive values of each; the loads of the
-        // next group (or of the next chunk's first) go out before this one is worked on, because a round trip to L2 takes
-        // as long as splitting three columns
         griddep_wait();
-        constexpr int V = CS * KS / 32, U = NC <= 24 ? NC / CONV_WARPS : NC / CONV_WARPS / 2;
-        const int w = warp - CONV_WARP0;
-        const int box = lane * V / KB, piece = lane * V % KB / 8, half = lane * V % 8;
-        // where a lane's values of the chunk [g, e) are: column n at k + n * ldx
-        struct At { int g, e, tile_end; int64_t k; };
-        auto chunk = [&](int g, int tile_end) {
-            At at{g, min(min(g1, tile_end), g + CS), tile_end, (int64_t)(g - tile_end + p.steps) * KS + lane * V};
-            return at;
-        };
-        auto load = [&](float (&v)[U][V], const At &at, int col) {
-            const bool live = at.g < g1 && at.k < p.K && box < 2 * (at.e - at.g);
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int i = 0; i < V; i += 4) {
-                    const bool in = live && col + u * CONV_WARPS < p.N;
-                    const float4 f = in ? *reinterpret_cast<const float4 *>(p.x + (int64_t)(col + u * CONV_WARPS) * p.ldx + at.k + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    v[u][i] = f.x; v[u][i + 1] = f.y; v[u][i + 2] = f.z; v[u][i + 3] = f.w;
-                }
-        };
-        int c = 0, n0 = w;
-        At at = chunk(g0, (tile_first + 1) * p.steps);
-        float nx[U][V];
-        load(nx, at, n0);
-        while (at.g < g1) {
-            const int buf = c & 1;
-            float v[U][V];
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int i = 0; i < V; i++) v[u][i] = nx[u][i];
-            const bool last = n0 + U * CONV_WARPS >= p.N;
-            const At to = last ? chunk(at.e, at.e == at.tile_end ? at.tile_end + p.steps : at.tile_end) : at;
-            load(nx, to, last ? w : n0 + U * CONV_WARPS);
-            if (n0 == w && c >= 2) mbar_wait_nap(&bar_bfree[buf], (uint32_t)(((c >> 1) & 1) ^ 1), fail, 0);
-            uint8_t *tile = smem + buf * b_chunk + box * b_tile + half * 2;
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int n = n0 + u * CONV_WARPS;
-                if (n >= p.N) break;
-                if (!BF16) {
-                    uint32_t m = 0;
-#pragma unroll
-                    for (int i = 0; i < V; i++) m = max(m, __float_as_uint(v[u][i]) & 0x7fffffffu);
-                    m = __reduce_max_sync(0xffffffffu, m) >> 23;
-                    // 2^(14 - exponent), kept within what f32 holds on both sides; 1 where nothing finite is to be scaled
-                    const int ex = m == 0 || m == 255 ? 0 : max(-112, min(120, 141 - (int)m));
-                    const float sc = __uint_as_float((uint32_t)(127 + ex) << 23);
-#pragma unroll
-                    for (int i = 0; i < V; i++) v[u][i] *= sc;
-                    if (lane == 0) inv[c & 3][n] = __uint_as_float((uint32_t)(127 - ex) << 23);
-                }
-#pragma unroll
-                for (int t = 0; t < 3; t++) {
-                    const int row = t * p.N + n;
-                    uint8_t *o = tile + row * 128 + ((piece ^ (row & 7)) << 4);
-                    if (V == 8) *reinterpret_cast<uint4 *>(o) = make_uint4(take_term<BF16>(v[u][0], v[u][1]), take_term<BF16>(v[u][2], v[u][3]), take_term<BF16>(v[u][4 % V], v[u][5 % V]), take_term<BF16>(v[u][6 % V], v[u][7 % V]));
-                    else *reinterpret_cast<uint2 *>(o) = make_uint2(take_term<BF16>(v[u][0], v[u][1]), take_term<BF16>(v[u][2], v[u][3]));
-                }
-            }
-            if (last) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> async-proxy (MMA) reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_b[buf]);
-                c++;
-                n0 = w;
-            } else {
-                n0 += U * CONV_WARPS;
-            }
-            at = to;
-        }
+        split_columns<BF16, NC, KS, CS, false>(p, smem, b_tile, b_chunk, inv, bar_b, bar_bfree, warp - CONV_WARP0, lane, g0, g1, tile_first, fail);
     }
     tc_fence_before();
     __syncthreads();
@@ -328,12 +206,17 @@ __global__ void __launch_bounds__(256) k_mm_plain_fixup(const float *__restrict_
     const int i = blockIdx.y * 256 + threadIdx.x, n = i / tc::ROWS, r = i % tc::ROWS;
     const int64_t row = (int64_t)blockIdx.x * tc::ROWS + r;
     if (n >= N || row >= M) return;
-    float s = 0.f;
+    // A tile of a matrix of few rows has up to a part per step: what an addition rounds off is carried along (56 parts: 1.4e-7 from f64
+    // without). Not in a sum that is no longer finite.
+    float s = 0.f, rest = 0.f;
     for (int c = c0; c <= c1; c++) {
         const bool first = plain_begin(c, total, ctas) >= t0;   // this tile is where the CTA's stretch begins
-        s += partial[((size_t)c * 2 + (first ? 0 : 1)) * N * tc::ROWS + (size_t)n * tc::ROWS + r];
+        const float v = partial[((size_t)c * 2 + (first ? 0 : 1)) * N * tc::ROWS + (size_t)n * tc::ROWS + r];
+        const float sum = __fadd_rn(s, v), got = __fsub_rn(sum, s);
+        rest = __fadd_rn(rest, __fadd_rn(__fsub_rn(s, __fsub_rn(sum, got)), __fsub_rn(v, got)));
+        s = sum;
     }
-    out[(size_t)n * ldy + row] = s;
+    out[(size_t)n * ldy + row] = fabsf(s) < __int_as_float(0x7f800000) ? s + rest : s;
 }
 
 // ---------------------------------------------------------------- host side
@@ -363,6 +246,11 @@ PlainPlan mm_plain_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
     t.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count, (int64_t)t.steps * t.tiles / 2));
     t.bytes = t.tiles % t.ctas ? (uint64_t)t.ctas * 2 * t.cols * tc::ROWS * 4 : 0;   // parts of cut tiles
     return t;
+}
+
+cudaError_t launch_mm_plain_fixup(const PlainPlan &t, int n, const float *partial, float *y, int64_t M, int64_t ldy, cudaStream_t st) {
+    if (t.tiles % t.ctas == 0) return cudaSuccess;
+    return launch_pdl(k_mm_plain_fixup, dim3((unsigned)t.tiles, (unsigned)((n * tc::ROWS + 255) / 256)), dim3(256), 0, st, partial, y, M, ldy, n, t.steps, t.tiles, t.ctas);
 }
 
 template <bool BF16>
@@ -405,9 +293,7 @@ cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64
         p.idesc = (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(p.n_mma >> 3) << 17) | ((uint32_t)(tc::ROWS >> 4) << 24);
         p.err = err;
         e = bf16 ? launch_plain_pass<true>(t, map, p, st, early) : launch_plain_pass<false>(t, map, p, st, early);
-        if (e == cudaSuccess && t.tiles % t.ctas != 0)
-            e = launch_pdl(k_mm_plain_fixup, dim3((unsigned)t.tiles, (unsigned)((n * tc::ROWS + 255) / 256)), dim3(256), 0, st, (const float *)p.partial, p.out, M, ldy, n, t.steps, t.tiles,
-                           t.ctas);
+        if (e == cudaSuccess) e = launch_mm_plain_fixup(t, n, p.partial, p.out, M, ldy, st);
     }
     return e;
 }

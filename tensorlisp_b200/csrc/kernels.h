@@ -118,7 +118,17 @@ bool mm_plain_supported(uint32_t type, int64_t K, int64_t M, int64_t N, uint64_t
 PlainPlan mm_plain_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_mm_plain(const PlainPlan &t, bool bf16, const void *W, uint64_t w_row_bytes, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx,
                             float *y, int64_t ldy, void *scratch, int *err, cudaStream_t st, bool early);
+cudaError_t launch_mm_plain_fixup(const PlainPlan &t, int n, const float *partial, float *y, int64_t M, int64_t ldy, cudaStream_t st);   // adds the parts of cut tiles, if any
 void mm_plain_configure();
+
+// ---------------------------------------------------------------- k_mm_q6.cu
+// Q6_K weights x f32 activations on tcgen05, for more columns than MM_Q6_FEW (k_gemv_q6.cu has the others)
+constexpr int MM_Q6_FEW = 4;
+bool mm_q6_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
+PlainPlan mm_q6_plan(int64_t K, int64_t M, int64_t N, int sm_count);
+cudaError_t launch_mm_q6(const PlainPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx, float *y, int64_t ldy, void *scratch, int *err,
+                         cudaStream_t st, bool early);
+void mm_q6_configure();
 
 // ---------------------------------------------------------------- k_fused.cu
 // One row (= activation column n) per CTA: produce the f32 row, quantize it to Q8_K into an ActLayout

@@ -49,7 +49,9 @@ TcPlan tc_plan(uint32_t wty, int64_t K, int64_t M, int64_t N, int sm) {
 
 // A product that the few-column kernel takes (k_gemv.cu): a 2-D matrix of whole super-blocks and the columns for which it is the faster
 // one (few_column_faster), or any number of them where no tensor-core kernel reads the type.
+bool plain_tc(const Graph &g, const Tensor &t);
 bool gemv_node(const Graph &g, const Tensor &t) {
+    if (plain_tc(g, t)) return false;
     if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || getenv("TLB_MM_GENERIC")) return false;
     const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
     if (tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] != 1 || tx.ne[2] * tx.ne[3] != 1 || tx.ty != TLB_TYPE_F32 || t.ty != TLB_TYPE_F32) return false;
@@ -414,7 +416,7 @@ bool allreduce_follows(const L &l) {
     return nx.op == "ALLREDUCE" && nx.src[0] == l.id;
 }
 
-// f16 / bf16 weights of an unbatched product whose rows and columns the copies of the tensor-core kernel can address
+// f16 / bf16 or Q6_K weights of an unbatched product (f32 activations) whose rows and columns the copies of the tensor-core kernels can address
 bool plain_tc(const Graph &g, const Tensor &t) {
     if (t.op != "MUL_MAT" || t.src[0] < 0 || t.src[1] < 0 || getenv("TLB_MM_GENERIC") || getenv("TLB_NO_TC")) return false;
     const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
@@ -422,7 +424,12 @@ bool plain_tc(const Graph &g, const Tensor &t) {
     uint64_t wo = 0, xo = 0;
     g.root(t.src[0], &wo);
     g.root(t.src[1], &xo);
-    return tx.nb[0] == 4 && tx.nb[1] % 16 == 0 && wo % 16 == 0 && xo % 16 == 0 && mm_plain_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1], tw.nb[1]);
+    if (tx.nb[0] != 4 || tx.nb[1] % 16 != 0 || wo % 16 != 0 || xo % 16 != 0) return false;
+    if (tw.ty == TLB_TYPE_Q6_K) return tw.nb[1] == tw.row_size() && mm_q6_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1]);
+    return mm_plain_supported(tw.ty, tw.ne[0], tw.ne[1], tx.ne[1], tw.nb[1]);
+}
+PlainPlan plain_plan(const Tensor &w, int64_t N, int sm) {
+    return w.ty == TLB_TYPE_Q6_K ? mm_q6_plan(w.ne[0], w.ne[1], N, sm) : mm_plain_plan(w.ne[0], w.ne[1], N, sm);
 }
 
 // ---- MUL_MAT (lower.rs:543-571). Quantized weights take int8 activations quantized once per
@@ -450,17 +457,18 @@ void lower_mul_mat(L &l) {
     g.r2 = t.ne[2] / tw.ne[2];
     g.r3 = t.ne[3] / tw.ne[3];
     if (plain_tc(*l.c.g, t)) {
-        const PlainPlan pp = mm_plain_plan(K, M, N, sm);
+        const PlainPlan pp = plain_plan(tw, N, sm);
         const int64_t sc = l.c.layout->scratch[l.pos];
         if (pp.bytes > 0 && sc < 0) throw std::string("mul_mat scratch was not planned");
         Place ps;
         ps.buf = BUF_ARENA;
         ps.off = sc < 0 ? 0 : (uint64_t)sc;
-        const bool bf16 = tw.ty == TLB_TYPE_BF16;
+        const bool bf16 = tw.ty == TLB_TYPE_BF16, q6 = tw.ty == TLB_TYPE_Q6_K;
         const uint64_t wrow = tw.nb[1];
         const int64_t ldx = N > 1 ? (int64_t)tx.nb[1] / 4 : K;
         l.push([=](const RunCtx &r) {
             if (((uintptr_t)r.at(pw) | (uintptr_t)r.at(px)) & 15) return launch_mm_generic(g, r.at(pw), r.at(px), r.at(pd), r.stream);   // a state block laid out by the caller
+            if (q6) return launch_mm_q6(pp, r.at(pw), K, M, N, (const float *)r.at(px), ldx, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early);
             return launch_mm_plain(pp, bf16, r.at(pw), wrow, K, M, N, (const float *)r.at(px), ldx, (float *)r.at(pd), M, r.at(ps), r.err, r.stream, early);
         });
         return;
@@ -1023,7 +1031,7 @@ uint64_t node_scratch_bytes(const Graph &g, int32_t id, int sm_count) {
     }
     if (plain_tc(g, t)) {
         const Tensor &tw = g.tensors[t.src[0]], &tx = g.tensors[t.src[1]];
-        return mm_plain_plan(tw.ne[0], tw.ne[1], tx.ne[1], sm_count).bytes;
+        return plain_plan(tw, tx.ne[1], sm_count).bytes;
     }
     if (t.op == "MUL_MAT" && t.src[0] >= 0 && t.src[1] >= 0 && t.src[2] >= 0 && is_qact(g.tensors[t.src[2]].op) &&
         g.tensors[t.src[2]].op_params[1] > 0) {

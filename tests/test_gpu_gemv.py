@@ -156,3 +156,49 @@ def test_q6_K_values_that_are_not_finite(oracle, bad, N):
     inf, fin = np.isinf(want), np.isfinite(want)
     assert np.array_equal(np.sign(got[inf]), np.sign(want[inf])) and np.allclose(got[fin], want[fin], atol=1e-5)
     m.close()
+
+
+@pytest.mark.parametrize("K,M,N", [(256, 8, 5), (512, 9, 6), (768, 135, 16), (4096, 1500, 17), (1024, 7, 12), (2048, 148 * 128 + 3, 9), (14336, 40, 22), (256, 130, 64), (4096, 20000, 21)])
+def test_q6_K_on_the_tensor_cores(oracle, K, M, N):
+    """More than four columns: rows in eights and what is left of them (fewer than eight rows stay with the other kernel), tiles cut between CTAs and
+    whole, several passes of columns. The sums of a super-block are exact, so the error is that of activations rounded to 2^-26 of the largest of their
+    256, four roundings per super-block and the addition of K / 256 of them: below 2.5e-7 of the result's norm."""
+    rng = np.random.default_rng(K + M + N)
+    Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32))
+    W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    X[1, :256] = 0.0
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    for scale in (1.0, 2.0 ** 100, 2.0 ** -60):
+        (got,) = m.run((X * np.float32(scale)).astype(np.float32))
+        want = (X * np.float32(scale)).astype(np.float64) @ W.T
+        assert np.linalg.norm(got.reshape(N, M) - want) <= 2.5e-7 * np.linalg.norm(want)
+    m.close()
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 1e-39])
+def test_q6_K_on_the_tensor_cores_unusual_values(oracle, bad):
+    """An infinite, undefined or denormal activation, and a row whose scale is infinite, where the digits cannot hold them."""
+    rng = np.random.default_rng(5)
+    K, M, N = 2048, 140, 7
+    Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32)).copy()
+    rows = Wq.view(np.uint8).reshape(M, K // 256, 210)
+    rows[3, 2, 208:210] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    if np.isfinite(bad):
+        X[2, 512:768] = bad * X[2, 512:768]   # a whole block of such values
+    else:
+        X[2, 777] = bad
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    (got,) = m.run(X)
+    with np.errstate(invalid="ignore"):
+        want = X.astype(np.float64) @ oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64).T
+    got = got.reshape(N, M)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    fin = np.isfinite(want)
+    assert np.allclose(got[fin], want[fin], atol=1e-5)
+    m.close()
