@@ -49,8 +49,10 @@ constexpr int A_RING = 4;                             // stages of A (8 blocks x
 //   d_a  f32  [8][NPAD]     activation scale per block and column                              NPAD*32
 static inline __host__ __device__ int tc8_blob_bytes(int npad) { return npad * 288; }
 
-__global__ void __launch_bounds__(256) k_act_pack_q80(const int8_t *__restrict__ qs, const float *__restrict__ ds, int64_t K, int N,
+__global__ void __launch_bounds__(256) k_act_pack_q80(const int8_t *qs, const float *ds, int64_t K, int N,
                                                        int npad, uint8_t *__restrict__ out) {
+    griddep_launch();
+    griddep_wait();
     // grid (stage, chunk of npad columns); blobs are laid out [chunk][stage]
     const int st = blockIdx.x;
     uint8_t *o = out + ((size_t)blockIdx.y * gridDim.x + st) * tc8_blob_bytes(npad);
@@ -1397,9 +1399,8 @@ cudaError_t launch_act_pack_tc8(const ActLayout &a, const void *act, int npad, v
             (const int8_t *)(ab + a.qs_off), (const float *)(ab + a.d_off), a.K, (int)a.N, a.kind == ACT_Q8_K ? 256 : 32, (uint8_t *)blobs);
         return cudaGetLastError();
     }
-    k_act_pack_q80<<<dim3((unsigned)(a.K / 256), (unsigned)((a.N + npad - 1) / npad)), 256, 0, st>>>((const int8_t *)(ab + a.qs_off), (const float *)(ab + a.d_off), a.K, (int)a.N, npad,
-                                                         (uint8_t *)blobs);
-    return cudaGetLastError();
+    return launch_pdl(k_act_pack_q80, dim3((unsigned)(a.K / 256), (unsigned)((a.N + npad - 1) / npad)), dim3(256), 0, st, (const int8_t *)(ab + a.qs_off), (const float *)(ab + a.d_off),
+                      a.K, (int)a.N, npad, (uint8_t *)blobs);
 }
 
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,

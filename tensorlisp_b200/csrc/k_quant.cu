@@ -21,6 +21,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace tlb {
 
@@ -704,8 +705,10 @@ __global__ void k_f32_to_bf16(const float *__restrict__ x, uint16_t *__restrict_
 //   qs int8 [N][K] | d f32 [N][K/blk] | (Q8_K only) bsums int16 [N][K/16]
 // Q8_0 flavour: d is the f16-rounded scale widened back to f32 (what the dot product reads).
 // x may be strided: column n starts at x + n*ldx (elements).
-__global__ void __launch_bounds__(256) k_act_q8_0(const float *__restrict__ x, int64_t ldx, int8_t *__restrict__ qs,
+__global__ void __launch_bounds__(256) k_act_q8_0(const float *x, int64_t ldx, int8_t *__restrict__ qs,
                                                    float *__restrict__ ds, int64_t K, int64_t N) {
+    griddep_launch();   // the product behind this starts on its weights (a call with a [4096 x 4096] Q4_0 product x 16: 59.0 -> 57.0 us)
+    griddep_wait();
     const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int64_t nblk = K / 32 * N;
     int64_t b = gid >> 3;
@@ -729,9 +732,11 @@ __global__ void __launch_bounds__(256) k_act_q8_0(const float *__restrict__ x, i
 }
 
 // One warp per 256-element block; lane holds 8 consecutive values (half of a 16-element bsum group).
-__global__ void __launch_bounds__(256) k_act_q8_K(const float *__restrict__ x, int64_t ldx, int8_t *__restrict__ qs,
+__global__ void __launch_bounds__(256) k_act_q8_K(const float *x, int64_t ldx, int8_t *__restrict__ qs,
                                                    float *__restrict__ ds, int16_t *__restrict__ bsums, int64_t K,
                                                    int64_t N) {
+    griddep_launch();
+    griddep_wait();
     const int lane = threadIdx.x & 31;
     const int64_t nblk = K / 256 * N;
     int64_t b = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -850,13 +855,10 @@ cudaError_t launch_act_quantize(const ActLayout &a, const float *x, int64_t ldx,
     char *o = (char *)out;
     if (a.kind == ACT_Q8_0) {
         const int64_t nb = a.K / 32 * a.N;
-        k_act_q8_0<<<(unsigned)((nb * 8 + 255) / 256), 256, 0, st>>>(x, ldx, (int8_t *)(o + a.qs_off), (float *)(o + a.d_off), a.K, a.N);
-    } else {
-        const int64_t nb = a.K / 256 * a.N;
-        k_act_q8_K<<<(unsigned)((nb + 7) / 8), 256, 0, st>>>(x, ldx, (int8_t *)(o + a.qs_off), (float *)(o + a.d_off),
-                                                            (int16_t *)(o + a.bsum_off), a.K, a.N);
+        return launch_pdl(k_act_q8_0, dim3((unsigned)((nb * 8 + 255) / 256)), dim3(256), 0, st, x, ldx, (int8_t *)(o + a.qs_off), (float *)(o + a.d_off), a.K, a.N);
     }
-    return cudaGetLastError();
+    const int64_t nb = a.K / 256 * a.N;
+    return launch_pdl(k_act_q8_K, dim3((unsigned)((nb + 7) / 8)), dim3(256), 0, st, x, ldx, (int8_t *)(o + a.qs_off), (float *)(o + a.d_off), (int16_t *)(o + a.bsum_off), a.K, a.N);
 }
 
 }  // namespace tlb
