@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cuda_fp16.h>
 
+#include "dequant.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "tc_common.cuh"
@@ -75,8 +76,8 @@ __device__ __forceinline__ int signed_byte(uint32_t w, uint32_t sel) {
 }
 
 // ---------------------------------------------------------------- activations as digits
-// Plane j of a column: its j-th digit (the highest first) of every value in order. Values of a block that are not all finite: infinities
-// as +-65537, the rest as 0, at the scale infinity; a NaN makes the scale one.
+// Plane j of a column: its j-th digit (the highest first) of every value in order. A block whose values are not all finite has the scale NaN:
+// its sums are taken value by value.
 template <int NC>
 __device__ __forceinline__ void load_digits(const Params &p, uint8_t *act) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -95,9 +96,9 @@ __device__ __forceinline__ void load_digits(const Params &p, uint8_t *act) {
         const int ex = max((int)(top >> 23) - 127, -120);
         float scale = 0.f;
         if (top >= 0x7f800000u) {
-            scale = top > 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float(0x7f800000u);
+            scale = __uint_as_float(0x7fc00000u);
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = isinf(v[e]) ? copysignf(65537.f, v[e]) : 0.f;   // a one in either half of the digits
+            for (int e = 0; e < 8; e++) v[e] = 0.f;
         } else if (top != 0) {
             const int up = 29 - ex, a = min(up, 127), b = up - a;   // 0 <= b <= 22; up >= -98
             const float fa = __uint_as_float((uint32_t)(a + 127) << 23), fb = __uint_as_float((uint32_t)(b + 127) << 23);
@@ -128,9 +129,10 @@ __device__ __forceinline__ void load_digits(const Params &p, uint8_t *act) {
 // {ql[128], qh[64], i8 scales[16], f16 d}; starts on 2-byte boundaries. Lane (g, t) brings words 4t of rows g and g + 8 and of column g of
 // the digits, and gets sums of those rows with columns 2t and 2t + 1. b: this lane's word of group 0 of this super-block.
 // NT = 0: one column; columns 0..3 are its digits against the first group of an instruction, 4..7 against the second.
-// f[2 * nt], f[2 * nt + 1]: rows g and g + 8, the part of this lane's two digits.
+// f[2 * nt], f[2 * nt + 1]: rows g and g + 8, the part of this lane's two digits. x: the columns' values of this super-block.
 template <int NT>
-__device__ __forceinline__ void unit_q6_K(const uint8_t *r0, const uint8_t *r1, const uint8_t *b, int pair_planes, const float *scale, int col_scales, float (&f)[NT ? 2 * NT : 2]) {
+__device__ __forceinline__ void unit_q6_K(const uint8_t *r0, const uint8_t *r1, const uint8_t *b, int pair_planes, const float *scale, int col_scales, const float *x, int64_t ldx,
+                                          float (&f)[NT ? 2 * NT : 2]) {
     constexpr int N = NT ? NT : 1;
     const int lane = threadIdx.x & 31, t = lane & 3;
     const bool second = NT == 0 && lane >= 16;
@@ -195,19 +197,19 @@ __device__ __forceinline__ void unit_q6_K(const uint8_t *r0, const uint8_t *r1, 
     for (int nt = 0; nt < N; nt++) {
         const float xs = scale[NT ? (2 * nt + (t >> 1)) * col_scales : 0];   // (multiplied last: it may be subnormal)
         float v0 = d0 * fmaf((float)acc[nt][0], 256.f, (float)acc[nt][1]) * weight, v1 = d1 * fmaf((float)acc[nt][2], 256.f, (float)acc[nt][3]) * weight;
-        if (__any_sync(0xffffffffu, !isfinite(xs))) {
-            // an infinite scale must meet the sum of all lanes' parts, of which some may be zero
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
-            if (NT == 0) {
-                v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
-                v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
+        if (xs != xs || !isfinite(d0) || !isfinite(d1)) {
+            // value by value, a quarter of the super-block per lane (of two columns: two quarters)
+            const float *const col = x + (NT ? 2 * nt + (t >> 1) : 0) * ldx;
+            for (int slot = NT ? 2 * (t & 1) : t, end = NT ? slot + 2 : slot + 1; slot < end; slot++) {
+                f[2 * nt] += q6_K_slot_sum(r0, col, slot);
+                f[2 * nt + 1] += q6_K_slot_sum(r1, col, slot);
             }
-            if (NT ? (t & 1) : t) continue;
+            continue;
         }
         f[2 * nt] = fmaf(v0, xs, f[2 * nt]);
         f[2 * nt + 1] = fmaf(v1, xs, f[2 * nt + 1]);
     }
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------- the kernel
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv_q6(const __grid_constant__ 
     const int gr = warp / per_group, u0 = warp % per_group;
     const bool works = gr < p.groups;
     // plane of this lane's column: digit g % 4 (of column g / 4 of the pair)
+    const float *const x = p.x + (int64_t)p.n0 * p.ldx;
     const uint8_t *const b0 = act + (NT ? g : g & 3) * p.plane + t4 * 4;
     int s = 0;
     uint32_t ph = 0;
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemv_q6(const __grid_constant__ 
                 if (works)
                     for (int u = u0; u < (p.boxes ? 8 : p.units); u += per_group) {
                         const int sb = seg * 8 + u;
-                        unit_q6_K<NT>(tile + u * BLOCK, tile + 8 * p.row_stride + u * BLOCK, b0 + sb * 256, 8 * p.plane, scales + sb, p.units, f);
+                        unit_q6_K<NT>(tile + u * BLOCK, tile + 8 * p.row_stride + u * BLOCK, b0 + sb * 256, 8 * p.plane, scales + sb, p.units, x + sb * 256, p.ldx, f);
                     }
                 __syncwarp();
                 if (lane == 0 && ok) mbar_arrive(&empty[s]);

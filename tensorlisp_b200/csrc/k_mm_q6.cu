@@ -64,13 +64,6 @@ __device__ __forceinline__ void cp_arrive(uint64_t *bar) {   // when this thread
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(su32(bar)) : "memory");
 }
 
-// A super-block of one row against one column where a factor is not finite: the scalar sum
-__device__ __noinline__ float plain_sum(const uint8_t *block, const float *x) {
-    float s = 0.f;
-    for (int k = 0; k < KS; k++) s += dq_elem(block, TLB_TYPE_Q6_K, k) * x[k];
-    return s;
-}
-
 // Four words of a row from word w0 on; sh: 16 where the super-block starts in the middle of a word
 __device__ __forceinline__ void words(const uint32_t *row, int w0, uint32_t sh, uint32_t (&o)[4]) {
     uint32_t prev = row[w0];
@@ -120,7 +113,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
     __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[2], bar_bfree[2], bar_acc[2], bar_accfree[2], bar_a[2], bar_afree[2];
-    __shared__ float inv[4][NC];      // per chunk in flight and column: what its sums are multiplied by (NaN: plain_sum)
+    __shared__ float inv[4][NC];      // per chunk in flight and column: what its sums are multiplied by (NaN: they are taken value by value)
     __shared__ float dsm[4][ROWS];    // and per row
     __shared__ float outer[NC][ROWS]; // sums of RUN super-blocks each: 56 added up one by one end 1.2e-7 from f64
     __shared__ uint32_t tmem_base_s;
@@ -264,11 +257,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
                         v = 0.f;
                         if (n0 + j < p.N && row < p.M) {
                             const int step = g - tile * p.steps;
-                            v = plain_sum(p.W + row * p.row_bytes + (int64_t)step * BLOCK, p.x + (int64_t)(n0 + j) * p.ldx + (int64_t)step * KS);
+                            for (int slot = 0; slot < 4; slot++) v += q6_K_slot_sum(p.W + row * p.row_bytes + (int64_t)step * BLOCK, p.x + (int64_t)(n0 + j) * p.ldx + (int64_t)step * KS, slot);
                         }
                     }
                     sum[n0 + j] += v;
                 }
+                __syncwarp();
             }
             tc_fence_before();
             __syncwarp();

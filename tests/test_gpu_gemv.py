@@ -158,6 +158,37 @@ def test_q6_K_values_that_are_not_finite(oracle, bad, N):
     m.close()
 
 
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 7])
+@pytest.mark.parametrize("K", [768, 2048])
+def test_q6_K_several_values_that_are_not_finite(oracle, K, N):
+    """Infinities of either sign side by side in a super-block, in two of them and over weights of zero (infinite, or undefined where they cancel or meet
+    a zero), and a row whose scale is infinite: the same kind of value as the sum of products, whichever kernel the columns take."""
+    rng = np.random.default_rng(K + N)
+    M = 170
+    Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32)).copy()
+    blocks = Wq.view(np.uint8).reshape(M, K // 256, 210)
+    blocks[5, 1, 208:210] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+    blocks[9, 0, :64] = blocks[9, 0, 128:160] = 0      # codes of 0 (a weight of -32 d sc) ...
+    blocks[10, 0, 192:200] = 0                         # ... and scales of 0
+    W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    for places in ([3, 70], [3, 4, 130], [7, 300], [255, 256, 600], [0, 1, 2, 3, 127, 511]):
+        for signs in ("++++++", "------", "+-+-+-"):
+            X = rng.standard_normal((N, K)).astype(np.float32)
+            for at, s in zip(places, signs):
+                X[N - 1, at] = np.inf if s == "+" else -np.inf
+            (got,) = m.run(X)
+            with np.errstate(invalid="ignore"):
+                want = np.stack([(W * x).sum(1) for x in X.astype(np.float64)])
+            got = got.reshape(N, M)
+            assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+            inf, fin = np.isinf(want), np.isfinite(want)
+            assert np.array_equal(np.sign(got[inf]), np.sign(want[inf])) and np.allclose(got[fin], want[fin], atol=1e-5)
+    m.close()
+
+
 @pytest.mark.parametrize("K,M,N", [(256, 8, 5), (512, 9, 6), (768, 135, 16), (4096, 1500, 17), (1024, 7, 12), (2048, 148 * 128 + 3, 9), (14336, 40, 22), (256, 130, 64), (4096, 20000, 21)])
 def test_q6_K_on_the_tensor_cores(oracle, K, M, N):
     """More than four columns: rows in eights and what is left of them (fewer than eight rows stay with the other kernel), tiles cut between CTAs and
