@@ -119,14 +119,14 @@ __device__ __forceinline__ float dq_elem(const uint8_t *row, uint32_t ty, int64_
     }
 }
 
-// A quarter of a Q6_K super-block (on any 2-byte boundary) against its 256 f32 values: decoded weights times values, one after the other. Slot
+// A quarter of a Q6_K super-block (on any 2-byte boundary) against its 256 f32 values: decoded weights times values, the four runs on their own. Slot
 // 2 h + is holds elements h * 128 + run * 32 + is * 16 + i, whose codes share 16 bytes of ql (two of the four runs each) and of qh.
 __device__ __noinline__ inline float q6_K_slot_sum(const uint8_t *b, const float *x, int slot) {
     const int h = slot >> 1, is = slot & 1;
     const int8_t *sc = reinterpret_cast<const int8_t *>(b + 192 + h * 8 + is);
     const float d = __half2float(*reinterpret_cast<const __half *>(b + 208));
     x += h * 128 + is * 16;
-    float s = 0.f;
+    float s[4] = {};
     for (int i = 0; i < 16; i += 2) {
         const uint32_t q0 = *reinterpret_cast<const uint16_t *>(b + h * 64 + is * 16 + i), q1 = *reinterpret_cast<const uint16_t *>(b + h * 64 + 32 + is * 16 + i),
                        qh = *reinterpret_cast<const uint16_t *>(b + 128 + h * 32 + is * 16 + i);
@@ -136,11 +136,11 @@ __device__ __noinline__ inline float q6_K_slot_sum(const uint8_t *b, const float
         for (int run = 0; run < 4; run++) {
             const float2 v = *reinterpret_cast<const float2 *>(x + run * 32 + i);
             const float ds = __fmul_rn(d, (float)sc[2 * run]);
-            s += __fmul_rn(ds, (float)((int)(c[run] & 0xff) - 32)) * v.x;
-            s += __fmul_rn(ds, (float)((int)(c[run] >> 8) - 32)) * v.y;
+            s[run] += __fmul_rn(ds, (float)((int)(c[run] & 0xff) - 32)) * v.x;
+            s[run] += __fmul_rn(ds, (float)((int)(c[run] >> 8) - 32)) * v.y;
         }
     }
-    return s;
+    return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 }  // namespace tlb

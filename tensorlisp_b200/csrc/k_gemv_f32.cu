@@ -1,6 +1,5 @@
 // MUL_MAT with Q6_K weights and a few f32 activation columns: decoded weights times the f32 values, the reference executor's
-// own arithmetic (crates/kernels/src/cuda/native/mm.cu:16-42). For rows that k_gemv_q6.cu has no tiles for: more than 28 super-blocks and not
-// a multiple of eight, or more than about 38000 weights.
+// own arithmetic (crates/kernels/src/cuda/native/mm.cu:16-42). For rows and columns that k_gemv_q6.cu does not take (gemv_q6_columns).
 //
 // What bounds it: decoding. A weight costs two integer operations (every other cycle each), a byte permutation that makes it an
 // f32 and half an add; the multiply-adds work on pairs. One CTA per SM takes a contiguous range of rows. A producer thread copies tiles
@@ -336,7 +335,7 @@ void gemv_f32_configure() {
 
 cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st) {
     if (g.n_mats != 1 || g.glu || g.act.mode != RQ_PLAIN) return cudaErrorInvalidValue;
-    if (gemv_q6_supported(g.K)) return launch_gemv_q6(g, sm_count, err, st);
+    if (g.N <= gemv_q6_columns(g.K)) return launch_gemv_q6(g, sm_count, err, st);
     gemvf::Params p{};
     p.W = (const uint8_t *)g.W[0];
     p.x = g.act.a;

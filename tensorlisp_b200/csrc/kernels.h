@@ -123,7 +123,7 @@ cudaError_t launch_mm_plain_fixup(const PlainPlan &t, int n, const float *partia
 void mm_plain_configure();
 
 // ---------------------------------------------------------------- k_mm_q6.cu
-// Q6_K weights x f32 activations on tcgen05, for more columns than MM_Q6_FEW (k_gemv_q6.cu has the others)
+// Q6_K weights x f32 activations on tcgen05, for more columns than MM_Q6_FEW (k_gemv_q6.cu and k_gemv_f32.cu have the others)
 constexpr int MM_Q6_FEW = 4;
 bool mm_q6_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 PlainPlan mm_q6_plan(int64_t K, int64_t M, int64_t N, int sm_count);
@@ -181,8 +181,8 @@ void gemv_configure();
 bool gemv_f32_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
 void gemv_f32_configure();
-// Q6_K on the integer matrix instruction (k_gemv_q6.cu): rows whose tiles fit, any number of columns
-bool gemv_q6_supported(int64_t K);
+// Q6_K on the integer matrix instruction (k_gemv_q6.cu): up to how many columns of K weights it takes (0 to 4)
+int gemv_q6_columns(int64_t K);
 cudaError_t launch_gemv_q6(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
 void gemv_q6_configure();
 bool row_quant_q80_supported(int64_t K, int mode);

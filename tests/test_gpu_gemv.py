@@ -119,9 +119,10 @@ def test_rows_quantized_in_the_launch_or_in_front_of_it(oracle, monkeypatch, ty,
 
 @pytest.mark.parametrize("K,M", [(256, 130), (768, 45), (1792, 300), (2048, 17), (4096, 148 * 32 + 5), (7168, 33), (7424, 40), (14336, 20)])
 def test_q6_K_against_f64(oracle, K, M):
-    """Activations as four digits of eight bits: rows of less than eight super-blocks (several row groups per tile), whole rows, segments of eight,
-    and 7424 (29 super-blocks), whose rows do not fit and take the kernel that decodes. Whole numbers are exact, so the error is that of one f32 sum
-    over the super-blocks and the eight warps: a few units in the last place of the result's root mean square, whatever the spread of the values."""
+    """Activations as eight digits of eight bits: rows of less than eight super-blocks (several row groups per tile), whole rows, segments of eight, one to four
+    columns of rows that have as many; and 7424 (29 super-blocks), whose rows do not fit and take the kernel that decodes, like the further columns of
+    longer rows. Whole numbers are exact, so the error is that of one f32 sum over the super-blocks and the eight warps: a few units in the last place of
+    the result's root mean square, whatever the spread of the values."""
     rng = np.random.default_rng(K + M)
     Wq = oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32))
     W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
@@ -186,6 +187,59 @@ def test_q6_K_several_values_that_are_not_finite(oracle, K, N):
             assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
             inf, fin = np.isinf(want), np.isfinite(want)
             assert np.array_equal(np.sign(got[inf]), np.sign(want[inf])) and np.allclose(got[fin], want[fin], atol=1e-5)
+    m.close()
+
+
+def outlier_rows(oracle, N, large, K=2048, M=150):
+    """Every row has weights of zero where a column's large values are; row sums in f64 and the norms of the rows' other terms."""
+    rng = np.random.default_rng(N)
+    W = (rng.standard_normal((M, K)) * 0.02).astype(np.float32)
+    at = rng.choice(K, 12, replace=False)
+    W[:, at] = 0
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    X[:, at] = (large * (1 + rng.random((N, 12)))).astype(np.float32)
+    Wq = oracle.quantize(Q6_K, W)
+    W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
+    assert not W[:, at].any()
+    terms = X.astype(np.float64)[:, None, :] * W
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    (got,) = m.run(X)
+    m.close()
+    return np.abs(got.reshape(N, M) - terms.sum(-1)), np.sqrt((terms ** 2).sum(-1))
+
+
+@pytest.mark.parametrize("large", [1e0, 1e2, 1e4, 1e6, 1e8, 1e15, 1e30])
+@pytest.mark.parametrize("N", [1, 2, 3, 4])
+def test_q6_K_large_values_over_weights_of_zero(oracle, N, large):
+    """Large activations under zero codes take no bits from the rest of their super-block. Row by row: the whole-number sums of a super-block are exact and get
+    four roundings, one more each as they and eight warps' parts are added up. Decoded, a lane adds 16 terms (value by value) or 64 in four sums, and a
+    warp's 32 lanes: about 40 roundings that a result goes through, of partial sums that stay below the norm of all terms for random signs. At 2^-24 of
+    that at most each and of random sign, three standard deviations are 3 x sqrt(40 / 3) = 11 of them."""
+    off, norm = outlier_rows(oracle, N, large)
+    assert (off <= 11 * 2.0 ** -24 * norm).all(), (off / norm).max()
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 4])
+def test_q6_K_single_terms(oracle, N):
+    """A row with one weight: the product of that weight and its activation to a few roundings (four with digits, three value by value, one in the bound for
+    both), however small the activation is beside the others of its super-block."""
+    rng = np.random.default_rng(N)
+    K, M = 1280, 900
+    W = np.zeros((M, K), np.float32)
+    at = rng.integers(0, K, M)
+    W[np.arange(M), at] = rng.standard_normal(M)
+    Wq = oracle.quantize(Q6_K, W)
+    W = oracle.dequantize(Q6_K, Wq, K).reshape(M, K).astype(np.float64)
+    g = G.Graph()
+    g.output(g.mul_mat(g.weight(Q6_K, [K, M], "W"), g.input(G.F32, [K, N], "x"), "y"))
+    m = Model(g, [Wq])
+    for spread in (1, 4, 12):
+        X = (rng.standard_normal((N, K)) * np.exp(spread * rng.standard_normal((N, K)))).astype(np.float32)
+        (got,) = m.run(X)
+        want = X.astype(np.float64) @ W.T
+        assert np.all(np.abs(got.reshape(N, M) - want) <= 5 * 2.0 ** -24 * np.abs(want))
     m.close()
 
 
