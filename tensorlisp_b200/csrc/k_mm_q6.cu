@@ -2,10 +2,12 @@
 // decoded weights times f32 activations, summed in f32).
 //
 // A weight is d * sc * (q - 32) with an 8-bit scale sc per 16 weights and d per 256. sc is cut into two digits of four bits, 16 s1 + s0, both in
-// [-8, 8]: (q - 32) * s1 and (q - 32) * s0 are whole numbers of at most 2^8. 256 activations of a column are 26-bit whole numbers at the scale of
-// their largest, three digits of nine bits (mm_terms.cuh). Products of a weight's and an activation's digit, and the sums of 256 of them, stay within
-// 2^24: exact in the f32 accumulators of kind::f16, which otherwise truncate (terms of f16 values in their place: 3.3e-7 relative error against
-// f64). So each super-block has two accumulators of three columns per activation; d and the scale come in as the sums leave tensor memory.
+// [-8, 8]: (q - 32) * s1 and (q - 32) * s0 are whole numbers of at most 2^8. 256 activations of a column are six digits of nine bits at the scale of
+// their largest (mm_terms.cuh), which hold every f32 down to 2^-29 of it to its last bit; a super-block with a smaller value, or one that is not finite, is
+// summed value by value. (Three digits, 26 bits, lost a large activation's neighbours where its weight is zero: 7.4e-5 of a row's norm beside 1e4, 0.68 beside
+// 1e8.) Products of a weight's and an activation's digit, and the sums of 256 of them, stay within 2^24: exact in the f32 accumulators of
+// kind::f16, which otherwise truncate (terms of f16 values in their place: 3.3e-7 relative error against f64). So each super-block has two
+// accumulators of six columns per activation; d and the scale come in as the sums leave tensor memory.
 //
 // Layout: one CTA per SM, a stretch of the (row tile of 128, super-block) sequence each (stream-K as in k_mm_plain.cu). Rows are 210 bytes per
 // super-block, so their pieces lie on 2-byte boundaries; eight rows together are a multiple of 16 bytes, so eight tensor copies, one per row of
@@ -13,13 +15,13 @@
 // copies, 256 or 64 instructions: 2.7 and 1.7 us per super-block). Eight warps unpack, two and a half instructions per weight, and store the two
 // digits into tensor memory, 128 weights of 128 rows at a time in two buffers; eight split activations, four add up, one issues MMAs.
 //
-// Relative error against f64, N(0, 1) activations, decoded weights in f32 (as before) and here: 1.0e-7 / 4.5e-8 at [300 x 4096], 9.9e-8 / 7.3e-8 at
-// [20000 x 4096], 1.1e-7 / 8.6e-8 at [20000 x 14336]; activations over five decades 1.0e-7 / 1.2e-7.
+// Relative error against f64, k_gemv_f32.cu and here, 5 to 40 columns: 9.9e-8 / 4.3e-8 at [300 x 4096], 9.8e-8 / 5.1e-8 at [20000 x 4096], 1.1e-7 / 5.1e-8 at [20000 x
+// 14336]; activations over five decades 8.3 to 10e-8 / 7.6 to 10e-8 at [20000 x 4096], 0.94 to 1.0e-7 / 7.1 to 8.7e-8 at [20000 x 14336].
 //
-// Measured, passes of four columns (k_gemv_q6.cu) and here, a launch timed alone, cold: [32000 x 4096] x 8 93 -> 66 us, x 16 174 -> 83, x 64 664 ->
-// 301; [4096 x 14336] x 16 206 -> 50, x 64 792 -> 164; [1500 x 2048] x 5 20 -> 17. Up to four columns it loses: 51 us there at [32000 x 4096] x 4, 62
-// here. What bounds it: issue slots (59% busy at 16 columns, a sixth of the stalls instruction fetch); copies alone take 44 us of the 83, unpacking
-// adds 13, splitting and adding 11, the MMAs 7.
+// Measured, passes of four columns of k_gemv_f32.cu and here, a launch timed alone, cold: [32000 x 4096] x 8 136 -> 74 us, x 16 260 -> 140, x 64 1003 -> 530;
+// [4096 x 14336] x 16 240 -> 81, x 64 929 -> 292; [1500 x 2048] x 5 20 -> 18 (three digits and passes of 21 columns: 67, 85, 302, 50, 164, 17). What bounds it:
+// issue slots. A pass of one column takes 66 us at [32000 x 4096], copies alone 44, unpacking adds 13; splitting and adding grow with columns times
+// digits, so that ten columns in one pass (113 us) gain little on two passes of five.
 #include <algorithm>
 #include <cuda_fp16.h>
 
@@ -44,12 +46,11 @@ constexpr int COPY_BYTES = ROWS / 8 * ROW_STRIDE;   // of one copy: every eighth
 constexpr int LEFT = 8 * COPY_BYTES;             // behind them the up to seven rows that are left at the end of the matrix
 constexpr int RAW_STAGE = (LEFT + 7 * ROW_STRIDE + 127) / 128 * 128;
 constexpr int MAX_STAGES = 6;
-constexpr int MAX_COLS = 21;                     // columns per pass: four accumulators of 64 columns (two super-blocks)
+constexpr int MAX_COLS = 8;                      // columns per pass, and what the adding warps hold in registers
 constexpr int CONV_WARP0 = 6, DEC_WARP0 = 14, DEC_WARPS = 8;
 constexpr int THREADS = 32 * (DEC_WARP0 + DEC_WARPS);
-constexpr int RUN = 8;
-// dynamic shared memory beside the static arrays of k_mm_q6<nc>
-constexpr int smem_room(int nc) { return 227 * 1024 - 3 * 1024 - nc * ROWS * 4; }
+// dynamic shared memory beside the static arrays
+constexpr int SMEM_ROOM = 227 * 1024 - 3 * 1024;
 constexpr uint32_t A_COL0 = 256, A_HALF = 128;   // tensor memory: accumulators in [0, 256), then per half of a super-block 64 columns of either digit
 
 struct Params : PlainParams {
@@ -107,15 +108,13 @@ __device__ __forceinline__ void unpack(const uint32_t *row, uint32_t sh, int h, 
     }
 }
 
-// NC: columns the adding warps hold in registers, a multiple of 8 and at least N
-template <int NC>
 __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CUtensorMap wmap, Params p) {
+    constexpr int NC = MAX_COLS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
     __shared__ uint64_t bar_raw[MAX_STAGES], bar_rawfree[MAX_STAGES], bar_b[2], bar_bfree[2], bar_acc[2], bar_accfree[2], bar_a[2], bar_afree[2];
     __shared__ float inv[4][NC];      // per chunk in flight and column: what its sums are multiplied by (NaN: they are taken value by value)
     __shared__ float dsm[4][ROWS];    // and per row
-    __shared__ float outer[NC][ROWS]; // sums of RUN super-blocks each: 56 added up one by one end 1.2e-7 from f64
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_fail;
     volatile int *fail = &s_fail;
@@ -216,69 +215,57 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
         // ---- adding warps: warp % 4 fixes the 32 rows a warp may read
         griddep_wait();
         const int q = warp & 3, r = 8 * (lane & 15) + 2 * q + (lane >> 4);
-        float sum[NC];
-        int run = 0;
-        bool flushed = false;
+        float sum[NC], rest[NC];   // what the additions of super-blocks round away is kept: without it 16 of them end up to 1.2e-7 from f64
         walk<1>(p.steps, g0, g1, tile_first, [&](int c, int g, int e, bool begins, bool ends) {
             const int buf = c & 1, tile = g / p.steps;
             const int64_t row = (int64_t)tile * ROWS + r;
             if (begins) {
 #pragma unroll
-                for (int n = 0; n < NC; n++) sum[n] = 0.f;
-                run = 0;
-                flushed = false;
+                for (int n = 0; n < NC; n++) sum[n] = rest[n] = 0.f;
             }
             mbar_wait_nap(&bar_acc[buf], (uint32_t)((c >> 1) & 1), fail, 32);
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)(2 * buf * p.acc_stride) + ((uint32_t)(q * 32) << 16);
             const float d = dsm[c & 3][q * 32 + lane];
             const bool d_finite = fabsf(d) < __int_as_float(0x7f800000);
+            float total[NC];
 #pragma unroll
-            for (int n0 = 0; n0 < NC; n0 += 8) {
-                if (n0 >= p.N) break;
-                float total[8];
+            for (int t = DIGITS - 1; t >= 0; t -= 3) {   // the smallest digit first, three in flight
+                float lo[3][NC], hi[3][NC];
 #pragma unroll
-                for (int t = 2; t >= 0; t--) {   // the smallest digit first
-                    float lo[8], hi[8];
-                    tmem_ld8(acc + (uint32_t)(t * p.N + n0), lo);
-                    tmem_ld8(acc + (uint32_t)(p.acc_stride + t * p.N + n0), hi);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const float v = fmaf(16.f, hi[j], lo[j]);
-                        total[j] = t == 2 ? v : fmaf(v, t == 1 ? 512.f : 262144.f, total[j]);
-                    }
+                for (int u = 0; u < 3; u++) {
+                    tmem_ld8(acc + (uint32_t)((t - u) * p.N), lo[u]);
+                    tmem_ld8(acc + (uint32_t)(p.acc_stride + (t - u) * p.N), hi[u]);
                 }
+                tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float f = inv[c & 3][n0 + j];
-                    float v = total[j] * d * f;
-                    if (!d_finite || f != f) {
-                        v = 0.f;
-                        if (n0 + j < p.N && row < p.M) {
-                            const int step = g - tile * p.steps;
-                            for (int slot = 0; slot < 4; slot++) v += q6_K_slot_sum(p.W + row * p.row_bytes + (int64_t)step * BLOCK, p.x + (int64_t)(n0 + j) * p.ldx + (int64_t)step * KS, slot);
-                        }
+                for (int u = 0; u < 3; u++)
+#pragma unroll
+                    for (int n = 0; n < NC; n++) {
+                        const float v = fmaf(16.f, hi[u][n], lo[u][n]);
+                        total[n] = t - u == DIGITS - 1 ? v : fmaf(total[n], 1.f / 512.f, v);
                     }
-                    sum[n0 + j] += v;
-                }
-                __syncwarp();
             }
+#pragma unroll
+            for (int n = 0; n < NC; n++) {
+                const float f = inv[c & 3][n];
+                float v = __fmul_rn(total[n] * 262144.f * d, f);
+                if (!d_finite || f != f) {
+                    v = 0.f;
+                    if (n < p.N && row < p.M) {
+                        const int step = g - tile * p.steps;
+                        for (int slot = 0; slot < 4; slot++)
+                            v += q6_K_slot_sum(p.W + row * p.row_bytes + (int64_t)step * BLOCK, p.x + (int64_t)n * p.ldx + (int64_t)step * KS, slot);
+                    }
+                }
+                const float s = __fadd_rn(sum[n], v), w = __fsub_rn(s, sum[n]);
+                rest[n] += __fadd_rn(__fsub_rn(sum[n], __fsub_rn(s, w)), __fsub_rn(v, w));
+                sum[n] = s;
+            }
+            __syncwarp();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_accfree[buf]);
-            if (++run == RUN || (ends && flushed)) {
-                run = 0;
-#pragma unroll
-                for (int n = 0; n < NC; n++) {
-                    if (n >= p.N) break;
-                    float &o = outer[n][q * 32 + lane];   // this thread's own
-                    const float v = flushed ? o + sum[n] : sum[n];
-                    o = v;
-                    sum[n] = ends ? v : 0.f;
-                }
-                flushed = true;
-            }
             if (!ends) return;
             const int t0 = tile * p.steps, t1 = t0 + p.steps, seg = max(g0, t0);
             const bool whole = seg == t0 && e == t1;
@@ -287,7 +274,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
             if (whole && row >= p.M) return;
 #pragma unroll
             for (int n = 0; n < NC; n++)
-                if (n < p.N) o[(size_t)n * ldo] = sum[n];
+                if (n < p.N) o[(size_t)n * ldo] = sum[n] + (fabsf(sum[n]) < __int_as_float(0x7f800000) ? rest[n] : 0.f);
         });
     } else if (warp < DEC_WARP0) {
         griddep_wait();
@@ -339,16 +326,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
 }  // namespace q6tc
 
 // ---------------------------------------------------------------- host side
-void mm_q6_configure() {
-    auto set = [](auto *k, int nc) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, q6tc::smem_room(nc)); };
-    set(q6tc::k_mm_q6<8>, 8);
-    set(q6tc::k_mm_q6<16>, 16);
-    set(q6tc::k_mm_q6<24>, 24);
-}
+void mm_q6_configure() { cudaFuncSetAttribute(q6tc::k_mm_q6, cudaFuncAttributeMaxDynamicSharedMemorySize, q6tc::SMEM_ROOM); }
 
+// From three columns on, where k_gemv_q6.cu has no more than that. us of a launch, cold, here / k_gemv_f32.cu, three and four columns: [32000 x 4096] 70 / 100 and
+// 72 / 74, [4096 x 4096] 27.1 / 25.5 and 25.2 / 22.4, [4096 x 14336] 44 / 64 and 42 / 67, [3000 x 2816] 23.5 / 22.4 and 21.2 / 21.4, [2000 x 8448] 29 / 32
+// and 28 / 42; two columns lose everywhere (67 / 57, 27 / 18, 44 / 39).
 bool mm_q6_supported(uint32_t type, int64_t K, int64_t M, int64_t N) {
-    return type == TLB_TYPE_Q6_K && K % q6tc::KS == 0 && K >= q6tc::KS && M >= 8 && N > MM_Q6_FEW && N <= (1 << 20) && K <= (1 << 20) && (M + tc::ROWS - 1) / tc::ROWS * (K / q6tc::KS) < (1ll << 31) &&
-           tc_available();
+    return type == TLB_TYPE_Q6_K && K % q6tc::KS == 0 && K >= q6tc::KS && M >= 8 && N > 2 && N > gemv_q6_columns(K) && N <= (1 << 20) && K <= (1 << 20) &&
+           (M + tc::ROWS - 1) / tc::ROWS * (K / q6tc::KS) < (1ll << 31) && tc_available();
 }
 
 PlainPlan mm_q6_plan(int64_t K, int64_t M, int64_t N, int sm_count) {
@@ -372,7 +357,7 @@ cudaError_t launch_mm_q6(const PlainPlan &t, const void *W, int64_t K, int64_t M
         const int64_t n0 = (int64_t)pass * t.cols;
         q6tc::Params p{};
         const int n = p.N = (int)std::min<int64_t>(t.cols, N - n0);
-        p.n_mma = (3 * n + 15) / 16 * 16;
+        p.n_mma = (plain::DIGITS * n + 15) / 16 * 16;
         p.acc_stride = 64;   // the adding warps read eight columns at a time: past the last digit's end what they read is not used
         p.x = x + n0 * ldx;
         p.out = y + n0 * ldy;
@@ -388,11 +373,9 @@ cudaError_t launch_mm_q6(const PlainPlan &t, const void *W, int64_t K, int64_t M
         p.W = (const uint8_t *)W;
         p.row_bytes = K / q6tc::KS * q6tc::BLOCK;
         const int b_bytes = 2 * q6tc::BOXES * p.n_mma * plain::KB * 2;
-        const int nc = (n + 7) / 8 * 8;
-        p.stages = std::min(q6tc::MAX_STAGES, (q6tc::smem_room(nc) - 1024 - b_bytes) / q6tc::RAW_STAGE);
+        p.stages = std::min(q6tc::MAX_STAGES, (q6tc::SMEM_ROOM - 1024 - b_bytes) / q6tc::RAW_STAGE);
         const size_t smem = (size_t)b_bytes + (size_t)p.stages * q6tc::RAW_STAGE + 1024;
-        auto go = [&](auto *k) { return launch_pdl_if(early, k, dim3((unsigned)t.ctas), dim3(q6tc::THREADS), smem, st, map, p); };
-        e = nc == 8 ? go(q6tc::k_mm_q6<8>) : (nc == 16 ? go(q6tc::k_mm_q6<16>) : go(q6tc::k_mm_q6<24>));
+        e = launch_pdl_if(early, q6tc::k_mm_q6, dim3((unsigned)t.ctas), dim3(q6tc::THREADS), smem, st, map, p);
         if (e == cudaSuccess) e = launch_mm_plain_fixup(t, n, p.partial, p.out, M, ldy, st);
     }
     return e;

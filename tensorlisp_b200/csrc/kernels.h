@@ -123,8 +123,7 @@ cudaError_t launch_mm_plain_fixup(const PlainPlan &t, int n, const float *partia
 void mm_plain_configure();
 
 // ---------------------------------------------------------------- k_mm_q6.cu
-// Q6_K weights x f32 activations on tcgen05, for more columns than MM_Q6_FEW (k_gemv_q6.cu and k_gemv_f32.cu have the others)
-constexpr int MM_Q6_FEW = 4;
+// Q6_K weights x f32 activations on tcgen05, from three columns on (k_gemv_q6.cu and k_gemv_f32.cu have the others)
 bool mm_q6_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 PlainPlan mm_q6_plan(int64_t K, int64_t M, int64_t N, int sm_count);
 cudaError_t launch_mm_q6(const PlainPlan &t, const void *W, int64_t K, int64_t M, int64_t N, const float *x, int64_t ldx, float *y, int64_t ldy, void *scratch, int *err,

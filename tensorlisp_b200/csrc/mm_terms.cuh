@@ -1,5 +1,5 @@
 // What the products of f32 activations on tcgen05 share (k_mm_plain.cu: f16 / bf16 weights, k_mm_q6.cu: Q6_K): the split of an activation
-// into three terms of a 16-bit type, and the walk over a CTA's stretch of the (tile, step) sequence.
+// into three terms of a 16-bit type or six digits, and the walk over a CTA's stretch of the (tile, step) sequence.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -38,13 +38,16 @@ __device__ __forceinline__ uint32_t take_term(float &a, float &b) {
     return bits;
 }
 
-// A whole number of magnitude at most 2^26 in three signed digits of nine bits: the digit at 2^SHIFT and what is left of it
-template <int SHIFT>
+// A value of magnitude at most 2^26 in signed digits of nine bits: digit t, at 2^(18 - 9t), and what is left of it, both exact (the digit and the rest have
+// no bits that the 24 of the value do not span)
+constexpr int DIGITS = 6;
+template <int T>
 __device__ __forceinline__ uint32_t take_digit(float &a, float &b) {
     constexpr float MAGIC = 12582912.f;   // 1.5 * 2^23: adding it rounds to a whole number
-    const float da = __fadd_rn(__fmaf_rn(a, 1.f / (1 << SHIFT), MAGIC), -MAGIC), db = __fadd_rn(__fmaf_rn(b, 1.f / (1 << SHIFT), MAGIC), -MAGIC);
-    a = __fmaf_rn(da, -(float)(1 << SHIFT), a);
-    b = __fmaf_rn(db, -(float)(1 << SHIFT), b);
+    constexpr float UP = T <= 2 ? (float)(1 << (T <= 2 ? 18 - 9 * T : 0)) : 1.f / (float)(1 << (T > 2 ? 9 * T - 18 : 0)), DOWN = 1.f / UP;
+    const float da = __fadd_rn(__fmaf_rn(a, DOWN, MAGIC), -MAGIC), db = __fadd_rn(__fmaf_rn(b, DOWN, MAGIC), -MAGIC);
+    a = __fmaf_rn(da, -UP, a);
+    b = __fmaf_rn(db, -UP, b);
     const __half2 h = __floats2half2_rn(da, db);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
@@ -83,9 +86,9 @@ __device__ __forceinline__ void walk(int steps, int g0, int g1, int tile_first, 
 
 // One of eight splitting warps: U columns of a chunk (CS steps of KS values) at a time, a lane holds V consecutive values of each; the
 // loads of the next group (or of the next chunk's first) go out before this one is worked on, because a round trip to L2 takes
-// as long as splitting three columns. DIGITS: not terms but digits of 26-bit whole numbers (the factor puts the largest magnitude into
-// [2^25, 2^26]); values that are not all finite, or all below 2^-95, have the factor NaN.
-template <bool BF16, int NC, int KS, int CS, bool DIGITS>
+// as long as splitting three columns. AS_DIGITS: not three terms but six digits (the factor puts the largest magnitude into [2^25, 2^26]); values
+// that these do not hold to the last bit (not finite, all below 2^-95, or with bits 2^53 below the largest) have the factor NaN.
+template <bool BF16, int NC, int KS, int CS, bool AS_DIGITS>
 __device__ __forceinline__ void split_columns(const PlainParams &p, uint8_t *smem, int b_tile, int b_chunk, float (&inv)[4][NC], uint64_t (&bar_b)[2], uint64_t (&bar_bfree)[2], int w,
                                               int lane, int g0, int g1, int tile_first, volatile int *fail) {
     constexpr int V = CS * KS / 32, U = NC <= 24 ? NC / CONV_WARPS : NC / CONV_WARPS / 2;
@@ -127,6 +130,8 @@ __device__ __forceinline__ void split_columns(const PlainParams &p, uint8_t *sme
         for (int u = 0; u < U; u++) {
             const int n = n0 + u * CONV_WARPS;
             if (n >= p.N) break;
+            bool lost = false;
+            float factor = 1.f;
             if (!BF16) {
                 uint32_t m = 0;
 #pragma unroll
@@ -135,16 +140,22 @@ __device__ __forceinline__ void split_columns(const PlainParams &p, uint8_t *sme
                 const bool zero = m == 0;
                 m >>= 23;
                 // 2^(14 - exponent), kept within what f32 holds on both sides; 1 where nothing finite is to be scaled
-                const int ex = m == 0 || m == 255 ? 0 : max(-112, min(120, (DIGITS ? 152 : 141) - (int)m));
+                const int ex = m == 0 || m == 255 ? 0 : max(-112, min(120, (AS_DIGITS ? 152 : 141) - (int)m));
                 const float sc = __uint_as_float((uint32_t)(127 + ex) << 23);
 #pragma unroll
-                for (int i = 0; i < V; i++) v[u][i] *= sc;
-                if (lane == 0) inv[c & 3][n] = DIGITS && (m == 255 || (m < 32 && !zero)) ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - ex) << 23);
+                for (int i = 0; i < V; i++) {
+                    const float f = v[u][i] * sc;
+                    lost |= f == 0.f && v[u][i] != 0.f;
+                    v[u][i] = f;
+                }
+                lost |= m == 255 || (m < 32 && !zero);
+                factor = __uint_as_float((uint32_t)(127 - ex) << 23);
             }
 #pragma unroll
-            for (int t = 0; t < 3; t++) {
+            for (int t = 0; t < (AS_DIGITS ? DIGITS : 3); t++) {
                 auto take = [&](float &a, float &b) {
-                    if constexpr (DIGITS) return t == 0 ? take_digit<18>(a, b) : (t == 1 ? take_digit<9>(a, b) : take_digit<0>(a, b));
+                    if constexpr (AS_DIGITS)
+                        return t == 0 ? take_digit<0>(a, b) : t == 1 ? take_digit<1>(a, b) : t == 2 ? take_digit<2>(a, b) : t == 3 ? take_digit<3>(a, b) : t == 4 ? take_digit<4>(a, b) : take_digit<5>(a, b);
                     else return take_term<BF16>(a, b);
                 };
                 const int row = t * p.N + n;
@@ -152,6 +163,12 @@ __device__ __forceinline__ void split_columns(const PlainParams &p, uint8_t *sme
                 if (V == 8) *reinterpret_cast<uint4 *>(o) = make_uint4(take(v[u][0], v[u][1]), take(v[u][2], v[u][3]), take(v[u][4 % V], v[u][5 % V]), take(v[u][6 % V], v[u][7 % V]));
                 else *reinterpret_cast<uint2 *>(o) = make_uint2(take(v[u][0], v[u][1]), take(v[u][2], v[u][3]));
             }
+            if constexpr (AS_DIGITS) {
+#pragma unroll
+                for (int i = 0; i < V; i++) lost |= v[u][i] != 0.f;
+                if (__any_sync(0xffffffffu, lost)) factor = __uint_as_float(0x7fc00000u);
+            }
+            if (!BF16 && lane == 0) inv[c & 3][n] = factor;
         }
         if (last) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> async-proxy (MMA) reads
