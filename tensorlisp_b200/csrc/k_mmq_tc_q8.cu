@@ -639,8 +639,8 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 //
 // Why pairs: the copies of B bound wide tiles of single CTAs. 148 of them, each with the B of its own 128 rows, read 11 to 12.5 TB/s out
 // of L2 (2.4 us per unit of 256 elements of K at 336 columns, 1.55 at 256, whose MMAs take 1.45 and 1.1); the pair reads each
-// column once for 256 rows. Arrivals on the leader's barriers must not be of cluster scope: nothing but tensor memory and
-// copied shared memory passes between the CTAs, and a release of that scope made a unit 2.0 us instead of 1.15 at 64 columns.
+// column once for 256 rows. The threads' arrivals on the leader's barriers are of CTA scope: they only pass tensor memory on, between tcgen05 fences (a release
+// of cluster scope made a unit 2.0 us instead of 1.15 at 64 columns). The columns of B that the other CTA copied arrive on the leader's barrier by themselves.
 // The expanding warps fetch and expand before they wait for their slot (the wait, fetch, expansion and store as one chain took
 // 1000 cycles of a slot's round). Narrow tiles are bound by the expansion's instructions (326 per warp and unit for Q4_K, 268 for Q8_0, four
 // warps per scheduler; 404 and 52 -> 47 us for gate and up of 14336 x 4096 at 128 columns while codes went through f32 one by one); wide ones by the tensor pipe: 16384 columns run at 1400 to 1456 TFLOP/s (1253 to 1346 before).
@@ -710,6 +710,7 @@ __global__ void __launch_bounds__(256) k_act_pack_q80_f16(const int8_t *__restri
 
 struct Tc8fMaps {
     CUtensorMap m[tc8f::MAX_MATS];
+    CUtensorMap act[2];   // pairs: the packed B as rows of eight columns x 64 of K, boxes of one CTA's share of a tile or of either half
 };
 // One pass of a pair: a tile's rows and columns and its stretch of K; part >= 0: the tile's sum is cut, this is its part's number.
 struct FoldItem {
@@ -794,6 +795,12 @@ __device__ __forceinline__ uint32_t of_leader(const void *p) {
 // on a barrier of this CTA, or at an address that of_leader gave
 __device__ __forceinline__ void arrive_at(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// a box of a tensor into this CTA's shared memory; its bytes arrive on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(tc::su32(dst)),
+                 "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
 }
 template <bool PAIR>
 __device__ __forceinline__ void fold_tmem_alloc(uint32_t *dst_smem, uint32_t cols) {
@@ -926,7 +933,7 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         for (int i = 0; i < MAX_STAGES; i++) {
             mbar_init(&bar_raw[i], 1);
             mbar_init(&bar_rawfree[i], tc8f::DEQ_WARPS);
-            mbar_init(&bar_b[i], PAIR && rank == 0 ? 2 : 1);   // the leader's: its own copy and word from the other CTA
+            mbar_init(&bar_b[i], 1);
             mbar_init(&bar_bfree[i], 1);
         }
         for (int i = 0; i < A_RING; i++) {
@@ -970,10 +977,12 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
             }
         }
     } else if (warp == tc8f::TMA_B_WARP) {
-        // ---- packed activations: this CTA's columns of each half (at the end only what there is: columns do not mix; a part
-        // that is not there at all gets the last columns once more)
+        // ---- packed activations: this CTA's columns of each half (at the end what there is, or what comes behind it: columns do not mix; a part
+        // that is not there at all gets the last columns once more). Of a pair the copies of both CTAs arrive on the leader's barrier: its matrix
+        // instruction reads both, so nothing but the copies themselves may stand between.
         if (lane == 0) {
             griddep_wait();
+            const uint32_t bar_lead = PAIR ? of_leader(bar_b) : 0u;
             int s = 0;
             uint32_t ph = 0;
             for (int t = pair; t < p.items; t += pairs) {
@@ -983,12 +992,15 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
                     for (int ct = 0; ct < CT; ct++) {
                         const int mine = (ct == 0 ? p.nw : p.width - p.nw) / (8 * CTAS);   // groups of eight columns
                         const int g0 = min((f.col_tile * p.width + ct * p.nw) / 8 + (int)rank * mine, p.groups - 1);
-                        const uint32_t bytes = (uint32_t)min(mine, p.groups - g0) * 1024u;
+                        const uint32_t bytes = (uint32_t)(PAIR ? mine : min(mine, p.groups - g0)) * 1024u;
                         mbar_wait_nap(&bar_bfree[s], ph ^ 1u, fail, 32);
-                        mbar_expect_tx(&bar_b[s], bytes * STEP);
+                        if (rank == 0) mbar_expect_tx(&bar_b[s], bytes * STEP * CTAS);
 #pragma unroll
-                        for (int k = 0; k < STEP; k++)
-                            bulk_g2s(bst + s * b_stage + k * b_half, p.act + ((size_t)(i + k) * p.groups + g0) * 1024, bytes, &bar_b[s]);
+                        for (int k = 0; k < STEP; k++) {
+                            uint8_t *dst = bst + s * b_stage + k * b_half;
+                            if constexpr (PAIR) tma_2d_pair(dst, &maps.act[ct], 0, (i + k) * p.groups + g0, bar_lead + (uint32_t)s * 8u);
+                            else bulk_g2s(dst, p.act + ((size_t)(i + k) * p.groups + g0) * 1024, bytes, &bar_b[s]);
+                        }
                         if (++s == p.b_stages) {
                             s = 0;
                             ph ^= 1u;
@@ -998,67 +1010,51 @@ __global__ void __launch_bounds__(tc8f::THREADS, 1) k_mm_q80_f16(const __grid_co
         }
     } else if (warp == tc8f::MMA_WARP) {
         // ---- MMA issuer: one thread of the pair. Its own instructions are what bounds tiles of any width (a warp that probed and issued
-        // with all lanes: 750 cycles per 64 elements of K, of which the four MMAs of 256 columns need 512). The other CTA's thread
-        // passes on that its columns have arrived.
-        if (elect_one()) {
+        // with all lanes: 750 cycles per 64 elements of K, of which the four MMAs of 256 columns need 512).
+        if (rank == 0 && elect_one()) {
             int bs = 0, as = 0;
             uint32_t bph = 0, aph = 0, it = 0;
-            if (PAIR && rank != 0) {
-                const uint32_t lead = of_leader(bar_b);
-                for (int t = pair; t < p.items; t += pairs) {
-                    const FoldItem f = p.item(t);
-                    for (int i = (f.k1 - f.k0) * 4 / STEP * CT; i > 0; i--) {
-                        mbar_wait_nap(&bar_b[bs], bph, fail, 0);
-                        arrive_at(lead + (uint32_t)bs * 8u);
+            const uint64_t b_desc0 = smem_desc(su32(bst), 128, 1024);
+            const uint32_t b_step = (uint32_t)b_stage >> 4;
+            uint32_t b_at = 0;
+            bool b_here = false, a_here = false;
+            for (int t = pair; t < p.items; t += pairs, it++) {
+                const FoldItem f = p.item(t);
+                const uint32_t ai = it % accs;
+                mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
+                uint32_t more = 0;
+#pragma unroll 1
+                for (int i = (f.k1 - f.k0) * 4 / STEP; i > 0; i--) {
+                    if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
+                    const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * (32u * STEP);
+                    uint64_t *const afree = &bar_afree[as];
+                    if (++as == A_RING) {
+                        as = 0;
+                        aph ^= 1u;
+                    }
+#pragma unroll
+                    for (int ct = 0; ct < CT; ct++) {
+                        if (!b_here) mbar_wait_nap(&bar_b[bs], bph, fail, 0);
+                        if (ct == 0) tc_fence_after();
+                        uint64_t *const bfree = &bar_bfree[bs];
+                        const uint64_t desc = b_desc0 + b_at;
+                        b_at += b_step;
                         if (++bs == p.b_stages) {
                             bs = 0;
+                            b_at = 0;
                             bph ^= 1u;
                         }
-                    }
-                }
-            } else {
-                const uint64_t b_desc0 = smem_desc(su32(bst), 128, 1024);
-                const uint32_t b_step = (uint32_t)b_stage >> 4;
-                uint32_t b_at = 0;
-                bool b_here = false, a_here = false;
-                for (int t = pair; t < p.items; t += pairs, it++) {
-                    const FoldItem f = p.item(t);
-                    const uint32_t ai = it % accs;
-                    mbar_wait_nap(&bar_accfree[ai], ((it / accs) & 1u) ^ 1u, fail, 32);   // the tile before in this accumulator has been drained
-                    uint32_t more = 0;
-#pragma unroll 1
-                    for (int i = (f.k1 - f.k0) * 4 / STEP; i > 0; i--) {
-                        if (!a_here) mbar_wait_nap(&bar_aready[as], aph, fail, 0);
-                        const uint32_t a0 = tmem_base + ACOLS + (uint32_t)as * (32u * STEP);
-                        uint64_t *const afree = &bar_afree[as];
-                        if (++as == A_RING) {
-                            as = 0;
-                            aph ^= 1u;
-                        }
+                        if (ct == CT - 1) a_here = mbar_test(su32(&bar_aready[as]), aph);
+                        b_here = mbar_test(su32(&bar_b[bs]), bph);
 #pragma unroll
-                        for (int ct = 0; ct < CT; ct++) {
-                            if (!b_here) mbar_wait_nap(&bar_b[bs], bph, fail, 0);
-                            if (ct == 0) tc_fence_after();
-                            uint64_t *const bfree = &bar_bfree[bs];
-                            const uint64_t desc = b_desc0 + b_at;
-                            b_at += b_step;
-                            if (++bs == p.b_stages) {
-                                bs = 0;
-                                b_at = 0;
-                                bph ^= 1u;
-                            }
-                            if (ct == CT - 1) a_here = mbar_test(su32(&bar_aready[as]), aph);
-                            b_here = mbar_test(su32(&bar_b[bs]), bph);
-#pragma unroll
-                            for (int k = 0; k < STEP; k++)
-                                umma4_f16<PAIR>(tmem_base + (CT == 1 ? ai : (uint32_t)ct) * ACC2, a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), idesc[ct], k ? 1u : more);
-                            fold_commit<PAIR>(bfree);
-                        }
-                        fold_commit<PAIR>(afree);
-                        more = 1;
+                        for (int k = 0; k < STEP; k++)
+                            umma4_f16<PAIR>(tmem_base + (CT == 1 ? ai : (uint32_t)ct) * ACC2, a0 + (uint32_t)k * 32u, desc + (uint64_t)(k * (b_half >> 4)), idesc[ct], k ? 1u : more);
+                        fold_commit<PAIR>(bfree);
                     }
-                    fold_commit<PAIR>(&bar_accfull[ai]);
+                    fold_commit<PAIR>(afree);
+                    more = 1;
                 }
+                fold_commit<PAIR>(&bar_accfull[ai]);
             }
         }
         __syncwarp();
@@ -1190,6 +1186,7 @@ __global__ void __launch_bounds__(256) k_fold_sum(const __grid_constant__ Tc8fPa
 
 cudaError_t tc_encode_2d(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows,
                          uint32_t elem_bytes);
+cudaError_t tc_encode_2d_bytes(CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows);
 // Time of a unit (256 elements of K) of a tile in us, all SMs at work. Measured, Q4_K / Q8_0: pairs 1.02 / 0.90 at 64 columns, 1.10 / 1.00 at 128,
 // 1.42 / 1.28 at 192, 1.72 / 1.70 at 256, in halves 2.20 / 2.10 at 352; single CTAs 1.15 at 80, 1.33 at 128, 2.1 at 256.
 static double fold_unit_us(bool q4k, int ctas, int width) {
@@ -1272,6 +1269,12 @@ cudaError_t launch_mm_fold_f16(bool q4k, int n_mats, const void *const *W, int64
     p.b_stages = std::min(tc8f::MAX_STAGES, (tc8f::SMEM - 1024 - p.raw_stages * raw_bytes) / (p.nw / plan.ctas * tc8f::KS * (shape == 0 ? 4 : 2)));
     if (p.b_stages < 2) return cudaErrorInvalidValue;
     p.groups = mm_fold_groups(N);
+    if (plan.ctas == 2)
+        for (int h = 0; h < 2; h++) {
+            const int cols = h == 0 || p.width == p.nw ? p.nw : p.width - p.nw;
+            const cudaError_t e = tc_encode_2d_bytes(&maps.act[h], blobs, 1024, (uint64_t)(K / tc8f::KS) * p.groups, 1024, (uint32_t)(cols / 16));
+            if (e != cudaSuccess) return e;
+        }
     p.err = err;
     const dim3 grid((unsigned)(plan.ctas * std::min(p.items, std::max(1, sms / plan.ctas))));
     auto go = [&](auto *k) { return launch_pdl_cluster(early, plan.ctas, k, grid, dim3(tc8f::THREADS), (size_t)tc8f::SMEM, st, maps, p); };
