@@ -1313,10 +1313,10 @@ void rewrite_graph(Graph &g, int sm_count) {
     // Quantize each distinct activation once: a QUANT_ACT node in front of the first quantized
     // MUL_MAT that reads it, shared by later ones until something writes its storage again.
     std::vector<int32_t> nodes;
-    // (activation tensor, kind) -> QUANT_ACT tensor. Q4_0 matrices and Q8_0 ones that read the same activation agree on the packed
-    // operand up to 64 columns; above, they take different ones, and the key says so.
-    std::map<std::pair<int32_t, int>, int32_t> cache;
-    constexpr int OTHER_OPERAND = 256;
+    // (activation tensor, kind) -> its QUANT_ACT tensors. A product on the tensor cores also reads the operand that is packed behind the block,
+    // and a QUANT_ACT packs one (op_params[1], 0: none). Products agree on it or take another QUANT_ACT: above 64 columns it differs between
+    // types, and between Q4_0 matrices of many and of few rows (mmq_tc8_plan).
+    std::map<std::pair<int32_t, int>, std::vector<int32_t>> cache;
     for (size_t i = 0; i < g.nodes.size(); i++) {
         if (dead[i]) continue;
         const int32_t id = g.nodes[i];
@@ -1340,12 +1340,13 @@ void rewrite_graph(Graph &g, int sm_count) {
             if (ok && tx.ne[2] > 1) ok = tx.nb[2] == tx.nb[1] * (uint64_t)tx.ne[1];
             if (ok && tx.ne[3] > 1) ok = tx.nb[3] == tx.nb[1] * (uint64_t)tx.ne[1] * (uint64_t)tx.ne[2];
             if (ok) {
-                auto key = std::make_pair(x, tw.ty == TLB_TYPE_Q4_0 && tx.ne[1] > 64 ? kind | OTHER_OPERAND : kind);
-                auto it = cache.find(key);
-                int32_t qa;
-                if (it != cache.end()) {
-                    qa = it->second;
-                } else {
+                const bool plain2d = tw.ne[2] * tw.ne[3] * t.ne[2] * t.ne[3] == 1 && tw.nb[1] == tw.row_size();
+                TcPlan tp{};
+                if (plain2d && tc_supported(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1]) && !getenv("TLB_NO_TC")) tp = tc_plan(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1], sm_count);
+                int32_t qa = -1;
+                for (int32_t c : cache[{x, kind}])
+                    if (qa < 0 && (tp.npad == 0 || g.tensors[c].op_params[1] == 0 || g.tensors[c].op_params[1] == tp.npad)) qa = c;
+                if (qa < 0) {
                     Tensor q;
                     q.ty = TLB_TYPE_I8;
                     q.op = "QUANT_ACT";
@@ -1359,14 +1360,10 @@ void rewrite_graph(Graph &g, int sm_count) {
                     qa = (int32_t)g.tensors.size();
                     g.tensors.push_back(q);
                     nodes.push_back(qa);
-                    cache[key] = qa;
+                    cache[{x, kind}].push_back(qa);
                 }
                 g.tensors[id].src[2] = qa;
-                // a consumer that takes the tensor-core path also needs the packed blobs behind the Q8_K block
-                const Tensor &mm = g.tensors[id];
-                const bool plain2d = tw.ne[2] * tw.ne[3] * mm.ne[2] * mm.ne[3] == 1 && tw.nb[1] == tw.row_size();
-                if (plain2d && tc_supported(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1]) && !getenv("TLB_NO_TC")) {
-                    const TcPlan tp = tc_plan(tw.ty, tx.ne[0], tw.ne[1], tx.ne[1], sm_count);
+                if (tp.npad) {
                     Tensor &q = g.tensors[qa];
                     q.op_params[1] = tp.npad;
                     q.opaque_bytes = act_layout(kind, tx.ne[0], tx.nrows()).bytes + tp.blob_bytes;

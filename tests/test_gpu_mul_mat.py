@@ -189,3 +189,31 @@ def test_q4_0_beside_q8_0(oracle, K, M, N):
     assert close(y4, oracle.mul_mat(Q4_0, Ws[0], K, X), TOL) <= 1e-5 * np.abs(y4).max()
     close(y8, oracle.mul_mat(Q8_0, Ws[1], K, X), TOL)
     m.close()
+
+
+@pytest.mark.parametrize("N", [65, 256, 768])
+@pytest.mark.parametrize("Ms", [(4096, 1024, 1024), (1024, 4096, 1024)])
+def test_q4_0_matrices_of_many_and_of_few_rows_on_one_activation(oracle, Ms, N):
+    """The projections of grouped-query attention. Above 64 columns a Q4_0 matrix of many rows takes tiles of 128 columns and one of few
+    rows passes of 32, each with its own packing of the activation that they share (at 256 columns on 148 SMs here: 64 and 16 tiles, the line
+    lies at 49). Behind a norm, as in a decoder. Integer sums of a block at every size: see test_q4_0_beside_q8_0."""
+    K = 512
+    rng = np.random.default_rng(N)
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    wn = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    Ws = [oracle.quantize(Q4_0, (rng.standard_normal((M, K)) * 0.02).astype(np.float32)) for M in Ms]
+    for normed in (False, True):
+        g = G.Graph()
+        tn = g.weight(G.F32, [K], "n")
+        tw = [g.weight(Q4_0, [K, M], "W%d" % i) for i, M in enumerate(Ms)]
+        x = g.input(G.F32, [K, N], "x")
+        a = g.mul(g.rms_norm(x, 1e-5), tn) if normed else x
+        for i, w in enumerate(tw):
+            g.output(g.mul_mat(w, a, "y%d" % i))
+        m = Model(g, [wn] + Ws)
+        got = m.run(X)
+        m.close()
+        A = oracle.rms_norm(X, 1e-5, wn) if normed else X
+        for y, w in zip(got, Ws):
+            # (a norm one unit in the last place off moves a code where it lies between two)
+            assert close(y, oracle.mul_mat(Q4_0, w, K, A), TOL) <= (1e-3 if normed else 1e-5) * np.abs(y).max()
