@@ -624,6 +624,8 @@ template <int PARTS>
 __global__ void k_argmax(TView a, const uint8_t *x, int32_t *out) {
     __shared__ float smax[32];
     __shared__ int sidx[32];
+    // shared memory of a CTA may be written once it is known to run: all of a cluster say so here, and it is waited for behind the scan
+    if constexpr (PARTS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int64_t row = blockIdx.x / PARTS;
     const int rank = (int)(blockIdx.x % PARTS);
     const float *xr = reinterpret_cast<const float *>(x + row * a.nb[1]);
@@ -676,6 +678,8 @@ __global__ void k_argmax(TView a, const uint8_t *x, int32_t *out) {
     if constexpr (PARTS > 1) {
         __shared__ float pmax[PARTS];
         __shared__ int pidx[PARTS];
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
         if (threadIdx.x == 0) {
             uint32_t m, i;
             asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(m) : "r"((uint32_t)__cvta_generic_to_shared(&pmax[rank])));
@@ -683,6 +687,7 @@ __global__ void k_argmax(TView a, const uint8_t *x, int32_t *out) {
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(m), "f"(mx) : "memory");
             asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(i), "r"(idx) : "memory");
         }
+        __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (rank == 0 && threadIdx.x == 0) {

@@ -188,6 +188,21 @@ def test_argmax_of_long_rows(n):
     assert np.array_equal(np.asarray(got).reshape(-1), want)
 
 
+@pytest.mark.parametrize("rows", [128, 129])
+def test_argmax_of_more_clusters_than_the_chip_holds(rows):
+    """Up to 128 long rows take a cluster of eight CTAs each, whose CTAs start at different times when the chip is full; one row more takes a CTA per row."""
+    n = 16384
+    x = np.random.default_rng(rows).standard_normal((rows, n)).astype(np.float32)
+    g = G.Graph()
+    tx = g.input(G.F32, [n, rows])
+    g.output(g.argmax(tx))
+    m = Model(g)
+    for _ in range(5):
+        (got,) = m.run(x)
+        assert np.array_equal(np.asarray(got).reshape(-1), x.argmax(1))
+    m.close()
+
+
 def test_masked_soft_max():
     rng = np.random.default_rng(3)
     x = rng.standard_normal((2, 5, 64)).astype(np.float32)       # [heads, rows, n]
