@@ -685,8 +685,20 @@ static void push_drop(tlb_program *p, const std::function<bool(const tlb_program
     p->pushed.erase(std::remove_if(p->pushed.begin(), p->pushed.end(), which), p->pushed.end());
     if (p->pushed.size() != before) push_table(p);
 }
+// Results that nobody reads any more: a push of up to 64 KB costs about 2 us a run, a block of its own 24 us per MB.
+static bool unread_long(const tlb_program::Pushed &o) { return o.unread > (o.block ? 2 : 64); }
 static void push_drop_unread(tlb_program *p) {
-    push_drop(p, [](const tlb_program::Pushed &o) { return o.unread > 64; });
+    for (const auto &o : p->pushed)
+        if (o.block && unread_long(o)) p->read_now_and_then[o.tensor] = 0;
+    push_drop(p, unread_long);
+}
+// While sequences use the page, such a block's entry is made one of no bytes (its length is one word) and dropped later.
+static void push_mute_unread(tlb_program *p) {
+    for (size_t i = 0; i < p->pushed.size(); i++)
+        if (p->pushed[i].block && unread_long(p->pushed[i])) {
+            *(volatile uint64_t *)&p->page->out[i].n16 = 0;
+            p->pushed[i].valid_from = UINT64_MAX;
+        }
 }
 
 // ------------------------------------------------------------------ programs
@@ -909,6 +921,7 @@ tlb_status tlb_program_enqueue(tlb_program *prog, tlb_buffer *const *weights, ui
     const bool idle = prog->page_seq <= prog->dev->done.load();
     for (auto &o : prog->pushed) o.unread++;
     if (idle) push_drop_unread(prog);
+    else push_mute_unread(prog);
     // Small inputs come in, the launches, results that are read after every run go out. A captured sequence always has
     // the two page kernels that it may need (their tables say what moves), a direct one launches them when there is something to move.
     auto sequence = [&](bool captured, bool prof) {
@@ -1073,8 +1086,16 @@ tlb_status tlb_program_read(tlb_program *prog, uint32_t tensor_id, uint64_t byte
         }
     if (pl.buf == BUF_IO) TLB_TRY_CUDA(flush_inputs(prog), TLB_EXECUTION);
     TLB_TRY_CUDA(copy_d2h(prog->ordinal, out, base + pl.off, bytes, prog->dev->stream), TLB_EXECUTION);
-    if (bytes <= IO_OUT_MAX && std::none_of(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; })) {
+    if (bytes <= IO_OUT_MAX) {
         TLB_TRY_CUDA(page_idle(prog), TLB_EXECUTION);
+        push_drop_unread(prog);
+        if (std::any_of(prog->pushed.begin(), prog->pushed.end(), [&](const tlb_program::Pushed &o) { return o.tensor == tensor_id; })) return TLB_OK;
+        auto it = prog->read_now_and_then.find(tensor_id);
+        if (it != prog->read_now_and_then.end() && it->second + 1 != prog->runs) {
+            it->second = prog->runs;
+            return TLB_OK;
+        }
+        if (it != prog->read_now_and_then.end()) prog->read_now_and_then.erase(it);
         push_add(prog, tensor_id, bytes);
     }
     return TLB_OK;

@@ -229,6 +229,8 @@ struct tlb_program {
         int unread;                      // runs since it was last read
     };
     std::vector<Pushed> pushed;
+    // results whose block was pushed for nothing, and the run of their last read: they get one again when two runs in a row were read
+    std::map<uint32_t, uint64_t> read_now_and_then;
     std::vector<uint32_t> no_push;       // tensors whose device address the caller holds
     uint64_t runs = 0;
 };

@@ -134,6 +134,57 @@ def test_a_result_that_the_run_has_written_is_handed_over_once(n):
     native.close()
 
 
+def test_a_large_result_that_is_read_now_and_then_is_not_pushed_every_run():
+    """Two runs that were not read end the pushing of a result above 64 KB, waited for or not; two runs in a row that were read bring it
+    back. Every read sees the last run."""
+    n = 65536
+    native = Native.load([])
+    g = G.Graph()
+    y = g.output(g.scale(g.input(G.F32, [n], "x"), 2.0))
+    prog = NativeProgram.compile(native, g)
+    a = np.arange(n, dtype=np.float32)
+
+    def go(wait=True):
+        nonlocal a
+        if not wait:
+            return prog.enqueue()       # (a new input would wait for the runs before)
+        a = a + 1
+        prog.set_input(0, a)
+        prog.run()
+
+    def read():
+        assert np.array_equal(prog.read(y).reshape(-1), 2 * a)
+
+    def pushed():
+        p = C.c_void_p()
+        check(native.L.tlb_program_take(prog.h, y, 4 * n, C.byref(p)))
+        if p.value:
+            assert np.array_equal(np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), (n,)), 2 * a)
+            native.L.tlb_host_free(p)
+        return bool(p.value)
+
+    for wait in (True, False):
+        for _ in range(3):
+            go()
+            read()
+        go()
+        assert pushed()
+        for _ in range(4):
+            go(wait)
+        assert not pushed()
+        read()              # one run is read, the next is not: not pushed
+        go()
+        go()
+        assert not pushed()
+        for _ in range(2):
+            read()
+            go()
+        assert pushed()
+        read()
+    prog.free()
+    native.close()
+
+
 @pytest.mark.parametrize("held", ["a view", "the tensor of a view", "the tensor itself"])
 def test_an_address_into_a_result_through_another_tensor_of_its_storage(held):
     """Who holds the address of a view writes into the root's memory (and the other way round): what read() returns then comes from
