@@ -263,6 +263,92 @@ uint64_t tlb_row_size(uint32_t type, int64_t ne0) {
 }
 
 // ------------------------------------------------------------------ device
+// A program's arena and io buffer. cudaMalloc maps new memory for each block of more than 1 MB (0.32 ms, and 0.27 when it goes), and for
+// smaller ones every 2 MB; a [4096 x 4096] Q4_0 product at 16 columns has 1.2 MB of parts of its sums, and a first call with a new shape took
+// 0.73 ms instead of 0.32. So blocks of up to SLAB_BLOCK_MAX are cut from slabs, which cost as much once. What the slabs cannot hold is a
+// cudaMalloc as before; slabs that nothing uses are given back when the last handle of their device closes.
+namespace {
+constexpr uint64_t SLAB_BYTES = 16ull << 20, SLAB_BLOCK_MAX = 4ull << 20, SLAB_ALIGN = 512;
+struct Slab {
+    char *base = nullptr;
+    std::map<uint64_t, uint64_t> gaps;   // offset -> bytes, no two of them touch
+};
+struct ProgramMemory {
+    Slab slabs[2];
+    std::map<char *, uint64_t> blocks;   // handed out
+    int devices = 0;                     // open handles
+};
+std::mutex program_memory_mutex;
+ProgramMemory &program_memory_of(int ordinal) {
+    static std::map<int, ProgramMemory> *all = new std::map<int, ProgramMemory>;   // never destroyed: programs may be freed while the process ends
+    return (*all)[ordinal];
+}
+void slabs_trim(ProgramMemory &m) {
+    for (Slab &s : m.slabs) {
+        if (m.devices > 0 || !s.base || s.gaps.size() != 1 || s.gaps.begin()->second != SLAB_BYTES) continue;
+        cudaFree(s.base);
+        s = Slab();
+    }
+}
+// (the device is current)
+cudaError_t program_malloc(int ordinal, void **out, uint64_t bytes) {
+    bytes = (bytes + SLAB_ALIGN - 1) / SLAB_ALIGN * SLAB_ALIGN;
+    if (bytes <= SLAB_BLOCK_MAX) {
+        std::lock_guard<std::mutex> lock(program_memory_mutex);
+        ProgramMemory &m = program_memory_of(ordinal);
+        for (Slab &s : m.slabs) {
+            if (!s.base) {
+                if (cudaMalloc(&s.base, SLAB_BYTES) != cudaSuccess) {
+                    cudaGetLastError();
+                    s.base = nullptr;
+                    break;
+                }
+                s.gaps[0] = SLAB_BYTES;
+            }
+            auto g = std::find_if(s.gaps.begin(), s.gaps.end(), [&](const auto &x) { return x.second >= bytes; });
+            if (g == s.gaps.end()) continue;
+            const uint64_t at = g->first, left = g->second - bytes;
+            s.gaps.erase(g);
+            if (left) s.gaps[at + bytes] = left;
+            m.blocks[s.base + at] = bytes;
+            *out = s.base + at;
+            return cudaSuccess;
+        }
+    }
+    return cudaMalloc(out, bytes);
+}
+// nothing on the device uses it any more
+void program_mfree(int ordinal, void *q) {
+    if (!q) return;
+    std::lock_guard<std::mutex> lock(program_memory_mutex);
+    ProgramMemory &m = program_memory_of(ordinal);
+    auto b = m.blocks.find((char *)q);
+    if (b == m.blocks.end()) {
+        cudaFree(q);
+        return;
+    }
+    for (Slab &s : m.slabs) {
+        if (!s.base || b->first < s.base || b->first >= s.base + SLAB_BYTES) continue;
+        uint64_t at = (uint64_t)(b->first - s.base), n = b->second;
+        auto next = s.gaps.lower_bound(at);
+        if (next != s.gaps.end() && next->first == at + n) {
+            n += next->second;
+            next = s.gaps.erase(next);
+        }
+        if (next != s.gaps.begin() && std::prev(next)->first + std::prev(next)->second == at) std::prev(next)->second += n;
+        else s.gaps[at] = n;
+    }
+    m.blocks.erase(b);
+    slabs_trim(m);
+}
+void program_memory_device(int ordinal, int by) {
+    std::lock_guard<std::mutex> lock(program_memory_mutex);
+    ProgramMemory &m = program_memory_of(ordinal);
+    m.devices += by;
+    slabs_trim(m);
+}
+}  // namespace
+
 tlb_status tlb_device_open(int ordinal, tlb_device **dev) {
     if (!dev) return fail(TLB_INVALID, "tlb_device_open: null output");
     *dev = nullptr;
@@ -306,6 +392,7 @@ tlb_status tlb_device_open(int ordinal, tlb_device **dev) {
     d->name = std::string("native ") + d->prop.name;
     configure_kernels_once(ordinal);   // cudaSetDevice(ordinal) above made it current
     pinned_device(ordinal);
+    program_memory_device(ordinal, 1);
     *dev = d;
     return TLB_OK;
 }
@@ -316,6 +403,7 @@ void tlb_device_close(tlb_device *dev) {
     cudaSetDevice(dev->ordinal);
     quant_space_free(dev);
     if (dev->stream) cudaStreamDestroy(dev->stream);
+    program_memory_device(dev->ordinal, -1);
     delete dev;
 }
 
@@ -766,12 +854,12 @@ tlb_status tlb_program_compile(tlb_device *dev, const tlb_graph *graph, const tl
         return bad(TLB_UNSUPPORTED, m);
     }
     cudaSetDevice(dev->ordinal);
-    cudaError_t e = cudaMalloc(&p->arena, align_up(std::max<uint64_t>(p->layout.arena_size, 1)) + 256 + align_up(sizeof(IoSync)));
+    cudaError_t e = program_malloc(p->ordinal, &p->arena, align_up(std::max<uint64_t>(p->layout.arena_size, 1)) + 256 + align_up(sizeof(IoSync)));
     if (e == cudaSuccess) {
         p->io_sync = (IoSync *)((char *)p->arena + align_up(std::max<uint64_t>(p->layout.arena_size, 1)) + 256);
         e = cudaMemsetAsync(p->io_sync, 0, sizeof(IoSync), dev->stream);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&p->io, std::max<uint64_t>(p->layout.io_size, 1));
+    if (e == cudaSuccess) e = program_malloc(p->ordinal, &p->io, std::max<uint64_t>(p->layout.io_size, 1));
     if (e != cudaSuccess) {
         cudaGetLastError();
         const uint64_t want = p->layout.arena_size + p->layout.io_size;
@@ -821,10 +909,10 @@ void tlb_program_free(tlb_program *prog) {
     cudaSetDevice(prog->ordinal);
     for (auto &c : prog->captured)
         if (c.exec) cudaGraphExecDestroy(c.exec);
-    if (prog->arena) cudaFree(prog->arena);
-    if (prog->io) cudaFree(prog->io);
+    cudaDeviceSynchronize();   // arena, io buffer and page may go to another program: no kernel may still use them
+    program_mfree(prog->ordinal, prog->arena);
+    program_mfree(prog->ordinal, prog->io);
     if (prog->page) {
-        cudaDeviceSynchronize();   // the page goes back to the pool: no kernel may still write to it
         pinned_free(prog->page);
         for (const auto &o : prog->pushed) pinned_free(o.block);
     }

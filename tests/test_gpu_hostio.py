@@ -262,3 +262,42 @@ def test_quantize_rows_in_pieces(oracle, ty, name, rows, n):
     some = np.unique(np.concatenate([[0, rows - 1], np.random.default_rng(1).integers(0, rows, 40)]))
     assert np.array_equal(got[some], oracle.quantize(ty, x[some]))
     native.close()
+
+
+def test_programs_of_many_sizes_come_and_go():
+    """Arenas and inputs of up to 4 MB are cut from slabs of 16 MB, two at most; what does not fit there, and larger ones, are blocks of
+    their own. Programs that live side by side share no bytes, in whatever order they come and go, and the memory goes back with the device."""
+    import torch
+
+    def cycle(rounds):
+        rng = np.random.default_rng(rounds)
+        native = Native.load([])
+        live = []
+        for _ in range(rounds):
+            for _ in range(int(rng.integers(1, 8))):
+                n = int(rng.choice([1, 100, 70001, 300000, 524288, 1048448, 1048576, 1048577, 1400000]))
+                g = G.Graph()
+                y = g.output(g.scale(g.input(G.F32, [n], "x"), 2.0))
+                prog = NativeProgram.compile(native, g)
+                a = rng.integers(-1000, 1000, n).astype(np.float32)
+                prog.set_input(0, a)
+                prog.enqueue()
+                live.append((prog, y, a))
+            for prog, y, a in live:
+                assert np.array_equal(prog.read(y).reshape(-1), 2 * a)
+            for prog, _, _ in live:     # the inputs are still there, too
+                prog.enqueue()
+            for i in rng.permutation(len(live))[:len(live) // 2]:
+                live[i][0].free()
+                live[i] = None
+            live = [x for x in live if x]
+            for prog, y, a in live:
+                assert np.array_equal(prog.read(y).reshape(-1), 2 * a)
+        for prog, _, _ in live:
+            prog.free()
+        native.close()
+
+    cycle(2)
+    before = torch.cuda.mem_get_info()[0]
+    cycle(12)
+    assert torch.cuda.mem_get_info()[0] >= before - (4 << 20)
