@@ -1731,7 +1731,7 @@ void fuse_gemv(Graph &g, bool groups, bool producers) {
         const Tensor W0 = g.tensors[A.src[0]];
         int members = 1;
         int last = (int)i;
-        if (groups && W0.row_size() % 16 == 0 && A.view_src < 0) {
+        if (groups && W0.row_size() % 16 == 0 && A.view_src < 0 && W0.ty != TLB_TYPE_Q6_K) {   // (k_gemv_q6.cu and k_gemv_f32.cu take one matrix)
             for (size_t j = i + 1; j < nn && members < 3; j++) {
                 const Tensor &B = g.tensors[g.nodes[j]];
                 if (B.is_view_op()) continue;

@@ -287,3 +287,30 @@ def test_q6_K_on_the_tensor_cores_unusual_values(oracle, bad):
     fin = np.isfinite(want)
     assert np.allclose(got[fin], want[fin], atol=1e-5)
     m.close()
+
+
+@pytest.mark.parametrize("N", [1, 2, 3])
+@pytest.mark.parametrize("K", [2048, 1792])
+def test_q6_K_matrices_on_one_activation(oracle, K, N):
+    """Projections of one activation, and gate and up in front of a gated product, with rows that are a multiple of 16 bytes (2048 weights) and that
+    are not: the few-column kernels of the other types take such matrices in one launch, the Q6_K ones take one each. Bound as in
+    test_q6_K_against_f64; the gate adds the exponential's and the division's two units in the last place, the second product's input rounding none (f32)."""
+    rng = np.random.default_rng(K + N)
+    X = rng.standard_normal((N, K)).astype(np.float32)
+    Ws = [oracle.quantize(Q6_K, (rng.standard_normal((M, K)) * 0.02).astype(np.float32)) for M in (512, 128, 512)]
+    D = [oracle.dequantize(Q6_K, w, K).reshape(-1, K).astype(np.float64) for w in Ws]
+    g = G.Graph()
+    x = g.input(G.F32, [K, N], "x")
+    ys = [g.mul_mat(g.weight(Q6_K, [K, len(d)], "W%d" % i), x, "y%d" % i) for i, d in enumerate(D)]
+    for y in ys:
+        g.output(y)
+    gate, up = (g.mul_mat(g.weight(Q6_K, [K, 512], n), x, n) for n in ("gate", "up"))
+    g.output(g.mul(g.silu(gate), up))
+    m = Model(g, Ws + [Ws[0], Ws[2]])
+    *got, h = m.run(X)
+    m.close()
+    want = [X.astype(np.float64) @ d.T for d in D]
+    for a, b in zip(got, want):
+        assert np.linalg.norm(a.reshape(b.shape) - b) <= 2.5e-7 * np.linalg.norm(b)
+    b = want[0] / (1 + np.exp(-want[0])) * want[2]
+    assert np.linalg.norm(h.reshape(b.shape) - b) <= 1e-6 * np.linalg.norm(b)
