@@ -335,7 +335,7 @@ void gemv_f32_configure() {
 
 cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st) {
     if (g.n_mats != 1 || g.glu || g.act.mode != RQ_PLAIN) return cudaErrorInvalidValue;
-    if (g.N <= gemv_q6_columns(g.K)) return launch_gemv_q6(g, sm_count, err, st);
+    if (g.N <= gemv_q6_columns(g.K, g.M[0])) return launch_gemv_q6(g, sm_count, err, st);
     gemvf::Params p{};
     p.W = (const uint8_t *)g.W[0];
     p.x = g.act.a;

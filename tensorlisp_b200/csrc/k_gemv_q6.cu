@@ -18,6 +18,7 @@
 // ring, eight warps take a super-block of 16 rows each. Rows of whole 8-super-block segments are copied by 2-D boxes of 16 x 1680
 // bytes (16 bytes past a multiple of 128: eight rows on different banks), shorter rows as 16 rows in one piece.
 #include <algorithm>
+#include <cstdlib>
 #include <cuda_fp16.h>
 
 #include "dequant.cuh"
@@ -344,12 +345,16 @@ static bool gemv_q6_geometry(gemvq6::Params &p, int64_t K, int nc, size_t &smem,
 }
 // One column, and as many as make 32 KB of digits. us of a launch, cold, this kernel / k_gemv_f32.cu: two columns of [30000 x 512] 16.6 / 21.1, [20000 x 1024]
 // 18.0 / 23.8, [1500 x 2048] 14.5 / 13.4, [3000 x 2816] 17.7 / 17.4, [4096 x 4096] 21.5 / 18.1, [4096 x 14336] 55.5 / 39.2; four of [30000 x 512] 18.7 /
-// 27.8, [20000 x 1024] 23.2 / 32.5, [1500 x 2048] 16.2 / 15.8, [4096 x 4096] 27.8 / 22.4.
-int gemv_q6_columns(int64_t K) {
+// 27.8, [20000 x 1024] 23.2 / 32.5, [1500 x 2048] 16.2 / 15.8, [4096 x 4096] 27.8 / 22.4. A CTA takes 16 rows at least, so fewer than 148 of these leave
+// SMs idle, and k_gemv_f32.cu spreads them further: one column in a row of launches [1024 x 4096] 8.8 / 5.2, [1500 x 2048] 5.9 / 4.8 (two: 7.9 / 5.5),
+// [4096 x 4096] 9.0 / 9.3.
+// (TLB_Q6_DIGITS: small matrices here and in k_mm_q6.cu all the same, for tests of their edges)
+constexpr int64_t Q6_ROWS = 16 * 148;
+int gemv_q6_columns(int64_t K, int64_t M) {
     gemvq6::Params p{};
     size_t smem;
     int per_sm, nc = 0;
-    if (!tc_available() || K % 256 != 0 || K < 256 || K > (1 << 20)) return 0;
+    if (!tc_available() || (M < Q6_ROWS && !getenv("TLB_Q6_DIGITS")) || K % 256 != 0 || K < 256 || K > (1 << 20)) return 0;
     while (nc < 4 && (nc == 0 || (nc + 1) * K <= 4096) && gemv_q6_geometry(p, K, nc + 1, smem, per_sm)) nc++;
     return nc;
 }
@@ -372,7 +377,7 @@ cudaError_t launch_gemv_q6(const GemvArgs &g, int sm_count, int *err, cudaStream
     CUtensorMap map{};
     size_t smem = 0;
     int per_sm = 1;
-    if (g.N < 1 || g.N > gemv_q6_columns(g.K) || !gemv_q6_geometry(p, g.K, (int)g.N, smem, per_sm)) return cudaErrorInvalidValue;
+    if (g.N < 1 || g.N > gemv_q6_columns(g.K, g.M[0]) || !gemv_q6_geometry(p, g.K, (int)g.N, smem, per_sm)) return cudaErrorInvalidValue;
     if (p.boxes) {
         const cudaError_t e = tc_encode_2d_bytes(&map, g.W[0], (uint64_t)p.row_bytes, (uint64_t)p.M, (uint32_t)p.row_stride, 16);
         if (e != cudaSuccess) return e;

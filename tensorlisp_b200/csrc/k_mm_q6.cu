@@ -23,6 +23,7 @@
 // issue slots. A pass of one column takes 66 us at [32000 x 4096], copies alone 44, unpacking adds 13; splitting and adding grow with columns times
 // digits, so that ten columns in one pass (113 us) gain little on two passes of five.
 #include <algorithm>
+#include <cstdlib>
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -328,11 +329,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_mm_q6(const __grid_constant__ CU
 // ---------------------------------------------------------------- host side
 void mm_q6_configure() { cudaFuncSetAttribute(q6tc::k_mm_q6, cudaFuncAttributeMaxDynamicSharedMemorySize, q6tc::SMEM_ROOM); }
 
-// From three columns on, where k_gemv_q6.cu has no more than that. us of a launch, cold, here / k_gemv_f32.cu, three and four columns: [32000 x 4096] 70 / 100 and
+// From three columns on, where k_gemv_q6.cu takes fewer. us of a launch, cold, here / k_gemv_f32.cu, three and four columns: [32000 x 4096] 70 / 100 and
 // 72 / 74, [4096 x 4096] 27.1 / 25.5 and 25.2 / 22.4, [4096 x 14336] 44 / 64 and 42 / 67, [3000 x 2816] 23.5 / 22.4 and 21.2 / 21.4, [2000 x 8448] 29 / 32
 // and 28 / 42; two columns lose everywhere (67 / 57, 27 / 18, 44 / 39).
+//
+// Small matrices, whose passes of four columns cost k_gemv_f32.cu less than half a pass of eight here. In a row of launches, us, there / here: [1500 x 2048] x 3
+// 7.9 / 10.0, x 4 7.3 / 9.9, x 5 11.7 / 10.0, x 12 17.8 / 19.9, x 16 23.4 / 19.8; [1024 x 4096] x 4 7.2 / 12.8, x 8 12.7 / 13.9, x 12 18.7 / 25.4, x 16 24.3 /
+// 25.5; [4096 x 4096] x 3 16.5 / 17.9, x 4 13.1 / 18.3, x 5 22.9 / 19.8, x 8 23.6 / 20.7, x 12 35.2 / 37.7, x 16 46.9 / 38.4; [30000 x 512] x 5 29 / 16; [32000 x 4096]
+// x 3 93 / 62, x 4 66 / 64. Both are a constant and a part that grows with the weights (here also with the parts of a tile's sum); rows of more than
+// 4096 weights have passes of two columns there.
+static bool decode_faster(int64_t K, int64_t M, int64_t N) {
+    if (K > 4096 || getenv("TLB_Q6_DIGITS")) return false;
+    const double x = (double)(K * M) * 1e-6;
+    const double pass1 = 4.0 + 0.33 * x, pass2 = 4.2 + 0.352 * x, pass4 = 5.2 + 0.461 * x;
+    const int64_t rest = N % 4, passes = N / 4 + (rest + 1) / 2;
+    const double there = (double)(N / 4) * pass4 + (rest & 1 ? pass1 : 0) + (rest & 2 ? pass2 : 0) - 1.5 * (double)(passes - 1) - (rest == 3 ? 1.5 : 0);
+    return there < (double)((N + q6tc::MAX_COLS - 1) / q6tc::MAX_COLS) * (6.3 + 0.31 * (double)(K / q6tc::KS) + 0.41 * x);
+}
 bool mm_q6_supported(uint32_t type, int64_t K, int64_t M, int64_t N) {
-    return type == TLB_TYPE_Q6_K && K % q6tc::KS == 0 && K >= q6tc::KS && M >= 8 && N > 2 && N > gemv_q6_columns(K) && N <= (1 << 20) && K <= (1 << 20) &&
+    return type == TLB_TYPE_Q6_K && K % q6tc::KS == 0 && K >= q6tc::KS && M >= 8 && N > 2 && N > gemv_q6_columns(K, M) && !decode_faster(K, M, N) && N <= (1 << 20) && K <= (1 << 20) &&
            (M + tc::ROWS - 1) / tc::ROWS * (K / q6tc::KS) < (1ll << 31) && tc_available();
 }
 

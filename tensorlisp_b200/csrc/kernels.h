@@ -180,8 +180,8 @@ void gemv_configure();
 bool gemv_f32_supported(uint32_t type, int64_t K, int64_t M, int64_t N);
 cudaError_t launch_gemv_f32(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
 void gemv_f32_configure();
-// Q6_K on the integer matrix instruction (k_gemv_q6.cu): up to how many columns of K weights it takes (0 to 4)
-int gemv_q6_columns(int64_t K);
+// Q6_K on the integer matrix instruction (k_gemv_q6.cu): up to how many columns of M rows of K weights it takes (0 to 4)
+int gemv_q6_columns(int64_t K, int64_t M);
 cudaError_t launch_gemv_q6(const GemvArgs &g, int sm_count, int *err, cudaStream_t st);
 void gemv_q6_configure();
 bool row_quant_q80_supported(int64_t K, int mode);

@@ -117,6 +117,20 @@ def test_rows_quantized_in_the_launch_or_in_front_of_it(oracle, monkeypatch, ty,
             assert a.tobytes() == b[:n].tobytes()
 
 
+# The Q6_K tests from here on run twice: with the kernel that a size takes, and with TLB_Q6_DIGITS, which sends matrices below the lines of gemv_q6_columns
+# and mm_q6_supported to the kernels behind them, too, so that their edges need no large matrices.
+def pytest_generate_tests(metafunc):
+    if metafunc.function.__name__.startswith("test_q6_K"):
+        metafunc.fixturenames.append("q6_route")
+        metafunc.parametrize("q6_route", ["by size", "digits"], indirect=True)
+
+
+@pytest.fixture
+def q6_route(request, monkeypatch):
+    if request.param == "digits":
+        monkeypatch.setenv("TLB_Q6_DIGITS", "1")
+
+
 @pytest.mark.parametrize("K,M", [(256, 130), (768, 45), (1792, 300), (2048, 17), (4096, 148 * 32 + 5), (7168, 33), (7424, 40), (14336, 20)])
 def test_q6_K_against_f64(oracle, K, M):
     """Activations as eight digits of eight bits: rows of less than eight super-blocks (several row groups per tile), whole rows, segments of eight, one to four
