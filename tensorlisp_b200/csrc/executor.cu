@@ -678,9 +678,9 @@ static std::string import_graph(const tlb_graph *graph, const tlb_leaves *leaves
 }
 
 // ------------------------------------------------------------------ the pinned page of a program
-// Inputs of at most IO_IN_MAX bytes wait in the page until the program's launch sequence fetches them (k_io_page):
+// Inputs of at most IO_IN_MAX bytes wait in the page until the program's launch sequence fetches them (k_io_fetch):
 // a blocking copy of the same bytes takes 10 to 12 us, most of it the wait. Kept results of at most IO_OUT_MAX bytes that
-// the caller reads after its runs are pushed by the sequence itself, the small ones into the page. Its kernels also write
+// the caller reads after its runs are pushed by the sequence itself (k_io_push), the small ones into the page. Its kernels also write
 // their error word there, so run() needs no copy to see it.
 static bool is_pushed_out(const tlb_program *p, uint32_t tensor) {
     const Place pl = p->layout.place[tensor];

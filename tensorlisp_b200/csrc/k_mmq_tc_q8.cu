@@ -639,11 +639,14 @@ __global__ void __launch_bounds__(tc8w::THREADS, 1) k_mmq_tc_q80_wide(const __gr
 //
 // Why pairs: the copies of B bound wide tiles of single CTAs. 148 of them, each with the B of its own 128 rows, read 11 to 12.5 TB/s out
 // of L2 (2.4 us per unit of 256 elements of K at 336 columns, 1.55 at 256, whose MMAs take 1.45 and 1.1); the pair reads each
-// column once for 256 rows. The threads' arrivals on the leader's barriers are of CTA scope: they only pass tensor memory on, between tcgen05 fences (a release
-// of cluster scope made a unit 2.0 us instead of 1.15 at 64 columns). The columns of B that the other CTA copied arrive on the leader's barrier by themselves.
-// The expanding warps fetch and expand before they wait for their slot (the wait, fetch, expansion and store as one chain took
-// 1000 cycles of a slot's round). Narrow tiles are bound by the expansion's instructions (326 per warp and unit for Q4_K, 268 for Q8_0, four
-// warps per scheduler; 404 and 52 -> 47 us for gate and up of 14336 x 4096 at 128 columns while codes went through f32 one by one); wide ones by the tensor pipe: 16384 columns run at 1400 to 1456 TFLOP/s (1253 to 1346 before).
+// column once for 256 rows. The threads' arrivals on the leader's barriers are of CTA scope: they only pass tensor memory on, between
+// tcgen05 fences (a release of cluster scope made a unit 2.0 us instead of 1.15 at 64 columns). The columns of B that the other CTA copied
+// arrive on the leader's barrier by themselves. The expanding warps fetch and expand before they wait for their slot (the wait, fetch,
+// expansion and store as one chain took 1000 cycles of a slot's round).
+//
+// What bounds it: narrow tiles the expansion's instructions (326 per warp and unit for Q4_K, 268 for Q8_0, four warps per scheduler; 404 with
+// codes through f32 one by one: gate and up of 14336 x 4096 at 128 columns 52 -> 47 us); wide ones the tensor pipe: 16384 columns run at
+// 1400 to 1456 TFLOP/s (1253 to 1346 with single CTAs).
 // The tile's width follows from rows, columns and the measured time of a unit; tiles that leave SMs idle are cut along K and their
 // parts added up by a second launch (mm_fold_plan). Matrices that share the activations are one launch. 333 columns, Q4_K, cold:
 // [4096 x 14336] 70 -> 50 us, gate and up (14336 x 4096) 86 -> 82, [4096 x 4096] 31 either way; 65 columns of [4096 x 14336] 68 -> 32.
@@ -1344,7 +1347,7 @@ TcPlan mmq_tc8_plan(uint32_t type, int64_t K, int64_t M, int64_t N, int sm_count
     TcPlan t;
     t.nsb = (int)(K / 256);
     if (type == TLB_TYPE_Q8_0 && N > 64 && !getenv("TLB_NO_WIDE_TC") && !getenv("TLB_PROMPT_EXACT")) {
-        // prompt-sized batches: 128 x 256 tiles, scales folded into f16 operands, one accumulator (k_mm_q80_f16)
+        // prompt-sized batches: scales folded into f16 operands (k_mm_q80_f16); tiles, pairs of CTAs and cuts of K by mm_fold_plan
         t.npad = tc8f::NW;
         t.n_split = 1;
         t.sb_per_split = t.nsb;
@@ -1356,7 +1359,9 @@ TcPlan mmq_tc8_plan(uint32_t type, int64_t K, int64_t M, int64_t N, int sm_count
         return t;
     }
     // Q4_0 in 128-column tiles once they are a third of the SMs; fewer leave so much of the chip idle that passes of 32 columns with K cut
-    // over the SMs are faster ([4096 x 14336] x 128, 32 tiles: 205 us against 100; x 256: 207 against 200)
+    // over the SMs are faster ([4096 x 14336] x 128, 32 tiles: 205 us against 100; x 256: 207 against 200). In a row of launches, tiles / passes (passes of eight
+    // columns in k_gemv.cu): [4096 x 4096] x 200 60 / 64 (134), x 256 60 / 74 (173); [14336 x 4096] x 128 60 / 86 (212); [32000 x 2048] x 65 63 / 73 (142); rows of
+    // 14336 weights cross later, a tile's K being one chain: [4096 x 14336] x 200 201 / 147 (377), x 400 202 / 273 (754).
     const bool wide = type == TLB_TYPE_Q8_0 || (M + tc8::ROWS - 1) / tc8::ROWS * ((N + tc8w::NW - 1) / tc8w::NW) >= sm_count / 3;
     if (N > 64 && wide && !getenv("TLB_NO_WIDE_TC")) {
         // the same batches with the reference's integer arithmetic (Q4_0, which has no other; TLB_PROMPT_EXACT=1): 128-column tiles, whole K per
@@ -1373,7 +1378,7 @@ TcPlan mmq_tc8_plan(uint32_t type, int64_t K, int64_t M, int64_t N, int sm_count
     }
     t.npad = N <= 16 ? 16 : 32;
     const int64_t tiles = (M + tc8::ROWS - 1) / tc8::ROWS;
-    // same model as the Q4_K kernel, with this kernel's time per stage
+    // same model as the Q4_K kernel, with the time per stage of Q8_0 (a stage of Q4_0 takes about 0.8 us instead of 1.0, so that it is cut a little more than it needs)
     int best = 1;
     double best_score = 1e30;
     for (int s = 1; s <= t.nsb && s <= 16; s++) {
