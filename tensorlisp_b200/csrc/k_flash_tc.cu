@@ -63,6 +63,10 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
+// a += the low half of p, b += the high one, in f32
+__device__ __forceinline__ void add_h2(uint32_t p, float &a, float &b) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.f16 %0, l, %0;\n\tadd.rn.f32.f16 %1, h, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(p));
+}
 // byte offset of (row, 16-byte chunk c of the row) inside a 128 x 128 f16 blob
 __device__ __forceinline__ int blob_off(int row, int c) { return (row >> 3) * 2048 + c * 128 + (row & 7) * 16; }
 }  // namespace fat
@@ -207,6 +211,7 @@ struct FaTcParams {
     const uint8_t *qp, *kp, *vt, *flags, *mask;   // flags and mask null without a mask
     TView m;              // rows on 16-byte boundaries
     int m_keys;           // keys that a mask row holds
+    float rescale_step;   // how far a row's maximum may outgrow its reference
     int m_ne2, m_ne3;
     float *out;
     int nq, nkv, nh, nhkv, nb, n_qt, n_kt;
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(fat::THREADS, 1) k_fa_tc(FaTcParams p) {
                     m_ref = mx;
                     have_ref = true;   // nothing has been accumulated for this row yet: O and l are zero
                 }
-            } else if (mx > m_ref + fat::RESCALE_STEP) {
+            } else if (mx > m_ref + p.rescale_step) {
                 alpha = fat::ex2(m_ref - mx);
                 m_ref = mx;
             }
@@ -417,16 +422,15 @@ __global__ void __launch_bounds__(fat::THREADS, 1) k_fa_tc(FaTcParams p) {
                 tmem_st_wait();
                 l *= alpha;
             }
-            // P = exp2(x - m_ref) as f16 pairs; this thread's part of the row sum in f32
+            // P = exp2(x - m_ref) as f16 pairs; this thread's part of the row sum in f32, of the values as they are rounded: O has the same roundings
             uint32_t pk[32];
-            float sum = 0.f;
+            float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
             for (int i = 0; i < 64; i += 2) {
-                const float e0 = fat::ex2(x[i] - m_ref), e1 = fat::ex2(x[i + 1] - m_ref);
-                sum += e0 + e1;
-                pk[i / 2] = fat::pack_h2(e0, e1);
+                pk[i / 2] = fat::pack_h2(fat::ex2(x[i] - m_ref), fat::ex2(x[i + 1] - m_ref));
+                fat::add_h2(pk[i / 2], sum0, sum1);
             }
-            l += sum;
+            l += sum0 + sum1;
             fat::tmem_st32(lane_base + fat::P_COL0 + (uint32_t)(s * 64 + half * 32), pk);
             tmem_st_wait();
             tc_fence_before();
@@ -484,7 +488,8 @@ bool flash_tc_supported(const FlashArgs &p, bool has_mask) {
     if (p.d != fat::T || p.dv != fat::T || p.k_ty != TLB_TYPE_F16 || p.v_ty != TLB_TYPE_F16 || p.softcap != 0.f || p.max_bias != 0.f) return false;
     // Few keys: the packing launch costs more than these tiles save. One node of 32 + 8 heads in us, this against k_flash.cu: 128 causal tokens
     // 21.6 / 17.0, 160: 20.0 / 18.9, 192: 19.6 / 20.5, 333: 23.3 / 30.9, 1001: 47 / 116, 2041: 103 / 354; eight prompts of 160: 49.6 / 43.9, of 192:
-    // 50.7 / 51.3, of 256: 55.6 / 74.9.
+    // 50.7 / 51.3, of 256: 55.6 / 74.9. In a chain of nodes, 192 keys: 16 + 4 heads 12.9 / 14.5, 8 + 8 13.1 / 14.4, 4 + 1 12.6 / 14.1, 64 + 8 14.6 / 18.9;
+    // 168: 12.3 to 13.4 on either, four and eight prompts of 32 + 8 24.6 / 23.4 and 44.8 / 37.8.
     if (p.nq < 64 || p.nkv <= 160 || (p.nkv + fat::T - 1) / fat::T > 512 || p.nh % p.nhkv != 0) return false;
     if (p.q.nb[1] % 16 || p.q.nb[2] % 16 || p.q.nb[3] % 16) return false;
     return !has_mask || !mask_needs_copy(p) || mask_copy_bytes(p) <= MASK_COPY_MAX;
@@ -542,7 +547,13 @@ cudaError_t launch_flash_attn_tc(const FlashArgs &p, const void *q, const void *
     a.mask = copy ? sc + L.m_off : (const uint8_t *)mask;
     a.m = p.m;
     a.m_keys = p.nkv;
+    a.rescale_step = fat::RESCALE_STEP;
     if (copy) {
+        // These masks took k_flash.cu before, whose reference is the maximum itself: a row's largest P is then 1 and rounds to itself. Relative error
+        // against f64, causal, that kernel / here with a lagging reference and sums of unrounded values / as it is: 333 keys 1.42e-4 / 1.46e-4 / 1.39e-4,
+        // 1001 keys 1.50e-4 / 1.57e-4 / 1.48e-4, with scores of standard deviation 3 instead of 1 7.5e-5 / 1.55e-4 / 7.5e-5, of 8 (333 keys) 4.2e-5 / 9.2e-5 /
+        // 4.3e-5. It costs 3 us of 44 at 1001 tokens and 7 of 101 at 2041 (k_flash.cu 116 and 354).
+        a.rescale_step = 0.f;
         a.m_keys = L.n_kt * fat::T;
         a.m.nb[1] = (int64_t)a.m_keys * 2;
         a.m.nb[2] = a.m.nb[1] * L.n_qt * fat::T;

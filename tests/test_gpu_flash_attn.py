@@ -262,3 +262,20 @@ def test_few_queries_over_a_long_cache_split_the_keys(nq, nkv, nh, nhkv, nb):
                                   (128, 64, 177, 2, 1, 1, "causal", 0.0, 0.0, G.F16), (128, 257, 401, 4, 2, 2, "causal", 0.0, 0.0, G.F16)], ids=lambda c: str(c[:7]))
 def test_mask_rows_of_any_alignment_on_the_tensor_cores(case):
     test_flash_attn_closed_form(case)
+
+
+@pytest.mark.parametrize("n,spread", [(333, 1.0), (1001, 1.0), (1001, 3.0)])
+def test_mask_rows_of_any_alignment_are_no_further_from_f64(n, spread, monkeypatch):
+    """Causal prompts of several key tiles whose mask rows do not start on 16 bytes, on the tcgen05 kernel and on the one that such masks took before it
+    had them: both round queries, keys, values and P to f16, and in both a row's largest P is exactly 1 when it is found."""
+    rng = np.random.default_rng(n)
+    q = (spread * rng.standard_normal((1, 8, n, 128))).astype(np.float32)
+    k, v = (rng.standard_normal((1, 2, n, 128)).astype(np.float16) for _ in range(2))
+    mask = np.triu(np.full((n, n), -np.inf, np.float16), 1)[None, None]
+    want = closed_form(q.astype(np.float16), k, v, mask, 128 ** -0.5).astype(np.float64)
+    err = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TLB_NO_FLASH_TC", "1")
+        err.append(np.linalg.norm(run_gpu(q, k, v, mask, 128 ** -0.5, 0.0, 0.0, G.F16) - want))
+    assert err[0] <= err[1]
