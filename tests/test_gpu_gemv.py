@@ -259,7 +259,7 @@ def test_q6_K_single_terms(oracle, N, K):
 
 @pytest.mark.parametrize("K,M,N", [(256, 8, 5), (512, 9, 6), (768, 135, 16), (4096, 1500, 17), (1024, 7, 12), (2048, 148 * 128 + 3, 9), (14336, 40, 22), (256, 130, 64), (4096, 20000, 21)])
 def test_q6_K_on_the_tensor_cores(oracle, K, M, N):
-    """More than four columns: rows in eights and what is left of them (fewer than eight rows stay with the other kernel), tiles cut between CTAs and
+    """The kernel of three columns and more: rows in eights and what is left of them (fewer than eight rows stay with the other kernel), tiles cut between CTAs and
     whole, several passes of columns. The sums of a super-block are exact, so the error is that of some eight roundings per super-block and of the
     addition of a tile's parts: below 2.5e-7 of the result's norm. (Row by row: test_q6_K_large_values_over_weights_of_zero.)"""
     rng = np.random.default_rng(K + M + N)
